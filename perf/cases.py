@@ -242,6 +242,11 @@ def _padded(a, n):
 
 def _pool(sim):
     pop, a = sim.read_pool()
+    gap = np.ones(len(a["state"]), dtype=bool)  # slots between the ranges hold nothing
+    for start, end in pop["ranges"]:
+        gap[start:end] = False
+    for v in a.values():
+        v[gap] = 0
     a = {k: v if v.dtype != np.uint32 else v.view(np.int32) for k, v in a.items()}
     return {"ranges": pop["ranges"].astype(np.int32), **{k: _padded(v, sim.capacity) for k, v in a.items()}}
 
