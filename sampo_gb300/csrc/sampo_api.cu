@@ -30,8 +30,9 @@ struct sampo_sim {
   RepParams* rep_dev = nullptr;        // this simulation as a batch of one
   BatchDev* bat_dev = nullptr;
   ModelConst* mc_dev = nullptr;
-  uint32_t* tile_mem = nullptr;
-  uint32_t max_tiles = 0;
+  void* span_mem = nullptr;            // span arrays (set_span_arrays)
+  uint32_t* small_mem = nullptr;       // the one-launch step's rows
+  bool wide = false;                   // the pool holds whole records (state_cols)
   float* T_dev = nullptr;
   sampo_environment* env_dev = nullptr;
   sampo_seeds* seeds_dev = nullptr;
@@ -50,7 +51,6 @@ struct sampo_sim {
   double last_run_ms = 0;
   SimDev host_state;                   // template for (re)initialisation
   uint32_t step = 0;                   // host mirror of the device step index
-  uint32_t epoch = 1;                  // host mirror of the device epoch
   bool have_pop = false;
   bool pending = false;                // steps queued by sampo_run_async, not yet synced
   int grid_count = 0, grid_scatter = 0;
@@ -123,7 +123,10 @@ static RepParams make_rep(sampo_sim* s) {
   r.sim = s->sim_dev;
   r.pool[0] = s->pool[0];
   r.pool[1] = s->pool[1];
-  set_tile_arrays(r, s->tile_mem, s->max_tiles);
+  r.dec = nullptr;
+  set_span_arrays(r, s->span_mem, (uint32_t)s->capacity);
+  r.smallRows = s->small_mem;
+  r.smallStride = units_of((uint32_t)s->capacity, 8);  // the tiles of any pool that fits, at 256 slots
   r.T = s->T_dev;
   r.env = s->env_dev;
   r.seeds = s->seeds_dev;
@@ -140,6 +143,7 @@ static KParams make_params(sampo_sim* s) {
   p.bat = s->bat_dev;
   p.mc = s->mc_dev;
   p.ks = s->species;
+  p.wide = s->wide ? 1u : 0u;
   return p;
 }
 
@@ -158,7 +162,7 @@ extern "C" int sampo_destroy(sampo_sim* s) {
   if (s->end_pinned) cudaFreeHost(s->end_pinned);
   for (auto& e : s->ev) if (e) cudaEventDestroy(e);
   cudaFree(s->pool_mem[0]); cudaFree(s->pool_mem[1]);
-  cudaFree(s->sim_dev); cudaFree(s->tile_mem);
+  cudaFree(s->sim_dev); cudaFree(s->span_mem); cudaFree(s->small_mem);
   cudaFree(s->rep_dev); cudaFree(s->bat_dev); cudaFree(s->mc_dev);
   cudaFree(s->T_dev); cudaFree(s->env_dev); cudaFree(s->seeds_dev); cudaFree(s->wt_dev);
   cudaFree(s->rows_dev); cudaFree(s->init_seeds_dev); cudaFree(s->hist_dev); cudaFree(s->flush_buf);
@@ -198,9 +202,12 @@ extern "C" int sampo_create(const sampo_config* cfg, sampo_sim** out) {
       P.flags = (uint8_t*)(m + 9 * col4);
     }
     if (rc) break;
-    s->max_tiles = (uint32_t)((C + kTileMin - 1) / kTileMin);  // room for the smaller tile's count
-    if ((e = cudaMalloc(&s->tile_mem, tile_array_words(s->max_tiles) * 4)) != cudaSuccess) { rc = cuda_fail(s, e, "tile arrays"); break; }
-    cudaMemsetAsync(s->tile_mem, 0, tile_array_words(s->max_tiles) * 4, s->stream);
+    if ((e = cudaMalloc(&s->span_mem, span_array_bytes((uint32_t)C))) != cudaSuccess ||
+        (e = cudaMalloc(&s->small_mem, (size_t)units_of((uint32_t)C, 8) * kSmallRowWords * 4)) != cudaSuccess) {
+      rc = cuda_fail(s, e, "span arrays");
+      break;
+    }
+    cudaMemsetAsync(s->span_mem, 0, span_array_bytes((uint32_t)C), s->stream);
     if ((e = cudaMalloc(&s->sim_dev, sizeof(SimDev))) != cudaSuccess ||
         (e = cudaMalloc(&s->rep_dev, sizeof(RepParams))) != cudaSuccess ||
         (e = cudaMalloc(&s->bat_dev, sizeof(BatchDev))) != cudaSuccess ||
@@ -308,11 +315,7 @@ static int reset_state(sampo_sim* s, const sampo_population& pop) {
   h.active = 1;
   h.step = 0;
   h.cur = 0;
-  // The look-back trusts a tile's inclusive prefix when its flag equals the
-  // running step's epoch. Epochs restart here, so flags left by an earlier
-  // run must go: clear the tile arrays before the first step.
-  h.epoch = 1;
-  CK(cudaMemsetAsync(s->tile_mem, 0, tile_array_words(s->max_tiles) * 4, s->stream), "tile reset");
+  CK(cudaMemsetAsync(s->span_mem, 0, span_array_bytes((uint32_t)s->capacity), s->stream), "span reset");
   // the one-launch step's grid barrier and exit counters start from zero
   CK(cudaMemsetAsync(&s->bat_dev->bar, 0, 2 * sizeof(uint32_t), s->stream), "barrier reset");
   CK(cudaMemcpyAsync(s->sim_dev, &h, sizeof(SimDev), cudaMemcpyHostToDevice, s->stream), "state reset");
@@ -320,13 +323,31 @@ static int reset_state(sampo_sim* s, const sampo_population& pop) {
   return SAMPO_OK;
 }
 
-static int publish_initial(sampo_sim* s) {
+static void drop_day_graph(sampo_sim* s);
+static void drop_small_graphs(sampo_sim* s);
+
+// The passes and grids for narrow or wide pools (state_cols).
+static void set_wide(sampo_sim* s, bool wide) {
+  if (wide == s->wide) return;
+  s->wide = wide;
+  s->grid_count = grid_blocks_count(1, s->species, s->items, wide);
+  s->grid_scatter = grid_blocks_scatter(1, s->species, s->items, wide);
+  drop_day_graph(s);  // captured with the other kernels
+  drop_small_graphs(s);
+}
+
+// Statistics and publish of the pool the caller has just put in buffer 0;
+// `loaded`: its records come from outside and may be wide.
+static int publish_initial(sampo_sim* s, bool loaded) {
   KParams p = make_params(s);
-  CK(launch_publish_start(p, s->stream), "initial statistics");
+  CK(launch_publish_start(p, loaded, s->stream), "initial statistics");
   CK(cudaMemcpyAsync(s->end_pinned, &s->sim_dev->pop.r[GRAVID].end, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream),
+     "initial statistics");
+  CK(cudaMemcpyAsync(s->end_pinned + 1, &s->sim_dev->wide, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream),
      "initial statistics");
   CK(cudaStreamSynchronize(s->stream), "initial statistics");
   s->known_end = s->end_pinned[0];
+  set_wide(s, s->end_pinned[1] != 0);
   s->have_pop = true;
   return SAMPO_OK;
 }
@@ -355,7 +376,7 @@ extern "C" int sampo_init_population(sampo_sim* s, uint32_t n, const sampo_seeds
   CK(cudaMemcpyAsync(s->init_seeds_dev, init_seeds, 4 * sizeof(sampo_seeds), cudaMemcpyHostToDevice, s->stream), "seeds");
   KParams p = make_params(s);
   CK(launch_init_eggs(p, n, s->T_host[0], s->init_seeds_dev, age_days_max, age_seed, s->stream), "initAgents");
-  return publish_initial(s);
+  return publish_initial(s, false);
 }
 
 extern "C" int sampo_load_pool(sampo_sim* s, const sampo_population* pop, const sampo_pool_view* v) {
@@ -383,7 +404,7 @@ extern "C" int sampo_load_pool(sampo_sim* s, const sampo_population* pop, const 
   for (uint32_t i = 0; i < n; i++) flags[i] = (uint8_t)((v->state[i] & 7u) | ((v->isFemale[i] ? 1u : 0u) << 3));
   CK(cudaMemcpyAsync(P.flags, flags.data(), n, cudaMemcpyHostToDevice, s->stream), "pool upload");
   CK(cudaStreamSynchronize(s->stream), "pool upload");
-  return publish_initial(s);
+  return publish_initial(s, true);
 }
 
 static int check_device(sampo_sim* s) {
@@ -398,11 +419,8 @@ static int check_device(sampo_sim* s) {
   return SAMPO_OK;
 }
 
-static cudaError_t launch_step(sampo_sim* s, const KParams& p) {
-  cudaError_t e = launch_count(p, s->grid_count, s->stream, s->items);
-  if (e != cudaSuccess) return e;
-  if ((e = launch_scatter(p, s->grid_scatter, s->stream, s->items)) != cudaSuccess) return e;
-  return launch_publish(p, PUB_AFTER_STEP, s->stream);
+static cudaError_t launch_hours(sampo_sim* s, const KParams& p, uint32_t nsteps, uint32_t* launches) {
+  return launch_steps(p, nsteps, true, s->grid_count, s->grid_scatter, s->items, s->stream, launches);
 }
 
 extern "C" int sampo_step(sampo_sim* s, const sampo_environment* env, float temperature, uint32_t world_time,
@@ -424,8 +442,9 @@ extern "C" int sampo_step(sampo_sim* s, const sampo_environment* env, float temp
   if (row) CK(cudaMemcpyAsync(row, s->rows_dev + slot, sizeof(sampo_stats_row), cudaMemcpyDeviceToHost, s->stream), "row");
   KParams p = make_params(s);
   CK(launch_publish(p, PUB_REFRESH, s->stream), "step constants");  // this step's inputs were just written
-  CK(launch_step(s, p), "step kernels");
-  s->launches += 4;
+  uint32_t n = 1;  // the refresh
+  CK(launch_hours(s, p, 1, &n), "step kernels");
+  s->launches += n;
   s->step++;
   return check_device(s);
 }
@@ -435,8 +454,7 @@ static int build_day_graph(sampo_sim* s) {
   KParams p = make_params(s);
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal), "capture");
-  cudaError_t e = cudaSuccess;
-  for (int h = 0; h < 24 && e == cudaSuccess; h++) e = launch_step(s, p);
+  cudaError_t e = launch_hours(s, p, 24, nullptr);
   cudaError_t e2 = cudaStreamEndCapture(s->stream, &g);
   if (e != cudaSuccess) { if (g) cudaGraphDestroy(g); return cuda_fail(s, e, "capture launch"); }
   if (e2 != cudaSuccess) return cuda_fail(s, e2, "end capture");
@@ -456,6 +474,13 @@ static void drop_day_graph(sampo_sim* s) {
     cudaGraphExecDestroy(s->day_graph);
     s->day_graph = nullptr;
   }
+}
+static void drop_small_graphs(sampo_sim* s) {
+  for (auto& row : s->small_graph)
+    for (auto& g : row) {
+      if (g) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
 }
 
 // A day on grid bucket b: one launch of 24 one-launch steps, cooperative
@@ -634,9 +659,10 @@ static int queue_run(sampo_sim* s, uint32_t nsteps, sampo_stats_row* rows, bool 
           }
         }
       }
-      for (; i < n; i++) {
-        CK(launch_step(s, p), "step kernels");
-        s->launches += 3;
+      if (i < n) {
+        uint32_t k = 0;
+        CK(launch_hours(s, p, n - i, &k), "step kernels");
+        s->launches += k;
       }
     }
     CK(cudaEventRecord(s->ev[2], s->stream), "event");
@@ -758,6 +784,7 @@ extern "C" int sampo_read_pool(sampo_sim* s, sampo_population* pop, sampo_pool_v
   CK(cudaStreamSynchronize(s->stream), "state");
   *pop = h.pop;
   if (!v) return SAMPO_OK;
+  CK(launch_widen(make_params(s), s->stream), "pool read");
   const uint32_t n = h.pop.r[7].end;
   const DevPool& P = s->pool[h.cur & 1u];
   const size_t b4 = (size_t)n * 4;
@@ -806,6 +833,7 @@ extern "C" int sampo_checkpoint_save(sampo_sim* s, const char* path) {
     hd.prev = prev.pop;
     hd.flags |= CK_PREV;
   }
+  CK(launch_widen(make_params(s), s->stream), "checkpoint");
   CK(cudaStreamSynchronize(s->stream), "state");
   const std::string err = ck_write(path, hd, s->pool[h.cur & 1u]);
   if (!err.empty()) return fail(s, SAMPO_ERR_IO, err);
@@ -857,10 +885,10 @@ extern "C" int sampo_checkpoint_load(sampo_sim* s, const char* path) {
   h.bnc = hd.bnc;
   h.step = hd.step;
   h.active = 1;
-  CK(cudaMemsetAsync(s->tile_mem, 0, tile_array_words(s->max_tiles) * 4, s->stream), "tile reset");
+  CK(cudaMemsetAsync(s->span_mem, 0, span_array_bytes((uint32_t)s->capacity), s->stream), "span reset");
   CK(cudaMemcpyAsync(s->sim_dev, &h, sizeof(SimDev), cudaMemcpyHostToDevice, s->stream), "state");
   s->step = hd.step;
-  const int rc = publish_initial(s);
+  const int rc = publish_initial(s, true);
   if (rc) return rc;
   sampo_population p;
   SimDev back;
@@ -907,8 +935,8 @@ extern "C" int sampo_set_species(sampo_sim* s, const sampo_species* sp) {
   if (s->species == sp) return SAMPO_OK;
   s->species = sp;
   if (sp) s->items = kItems;  // a run-time species is built for 4 slots per thread
-  s->grid_count = grid_blocks_count(1, sp, s->items);
-  s->grid_scatter = grid_blocks_scatter(1, sp, s->items);
+  s->grid_count = grid_blocks_count(1, sp, s->items, s->wide);
+  s->grid_scatter = grid_blocks_scatter(1, sp, s->items, s->wide);
   drop_day_graph(s);  // captured with the other kernels
   return SAMPO_OK;
 }
@@ -920,8 +948,8 @@ extern "C" int sampo_set_grids(sampo_sim* s, uint32_t count_ctas_per_sm, uint32_
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
   if (sms <= 0) sms = 1;
-  const uint32_t max_c = (uint32_t)(grid_blocks_count(1, s->species, s->items) / sms);
-  const uint32_t max_s = (uint32_t)(grid_blocks_scatter(1, s->species, s->items) / sms);
+  const uint32_t max_c = (uint32_t)(grid_blocks_count(1, s->species, s->items, s->wide) / sms);
+  const uint32_t max_s = (uint32_t)(grid_blocks_scatter(1, s->species, s->items, s->wide) / sms);
   if (count_ctas_per_sm < 1 || count_ctas_per_sm > max_c || scatter_ctas_per_sm < 1 || scatter_ctas_per_sm > max_s)
     return fail(s, SAMPO_ERR_ARG, "CTAs per SM outside 1.." + std::to_string(max_c) + " (count) / 1.." + std::to_string(max_s) +
                                       " (update/scatter)");
@@ -942,8 +970,8 @@ extern "C" int sampo_set_items_per_thread(sampo_sim* s, uint32_t items) {
   cudaSetDevice(s->device);
   if ((int)items != s->items) {
     s->items = (int)items;
-    s->grid_count = grid_blocks_count(1, s->species, s->items);
-    s->grid_scatter = grid_blocks_scatter(1, s->species, s->items);
+    s->grid_count = grid_blocks_count(1, s->species, s->items, s->wide);
+    s->grid_scatter = grid_blocks_scatter(1, s->species, s->items, s->wide);
     drop_day_graph(s);
   }
   return SAMPO_OK;

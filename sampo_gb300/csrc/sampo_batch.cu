@@ -26,21 +26,19 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Byte layout of one replicate's allocation.
 struct RepLayout {
-  size_t col4, col1, pool, tiles, T, env, seeds, wt, rows, total;
-  uint32_t max_tiles;
+  size_t col4, col1, pool, spans, T, env, seeds, wt, rows, total;
   RepLayout(uint64_t capacity, uint32_t ring) {
     // 16 bytes of slack per column: tile copies round up to 16 bytes
     col4 = align256(capacity * 4 + 16);
     col1 = align256(capacity + 16);
     pool = 9 * col4 + col1;
-    max_tiles = (uint32_t)((capacity + kTileMin - 1) / kTileMin);  // room for the smaller tile's count
-    tiles = align256(tile_array_words(max_tiles) * 4);
+    spans = align256(span_array_bytes((uint32_t)capacity));
     T = align256((size_t)ring * sizeof(float));
     env = align256((size_t)ring * sizeof(sampo_environment));
     seeds = align256((size_t)ring * 4 * sizeof(sampo_seeds));
     wt = align256((size_t)ring * sizeof(uint32_t));
     rows = align256((size_t)ring * sizeof(sampo_stats_row));
-    total = 2 * pool + tiles + T + env + seeds + wt + rows;
+    total = 2 * pool + spans + T + env + seeds + wt + rows;
   }
 };
 
@@ -51,6 +49,7 @@ struct Replicate {
   uint32_t step = 0;           // host mirror of SimDev::step
   uint32_t stop_step = 0xffffffffu;
   uint64_t capacity = 0;
+  uint32_t known_end = 0;      // its pool's end as the host last saw it
   float cc = 0.0f;
   void* mem = nullptr;
   RepParams rp;                // host copy of the kernels' view
@@ -77,8 +76,9 @@ struct sampo_batch {
   std::vector<uint32_t> wt_staging;
   int grid_count = 0, grid_scatter = 0;
   int items = kItems;                // slots per thread of the count and update/scatter passes (2 or 4)
-  cudaGraphExec_t day_graph = nullptr;
-  uint32_t day_graph_kernels = 0;    // kernel nodes of day_graph
+  bool wide = false;                 // every slot's pool holds whole records (state_cols): set by the first loaded one that has to
+  cudaGraphExec_t day_graph[2] = {nullptr, nullptr};  // three kernels every hour, and deciding ahead
+  uint32_t day_graph_kernels[2] = {0, 0};             // kernel nodes of each
   uint64_t launches = 0;             // kernels sampo_batch_run launched
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool timed = false;
@@ -102,6 +102,7 @@ static KParams all_params(sampo_batch* b) {
   p.bat = b->bat_dev;
   p.mc = b->mc_dev;
   p.ks = b->species;
+  p.wide = b->wide ? 1u : 0u;
   return p;
 }
 static KParams slot_params(sampo_batch* b, uint32_t slot) {
@@ -122,11 +123,18 @@ extern "C" uint64_t sampo_batch_replicate_bytes(uint64_t capacity, uint32_t ring
 
 extern "C" const char* sampo_batch_last_error(const sampo_batch* b) { return b ? b->err.c_str() : "null handle"; }
 
+static void drop_day_graphs(sampo_batch* b) {
+  for (auto& g : b->day_graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
+}
+
 extern "C" int sampo_batch_destroy(sampo_batch* b) {
   if (!b) return SAMPO_OK;
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
-  if (b->day_graph) cudaGraphExecDestroy(b->day_graph);
+  drop_day_graphs(b);
   for (auto& r : b->reps)
     if (r.mem) cudaFreeAsync(r.mem, b->stream);
   if (b->stream) cudaStreamSynchronize(b->stream);
@@ -211,7 +219,7 @@ extern "C" int sampo_batch_create(const sampo_batch_config* cfg, sampo_batch** o
 }
 
 // The kernels' view of one replicate's allocation `mem` (layout L).
-static RepParams carve(const RepLayout& L, void* mem, SimDev* sim, uint32_t ring) {
+static RepParams carve(const RepLayout& L, void* mem, SimDev* sim, uint64_t capacity, uint32_t ring) {
   RepParams rp;
   memset(&rp, 0, sizeof(rp));
   char* m = (char*)mem;
@@ -225,8 +233,8 @@ static RepParams carve(const RepLayout& L, void* mem, SimDev* sim, uint32_t ring
     P.flags = (uint8_t*)(q + 9 * L.col4);
   }
   char* q = m + 2 * L.pool;
-  set_tile_arrays(rp, (uint32_t*)q, L.max_tiles);
-  q += L.tiles;
+  set_span_arrays(rp, q, (uint32_t)capacity);
+  q += L.spans;
   rp.T = (const float*)q; q += L.T;
   rp.env = (const sampo_environment*)q; q += L.env;
   rp.seeds = (sampo_seeds*)q; q += L.seeds;
@@ -234,6 +242,14 @@ static RepParams carve(const RepLayout& L, void* mem, SimDev* sim, uint32_t ring
   rp.rows = (sampo_stats_row*)q;
   rp.ring = ring;
   return rp;
+}
+
+// The largest grids of the passes the batch runs; a day graph captured with
+// other kernels or grids goes.
+static void size_grids(sampo_batch* b) {
+  b->grid_count = grid_blocks_count(b->nslots, b->species, b->items, b->wide);
+  b->grid_scatter = grid_blocks_scatter(b->nslots, b->species, b->items, b->wide);
+  drop_day_graphs(b);
 }
 
 // The device state of every slot up to its step constants (one strided copy).
@@ -256,6 +272,7 @@ static int refresh_mirrors(sampo_batch* b) {
     if (!r.used || !r.have_pop) continue;
     r.step = h[i].step;
     r.active = h[i].active != 0;
+    r.known_end = h[i].pop.r[7].end;
   }
   return SAMPO_OK;
 }
@@ -291,8 +308,8 @@ extern "C" int sampo_batch_add(sampo_batch* b, const sampo_replicate_config* rc,
   r.seed_step.assign(b->ring, 0xffffffffu);
   r.T_host.assign(b->ring, 0.0f);
   RepParams& rp = r.rp;
-  rp = carve(L, mem, b->sims_dev + i, b->ring);
-  BCK(cudaMemsetAsync(rp.tilePre, 0, tile_array_words(L.max_tiles) * 4, b->stream), "tile arrays");
+  rp = carve(L, mem, b->sims_dev + i, rc->capacity, b->ring);
+  BCK(cudaMemsetAsync(rp.supers, 0, span_array_bytes((uint32_t)rc->capacity), b->stream), "span arrays");
   SimDev h = initial_sim_state((uint32_t)rc->capacity, rc->carrying_capacity);
   h.stop_step = rc->stop_step;
   const int st = upload_slot(b, i, h);
@@ -393,13 +410,14 @@ extern "C" int sampo_batch_init_population(sampo_batch* b, uint32_t slot, uint32
   h.stop_step = r->stop_step;
   const int st = upload_slot(b, slot, h);
   if (st) return st;
-  BCK(cudaMemsetAsync(r->rp.tilePre, 0, tile_array_words(r->rp.maxTiles) * 4, b->stream), "tile arrays");
+  BCK(cudaMemsetAsync(r->rp.supers, 0, span_array_bytes((uint32_t)r->capacity), b->stream), "span arrays");
   BCK(cudaMemcpyAsync(b->init_seeds_dev + (size_t)slot * 4, init_seeds, 4 * sizeof(sampo_seeds), cudaMemcpyHostToDevice, b->stream),
       "seeds");
   const KParams p = slot_params(b, slot);
   BCK(launch_init_eggs(p, n, r->T_host[0], b->init_seeds_dev + (size_t)slot * 4, age_days_max, age_seed, b->stream), "initAgents");
-  BCK(launch_publish_start(p, b->stream), "initial statistics");
+  BCK(launch_publish_start(p, false, b->stream), "initial statistics");
   r->have_pop = true;
+  r->known_end = pop.r[7].end;
   r->step = 0;
   r->active = r->stop_step > 0;
   r->dev_seeds = false;
@@ -457,6 +475,8 @@ extern "C" int sampo_batch_checkpoint_save(sampo_batch* b, uint32_t slot, const 
       hd.flags |= CK_COMING_SEEDS;
     }
   }
+  BCK(launch_widen(slot_params(b, slot), b->stream), "checkpoint");
+  BCK(cudaStreamSynchronize(b->stream), "checkpoint");
   const std::string err = ck_write(path, hd, r->rp.pool[h.cur & 1u]);
   if (!err.empty()) return bfail(b, SAMPO_ERR_IO, err);
   return SAMPO_OK;
@@ -495,15 +515,23 @@ extern "C" int sampo_batch_checkpoint_load(sampo_batch* b, uint32_t slot, const 
   }
   const int st = upload_slot(b, slot, h);
   if (st) return st;
-  BCK(cudaMemsetAsync(r->rp.tilePre, 0, tile_array_words(r->rp.maxTiles) * 4, b->stream), "tile arrays");
-  BCK(launch_publish_start(slot_params(b, slot), b->stream), "checkpoint statistics");
+  BCK(cudaMemsetAsync(r->rp.supers, 0, span_array_bytes((uint32_t)r->capacity), b->stream), "span arrays");
+  BCK(launch_publish_start(slot_params(b, slot), true, b->stream), "checkpoint statistics");
   SimDev back;
   BCK(cudaMemcpyAsync(&back, b->sims_dev + slot, sizeof(SimDev), cudaMemcpyDeviceToHost, b->stream), "state");
   BCK(cudaStreamSynchronize(b->stream), "state");
   if (back.pop.numLarvae1DayEquiv != hd.pop.numLarvae1DayEquiv || back.pop.numFemale != hd.pop.numFemale ||
       back.pop.numPotentiallyInfective != hd.pop.numPotentiallyInfective)
     return bfail(b, SAMPO_ERR_INTERNAL, "checkpoint statistics do not match its pool");
+  if (back.wide && !b->wide) {
+    // the passes for whole records take over: the other slots' pools get theirs
+    for (uint32_t i = 0; i < b->nslots; i++)
+      if (i != slot && b->reps[i].used && b->reps[i].have_pop) BCK(launch_widen(slot_params(b, i), b->stream), "whole records");
+    b->wide = true;
+    size_grids(b);
+  }
   r->have_pop = true;
+  r->known_end = hd.pop.r[7].end;
   r->step = hd.step;
   r->active = h.active != 0;
   return SAMPO_OK;
@@ -522,20 +550,28 @@ extern "C" int sampo_batch_seed_state(sampo_batch* b, uint32_t slot, sampo_rand_
   return SAMPO_OK;
 }
 
-static cudaError_t launch_batch_step(sampo_batch* b, const KParams& p) {
-  cudaError_t e = launch_count(p, b->grid_count, b->stream, b->items);
-  if (e == cudaSuccess) e = launch_scatter(p, b->grid_scatter, b->stream, b->items);
-  if (e == cudaSuccess) e = launch_publish(p, PUB_AFTER_STEP, b->stream);
-  return e;
+static cudaError_t launch_hours(sampo_batch* b, const KParams& p, uint32_t nsteps, bool ahead, uint32_t* launches) {
+  return launch_steps(p, nsteps, ahead, b->grid_count, b->grid_scatter, b->items, b->stream, launches);
 }
 
-static int build_batch_graph(sampo_batch* b) {
-  if (b->day_graph) return SAMPO_OK;
+// Whether a run's days decide ahead: the pools the host has last seen come to
+// more than kAheadSlots slots. Below that a step is three launches' latency
+// either way.
+constexpr uint64_t kAheadSlots = 65536;
+static bool decides_ahead(const sampo_batch* b) {
+  uint64_t slots = 0;
+  for (const Replicate& r : b->reps)
+    if (r.used && r.have_pop && r.active) slots += r.known_end;
+  return slots > kAheadSlots;
+}
+
+static int build_batch_graph(sampo_batch* b, bool ahead) {
+  cudaGraphExec_t& day_graph = b->day_graph[ahead ? 1 : 0];
+  if (day_graph) return SAMPO_OK;
   const KParams p = all_params(b);
   cudaGraph_t g = nullptr;
   BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal), "capture");
-  cudaError_t e = cudaSuccess;
-  for (int h = 0; h < 24 && e == cudaSuccess; h++) e = launch_batch_step(b, p);
+  cudaError_t e = launch_hours(b, p, 24, ahead, nullptr);
   cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
   if (e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
@@ -548,11 +584,11 @@ static int build_batch_graph(sampo_batch* b) {
     cudaGraphDestroy(g);
     return bfail(b, SAMPO_ERR_CUDA, std::string("graph nodes: ") + cudaGetErrorString(e));
   }
-  b->day_graph_kernels = kernels;
-  e = cudaGraphInstantiate(&b->day_graph, g, 0);
+  b->day_graph_kernels[ahead ? 1 : 0] = kernels;
+  e = cudaGraphInstantiate(&day_graph, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) {
-    b->day_graph = nullptr;
+    day_graph = nullptr;
     return bfail(b, SAMPO_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
   }
   return SAMPO_OK;
@@ -577,18 +613,20 @@ extern "C" int sampo_batch_run(sampo_batch* b, uint32_t nsteps, int wait) {
   BCK(cudaEventRecord(b->ev0, b->stream), "event");
   BCK(launch_publish(p, PUB_REFRESH, b->stream), "step constants");  // inputs may postdate the last publish
   b->launches += 1;
+  const bool ahead = decides_ahead(b);
   uint32_t i = 0;
   if (nsteps >= 24) {
-    const int rc = build_batch_graph(b);
+    const int rc = build_batch_graph(b, ahead);
     if (rc) return rc;
     for (; i + 24 <= nsteps; i += 24) {
-      BCK(cudaGraphLaunch(b->day_graph, b->stream), "day graph");
-      b->launches += b->day_graph_kernels;
+      BCK(cudaGraphLaunch(b->day_graph[ahead ? 1 : 0], b->stream), "day graph");
+      b->launches += b->day_graph_kernels[ahead ? 1 : 0];
     }
   }
-  for (; i < nsteps; i++) {
-    BCK(launch_batch_step(b, p), "step kernels");
-    b->launches += 3;
+  if (i < nsteps) {
+    uint32_t n = 0;
+    BCK(launch_hours(b, p, nsteps - i, ahead, &n), "step kernels");
+    b->launches += n;
   }
   BCK(cudaEventRecord(b->ev1, b->stream), "event");
   b->timed = true;
@@ -631,10 +669,7 @@ extern "C" int sampo_batch_autotune(sampo_batch* b, uint32_t* count_ctas_per_sm,
     b->grid_count = gc;
     b->grid_scatter = gs;
     b->items = items;
-    if (b->day_graph) {
-      cudaGraphExecDestroy(b->day_graph);
-      b->day_graph = nullptr;
-    }
+    drop_day_graphs(b);
   }
   if (count_ctas_per_sm) *count_ctas_per_sm = (uint32_t)(gc / sms);
   if (scatter_ctas_per_sm) *scatter_ctas_per_sm = (uint32_t)(gs / sms);
@@ -648,12 +683,7 @@ extern "C" int sampo_batch_set_species(sampo_batch* b, const sampo_species* sp) 
   if (b->species == sp) return SAMPO_OK;
   b->species = sp;
   if (sp) b->items = kItems;  // a run-time species is built for 4 slots per thread
-  b->grid_count = grid_blocks_count(b->nslots, sp, b->items);
-  b->grid_scatter = grid_blocks_scatter(b->nslots, sp, b->items);
-  if (b->day_graph) {
-    cudaGraphExecDestroy(b->day_graph);
-    b->day_graph = nullptr;
-  }
+  size_grids(b);
   return SAMPO_OK;
 }
 
@@ -663,8 +693,8 @@ extern "C" int sampo_batch_set_grids(sampo_batch* b, uint32_t count_ctas_per_sm,
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
   if (sms <= 0) sms = 1;
-  const uint32_t max_c = (uint32_t)(grid_blocks_count(b->nslots, b->species, b->items) / sms);
-  const uint32_t max_s = (uint32_t)(grid_blocks_scatter(b->nslots, b->species, b->items) / sms);
+  const uint32_t max_c = (uint32_t)(grid_blocks_count(b->nslots, b->species, b->items, b->wide) / sms);
+  const uint32_t max_s = (uint32_t)(grid_blocks_scatter(b->nslots, b->species, b->items, b->wide) / sms);
   if (count_ctas_per_sm < 1 || count_ctas_per_sm > max_c || scatter_ctas_per_sm < 1 || scatter_ctas_per_sm > max_s)
     return bfail(b, SAMPO_ERR_ARG, "CTAs per SM outside 1.." + std::to_string(max_c) + " (count) / 1.." +
                                        std::to_string(max_s) + " (update/scatter)");
@@ -672,10 +702,7 @@ extern "C" int sampo_batch_set_grids(sampo_batch* b, uint32_t count_ctas_per_sm,
   if (gc != b->grid_count || gs != b->grid_scatter) {
     b->grid_count = gc;
     b->grid_scatter = gs;
-    if (b->day_graph) {
-      cudaGraphExecDestroy(b->day_graph);
-      b->day_graph = nullptr;
-    }
+    drop_day_graphs(b);
   }
   return SAMPO_OK;
 }
@@ -687,12 +714,7 @@ extern "C" int sampo_batch_set_items_per_thread(sampo_batch* b, uint32_t items) 
   cudaSetDevice(b->device);
   if ((int)items != b->items) {
     b->items = (int)items;
-    b->grid_count = grid_blocks_count(b->nslots, b->species, b->items);
-    b->grid_scatter = grid_blocks_scatter(b->nslots, b->species, b->items);
-    if (b->day_graph) {
-      cudaGraphExecDestroy(b->day_graph);
-      b->day_graph = nullptr;
-    }
+    size_grids(b);
   }
   return SAMPO_OK;
 }
@@ -747,7 +769,7 @@ extern "C" int sampo_batch_grow(sampo_batch* b, uint32_t slot, uint64_t capacity
     cudaGetLastError();
     return bfail(b, SAMPO_ERR_CAPACITY, std::string("grown replicate buffers: ") + cudaGetErrorString(e));
   }
-  const RepParams rp = carve(L, mem, b->sims_dev + slot, b->ring);
+  const RepParams rp = carve(L, mem, b->sims_dev + slot, capacity, b->ring);
   const RepParams& old = r->rp;
   // the current pool into buffer 0, column by column: slot indices unchanged
   const DevPool& S = old.pool[h.cur & 1u];
@@ -768,8 +790,7 @@ extern "C" int sampo_batch_grow(sampo_batch* b, uint32_t slot, uint64_t capacity
   // the rings of inputs, seeds and rows (same ring length, same layout)
   BCK(cudaMemcpyAsync((void*)rp.T, old.T, L.T + L.env + L.seeds + L.wt + L.rows, cudaMemcpyDeviceToDevice, b->stream),
       "grow rings");
-  // fresh look-back arrays: zero epochs never match the running step's
-  BCK(cudaMemsetAsync(rp.tilePre, 0, tile_array_words(L.max_tiles) * 4, b->stream), "tile arrays");
+  BCK(cudaMemsetAsync(rp.supers, 0, span_array_bytes((uint32_t)capacity), b->stream), "span arrays");
   h.capacity = (uint32_t)capacity;
   h.cur = 0;
   h.error &= ~SAMPO_DEV_ERR_CAPACITY;
@@ -852,6 +873,7 @@ extern "C" int sampo_batch_read_pool(sampo_batch* b, uint32_t slot, sampo_popula
   BCK(cudaStreamSynchronize(b->stream), "state");
   *pop = h.pop;
   if (!v) return SAMPO_OK;
+  BCK(launch_widen(slot_params(b, slot), b->stream), "pool read");
   const uint32_t n = h.pop.r[7].end;
   const DevPool& P = r->rp.pool[h.cur & 1u];
   const size_t b4 = (size_t)n * 4;

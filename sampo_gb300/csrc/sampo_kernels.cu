@@ -9,67 +9,62 @@
 namespace sampo {
 
 // ------------------------------------------------------------------------
-// Per-device set-up, once per device under a once_flag: the SM count and the
-// dynamic shared memory limit of the two persistent kernels (a function
-// attribute applies to the device that is current when it is set, so every
-// device the library runs on gets its own). Devices beyond kMaxDevices are
-// set up on every call under a mutex.
-// The built-in count and update/scatter passes for `items` slots per thread.
-static const void* count_fn(int items) { return items == 2 ? (const void*)k_count<2> : (const void*)k_count<4>; }
-static const void* scatter_fn(int items) { return items == 2 ? (const void*)k_scatter<2> : (const void*)k_scatter<4>; }
-
-namespace {
-constexpr int kMaxDevices = 64;
-struct DeviceSetup {
-  std::once_flag once;
-  int sms = 1;
-};
-DeviceSetup g_setup[kMaxDevices];
-std::mutex g_setup_mu;
-
-int setup_current_device(int dev) {
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  for (int items : {2, 4}) {
-    cudaFuncSetAttribute(count_fn(items), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(count_smem(items) + plan_bytes(kMaxRep)));
-    cudaFuncSetAttribute(scatter_fn(items), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(scatter_smem(items) + plan_bytes(kMaxRep)));
-  }
-  return sms > 0 ? sms : 1;
+// The built-in count and update/scatter passes for `items` rows at once.
+// (the passes for whole records come with 4 only)
+static const void* count_fn(int items, bool wide) {
+  return wide ? (const void*)k_count<4, true> : items == 2 ? (const void*)k_count<2, false> : (const void*)k_count<4, false>;
 }
-}  // namespace
+static const void* scatter_fn(int items, bool wide, bool ahead = false) {
+  if (wide) return (const void*)k_scatter<4, true, false>;
+  if (ahead) return items == 2 ? (const void*)k_scatter<2, false, true> : (const void*)k_scatter<4, false, true>;
+  return items == 2 ? (const void*)k_scatter<2, false, false> : (const void*)k_scatter<4, false, false>;
+}
 
-// The SM count of the current device, after its one-time set-up.
+// The SM count of the current device, after its one-time set-up: the dynamic
+// shared memory limit of the two passes (a function attribute applies to the
+// device that is current when it is set, so every device the library runs on
+// gets its own; devices beyond kMaxDevices are set up on every call).
+static int setup_device(int dev) {
+  int n = 0;
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  const int smem = (int)pass_smem(kMaxRep);
+  for (int items : {2, 4})
+    for (bool wide : {false, true}) {
+      cudaFuncSetAttribute(count_fn(items, wide), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      for (bool ahead : {false, true})
+        cudaFuncSetAttribute(scatter_fn(items, wide, ahead), cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    }
+  return n > 0 ? n : 1;
+}
 static int sm_count() {
+  constexpr int kMaxDevices = 64;
+  static std::once_flag once[kMaxDevices];
+  static int sms[kMaxDevices];
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= kMaxDevices) {
-    std::lock_guard<std::mutex> lk(g_setup_mu);
-    return setup_current_device(dev);
-  }
-  DeviceSetup& d = g_setup[dev];
-  std::call_once(d.once, [&] { d.sms = setup_current_device(dev); });
-  return d.sms;
+  if (dev < 0 || dev >= kMaxDevices) return setup_device(dev);
+  std::call_once(once[dev], [&] { sms[dev] = setup_device(dev); });
+  return sms[dev];
 }
-static void set_smem_attrs() { (void)sm_count(); }
-size_t count_smem_max() { return kCountSmem + plan_bytes(kMaxRep); }
-size_t scatter_smem_max() { return kScatterSmem + plan_bytes(kMaxRep); }
+size_t pass_smem_max() { return pass_smem(kMaxRep); }
 
-// Resident CTAs per SM of a persistent kernel, built in (for `items` slots
-// per thread) or of p.ks (4 slots per thread).
-static int occupancy(const void* ks, int kid, int items, int threads, size_t smem) {
-  if (ks) return species_occupancy(ks, kid, threads, smem);
-  set_smem_attrs();
+// Resident CTAs per SM of a pass, built in or of ks (4 rows at once).
+static int occupancy(const void* ks, bool scatter, int items, bool wide, uint32_t nrep) {
+  if (ks)
+    return species_occupancy(ks, scatter ? (wide ? KID_SCATTER_WIDE : KID_SCATTER) : (wide ? KID_COUNT_WIDE : KID_COUNT), kBlock,
+                             pass_smem(nrep));
+  (void)sm_count();  // the set-up
   int per = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kid == KID_COUNT ? count_fn(items) : scatter_fn(items), threads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scatter ? scatter_fn(items, wide) : count_fn(items, wide), kBlock,
+                                                pass_smem(nrep));
   return per;
 }
-int grid_blocks_count(uint32_t nrep, const void* ks, int items) {
-  const int per = occupancy(ks, KID_COUNT, items, kBlock, count_smem(items) + plan_bytes(nrep));
+int grid_blocks_count(uint32_t nrep, const void* ks, int items, bool wide) {
+  const int per = occupancy(ks, false, items, wide, nrep);
   return sm_count() * (per > 0 ? per : 1);
 }
-int grid_blocks_scatter(uint32_t nrep, const void* ks, int items) {
-  const int per = occupancy(ks, KID_SCATTER, items, kScatterThreads, scatter_smem(items) + plan_bytes(nrep));
+int grid_blocks_scatter(uint32_t nrep, const void* ks, int items, bool wide) {
+  const int per = occupancy(ks, true, items, wide, nrep);
   return sm_count() * (per > 0 ? per : 1);
 }
 
@@ -77,21 +72,44 @@ int grid_blocks_scatter(uint32_t nrep, const void* ks, int items) {
 static cudaError_t launch(const KParams& p, int kid, const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                           void** args) {
   if (p.ks) return species_launch(p.ks, kid, grid, block, smem, st, args);
-  set_smem_attrs();
+  (void)sm_count();  // the set-up
   return cudaLaunchKernel(fn, grid, block, args, smem, st);
 }
 
 cudaError_t launch_count(const KParams& p, int grid, cudaStream_t st, int items) {
   KParams q = p;
   void* args[] = {&q};
-  if (p.ks) items = kItems;  // a run-time species is built for 4 slots per thread
-  return launch(p, KID_COUNT, count_fn(items), grid, kBlock, count_smem(items) + plan_bytes(p.nrep), st, args);
+  return launch(p, p.wide ? KID_COUNT_WIDE : KID_COUNT, count_fn(items, p.wide), grid, kBlock, pass_smem(p.nrep), st, args);
 }
-cudaError_t launch_scatter(const KParams& p, int grid, cudaStream_t st, int items) {
+cudaError_t launch_scatter(const KParams& p, int grid, cudaStream_t st, int items, bool ahead) {
   KParams q = p;
   void* args[] = {&q};
-  if (p.ks) items = kItems;
-  return launch(p, KID_SCATTER, scatter_fn(items), grid, kScatterThreads, scatter_smem(items) + plan_bytes(p.nrep), st, args);
+  return launch(p, p.wide ? KID_SCATTER_WIDE : KID_SCATTER, scatter_fn(items, p.wide, ahead), grid, kBlock, pass_smem(p.nrep), st,
+                args);
+}
+cudaError_t launch_steps(const KParams& p, uint32_t nsteps, bool ahead, int grid_count, int grid_scatter, int items, cudaStream_t st,
+                         uint32_t* launches) {
+  cudaError_t e = cudaSuccess;
+  uint32_t n = 0;
+  auto run = [&](cudaError_t x) {
+    e = x;
+    n++;
+    return x == cudaSuccess;
+  };
+  if (ahead && can_decide_ahead(p) && nsteps > 1) {
+    // one count pass; every pass but the last decides the hour after its own
+    bool ok = run(launch_count(p, grid_count, st, items)) && run(launch_publish(p, PUB_DECIDED | PUB_AHEAD, st));
+    for (uint32_t i = 0; i < nsteps && ok; i++)
+      ok = run(launch_scatter(p, grid_scatter, st, items, true)) &&
+           run(launch_publish(p, PUB_AFTER_STEP | (i + 2 < nsteps ? PUB_AHEAD : 0), st));
+  } else {
+    for (uint32_t i = 0; i < nsteps; i++)
+      if (!run(launch_count(p, grid_count, st, items)) || !run(launch_scatter(p, grid_scatter, st, items, false)) ||
+          !run(launch_publish(p, PUB_AFTER_STEP, st)))
+        break;
+  }
+  if (launches) *launches += n;
+  return e;
 }
 cudaError_t launch_publish(const KParams& p, int mode, cudaStream_t st) {
   KParams q = p;
@@ -104,14 +122,20 @@ cudaError_t launch_init_eggs(const KParams& p, uint32_t n, float T0, const sampo
   void* args[] = {&q, &n, &T0, &seeds_dev, &age_days_max, &age_seed};
   return launch(p, KID_INIT_EGGS, (const void*)k_init_eggs, sm_count() * 4, 256, 0, st, args);
 }
-cudaError_t launch_publish_start(const KParams& p, cudaStream_t st) {
+cudaError_t launch_publish_start(const KParams& p, bool check, cudaStream_t st) {
   KParams q = p;
-  void* args[] = {&q};
+  int ck = check ? 1 : 0;
+  void* args[] = {&q, &ck};
   cudaError_t e = launch(p, KID_POOL_STATS, (const void*)k_pool_stats, sm_count() * 4, 256, 0, st, args);
   if (e != cudaSuccess) return e;
   int mode = PUB_INITIAL;
   void* args2[] = {&q, &mode};
   return launch(p, KID_PUBLISH, (const void*)k_publish, 1, kPublishThreads, 0, st, args2);
+}
+cudaError_t launch_widen(const KParams& p, cudaStream_t st) {
+  KParams q = p;
+  void* args[] = {&q};
+  return launch(p, KID_WIDEN, (const void*)k_widen, sm_count() * 4, 256, 0, st, args);
 }
 cudaError_t launch_histogram(const KParams& p, uint32_t* hist_dev, cudaStream_t st) {
   KParams q = p;
@@ -123,17 +147,11 @@ static cudaError_t launch_trial_reset(const KParams& p, cudaStream_t st) {
   void* args[] = {&q};
   return launch(p, KID_TRIAL_RESET, (const void*)k_trial_reset, (int)((p.nrep + 255) / 256), 256, 0, st, args);
 }
-// The built-in kernels only: a run-time species is tuned at one tile size.
-static cudaError_t launch_clear_lookback(const KParams& p, cudaStream_t st) {
-  KParams q = p;
-  void* args[] = {&q};
-  return cudaLaunchKernel((const void*)k_clear_lookback, sm_count() * 4, 256, args, 0, st);
-}
-// The grid tuner of one tile size: see tune_grids.
+// The grid tuner of one number of rows at once: see tune_grids.
 static cudaError_t tune_grids_items(const KParams& p, cudaStream_t st, int items, cudaEvent_t* ev, int* grid_count,
                                     int* grid_scatter, double* best_ms) {
-  int max_c = occupancy(p.ks, KID_COUNT, items, kBlock, count_smem(items) + plan_bytes(p.nrep));
-  int max_s = occupancy(p.ks, KID_SCATTER, items, kScatterThreads, scatter_smem(items) + plan_bytes(p.nrep));
+  int max_c = occupancy(p.ks, false, items, p.wide, p.nrep);
+  int max_s = occupancy(p.ks, true, items, p.wide, p.nrep);
   if (max_c < 1) max_c = 1;
   if (max_s < 1) max_s = 1;
   const int sms = sm_count();
@@ -205,16 +223,14 @@ cudaError_t tune_grids(const KParams& p, cudaStream_t st, int* grid_count, int* 
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < 3 && e == cudaSuccess; i++) e = cudaEventCreate(&ev[i]);
-  // tile sizes: 1024-slot tiles (4 slots per thread) and, for the built-in
-  // species, 512-slot tiles; the step as a whole decides
+  // 4 rows at once and, for the built-in species, 2; the step as a whole decides
   double best = 1e30;
   int bi = kItems, bgc = 0, bgs = 0;
   for (int it : {4, 2}) {
     if (e != cudaSuccess || (it != kItems && p.ks)) break;
     int gc = 0, gs = 0;
     double ms = 1e30;
-    if (!p.ks) e = launch_clear_lookback(p, st);  // the other tile size's trial prefixes
-    if (e == cudaSuccess) e = tune_grids_items(p, st, it, ev, &gc, &gs, &ms);
+    e = tune_grids_items(p, st, it, ev, &gc, &gs, &ms);
     if (e == cudaSuccess && ms < best) {
       best = ms;
       bi = it;
@@ -223,7 +239,6 @@ cudaError_t tune_grids(const KParams& p, cudaStream_t st, int* grid_count, int* 
     }
   }
   if (e == cudaSuccess) e = launch_trial_reset(p, st);
-  if (e == cudaSuccess && !p.ks) e = launch_clear_lookback(p, st);  // the step may run at either tile size
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   for (int i = 0; i < 3; i++)
     if (ev[i]) cudaEventDestroy(ev[i]);

@@ -17,9 +17,8 @@
 namespace sampo {
 
 constexpr int kBlock = 256;                 // threads per CTA
-constexpr int kItems = 4;                   // slots per thread per tile (striped by kBlock); 2 or 4 in the count and update/scatter passes
-constexpr int kTile = kBlock * kItems;      // slots per tile
-constexpr int kTileMin = kBlock * 2;        // the smallest tile the passes run with (the tile arrays have room for its count)
+constexpr int kItems = 4;                   // rows of 32 slots a warp of the count and update/scatter passes loads at once (2 or 4)
+constexpr int kTile = kBlock * 4;           // slots per tile of the one-launch step at its largest
 constexpr int kWarps = kBlock / 32;
 constexpr uint32_t kMaxRep = 1024;          // replicates per batch
 
@@ -41,73 +40,90 @@ struct DevSeedStream {
 };
 constexpr uint32_t kNoStream = 0xffffffffu;
 
+// What the decisions of one step add up to, besides the survivor counts.
+struct Decided {
+  uint32_t newEggs;           // eggs laid (EggsNbiomass.newEggs)
+  uint32_t L1de, dmin, dmax;  // the larvae of the pool it makes: L1de, youngest and oldest age in days
+};
+
 struct SimDev {
   sampo_population pop;       // ranges + stats of the current pool (reference pop[0] at step start)
   sampo_bites_cycles bnc;     // counters of the last update (printed with the next row)
   uint32_t step;              // index of the next step
   uint32_t cur;               // current pool buffer (0/1)
-  uint32_t epoch;             // look-back flag value of the running step (never reused)
-  uint32_t cnt[8];            // count pass: survivors by next state
-  uint32_t newEggs;           // count pass: eggs laid (EggsNbiomass.newEggs)
-  uint32_t acc_bnc[4];        // scatter pass: numCycles, sumCycles, numBites, numInfectBites
-  uint32_t acc_L1de, acc_fem, acc_inf, acc_dmin, acc_dmax;  // stats of the next pool
+  // The decided step: what its decisions (count pass, or the update/scatter
+  // pass of the step before) make of the pool.
+  Decided dec;
+  uint32_t cnt[8];            // its survivors by next state
+  Decided ahead_dec;          // the same of the step after, while a pass decides ahead
+  uint32_t ahead;             // the running step's update/scatter pass decides the step after
+  uint32_t rot;               // the span counts of the decided step: RepParams::spans + rot * spanStride
+  uint32_t dirty[3];          // spans of each of the three that may not be zero
+  uint32_t spans_done;        // count pass: spans counted so far
+  uint32_t acc_bnc[4];        // update/scatter pass: numCycles, sumCycles, numBites, numInfectBites
+  uint32_t acc_fem, acc_inf;  // females and potentially infective ones of the next pool
   uint32_t error;             // sticky SAMPO_DEV_ERR_* bits
   uint32_t warn;              // sticky SAMPO_DEV_WARN_* bits
   uint32_t capacity;
   float cc;                   // carrying capacity (constant per run, src/abms.c:19,132)
   uint32_t active;            // 1: the replicate takes part in the batch's steps
   uint32_t stop_step;         // becomes inactive once step reaches this
+  uint32_t wide;              // k_pool_stats: the pool holds a record its state does not imply (state_cols)
   DevSeedStream rnd;          // the replicate's own rand() stream, when its seeds are drawn on the device
-  StepCtx ctx;                // constants of step `step` (valid while active)
-  float larvaHMR[100];        // larval hourly mortality of step `step` by age in days
+  StepCtx ctx[2];             // constants of step s at s % 2 (the coming step's valid while active)
+  uint32_t larvaKill[2][100]; // larval mortality of step s by age in days (kill_threshold), at s % 2
 };
 
-// Batch-wide counters of the persistent kernels (tickets reset by k_publish).
+// Batch-wide counters.
 struct BatchDev {
-  uint32_t ticket1;           // count pass tile ticket
-  uint32_t ticket2;           // scatter pass tile ticket
   uint32_t bar;               // one-launch step: CTAs past the decision phase (reset by its last CTA)
   uint32_t done;              // one-launch step: CTAs finished (reset by its last CTA)
 };
 
-// The count pass's in-tile prefix table of one tile: for each (round, warp)
-// chunk of 32 slots (slot k * kBlock + tid is round k of warp tid / 32) and a
-// final entry for the whole tile, the survivors of the chunks before it by next
-// state (16-bit pairs: states 0-1, 2-3, 4-5, 6-7) and over all states.
-constexpr uint32_t kChunks = kItems * kWarps;
-constexpr uint32_t kPreEntryWords = 5;
-constexpr uint32_t kPreWords = ((kChunks + 1) * kPreEntryWords + 3) / 4 * 4;  // whole 16-byte units
-constexpr uint32_t kPreWordsMax = kPreWords;  // prefix-table words of one tile at I = 4, the largest
-constexpr uint32_t kPreWordsMin = ((2 * kWarps + 1) * kPreEntryWords + 3) / 4 * 4;  // at I = 2
-// Words of a pool's tile arrays for max_tiles tiles of kTileMin slots: the
-// prefix tables (max_tiles of the smaller tile's tables, plus one larger
-// table: ceil(C / kTile) tables of kPreWordsMax words fit in that too),
-// aggregates (8 per tile) and inclusive prefixes with their epochs (8 x 64 bits
-// per tile).
-constexpr uint32_t kPreRegionPad = kPreWordsMax;
-__host__ __device__ constexpr size_t tile_pre_words(uint32_t max_tiles) {
-  return (size_t)max_tiles * kPreWordsMin + kPreRegionPad;
+// Spans: the slots a warp of the two passes takes at once, 2^span_shift(end)
+// of a pool that ends at `end`. Small enough that every warp of the largest
+// grid (4,864) gets several, so that the last round is a small part of the
+// pass; large enough that a span's fixed work (its prefix, about a hundred
+// instructions) stays a small part of its own.
+constexpr uint32_t kSpanMinShift = 7, kSpanMaxShift = 10, kSpanTarget = 16384;
+__host__ __device__ constexpr uint32_t units_of(uint32_t n, uint32_t shift) { return (n >> shift) + ((n & ((1u << shift) - 1u)) ? 1u : 0u); }
+__host__ __device__ constexpr uint32_t span_shift(uint32_t end) {
+  uint32_t s = kSpanMinShift;
+  while (s < kSpanMaxShift && units_of(end, s) > kSpanTarget) s++;
+  return s;
 }
-__host__ __device__ constexpr size_t tile_array_words(uint32_t max_tiles) {
-  return tile_pre_words(max_tiles) + (size_t)max_tiles * (8 + 16);
+__host__ __device__ constexpr uint32_t span_count(uint32_t end) { return units_of(end, span_shift(end)); }
+// The most spans any pool of up to `capacity` slots has.
+__host__ __device__ constexpr uint32_t max_spans(uint32_t capacity) {
+  const uint32_t most = units_of(capacity, kSpanMaxShift), small = units_of(capacity, kSpanMinShift);
+  return small <= kSpanTarget ? small : most > kSpanTarget ? most : kSpanTarget;
 }
-static_assert(kPreWordsMin % 4 == 0 && kPreRegionPad % 4 == 0, "the inclusive prefixes start on a 16-byte boundary");
-static_assert(2 * kPreWordsMin >= kPreWordsMax, "two small tables hold one large table");
+// The span arrays of a pool of `capacity` slots, in 16-byte words: a span's
+// survivors by next state (one word, for each of three steps), a super's (32
+// spans) the same, and its exclusive prefix (two).
+__host__ __device__ constexpr uint32_t max_supers(uint32_t capacity) { return (max_spans(capacity) + 31u) / 32u; }
+__host__ __device__ constexpr size_t span_array_words(uint32_t capacity) {
+  return 3 * ((size_t)max_spans(capacity) + max_supers(capacity));
+}
 
 // Everything the kernels need of one replicate.
 struct RepParams {
   SimDev* sim;
   DevPool pool[2];
-  uint32_t* tilePre;          // [tiles][pre_words(I)] in-tile prefix tables (count pass), tile_pre_words(maxTiles) words
-  uint32_t* tileAgg;          // [maxTiles][8] per-tile survivor counts (count pass)
-  unsigned long long* tileIncl;  // [maxTiles][8] inclusive prefixes | epoch << 32 (scatter pass)
+  uint8_t* dec;               // caller-owned pools: [slots] the count pass's decisions; null: they are in the flags
+  uint4* spans;               // [3][spanStride] survivors by next state, 16 bits each: of the decided step, of the step
+                              // after (while deciding ahead), and the one cleared for the step after that
+  uint4* supers;              // [max_supers] the same of 32 spans, while they are being counted; zero otherwise
+  uint32_t* superPre;         // [max_supers][8] survivors of the supers before, of the decided step
+  uint32_t spanStride;
+  uint32_t* smallRows;        // one-launch step: [kSmallRows + kSmallStats][smallStride], or null
+  uint32_t smallStride;
   const float* T;             // [ring] temperature per step
   const sampo_environment* env;  // [ring]
   sampo_seeds* seeds;         // [ring][4] (written by the device for a device seed stream)
   const uint32_t* wt;         // [ring] world time per step
   sampo_stats_row* rows;      // [ring] stats at the start of each step
   uint32_t ring;
-  uint32_t maxTiles;
 };
 
 struct KParams {
@@ -116,13 +132,16 @@ struct KParams {
   BatchDev* bat;
   const ModelConst* mc;
   const void* ks;             // host: the kernels compiled for a user species (sampo_species.cu), or null
+  uint32_t wide;              // the pools hold whole records (state_cols)
 };
 
 // Modes of k_publish: PUB_AFTER_STEP turns the step's counts into the next
 // pool's start; PUB_INITIAL publishes the current pool (after init/load);
 // PUB_REFRESH recomputes the coming step's input-dependent constants (run it
-// after writing that step's inputs).
-enum : int { PUB_INITIAL = 0, PUB_AFTER_STEP = 1, PUB_REFRESH = 2 };
+// after writing that step's inputs); PUB_DECIDED follows a count pass whose
+// update/scatter pass decides ahead. PUB_DECIDED and PUB_AFTER_STEP take
+// PUB_AHEAD when the update/scatter pass that comes next decides ahead.
+enum : int { PUB_INITIAL = 0, PUB_AFTER_STEP = 1, PUB_REFRESH = 2, PUB_DECIDED = 3, PUB_MODE = 3, PUB_AHEAD = 4 };
 
 #ifndef __CUDACC_RTC__  // host side (the run-time compiler sees the device part only)
 
@@ -136,24 +155,23 @@ inline void fill_constant_tables(ModelConst& h) {
     float dmr = (a * e) / (1.0f + (a * B * sg * (e - 1.0f)));
     float dsr = 1.0f - dmr;
     float hsr = sampo_powf(dsr, 1.0f / 24.0f);
-    h.kill.adultHMR[d] = 1.0f - hsr;
+    h.kill.adult[d] = kill_threshold(1.0f - hsr);
   }
   float dmr = 0.1f;
   float dsr = 1.0f - dmr;
-  h.kill.aquaticHMR = 1.0f - sampo_powf(dsr, 1.0f / 24.0f);
+  h.kill.aquatic = kill_threshold(1.0f - sampo_powf(dsr, 1.0f / 24.0f));
   for (uint32_t k = 0; k < kEggBatchTable; k++) h.eggBatchScale[k] = egg_batch_scale(k);
 }
 
-// The tile arrays of a pool of max_tiles tiles of kTileMin slots at base
-// (16-byte aligned, for the bulk copies of the prefix tables): the prefix
-// tables (tile_pre_words words, indexed by the running tile size's table
-// length), then aggregates and inclusive prefixes.
-inline void set_tile_arrays(RepParams& r, uint32_t* base, uint32_t max_tiles) {
-  r.tilePre = base;
-  r.tileAgg = base + tile_pre_words(max_tiles);
-  r.tileIncl = reinterpret_cast<unsigned long long*>(r.tileAgg + (size_t)max_tiles * 8);
-  r.maxTiles = max_tiles;
+// The span arrays of a pool of `capacity` slots at base (16-byte aligned,
+// span_array_words words; they start as zeros).
+inline void set_span_arrays(RepParams& r, void* base, uint32_t capacity) {
+  r.supers = reinterpret_cast<uint4*>(base);
+  r.superPre = reinterpret_cast<uint32_t*>(r.supers + max_supers(capacity));
+  r.spans = r.supers + 3 * (size_t)max_supers(capacity);
+  r.spanStride = max_spans(capacity);
 }
+inline size_t span_array_bytes(uint32_t capacity) { return span_array_words(capacity) * sizeof(uint4); }
 
 // Why a pool's ranges cannot be stepped, or null when they can: the egg
 // range starts at slot 0, no range ends before it starts, the ranges are
@@ -177,8 +195,8 @@ inline SimDev initial_sim_state(uint32_t capacity, float cc) {
   memset(&h, 0, sizeof(h));
   h.capacity = capacity;
   h.cc = cc;
-  h.acc_dmin = 0xffffffffu;
-  h.epoch = 1;
+  h.dec.dmin = 0xffffffffu;
+  h.ahead_dec.dmin = 0xffffffffu;
   h.stop_step = 0xffffffffu;
   h.rnd.next = kNoStream;
   return h;
@@ -188,30 +206,46 @@ inline SimDev initial_sim_state(uint32_t capacity, float cc) {
 // p; init, pool statistics and the histogram take p.reps[0] only. They launch
 // the built-in kernels, or p.ks's when a species was compiled at run time.
 // persistent grid sizes (CTAs resident on all SMs) for batches of nrep replicates
-int grid_blocks_count(uint32_t nrep, const void* ks = nullptr, int items = kItems);
-int grid_blocks_scatter(uint32_t nrep, const void* ks = nullptr, int items = kItems);
+int grid_blocks_count(uint32_t nrep, const void* ks = nullptr, int items = kItems, bool wide = false);
+int grid_blocks_scatter(uint32_t nrep, const void* ks = nullptr, int items = kItems, bool wide = false);
 // The kernels of a run-time species (sampo_species.cu): launch one, and its
 // resident CTAs per SM.
-enum : int { KID_COUNT, KID_SCATTER, KID_PUBLISH, KID_INIT_EGGS, KID_POOL_STATS, KID_HISTOGRAM, KID_TRIAL_RESET, KID_N };
+enum : int {
+  KID_COUNT, KID_SCATTER, KID_COUNT_WIDE, KID_SCATTER_WIDE, KID_PUBLISH, KID_INIT_EGGS, KID_POOL_STATS, KID_HISTOGRAM,
+  KID_TRIAL_RESET, KID_WIDEN, KID_N
+};
 cudaError_t species_launch(const void* ks, int kid, dim3 grid, dim3 block, size_t smem, cudaStream_t st, void** args);
 int species_occupancy(const void* ks, int kid, int threads, size_t smem);
-// dynamic shared memory the persistent kernels may request
-size_t count_smem_max();
-size_t scatter_smem_max();
-// (the built-in passes for `items` = 2 or 4 slots per thread; a run-time
-// species is built for 4)
+// dynamic shared memory the two passes may request
+size_t pass_smem_max();
+// (the built-in passes for `items` = 2 or 4 rows at once; a run-time species
+// is built for 4; p.wide picks the passes that move whole records)
 cudaError_t launch_count(const KParams& p, int grid, cudaStream_t st, int items = kItems);
-cudaError_t launch_scatter(const KParams& p, int grid, cudaStream_t st, int items = kItems);
+cudaError_t launch_scatter(const KParams& p, int grid, cudaStream_t st, int items = kItems, bool ahead = false);
+// Whether the passes decide ahead over several hours (launch_steps): the
+// built-in species on narrow pools.
+inline bool can_decide_ahead(const KParams& p) { return !p.ks && !p.wide; }
+// `nsteps` hourly steps of every replicate of p. Deciding ahead: one count
+// pass, then an update/scatter pass and a publish per hour; otherwise the
+// three kernels every hour.
+cudaError_t launch_steps(const KParams& p, uint32_t nsteps, bool ahead, int grid_count, int grid_scatter, int items, cudaStream_t st,
+                         uint32_t* launches);
 // k_publish over every replicate of p (modes PUB_*, above).
 cudaError_t launch_publish(const KParams& p, int mode, cudaStream_t st);
 cudaError_t launch_init_eggs(const KParams& p, uint32_t n, float T0, const sampo_seeds* seeds_dev,
                              int age_days_max, uint64_t age_seed, cudaStream_t st);
-// statistics of p.reps[0]'s current pool, then its publish (PUB_INITIAL)
-cudaError_t launch_publish_start(const KParams& p, cudaStream_t st);
+// statistics of p.reps[0]'s current pool, then its publish (PUB_INITIAL);
+// `check` also finds out whether the pool is a wide one (SimDev::wide)
+cudaError_t launch_publish_start(const KParams& p, bool check, cudaStream_t st);
+// the columns that the records of p's narrow pools imply, written out, and
+// the decisions taken out of the flags (before a pool is read back)
+cudaError_t launch_widen(const KParams& p, cudaStream_t st);
 cudaError_t launch_histogram(const KParams& p, uint32_t* hist_dev, cudaStream_t st);
 cudaError_t launch_eval_math(int fn, const float* x, const float* y, float* out, uint32_t n, cudaStream_t st);
 // Kernel nodes in a captured graph (the launches one replay makes).
 cudaError_t graph_kernel_nodes(cudaGraph_t g, uint32_t* kernels);
+// Words of the one-launch step's rows per tile (sampo_small_step.cuh).
+constexpr uint32_t kSmallRowWords = 18;
 // The one-launch steps of a single simulation (sampo_small_step.cuh) with
 // tiles of kBlock * items slots (items 1, 2 or 4): the largest grid (CTAs
 // resident on all SMs, 0 if it cannot run) and a launch of `nsteps` hourly
@@ -219,10 +253,9 @@ cudaError_t graph_kernel_nodes(cudaGraph_t g, uint32_t* kernels);
 int grid_blocks_small(int items = kItems);
 cudaError_t launch_small(const KParams& p, int grid, bool cooperative, uint32_t nsteps, cudaStream_t st,
                          int items = kItems);
-// Times count + scatter of the coming step for each tile size (4 and, for
-// the built-in species, 2 slots per thread) at every (count, scatter) number
-// of CTAs per SM the occupancy allows, and returns the fastest tile size and
-// grids. The trials leave the simulations' course unchanged (k_trial_reset);
+// Times count + scatter of the coming step for each number of rows at once
+// (4 and, for the built-in species, 2) at every (count, scatter) number of
+// CTAs per SM the occupancy allows, and returns the fastest. The trials leave the simulations' course unchanged (k_trial_reset);
 // the coming step's constants must be current (PUB_REFRESH) before the call.
 cudaError_t tune_grids(const KParams& p, cudaStream_t st, int* grid_count, int* grid_scatter, int* items, double* best_ms);
 

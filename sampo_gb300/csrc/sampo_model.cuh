@@ -12,10 +12,12 @@
 //
 // update_agent<FULL> is used twice per step: FULL=false by the counting pass
 // (only the fields that decide survival, the next state and the number of
-// eggs laid) and FULL=true by the scatter pass (the complete record). Both
-// instantiations run the same decision code on the same inputs, so they
-// agree bit for bit. EGGS adds the eggs laid to Acc::newEggs (the counting
-// pass, and the one-launch step, whose single update decides and writes).
+// eggs laid) and FULL=true by the scatter pass (the complete record), which
+// takes the counting pass's decision (DECIDED: `code`, DEC_STAYS or
+// DEC_MOVES) instead of drawing it again. EGGS adds the eggs laid to
+// Acc::newEggs (the counting pass, and the one-launch step, whose single
+// update decides and writes).
+// WHOLE: the ages are whole hours (a narrow pool).
 // LDG reads the larval mortality table through the read-only cache; the
 // one-launch step, which rewrites the table between the hours of one launch,
 // keeps a copy in shared memory instead.
@@ -28,6 +30,14 @@
 namespace sampo {
 
 enum : int { EGG = 0, LARVA, PUPA, IMMATURE, MATESEEKING, BMS, BMD, GRAVID, NSTATE };
+// An hour's decision about an agent: it dies, stays in its state, moves on to
+// next_state(state), the one state it can leave for, or (a gravid caught by
+// an oviposition trap) dies and still reports its cycle.
+enum : uint32_t { DEC_DIES = 0, DEC_STAYS = 1, DEC_MOVES = 2, DEC_TRAPPED = 3 };
+__host__ __device__ constexpr int next_state(int rg) { return rg == GRAVID ? BMS : rg + 1; }
+__host__ __device__ constexpr uint32_t decision_code(int rg, int ns) {
+  return ns == rg ? DEC_STAYS : ns >= 0 ? DEC_MOVES : ns == -2 ? DEC_TRAPPED : DEC_DIES;
+}
 constexpr uint32_t kLayoutAlign = 64;  // LOCAL_SIZE (include/agent.h:9-17): a layout constant
 constexpr uint32_t kEggBatchTable = 64;  // batches with a tabulated 0.8^(n-1)
 
@@ -54,8 +64,8 @@ enum : uint32_t { BM_NONE = 0, BM_LARVA_DELAY = 1, BM_EGG_BATCH = 2 };
 // simulation (kernel/killAgents.cl:84-115,135-147; include/properties.h:262).
 // The count pass needs only the mortality part (KillConst, a prefix).
 struct KillConst {
-  float aquaticHMR;            // eggs and pupae (kernel/killAgents.cl:103-115,135-147)
-  float adultHMR[100];
+  uint32_t aquatic;            // eggs and pupae (kernel/killAgents.cl:103-115,135-147): kill_threshold of their hourly mortality
+  uint32_t adult[100];         // by age in days
 };
 struct ModelConst {
   KillConst kill;
@@ -68,7 +78,8 @@ struct ModelConst {
 struct alignas(16) StepCtx {
   // HybridTaus (include/gpuRand.h:33-50): z1 and z3 do not depend on the
   // work-item, so their Tausworthe steps are folded per seed slot.
-  uint32_t rng_c13[4], rng_z2[4], rng_z4[4];
+  // The linear generator's multiplier is folded too: rng_k4 = 1664525 * z4.
+  uint32_t rng_c13[4], rng_z2[4], rng_k4[4];
   sampo_environment env;
   float T;
   uint32_t wt;                 // world time = step % 24
@@ -82,7 +93,7 @@ struct alignas(16) StepCtx {
   float sporoH, sporoM, sporoL;  // sporoInc = sporoH + sporoM + sporoL exactly
   uint32_t sporoOn;            // T > 16
   uint32_t devOOB;             // T >= 44: the reference reads past devRates
-  const float* larvaHMR;       // [100] in global memory; NaN outside the larvae's age range of the step
+  const uint32_t* larvaKill;   // [100] in global memory: kill_threshold by age in days; 0 outside the larvae's ages of the step
 };
 
 // Counters an agent update contributes to (BitesNcycles, EggsNbiomass).
@@ -126,13 +137,33 @@ __device__ __forceinline__ float trunc_sat_fast(float x) {
   return r > x ? __fadd_rn(r, -1.0f) : r;
 }
 
-// HybridTaus of one seed slot whose z1 and z3 parts are folded into c13.
-__device__ __forceinline__ float rng_folded(uint32_t c13, uint32_t z2, uint32_t z4, uint32_t gid) {
-  uint32_t v = c13 ^ taus_step(z2 + gid, 2, 25, 4, 4294967288u) ^ (1664525u * (z4 * gid) + 1013904223u);
-  return 2.3283064365387e-10f * u32_to_f32_rn(v);  // (float)v * 2^-32
+// HybridTaus of one seed slot whose z1 and z3 parts are folded into c13 and
+// the linear part's multiplier into k4: the 32 bits of the draw, and the draw.
+__device__ __forceinline__ uint32_t rng_bits(uint32_t c13, uint32_t z2, uint32_t k4, uint32_t gid) {
+  return c13 ^ taus_step(z2 + gid, 2, 25, 4, 4294967288u) ^ (k4 * gid + 1013904223u);
+}
+__device__ __forceinline__ float rng_folded(uint32_t c13, uint32_t z2, uint32_t k4, uint32_t gid) {
+  return 2.3283064365387e-10f * u32_to_f32_rn(rng_bits(c13, z2, k4, gid));  // (float)v * 2^-32
 }
 __device__ __forceinline__ float rng(const StepCtx& c, int slot, uint32_t gid) {
-  return rng_folded(c.rng_c13[slot], c.rng_z2[slot], c.rng_z4[slot], gid);
+  return rng_folded(c.rng_c13[slot], c.rng_z2[slot], c.rng_k4[slot], gid);
+}
+
+// The mortality test `(float)v * 2^-32 <= hmr` on a draw's 32 bits: it holds
+// exactly for v < kill_threshold(hmr). Rounding v to binary32 is monotonic,
+// so the draws that pass are those up to hmr * 2^32 (exact: a power of two)
+// plus, from 2^24 on, the ones that round down to it: half a unit in the
+// last place more, the tie included when the last bit is even. 0 (no draw
+// dies) for NaN; a mortality of 1 or more does not occur.
+__host__ __device__ __forceinline__ uint32_t kill_threshold(float hmr) {
+  if (!(hmr >= 0.0f)) return 0u;
+  const float h = hmr * 4294967296.0f;
+  if (!(h < 4294967040.0f)) return 0xffffffffu;
+  const uint32_t n = (uint32_t)h;
+  if (h < 16777216.0f) return n + 1u;
+  uint32_t half = 1u;  // half a unit in the last place of h
+  for (uint32_t m = n >> 25; m; m >>= 1) half <<= 1;
+  return n + half + ((n / (2u * half)) & 1u ? 0u : 1u);
 }
 
 // BoxMuller (include/gpuRand.h:56-63) of two uniform draws.
@@ -152,31 +183,49 @@ __device__ __forceinline__ float box_muller(const StepCtx& c, uint32_t gid, floa
 
 namespace sampo {
 
+// (UINT)(age / 24.0f) of a whole number of hours below 2^21 (the ages of
+// narrow pools, see state_cols): half an hour past it the quotient is at
+// least 1/48 away from every whole number, far more than the two roundings,
+// so truncating it gives the same days as the exact division.
+__device__ __forceinline__ uint32_t whole_age_days(float age) {
+  return __float_as_uint(__fadd_rz(__fmul_rn(__fadd_rn(age, 0.5f), 1.0f / 24.0f), 8388608.0f)) - 0x4B000000u;
+}
+template <bool WHOLE = false>
 __device__ __forceinline__ uint32_t age_days(float age) {
+  if (WHOLE) {
+    const uint32_t d = whole_age_days(age);
+    return d < 99u ? d : 99u;
+  }
   return f32_to_u32_small(sampo_fminf(age / 24.0f, 99.0f));  // kernel/killAgents.cl:55
 }
 // (UINT)(age / 24.0f) without the 99-day cap (kernel/calcL1de.cl:30)
+template <bool WHOLE = false>
 __device__ __forceinline__ uint32_t age_days_uncapped(float age) {
-  return f2u_sat_fast(age / 24.0f);
+  return WHOLE ? whole_age_days(age) : f2u_sat_fast(age / 24.0f);
 }
 
 // Kill then update one valid agent of range rg at slot gid.
-// Returns the next state (0..7), or -1 when the agent dies this step.
-template <bool FULL, bool EGGS = !FULL, bool LDG = true>
-__device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& mc, int rg, uint32_t gid, Rec& a, Acc& acc) {
+// Returns the next state (0..7), or a negative value when the agent dies
+// this step (-2: a gravid caught by an oviposition trap, whose cycle is
+// still reported).
+template <bool FULL, bool EGGS = !FULL, bool LDG = true, bool DECIDED = false, bool WHOLE = false>
+__device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& mc, int rg, uint32_t gid, Rec& a, Acc& acc,
+                                            uint32_t code = DEC_STAYS) {
+  const bool moves = code == DEC_MOVES;  // DECIDED only
   // ---- killAgents (kernel/killAgents.cl:52-147) ----
-  {
-    float prob = rng(c, 0, gid);
-    float hmr;
+  if (!DECIDED) {
+    const uint32_t v = rng_bits(c.rng_c13[0], c.rng_z2[0], c.rng_k4[0], gid);
+    uint32_t kill;
     if (rg >= IMMATURE) {
-      hmr = mc.adultHMR[age_days(a.age)];
+      kill = mc.adult[age_days<WHOLE>(a.age)];
     } else if (rg == LARVA) {
-      hmr = LDG ? __ldg(c.larvaHMR + age_days(a.age)) : c.larvaHMR[age_days(a.age)];
-      if (hmr != hmr) acc.bad = 1;  // table entry not prepared
+      const uint32_t d = age_days<WHOLE>(a.age);
+      kill = LDG ? __ldg(c.larvaKill + d) : c.larvaKill[d];
+      if (kill == 0u) acc.bad = 1;  // table entry not prepared
     } else {
-      hmr = mc.aquaticHMR;
+      kill = mc.aquatic;
     }
-    if (prob <= hmr) return -1;
+    if (v < kill) return -1;
   }
   // ---- updateAgents (kernel/updateAgents.cl:57-270), elapsedTimeInHours = 1.0f ----
   a.age = a.age + 1.0f;
@@ -185,7 +234,7 @@ __device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& m
     a.sporo = sampo_sporo_add(a.sporo, c.sporoH, c.sporoM, c.sporoL, c.sporoInc);
   switch (rg) {
     case EGG:
-      if (a.his >= a.delay && (c.tt & TT_EGG)) {
+      if (DECIDED ? moves : a.his >= a.delay && (c.tt & TT_EGG)) {
         if (FULL) {
           a.age = 24.0f; a.his = 0.0f;
 #ifdef SAMPO_USER_SPECIES
@@ -198,40 +247,40 @@ __device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& m
       }
       return EGG;
     case LARVA: {
-      if (c.env.larvacideValue > 0.0f && a.his == 1.0f) {
+      if (!DECIDED && c.env.larvacideValue > 0.0f && a.his == 1.0f) {
         if (rng(c, 2, gid) <= c.env.larvacideValue) return -1;
       }
       float cld = __uint_as_float(a.uni) + c.larvaDev;
       if (FULL) a.uni = __float_as_uint(cld);
-      if (cld >= a.delay && (c.tt & TT_LARVA)) {
+      if (DECIDED ? moves : cld >= a.delay && (c.tt & TT_LARVA)) {
         if (FULL) { a.his = 0.0f; a.delay = c.pupaDelay; }
         return PUPA;
       }
       return LARVA;
     }
     case PUPA:
-      if (a.his >= a.delay && (c.tt & TT_PUPA)) {
+      if (DECIDED ? moves : a.his >= a.delay && (c.tt & TT_PUPA)) {
         if (FULL) { a.age = 0.0f; a.his = 0.0f; a.delay = c.immatureDelay; }
         return IMMATURE;
       }
       return PUPA;
     case IMMATURE:
-      if (a.his >= a.delay && (c.tt & TT_IMMATURE)) {
+      if (DECIDED ? moves : a.his >= a.delay && (c.tt & TT_IMMATURE)) {
         if (FULL) { a.delay = c.mateDelay; a.his = 0.0f; }
         return MATESEEKING;
       }
       return IMMATURE;
     case MATESEEKING:
-      if (a.his >= a.delay && a.female && (c.tt & TT_MATESEEKING)) {
+      if (DECIDED ? moves : a.his >= a.delay && a.female && (c.tt & TT_MATESEEKING)) {
         if (FULL) { a.his = 0.0f; a.delay = c.bmsDelay; }
         return BMS;
       }
       return MATESEEKING;
     case BMS:
       if (FULL) a.cycle += 1u;
-      if (a.his >= a.delay && (c.tt & TT_BMS)) {
-        if (rng(c, 1, gid) <= c.env.bloodmealSuccess) {
-          if (c.env.ITNValue * SAMPO_BITE_HUMAN * SAMPO_BITE_INDOOR > 0.0f) {
+      if (DECIDED ? moves : a.his >= a.delay && (c.tt & TT_BMS)) {
+        if (DECIDED || rng(c, 1, gid) <= c.env.bloodmealSuccess) {
+          if (!DECIDED && c.env.ITNValue * SAMPO_BITE_HUMAN * SAMPO_BITE_INDOOR > 0.0f) {
             if (rng(c, 2, gid) <= c.env.ITNValue * SAMPO_BITE_HUMAN * SAMPO_BITE_INDOOR) return -1;
           }
           if (FULL) {
@@ -247,11 +296,11 @@ __device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& m
       }
       return BMS;
     case BMD:
-      if (c.env.IRSValue * SAMPO_REST_INDOOR > 0.0f) {
+      if (!DECIDED && c.env.IRSValue * SAMPO_REST_INDOOR > 0.0f) {
         if (rng(c, 2, gid) <= c.env.IRSValue * SAMPO_REST_INDOOR) return -1;
       }
       if (FULL) a.cycle += 1u;
-      if (a.his >= a.delay && (c.tt & TT_BMD)) {
+      if (DECIDED ? moves : a.his >= a.delay && (c.tt & TT_BMD)) {
         if (FULL) {
           if (a.avail <= 0u && a.female) {
 #ifdef SAMPO_USER_SPECIES
@@ -270,11 +319,20 @@ __device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& m
       return BMD;
     default: {  // GRAVID
       if (FULL) a.cycle += 1u;
+      // a trapped gravid loses her eggs and dies, so a decided one was not trapped
+      if (DECIDED && moves) {  // she has laid her last eggs
+        if (FULL) {
+          a.uni += 1u; a.avail = 0u;
+          acc.cycles += 1u; acc.sumCycles += a.cycle;
+          a.cycle = 0u; a.his = 0.0f; a.delay = c.bmsDelay;
+        }
+        return BMS;
+      }
       if (c.tt & TT_LAY) {
         if (rng(c, 1, gid) < 0.25f) {
           uint32_t avail = a.avail;
           bool trapped = false;
-          if (c.env.oviTrapValue > 0.0f) {
+          if (!DECIDED && c.env.oviTrapValue > 0.0f) {
             if (rng(c, 2, gid) <= c.env.oviTrapValue) { trapped = true; avail = 0u; }
           }
           if (!trapped) {
@@ -297,7 +355,7 @@ __device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& m
               acc.cycles += 1u; acc.sumCycles += a.cycle;
               a.cycle = 0u; a.his = 0.0f; a.delay = c.bmsDelay;
             }
-            if (trapped) return -1;
+            if (trapped) return -2;
             return BMS;
           }
         }

@@ -19,7 +19,6 @@ using namespace sampo;
 
 namespace {
 
-constexpr uint32_t kMaxTiles = SAMPO_NOALLOC_MAX_SLOTS / kTileMin;  // tile arrays in kTileMin-slot tiles
 
 // One step of inputs (ring of two, as the kernels index step % ring).
 struct InputBlock {
@@ -30,7 +29,8 @@ struct InputBlock {
 };
 
 struct Scratch {
-  __align__(16) uint32_t tiles[tile_array_words(kMaxTiles)];  // prefix tables | counts | inclusive prefixes
+  __align__(16) uint4 spans[span_array_words(SAMPO_NOALLOC_MAX_SLOTS)];
+  uint8_t dec[SAMPO_NOALLOC_MAX_SLOTS];  // the count pass's decisions (the caller's pool is only read)
   SimDev sim;
   RepParams rep;
   BatchDev bat;
@@ -123,15 +123,17 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
   ib.env[0] = *env;
   for (int k = 0; k < 4; k++) ib.seeds[k] = seeds[k];
 
-  // The array keeps the previous call's contents: reset the state, and clear
-  // the inclusive prefixes of the tiles this step uses (a stale word carrying
-  // this step's epoch would be taken for a published prefix).
-  const uint32_t ntiles = (pop_in->r[7].end + kTile - 1) / kTile;
+  // The array keeps the previous call's contents: reset the state and clear
+  // the supers this step adds to.
+  const uint32_t nsup = (span_count(pop_in->r[7].end) + 31u) / 32u;
   RepParams rp;
   rp.sim = &sc->sim;
   rp.pool[0] = to_dev(in);
   rp.pool[1] = to_dev(out);
-  set_tile_arrays(rp, sc->tiles, kMaxTiles);
+  rp.dec = sc->dec;
+  set_span_arrays(rp, sc->spans, SAMPO_NOALLOC_MAX_SLOTS);
+  rp.smallRows = nullptr;
+  rp.smallStride = 0;
   rp.T = sc->in.T;
   rp.env = sc->in.env;
   rp.seeds = sc->in.seeds;
@@ -144,7 +146,7 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
       cudaMemcpyAsync(&sc->mc, &mc, sizeof(mc), cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(&sc->in, &ib, sizeof(ib), cudaMemcpyHostToDevice, st) != cudaSuccess)
     return SAMPO_ERR_CUDA;
-  if (ntiles && cudaMemsetAsync(rp.tileIncl, 0, (size_t)ntiles * 8 * sizeof(unsigned long long), st) != cudaSuccess)
+  if (nsup && cudaMemsetAsync(rp.supers, 0, (size_t)nsup * sizeof(uint4), st) != cudaSuccess)
     return SAMPO_ERR_CUDA;
 
   KParams p;
@@ -153,9 +155,10 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
   p.bat = &sc->bat;
   p.mc = &sc->mc;
   p.ks = nullptr;  // the built-in species
-  if (launch_publish_start(p, st) != cudaSuccess) return SAMPO_ERR_CUDA;
-  if (launch_count(p, grid_blocks_count(1), st) != cudaSuccess) return SAMPO_ERR_CUDA;
-  if (launch_scatter(p, grid_blocks_scatter(1), st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  p.wide = 1u;     // the caller's columns hold whole records
+  if (launch_publish_start(p, false, st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  if (launch_count(p, grid_blocks_count(1, nullptr, kItems, true), st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  if (launch_scatter(p, grid_blocks_scatter(1, nullptr, kItems, true), st) != cudaSuccess) return SAMPO_ERR_CUDA;
   if (launch_publish(p, PUB_AFTER_STEP, st) != cudaSuccess) return SAMPO_ERR_CUDA;
 
   uint32_t err = 0;

@@ -45,9 +45,19 @@ constexpr uint32_t kSmallHours = 24;       // hours whose inputs a CTA holds in 
 // L1de, females, infective, cycles, sum of cycles, bites, infective bites
 // (sums) and the min and max larva age in days.
 enum : uint32_t { SA_L1 = 0, SA_FEM, SA_INF, SA_CYC, SA_SUMCYC, SA_BITES, SA_IBITES, SA_DMIN, SA_DMAX, kSmallStats };
-// The rows' stride is twice the pool's count of 512-slot tiles (room for
-// 256-slot tiles): they fit the prefix-table array.
-static_assert(2 * (kSmallRows + kSmallStats) <= kPreWordsMin, "the per-tile rows fit the prefix-table array");
+static_assert(kSmallRows + kSmallStats == kSmallRowWords, "the rows' array has a word per row and tile");
+// The sizes of a kernel built for I slots per thread. A tile's prefix table
+// has, for each (round, warp) chunk of 32 slots (slot k * kBlock + tid is
+// round k of warp tid / 32) and for the whole tile, the survivors of the
+// chunks before it by next state (16-bit pairs) and over all states.
+constexpr uint32_t kPreEntryWords = 5;
+#define SAMPO_TILE_CONSTANTS(I)                    \
+  constexpr int kItems = (I);                      \
+  constexpr int kTile = kBlock * (I);              \
+  constexpr uint32_t kChunks = (uint32_t)(I) * kWarps; \
+  constexpr uint32_t kColBytes = (uint32_t)kTile * 4;  \
+  static_assert(kChunks <= 32, "one chunk per lane");  \
+  (void)kItems; (void)kChunks; (void)kColBytes
 
 __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
   uint32_t v;
@@ -98,7 +108,7 @@ struct SmallAcc {
 // counters and the next pool's statistics go to sa (a tile updated twice
 // counts its eggs the first time and the rest the second).
 template <int I, bool KEEP, bool EGGS, bool STATS>
-__device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelConst& mc, const sampo_population& pop,
+__device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelConst& mc, const sampo_population& pop, bool wide,
                                                   uint8_t* st, uint32_t lo, uint32_t end, uint2* s_ent, SmallAcc& sa) {
   SAMPO_TILE_CONSTANTS(I);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -127,6 +137,12 @@ __device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelC
       a.batches = c_batches[i];
       a.female = (c_flags[i] >> 3) & 1u;
       a.bm = BM_NONE;
+      if (!wide && rg < BMS) {  // a narrow record's implied fields (state_cols): the columns hold anything
+        a.sporo = 0.0f;
+        a.avail = a.cycle = a.hbc = a.batches = 0u;
+        if (rg == EGG) { a.his = a.age; a.uni = 0u; }
+        if (rg == LARVA) a.his = a.age - 24.0f;
+      }
       sa.devoob |= (rg == LARVA) & c.devOOB;
       const int ns = update_agent<true, true, false>(c, mc.kill, rg, g, a, t);
       if (ns >= 0) {
@@ -393,10 +409,8 @@ __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence
 // hold a tile, also writes them to the replicate's state for the host) before
 // it waits there; then the next hour's tile copies go out. The step inputs of
 // the launch's hours are read into shared memory at its start (the host
-// writes them before the launch). The rows use the replicate's prefix-table
-// array (tilePre: kSmallRows + kSmallStats words per column, at a stride of
-// twice its count of 512-slot tiles), which the three-kernel step rewrites
-// before it reads it. The pool the scatter wrote with ordinary stores is
+// writes them before the launch). The rows (smallRows: kSmallRows +
+// kSmallStats words per column) are read through L2. The pool the scatter wrote with ordinary stores is
 // read by the next hour's bulk copies after proxy fences.
 template <int I>
 __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(KParams p, uint32_t nsteps) {
@@ -404,7 +418,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
   extern __shared__ __align__(128) uint8_t stage[];
   __shared__ StepCtx s_c;
   __shared__ ModelConst s_mc;
-  __shared__ float s_hmr[100];
+  __shared__ uint32_t s_kill[100];
   __shared__ sampo_population s_pop;
   __shared__ CtxInputs s_in[kSmallHours];
   __shared__ __align__(8) uint64_t s_mbar;
@@ -413,7 +427,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
   __shared__ uint32_t s_ex[kSmallRows], s_tot[kSmallRows + kSmallStats], s_d0[8], s_ne[kWarps];
   __shared__ uint32_t s_red[kWarps][kSmallStats], s_part[kWarps][kSumWords];
   __shared__ uint32_t s_flag, s_ok, s_last;
-  __shared__ uint32_t s_active, s_end, s_nold, s_cur, s_cap, s_step, s_epoch, s_stop;
+  __shared__ uint32_t s_active, s_end, s_nold, s_cur, s_cap, s_step, s_stop;
   __shared__ float s_cc;
   const RepParams& rp = p.reps[0];
   SimDev* sim = rp.sim;
@@ -421,8 +435,9 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
   const uint32_t G = gridDim.x, b = blockIdx.x;
   uint32_t phase = 0, barriers = 0;
   bool met = true, ok = true;
-  const uint32_t stride = 2u * rp.maxTiles;  // >= the tiles of any pool that fits, at 256-slot tiles
-  uint32_t* rows = rp.tilePre;  // [kSmallRows + kSmallStats][stride]
+  const bool wide = p.wide != 0;
+  const uint32_t stride = rp.smallStride;  // >= the tiles of any pool that fits, at 256-slot tiles
+  uint32_t* rows = rp.smallRows;  // [kSmallRows + kSmallStats][stride]
 
   // ---- the replicate's state at the launch (the previous kernel wrote it) ----
   if (tid == 0) {
@@ -436,7 +451,6 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     s_cur = sim->cur;
     s_cap = sim->capacity;
     s_step = sim->step;
-    s_epoch = sim->epoch;
     s_stop = sim->stop_step;
     s_cc = sim->cc;
     if (b < s_nold) {
@@ -444,11 +458,11 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
       small_issue_tile<I>(rp.pool[s_cur], stage, &s_mbar, lo, min((uint32_t)kTile, s_end - lo));
     }
   }
-  copy16(&s_c, &sim->ctx, (int)sizeof(StepCtx), tid, blockDim.x);
-  for (int k = tid; k < 100; k += blockDim.x) s_hmr[k] = sim->larvaHMR[k];
+  copy16(&s_c, &sim->ctx[sim->step & 1u], (int)sizeof(StepCtx), tid, blockDim.x);
+  for (int k = tid; k < 100; k += blockDim.x) s_kill[k] = sim->larvaKill[sim->step & 1u][k];
   load_model_const(p.mc, s_mc);
   __syncthreads();
-  if (tid == 0) s_c.larvaHMR = s_hmr;
+  if (tid == 0) s_c.larvaKill = s_kill;
   // the inputs of the steps that follow the launch's hours
   for (uint32_t j = tid; j < min(nsteps, kSmallHours); j += blockDim.x) load_ctx_inputs(rp, s_step + 1u + j, s_in[j]);
   __syncthreads();
@@ -477,7 +491,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           if (!ok) break;
         }
         const uint32_t eggs_before = sa.acc.newEggs;
-        small_update_tile<I, false, true, true>(s_c, s_mc, s_pop, stage, t * kTile, end, s_ent, sa);
+        small_update_tile<I, false, true, true>(s_c, s_mc, s_pop, wide, stage, t * kTile, end, s_ent, sa);
         const uint32_t ne = __reduce_add_sync(0xffffffffu, sa.acc.newEggs - eggs_before);
         if (lane == 0) s_ne[warp] = ne;
         __syncthreads();
@@ -497,7 +511,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
         }
         ok = small_wait_stage(&s_mbar, phase);
         if (ok) {
-          small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, stage, b * kTile, end, s_ent, sa);  // counted above
+          small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, wide, stage, b * kTile, end, s_ent, sa);  // counted above
           small_stats_warps(sa, s_red);
           __syncthreads();
           if (warp == 0) (void)small_build_table<I>(s_ent, s_tab);
@@ -508,7 +522,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
       ok = small_wait_stage(&s_mbar, phase);
       if (ok) {
         const uint32_t eggs_before = sa.acc.newEggs;
-        small_update_tile<I, true, true, true>(s_c, s_mc, s_pop, stage, b * kTile, end, s_ent, sa);
+        small_update_tile<I, true, true, true>(s_c, s_mc, s_pop, wide, stage, b * kTile, end, s_ent, sa);
         const uint32_t ne = __reduce_add_sync(0xffffffffu, sa.acc.newEggs - eggs_before);
         if (lane == 0) s_ne[warp] = ne;
         small_stats_warps(sa, s_red);
@@ -553,7 +567,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           small_issue_tile<I>(rp.pool[s_cur], stage, &s_mbar, t * kTile, min((uint32_t)kTile, end - t * kTile));
         }
         if (!small_wait_stage(&s_mbar, phase)) { ok = false; break; }
-        small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, stage, t * kTile, end, s_ent, sa);
+        small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, wide, stage, t * kTile, end, s_ent, sa);
         small_sum_rows(rows, stride, nold, t, false, s_ex, s_tot, s_part);
         if (warp == 0) {
           const uint32_t tw = small_build_table<I>(s_ent, s_tab);
@@ -615,12 +629,12 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     np.numLarvae1DayEquiv = (np.r[LARVA].end > np.r[LARVA].start) ? st[SA_L1] : 0u;
     np.numFemale = st[SA_FEM];
     np.numPotentiallyInfective = st[SA_INF];
-    __syncthreads();  // every thread is past its last read of s_c, s_hmr and s_pop
+    __syncthreads();  // every thread is past its last read of s_c, s_kill and s_pop
     if (tid == 0) {
       CtxInputs& in = s_in[hour % kSmallHours];
       if (hour >= kSmallHours) load_ctx_inputs(rp, step, in);  // (its slot's hour is done)
       StepCtx c;
-      make_ctx(in, sim->larvaHMR, np, c);  // the global table: the last CTA stores this one
+      make_ctx(in, sim->larvaKill[step & 1u], np, c);  // the global table: the last CTA stores this one
       if (b == G - 1u) {
         // the replicate's state and the coming step's row for the host
         sampo_bites_cycles nbnc;
@@ -636,23 +650,21 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           moved += s_tot[k];
         }
         if (shared_end && moved) sim->warn = __ldcg(&sim->warn) | SAMPO_DEV_WARN_REF_LAYOUT;
-        sim->ctx = c;
+        sim->ctx[step & 1u] = c;
         sim->pop = np;
         sim->bnc = nbnc;
         sim->step = step;
         sim->cur = s_cur ^ 1u;
-        sim->epoch = s_epoch + 1u;
         sampo_stats_row row;
         row.pop = np;
         row.bnc = nbnc;
         rp.rows[step % rp.ring] = row;
         if (!active) sim->active = 0;
       }
-      c.larvaHMR = s_hmr;
+      c.larvaKill = s_kill;
       s_c = c;
       s_pop = np;
       s_step = step;
-      s_epoch += 1u;
       s_cur ^= 1u;
       s_end = next_end;
       s_nold = next_nold;
@@ -661,9 +673,9 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     {  // the next hour's larval table (every CTA; the last one also stores it)
       const uint32_t dmin = st[SA_DMIN], dmax = st[SA_DMAX], l1 = np.numLarvae1DayEquiv;
       for (int d = tid - 32; d >= 0 && d < 100; d += blockDim.x - 32) {
-        const float h = larva_hmr_entry((uint32_t)d, dmin, dmax, l1, s_cc);
-        s_hmr[d] = h;
-        if (b == G - 1u) sim->larvaHMR[d] = h;
+        const uint32_t k = larva_kill_entry((uint32_t)d, dmin, dmax, l1, s_cc);
+        s_kill[d] = k;
+        if (b == G - 1u) sim->larvaKill[step & 1u][d] = k;
       }
     }
     if (!more) break;  // (no copy is in flight)

@@ -115,9 +115,11 @@ void open_driver(Driver& d) {
 }
 
 // the kernels of one compiled species, in KID_* order
-const char* const kKernelNames[KID_N] = {"&sampo::k_count<4>",   "&sampo::k_scatter<4>", "&sampo::k_publish",
-                                         "&sampo::k_init_eggs",  "&sampo::k_pool_stats", "&sampo::k_histogram",
-                                         "&sampo::k_trial_reset"};
+const char* const kKernelNames[KID_N] = {"&sampo::k_count<4, false>", "&sampo::k_scatter<4, false, false>",
+                                         "&sampo::k_count<4, true>",  "&sampo::k_scatter<4, true, false>",
+                                         "&sampo::k_publish",         "&sampo::k_init_eggs",
+                                         "&sampo::k_pool_stats",      "&sampo::k_histogram",
+                                         "&sampo::k_trial_reset",     "&sampo::k_widen"};
 
 // standard headers the kernel sources include, reduced to what NVRTC lacks,
 // and the reference's headers a species header includes (the prelude defines
@@ -260,9 +262,8 @@ extern "C" int sampo_species_compile_text(const char* name, const char* text, in
     r = drv.get_function(&sp->fn[k], sp->module, lowered);
   }
   rt.destroy(&prog);
-  if (r == CUDA_SUCCESS) r = drv.set_attr(sp->fn[KID_COUNT], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)count_smem_max());
-  if (r == CUDA_SUCCESS)
-    r = drv.set_attr(sp->fn[KID_SCATTER], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)scatter_smem_max());
+  for (int k : {KID_COUNT, KID_SCATTER, KID_COUNT_WIDE, KID_SCATTER_WIDE})
+    if (r == CUDA_SUCCESS) r = drv.set_attr(sp->fn[k], CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)pass_smem_max());
   if (r != CUDA_SUCCESS) {
     if (sp->module) drv.module_unload(sp->module);
     delete sp;

@@ -107,7 +107,7 @@ __device__ __forceinline__ void user_seeds(const StepCtx& c, uint32_t gid, sampo
   for (int k = 0; k < 4; k++) {
     s[k].c13 = c.rng_c13[k];
     s[k].z2 = c.rng_z2[k];
-    s[k].z4 = c.rng_z4[k];
+    s[k].k4 = c.rng_k4[k];
     s[k].gid = gid;
   }
 }

@@ -66,10 +66,10 @@ struct AgentState {
 };
 
 struct Seeds {
-  uint c13, z2, z4, gid;
+  uint c13, z2, k4, gid;
 };
 
-static inline REAL HybridTaus(const struct Seeds* s) { return ::sampo::rng_folded(s->c13, s->z2, s->z4, s->gid); }
+static inline REAL HybridTaus(const struct Seeds* s) { return ::sampo::rng_folded(s->c13, s->z2, s->k4, s->gid); }
 static inline REAL BoxMuller(const struct Seeds* s, REAL mean, REAL stdDev) {
   return ::sampo::box_muller_u(HybridTaus(&s[0]), HybridTaus(&s[1]), mean, stdDev);
 }

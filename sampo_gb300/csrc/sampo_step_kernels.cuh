@@ -3,37 +3,24 @@
 // the library by nvcc (sampo_kernels.cu) and, for a user species header, at
 // run time by NVRTC (sampo_species.cu).
 //
-// A step of a batch of simulations is two persistent-CTA kernels over every
-// active replicate's current pool buffer, whose 1024-slot tiles they take
-// from one ticket counter, and a small one with a CTA per replicate:
+// A step of a batch of simulations is two kernels over every active
+// replicate's current pool buffer and a small one with a CTA per replicate:
 //
-//  k_count   reads the ~12 bytes per agent that decide survival, the next
+//  k_count   reads the ~8-12 bytes per agent that decide survival, the next
 //            state and the eggs laid (killAgents + the decision part of
-//            updateAgents), and publishes per tile the number of survivors
-//            per next state, the tile's prefix table over its (round, warp)
-//            chunks, and the replicate's newEggs total.
-//  k_scatter recomputes the same decisions with the complete record,
-//            obtains each survivor's stable rank within its next state
-//            (warp match/popc, the tile's prefix table, and a decoupled
-//            look-back over the tile counts that k_count already published,
-//            within the replicate, so no CTA ever waits on another and the
-//            consumer warps share no barrier), writes the updated
-//            record to its slot in the other buffer (the reference's
-//            oldToNewAgents layout, kernel/oldToNewAgents.cl:57-95,126-226),
-//            writes the new eggs at [0, newEggs) (initAgents,
-//            kernel/initAgents.cl:26-65), and accumulates the next step's
-//            statistics (calcL1de.cl, calcGender.cl).
+//            updateAgents), notes each decision in two bits of the agent's
+//            flags, and counts the survivors by next state per span of slots
+//            and the replicate's new eggs.
+//  k_scatter applies the decisions to the complete records, obtains each
+//            survivor's stable rank within its next state (the span counts
+//            of k_count, then ballots), writes the updated record to its
+//            slot in the other buffer (the reference's oldToNewAgents
+//            layout, kernel/oldToNewAgents.cl:57-95,126-226), writes the new
+//            eggs at [0, newEggs) (initAgents, kernel/initAgents.cl:26-65),
+//            and accumulates the next step's statistics (calcL1de.cl,
+//            calcGender.cl).
 //  k_publish turns each replicate's counts into its next population, stats
 //            row, step constants and larval mortality table.
-//
-// Both kernels stream tiles through shared memory with TMA bulk copies
-// (cp.async.bulk + mbarrier, double-buffered: tile j+1 is in flight while
-// tile j is processed). k_count loads only the columns the tile's ranges
-// need. In k_scatter a producer warp claims and describes tiles ahead and
-// issues their loads; the eight consumer warps release a stage as soon as
-// they have read it and write every survivor from registers straight to its
-// slot in the next buffer (a next state's survivors are contiguous within a
-// warp, so these stores coalesce).
 //
 // This replaces the reference's 19 kernels per step (killAgents,
 // updateAgents, initAgents, 3 x preScan + 3 x Bolt scan-by-key,
@@ -44,38 +31,9 @@
 namespace sampo {
 
 
-constexpr uint32_t kColBytes = kTile * 4;                    // one 4-byte column of a tile
-constexpr uint32_t kCountStage = 5 * kColBytes + kTile;      // age, his, delay, uni, avail, flags
-constexpr uint32_t kPreOff = 9 * kColBytes + kTile;          // the nine 4-byte columns and the flags,
-constexpr uint32_t kScatterStage = kPreOff + kPreWords * 4;   // then the tile's prefix table
-static_assert(kPreOff % 16 == 0 && kScatterStage % 16 == 0, "bulk copies land on 16-byte boundaries");
-
-// The count and update/scatter passes are built for I slots per thread
-// (tiles of 256 * I slots: I = 2 or 4, picked per workload by the
-// autotuner). Inside them these local constants stand for the tile sizes
-// above, which are those of I = 4.
-#define SAMPO_TILE_CONSTANTS(I)                                                         \
-  constexpr int kItems = (I);                                                         \
-  constexpr int kTile = kBlock * (I);                                                 \
-  constexpr uint32_t kChunks = (uint32_t)(I) * kWarps;                                \
-  constexpr uint32_t kPreWords = ((kChunks + 1) * kPreEntryWords + 3) / 4 * 4;        \
-  constexpr uint32_t kColBytes = (uint32_t)kTile * 4;                                 \
-  constexpr uint32_t kCountStage = 5 * kColBytes + kTile;                             \
-  constexpr uint32_t kPreOff = 9 * kColBytes + kTile;                                 \
-  constexpr uint32_t kScatterStage = kPreOff + kPreWords * 4;                         \
-  constexpr size_t kCountSmem = 2 * (size_t)kCountStage;                              \
-  constexpr size_t kScatterSmem = 2 * (size_t)kScatterStage;                          \
-  static_assert(kPreOff % 16 == 0 && kScatterStage % 16 == 0 && kChunks <= 32 && kPreWords <= kPreWordsMax, \
-                "bulk copies land on 16-byte boundaries; one chunk per lane; tables fit the tile arrays"); \
-  (void)kItems; (void)kChunks; (void)kCountSmem; (void)kScatterSmem
 constexpr uint32_t kWaitLimit = 1u << 22;                    // bounded mbarrier waits
 
 // ---------------- memory-model and TMA helpers ----------------
-__device__ __forceinline__ uint4 ld_cg_v4(const uint32_t* p) {
-  uint4 v;
-  asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ uint32_t lanemask_lt() {
   uint32_t m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -89,12 +47,6 @@ __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_init_count(uint64_t* bar, uint32_t n) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(n) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 // 1-D bulk copy global -> shared, completion counted on bar (both addresses
 // 16-byte aligned, bytes a multiple of 16).
@@ -172,13 +124,13 @@ __device__ __forceinline__ void load_ctx_inputs(const RepParams& rp, uint32_t st
 // (include/properties.h) and the biomass of the pool
 // (kernel/killAgents.cl:42-43). The larval mortality table is filled
 // separately (k_publish).
-__device__ void make_ctx(const CtxInputs& in, const float* larvaHMR, const sampo_population& pop, StepCtx& c) {
-  c.larvaHMR = larvaHMR;
+__device__ void make_ctx(const CtxInputs& in, const uint32_t* larvaKill, const sampo_population& pop, StepCtx& c) {
+  c.larvaKill = larvaKill;
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     c.rng_c13[k] = taus_step(in.sd[k].z1 + 128u, 13, 19, 12, 4294967294u) ^ taus_step(in.sd[k].z3 + 128u, 3, 11, 17, 4294967280u);
     c.rng_z2[k] = in.sd[k].z2 + 128u;
-    c.rng_z4[k] = in.sd[k].z4;
+    c.rng_k4[k] = 1664525u * in.sd[k].z4;
   }
   c.env = in.env;
   const float T = in.T;
@@ -303,438 +255,665 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, int bytes, in
 static_assert(sizeof(StepCtx) % 16 == 0, "StepCtx is copied in 16-byte words");
 
 // ------------------------------------------------------------------------
-// Count pass
+// The two passes of a step
 // ------------------------------------------------------------------------
-enum : uint32_t { CA_AGE = 1, CA_HIS = 2, CA_DELAY = 4, CA_UNI = 8, CA_AVAIL = 16, CA_FLAGS = 32 };
-
-// Columns the decision part of the update reads, by range (see update_agent<false>).
-__device__ __forceinline__ uint32_t count_cols(int rg, bool larvicide) {
-  switch (rg) {
-    case EGG: case PUPA: return CA_HIS | CA_DELAY;
-    case LARVA: return CA_AGE | CA_UNI | CA_DELAY | (larvicide ? CA_HIS : 0u);
-    case MATESEEKING: return CA_AGE | CA_HIS | CA_DELAY | CA_FLAGS;
-    case GRAVID: return CA_AGE | CA_AVAIL | CA_UNI;
-    default: return CA_AGE | CA_HIS | CA_DELAY;  // IMMATURE, BMS, BMD
-  }
-}
-
-template <int I>
-__device__ void issue_count_tile(const DevPool& src, uint8_t* st, uint64_t* bar, const sampo_population& pop,
-                                 uint32_t lo, uint32_t n, bool larvicide) {
-  SAMPO_TILE_CONSTANTS(I);
-  uint32_t m = 0;
-  for (int k = 0; k < 8; k++)
-    if (pop.r[k].end > pop.r[k].start && pop.r[k].start < lo + n && pop.r[k].end > lo) m |= count_cols(k, larvicide);
-  const uint32_t b4 = (n * 4 + 15) & ~15u, b1 = (n + 15) & ~15u;
-  uint32_t tx = __popc(m & 31u) * b4 + ((m & CA_FLAGS) ? b1 : 0u);
-  mbar_arrive_tx(bar, tx);
-  if (m & CA_AGE) bulk_load(st + 0 * kColBytes, src.age + lo, b4, bar);
-  if (m & CA_HIS) bulk_load(st + 1 * kColBytes, src.his + lo, b4, bar);
-  if (m & CA_DELAY) bulk_load(st + 2 * kColBytes, src.delay + lo, b4, bar);
-  if (m & CA_UNI) bulk_load(st + 3 * kColBytes, src.uni + lo, b4, bar);
-  if (m & CA_AVAIL) bulk_load(st + 4 * kColBytes, src.avail + lo, b4, bar);
-  if (m & CA_FLAGS) bulk_load(st + 5 * kColBytes, src.flags + lo, b1, bar);
-}
-
-// One tile in flight or in work in a count stage. The replicate's part
-// (c .. larv) is reloaded only when the stage moves on to another replicate.
-struct alignas(16) CountStage {
-  StepCtx c;
-  sampo_population pop;
-  DevPool src;
-  uint32_t* tileAgg;
-  uint32_t* tilePre;
-  uint32_t rep, lt, end, larv;    // replicate, its tile index, its pool end, larvicide on
-  uint32_t tick;                  // the tile's ticket; >= the ticket total: no more tiles
-  int urg;                        // the range that holds every slot of the tile, or -1
-  uint32_t left;                  // warps that have not finished the tile
-  uint32_t crep;                  // replicate whose survivor counts `cnt` holds
-  uint32_t cnt[8];                // survivors by next state of the stage's tiles of crep, not yet added to its totals
-};
-
-// Dynamic shared memory of the persistent kernels: the two stages, then the
-// batch's ticket prefix (nrep + 1 words), sized at launch so that a single
-// simulation pays 8 bytes for it.
-constexpr size_t kCountSmem = 2 * kCountStage;
-constexpr size_t kScatterSmem = 2 * kScatterStage;
-// the same for I slots per thread (the stages scale with the tile; the
-// prefix table has 8 I + 1 entries)
-__host__ __device__ constexpr uint32_t pre_words(int items) { return ((items * kWarps + 1) * kPreEntryWords + 3) / 4 * 4; }
-__host__ __device__ constexpr size_t count_smem(int items) { return 2 * (size_t)(5 * kBlock * items * 4 + kBlock * items); }
-__host__ __device__ constexpr size_t scatter_smem(int items) {
-  return 2 * (size_t)(9 * kBlock * items * 4 + kBlock * items + pre_words(items) * 4);
-}
-static_assert(count_smem(kItems) == kCountSmem && scatter_smem(kItems) == kScatterSmem, "one definition");
-__host__ __device__ constexpr size_t plan_bytes(uint32_t nrep) { return ((size_t)(nrep + 1) * 4 + 15) & ~(size_t)15; }
+// Both passes cut every active replicate's pool into spans of
+// 2^span_shift(end) slots and give the spans of the batch to the warps of a
+// grid of resident CTAs in turn (warp w takes units w, w + W, ...). A warp
+// walks its span range by range, 32 slots of one state at a time, with code
+// specialised for the state, and shares nothing with the other warps but the
+// span counts, so neither pass has a barrier, a ticket or a staged tile in
+// its loop.
+//
+// What bounds them is the number of instructions per agent and the bytes of
+// its record, so both are kept to what the state needs (state_cols): an egg
+// or a larva carries its age and delay (hoursInState follows from the age),
+// the sporogonic and gonotrophic fields are zero until a female seeks blood,
+// and the columns of a field that a state implies are neither read
+// nor written. A pool whose loaded records do not obey that (k_pool_stats
+// checks) and the caller-owned pools of sampo_step_noalloc take the WIDE
+// passes, which move whole records.
 constexpr uint32_t kNoRep = 0xffffffffu;
 
-// One warp's items of a count-pass tile in stage memory st: the decision
-// part of the update for each of its slots, and per (round, warp) chunk the
-// survivors by next state into ent (8-bit fields, states 0-3 | 4-7).
-// RG >= 0: every slot of the tile lies in range RG, so only that state's
-// code is compiled in; RG = -1: a tile that spans ranges.
-template <int I, int RG>
-__device__ __forceinline__ void count_items(const CountStage& cs, const uint8_t* st, const KillConst& mc, uint32_t lo,
-                                            uint32_t end, int tid, uint2* ent, Acc& acc, uint32_t& devoob) {
-  SAMPO_TILE_CONSTANTS(I);
-  const int lane = tid & 31, warp = tid >> 5;
-  const StepCtx& c = cs.c;
-  const bool larvicide = c.env.larvacideValue > 0.0f;
-  const float* s_age = (const float*)(st + 0 * kColBytes);
-  const float* s_his = (const float*)(st + 1 * kColBytes);
-  const float* s_delay = (const float*)(st + 2 * kColBytes);
-  const uint32_t* s_uni = (const uint32_t*)(st + 3 * kColBytes);
-  const uint32_t* s_avail = (const uint32_t*)(st + 4 * kColBytes);
-  const uint8_t* s_flags = st + 5 * kColBytes;
+enum : uint32_t {
+  C_AGE = 1, C_HIS = 2, C_DELAY = 4, C_SPORO = 8, C_UNI = 16, C_AVAIL = 32, C_CYCLE = 64, C_HBC = 128, C_BATCHES = 256,
+  C_ALL = 511
+};
+// Columns that hold an agent's record in state rg; the others are implied:
+// zero, or hoursInState = ageInHours (eggs) and ageInHours - 24 (larvae).
+__host__ __device__ constexpr uint32_t state_cols(int rg, bool wide) {
+  return wide || rg >= BMS ? (uint32_t)C_ALL
+         : rg == EGG       ? (uint32_t)(C_AGE | C_DELAY)
+         : rg == LARVA     ? (uint32_t)(C_AGE | C_DELAY | C_UNI)
+                           : (uint32_t)(C_AGE | C_HIS | C_DELAY | C_UNI);
+}
+// Columns the decision part of the update reads (update_agent<false>).
+__host__ __device__ constexpr uint32_t decide_cols(int rg, bool wide) {
+#ifdef SAMPO_USER_SPECIES
+  if (rg == GRAVID) return C_ALL;  // the header's layEggs may read any of the agent's fields
+#endif
+  return rg == EGG     ? (uint32_t)(C_DELAY | (wide ? C_HIS : C_AGE))
+         : rg == LARVA ? (uint32_t)(C_AGE | C_DELAY | C_UNI | (wide ? C_HIS : 0))
+         : rg == PUPA  ? (uint32_t)(C_HIS | C_DELAY)
+         : rg == GRAVID ? (uint32_t)(C_AGE | C_AVAIL | C_UNI)
+                        : (uint32_t)(C_AGE | C_HIS | C_DELAY);
+}
+__host__ __device__ constexpr uint32_t num_cols(uint32_t cols) {
+  uint32_t n = 0;
+  for (; cols; cols &= cols - 1u) n++;
+  return n;
+}
+
+// The columns of a range stream through a ring of chunks in the warp's own
+// piece of shared memory (cp.async, 16 bytes per lane), so that the loads of
+// the next chunks are in flight while one is worked on and cost no registers
+// (without the ring a warp waited a full memory latency for every four rows:
+// 57 % of its cycles). The chunk is the largest of 32 * I, 64 or 32 slots of
+// which at least two fit (I = 4 or 2, the "slots per thread").
+constexpr int kRowUnroll = 2;  // rows of a chunk unrolled together
+constexpr uint32_t kRingBytes = 4096;
+// Dynamic shared memory of the two passes: the rings and the batch's unit
+// prefix (nrep + 1 words), sized at launch so that a single simulation pays 8
+// bytes for it.
+__host__ __device__ constexpr size_t pass_smem(uint32_t nrep) {
+  return kWarps * (size_t)kRingBytes + (((size_t)(nrep + 1) * 4 + 15) & ~(size_t)15);
+}
+template <uint32_t COLS, uint32_t BYTE_COLS, int I>
+struct Ring {
+  static constexpr uint32_t kSlotBytes = 4 * num_cols(COLS) + BYTE_COLS;
+  __host__ __device__ static constexpr uint32_t fits(uint32_t slots) { return kRingBytes / (slots * kSlotBytes); }
+  static constexpr uint32_t kSlots = (I == 4 && fits(128) >= 2) ? 128u : fits(64) >= 2 ? 64u : 32u;
+  static constexpr uint32_t kStages = fits(kSlots) > 4 ? 4u : fits(kSlots);
+  static constexpr uint32_t kStageBytes = kSlots * kSlotBytes;
+  static_assert(kStages >= 2 && kStageBytes % 16 == 0, "two chunks at least, on 16-byte boundaries");
+  __host__ __device__ static constexpr uint32_t offset(uint32_t col) { return num_cols(COLS & (col - 1u)) * kSlots * 4u; }
+  static constexpr uint32_t kByteOffset = num_cols(COLS) * kSlots * 4u;
+};
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+// Starts the copies of the chunk at slot g0 (a multiple of 32) into the
+// stage: four slots per lane, as far as the range reaches (rounded up to four
+// slots, inside the columns' slack).
+template <class RING, uint32_t COLS>
+__device__ __forceinline__ void issue_chunk(uint8_t* st, const DevPool& s, const uint8_t* bytes0, const uint8_t* bytes1, uint32_t g0, uint32_t hi) {
+  const uint32_t i = 4u * (threadIdx.x & 31u);
+  const size_t g = (size_t)g0 + i;
+  if (i < RING::kSlots && g < hi) {
+    if (COLS & C_AGE) cp_async16(st + RING::offset(C_AGE) + 4 * i, s.age + g);
+    if (COLS & C_HIS) cp_async16(st + RING::offset(C_HIS) + 4 * i, s.his + g);
+    if (COLS & C_DELAY) cp_async16(st + RING::offset(C_DELAY) + 4 * i, s.delay + g);
+    if (COLS & C_SPORO) cp_async16(st + RING::offset(C_SPORO) + 4 * i, s.sporo + g);
+    if (COLS & C_UNI) cp_async16(st + RING::offset(C_UNI) + 4 * i, s.uni + g);
+    if (COLS & C_AVAIL) cp_async16(st + RING::offset(C_AVAIL) + 4 * i, s.avail + g);
+    if (COLS & C_CYCLE) cp_async16(st + RING::offset(C_CYCLE) + 4 * i, s.cycle + g);
+    if (COLS & C_HBC) cp_async16(st + RING::offset(C_HBC) + 4 * i, s.hbc + g);
+    if (COLS & C_BATCHES) cp_async16(st + RING::offset(C_BATCHES) + 4 * i, s.batches + g);
+    if (bytes0) cp_async4(st + RING::kByteOffset + i, bytes0 + g);
+    if (bytes1) cp_async4(st + RING::kByteOffset + RING::kSlots + i, bytes1 + g);
+  }
+  cp_async_commit();
+}
+template <class RING, uint32_t COLS>
+__device__ __forceinline__ void read_chunk(const uint8_t* st, uint32_t i, Rec& a) {
+  const float* f = reinterpret_cast<const float*>(st) + i;
+  const uint32_t* u = reinterpret_cast<const uint32_t*>(st) + i;
+  a.age = (COLS & C_AGE) ? f[RING::offset(C_AGE) / 4] : 0.0f;
+  a.his = (COLS & C_HIS) ? f[RING::offset(C_HIS) / 4] : 0.0f;
+  a.delay = (COLS & C_DELAY) ? f[RING::offset(C_DELAY) / 4] : 0.0f;
+  a.sporo = (COLS & C_SPORO) ? f[RING::offset(C_SPORO) / 4] : 0.0f;
+  a.uni = (COLS & C_UNI) ? u[RING::offset(C_UNI) / 4] : 0u;
+  a.avail = (COLS & C_AVAIL) ? u[RING::offset(C_AVAIL) / 4] : 0u;
+  a.cycle = (COLS & C_CYCLE) ? u[RING::offset(C_CYCLE) / 4] : 0u;
+  a.hbc = (COLS & C_HBC) ? u[RING::offset(C_HBC) / 4] : 0u;
+  a.batches = (COLS & C_BATCHES) ? u[RING::offset(C_BATCHES) / 4] : 0u;
+  a.female = 0u;
+  a.bm = BM_NONE;
+}
+// Walks slots [lo, hi) of the current buffer in chunks: f(stage, first slot)
+// for each, with the copies of the following chunks in flight. Every lane
+// calls it; the stage may be read by any lane until f returns.
+template <class RING, uint32_t COLS, class F>
+__device__ __forceinline__ void stream_range(uint8_t* ring, const DevPool& s, const uint8_t* bytes0, const uint8_t* bytes1, uint32_t lo,
+                                             uint32_t hi, F&& f) {
+  constexpr uint32_t N = RING::kStages;
+  const uint32_t first = lo & ~31u;
 #pragma unroll
-  for (int k = 0; k < kItems; k++) {
-    const uint32_t i = k * kBlock + tid;
-    const uint32_t g = lo + i;
-    int rg;
-    bool valid;
-    if (RG >= 0) {
-      rg = RG;
-      valid = g < end;
-    } else {
-      rg = g < end ? range_of(cs.pop, g) : -1;
-      valid = rg >= 0;
+  for (uint32_t j = 0; j < N - 1; j++) issue_chunk<RING, COLS>(ring + j * RING::kStageBytes, s, bytes0, bytes1, first + j * RING::kSlots, hi);
+  uint32_t rd = 0, wr = N - 1;
+  for (uint32_t g0 = first; g0 < hi; g0 += RING::kSlots) {
+    issue_chunk<RING, COLS>(ring + wr * RING::kStageBytes, s, bytes0, bytes1, g0 + (N - 1) * RING::kSlots, hi);
+    cp_async_wait<N - 1>();
+    __syncwarp();  // every lane's copies of this chunk are in
+    f(ring + rd * RING::kStageBytes, g0);
+    __syncwarp();  // the stage is read before its next copies start
+    rd = rd + 1 == N ? 0 : rd + 1;
+    wr = wr + 1 == N ? 0 : wr + 1;
+  }
+  cp_async_wait<0>();
+}
+// The fields a narrow record implies.
+template <int RG, bool WIDE>
+__device__ __forceinline__ void implied_fields(Rec& a) {
+  if (!WIDE && RG == EGG) a.his = a.age;
+  if (!WIDE && RG == LARVA) a.his = a.age - 24.0f;
+}
+// Stores to a pool that the kernel does not read: as global stores that the
+// compiler need not order against the warps' state in shared memory (through
+// the pools' pointers, which it reads from memory, it would take them for
+// stores to anywhere, and read the step's constants again after each).
+__device__ __forceinline__ void put(float* p, float v) { asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(v)); }
+__device__ __forceinline__ void put(uint32_t* p, uint32_t v) { asm volatile("st.global.u32 [%0], %1;" ::"l"(p), "r"(v)); }
+__device__ __forceinline__ void put(uint8_t* p, uint32_t v) { asm volatile("st.global.u8 [%0], %1;" ::"l"(p), "r"(v)); }
+template <uint32_t COLS>
+__device__ __forceinline__ void store_cols(const DevPool& d, uint32_t g, const Rec& a) {
+  if (COLS & C_AGE) put(d.age + g, a.age);
+  if (COLS & C_HIS) put(d.his + g, a.his);
+  if (COLS & C_DELAY) put(d.delay + g, a.delay);
+  if (COLS & C_SPORO) put(d.sporo + g, a.sporo);
+  if (COLS & C_UNI) put(d.uni + g, a.uni);
+  if (COLS & C_AVAIL) put(d.avail + g, a.avail);
+  if (COLS & C_CYCLE) put(d.cycle + g, a.cycle);
+  if (COLS & C_HBC) put(d.hbc + g, a.hbc);
+  if (COLS & C_BATCHES) put(d.batches + g, a.batches);
+}
+
+// Survivors by next state, 16 bits each: states 0-1, 2-3, 4-5, 6-7. A span
+// has at most 2^10 slots and a super (32 spans) 2^15, so no field carries.
+__device__ __forceinline__ uint32_t state_count(const uint4& v, int b) {
+  const uint32_t w = b < 2 ? v.x : b < 4 ? v.y : b < 6 ? v.z : v.w;
+  return (w >> (16 * (b & 1))) & 0xffffu;
+}
+template <int B>
+__device__ __forceinline__ void add_count(uint4& v, uint32_t n) {
+  const uint32_t x = n << (16 * (B & 1));
+  if (B < 2) v.x += x;
+  else if (B < 4) v.y += x;
+  else if (B < 6) v.z += x;
+  else v.w += x;
+}
+// One lane: adds a span's counts to its super's.
+__device__ __forceinline__ void add_super(uint4* sup, const uint4& v) {
+  unsigned long long* q = reinterpret_cast<unsigned long long*>(sup);
+  const unsigned long long a = v.x | ((unsigned long long)v.y << 32), b = v.z | ((unsigned long long)v.w << 32);
+  if (a) atomicAdd(q, a);
+  if (b) atomicAdd(q + 1, b);
+}
+
+// Once every span of the replicate is counted: the exclusive prefix by state
+// of each super and the totals (cnt, 8 words); the raw counts are cleared for
+// the next step. The calling threads (nt of them, thread t) take contiguous
+// runs of supers: one pass of independent loads, one scan over the threads
+// (`scan` returns a thread's exclusive prefix of a value and the total), one
+// pass back.
+template <class Scan>
+__device__ __forceinline__ void scan_supers(const RepParams& rp, uint32_t nspans, uint32_t* cnt, uint32_t t, uint32_t nt, Scan scan) {
+  const uint32_t nsup = (nspans + 31u) / 32u, per = (nsup + nt - 1u) / nt;
+  const uint32_t i0 = min(t * per, nsup), i1 = min(i0 + per, nsup);
+  uint32_t sum[8];
+#pragma unroll
+  for (int b = 0; b < 8; b++) sum[b] = 0;
+#pragma unroll 4
+  for (uint32_t i = i0; i < i1; i++) {
+    const uint4 v = __ldcg(rp.supers + i);
+#pragma unroll
+    for (int b = 0; b < 8; b++) sum[b] += state_count(v, b);
+  }
+  uint32_t run[8];
+  scan(sum, run, cnt);
+#pragma unroll 2
+  for (uint32_t i = i0; i < i1; i++) {
+    const uint4 v = __ldcg(rp.supers + i);
+    uint4* o = reinterpret_cast<uint4*>(rp.superPre + (size_t)i * 8);
+    o[0] = make_uint4(run[0], run[1], run[2], run[3]);
+    o[1] = make_uint4(run[4], run[5], run[6], run[7]);
+    rp.supers[i] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int b = 0; b < 8; b++) run[b] += state_count(v, b);
+  }
+}
+// The eight sums of the lanes of a warp: exclusive prefixes; lane 31 has the totals in incl.
+__device__ __forceinline__ void warp_scan8(const uint32_t (&sum)[8], uint32_t (&run)[8], uint32_t (&incl)[8]) {
+  const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int b = 0; b < 8; b++) {
+    uint32_t x = sum[b];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= (uint32_t)o) x += y;
     }
-    uint32_t pk0 = 0, pk1 = 0;  // this slot's next state as an 8-bit counter: states 0-3, 4-7
-    if (valid) {
-      Rec a;
-      a.age = (rg == LARVA || rg >= IMMATURE) ? s_age[i] : 0.0f;
-      a.his = (rg != GRAVID && (rg != LARVA || larvicide)) ? s_his[i] : 0.0f;
-      a.delay = rg != GRAVID ? s_delay[i] : 0.0f;
-      a.uni = (rg == LARVA || rg == GRAVID) ? s_uni[i] : 0u;
-      a.avail = rg == GRAVID ? s_avail[i] : 0u;
-      a.female = rg == MATESEEKING ? (s_flags[i] >> 3) & 1u : 0u;
-      a.sporo = 0.0f; a.cycle = 0u; a.hbc = 0u; a.batches = 0u;
-      devoob |= (rg == LARVA) & c.devOOB;
-      const int ns = update_agent<false>(c, mc, rg, g, a, acc);
-      if (ns >= 0) {
-        if (ns < 4) pk0 = 1u << (8 * ns);
-        else pk1 = 1u << (8 * (ns - 4));
+    incl[b] = x;
+    run[b] = x - sum[b];
+  }
+}
+// scan_supers by one warp.
+__device__ void scan_supers_warp(const RepParams& rp, uint32_t nspans, uint32_t* cnt) {
+  const uint32_t lane = threadIdx.x & 31u;
+  scan_supers(rp, nspans, cnt, lane, 32u, [&](const uint32_t (&sum)[8], uint32_t (&run)[8], uint32_t* tot) {
+    uint32_t incl[8];
+    warp_scan8(sum, run, incl);
+    if (lane == 31u) {
+#pragma unroll
+      for (int b = 0; b < 8; b++) tot[b] = incl[b];
+    }
+  });
+}
+// scan_supers by a CTA of at most 32 warps (all threads; ends synchronised).
+// s_part: 32 x 8 words.
+__device__ void scan_supers_block(const RepParams& rp, uint32_t nspans, uint32_t* cnt, uint32_t (*s_part)[8]) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  scan_supers(rp, nspans, cnt, threadIdx.x, blockDim.x, [&](const uint32_t (&sum)[8], uint32_t (&run)[8], uint32_t* tot) {
+    uint32_t incl[8];
+    warp_scan8(sum, run, incl);
+    if (lane == 31u) {
+#pragma unroll
+      for (int b = 0; b < 8; b++) s_part[warp][b] = incl[b];
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {  // one state per thread over the warps
+      uint32_t x = 0;
+      for (uint32_t i = 0; i < nw; i++) {
+        const uint32_t y = s_part[i][threadIdx.x];
+        s_part[i][threadIdx.x] = x;
+        x += y;
+      }
+      tot[threadIdx.x] = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < 8; b++) run[b] += s_part[warp][b];
+  });
+  __syncthreads();
+}
+
+// What a warp holds of the replicate its unit belongs to; reloaded only when
+// its next unit belongs to another one.
+struct alignas(16) WarpRep {
+  StepCtx c;                    // constants of the step
+  StepCtx c1;                   // and of the step after, while deciding ahead
+  sampo_population pop, next;   // current ranges; the next pool's (update/scatter pass)
+  DevPool src, dst;
+  uint8_t* dec;                 // decisions of caller-owned pools, or null: in the flags
+  uint4 *spans, *spans1, *spans2;  // span counts of the step, of the step after, and the ones to clear
+  uint4* supers;
+  const uint32_t* superPre;
+  uint32_t shift, nspans, newEggs, ahead;
+  uint32_t shift1, clear, clearPer;  // span size of the next pool; spans to clear, and of them per unit
+};
+// Words of src to dst by the lanes of a warp.
+template <class T>
+__device__ __forceinline__ void warp_copy(T* dst, const T* src) {
+  static_assert(sizeof(T) % 4 == 0, "whole words");
+  uint32_t* d = reinterpret_cast<uint32_t*>(dst);
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(src);
+  for (int k = threadIdx.x & 31; k < (int)(sizeof(T) / 4); k += 32) d[k] = q[k];
+}
+// (PASS2: also what the update/scatter pass needs)
+template <bool PASS2, bool AHEAD>
+__device__ __forceinline__ void load_warp_rep(const RepParams& rp, WarpRep& w) {
+  const SimDev* sim = rp.sim;
+  const uint32_t cur = sim->cur, par = sim->step & 1u;
+  __syncwarp();  // every lane is past its reads of the last replicate's
+  warp_copy(&w.c, &sim->ctx[par]);
+  if (AHEAD) warp_copy(&w.c1, &sim->ctx[par ^ 1u]);
+  warp_copy(&w.pop, &sim->pop);
+  warp_copy(&w.src, &rp.pool[cur]);
+  if (PASS2) warp_copy(&w.dst, &rp.pool[cur ^ 1u]);
+  if ((threadIdx.x & 31) == 0) {
+    const uint32_t end = sim->pop.r[GRAVID].end, rot = sim->rot;
+    w.dec = rp.dec;
+    w.spans = rp.spans + (size_t)rot * rp.spanStride;
+    w.supers = rp.supers;
+    w.superPre = rp.superPre;
+    w.shift = span_shift(end);
+    w.nspans = span_count(end);
+    w.newEggs = sim->dec.newEggs;
+    if (PASS2) {
+      uint32_t tc[8], base[8];
+      for (int k = 0; k < 8; k++) tc[k] = sim->cnt[k];
+      sampo_population np;
+      next_layout(tc, w.newEggs, np, base);
+      w.next = np;
+      if (AHEAD) {
+        w.ahead = sim->ahead;
+        w.shift1 = span_shift(np.r[GRAVID].end);
+        w.spans1 = rp.spans + (size_t)(rot == 2u ? 0u : rot + 1u) * rp.spanStride;
+        const uint32_t old = rot == 0u ? 2u : rot - 1u, units = w.nspans + units_of(w.newEggs, w.shift);
+        w.spans2 = rp.spans + (size_t)old * rp.spanStride;
+        w.clear = w.ahead ? sim->dirty[old] : 0u;
+        w.clearPer = units ? (w.clear + units - 1u) / units : 0u;
       }
     }
-    pk0 = __reduce_add_sync(0xffffffffu, pk0);
-    pk1 = __reduce_add_sync(0xffffffffu, pk1);
-    if (lane == 0) ent[k * kWarps + warp] = make_uint2(pk0, pk1);
+  }
+  __syncwarp();
+}
+
+// What a warp adds to its replicate, gathered range by range in shared memory
+// (written by lane 0).
+struct WarpSum {
+  Decided dec;                 // of the step being decided
+  uint32_t fem, inf, bnc[4];   // of the pool being written
+  uint32_t error;
+};
+__device__ __forceinline__ void clear_sum(WarpSum& t) {
+  t.dec = Decided{0u, 0u, 0xffffffffu, 0u};
+  t.fem = t.inf = t.error = 0;
+  t.bnc[0] = t.bnc[1] = t.bnc[2] = t.bnc[3] = 0;
+}
+// Lane 0: the warp's sums into its replicate, and cleared.
+__device__ __forceinline__ void flush_sum(WarpSum& t, SimDev* sim, Decided* to) {
+  if (t.dec.newEggs) atomicAdd(&to->newEggs, t.dec.newEggs);
+  if (t.dec.L1de) atomicAdd(&to->L1de, t.dec.L1de);
+  if (t.dec.dmin != 0xffffffffu) { atomicMin(&to->dmin, t.dec.dmin); atomicMax(&to->dmax, t.dec.dmax); }
+  if (t.fem) atomicAdd(&sim->acc_fem, t.fem);
+  if (t.inf) atomicAdd(&sim->acc_inf, t.inf);
+  for (int j = 0; j < 4; j++)
+    if (t.bnc[j]) atomicAdd(&sim->acc_bnc[j], t.bnc[j]);
+  if (t.error) atomicOr(&sim->error, t.error);
+  clear_sum(t);
+}
+
+// What a lane's decisions in one range add up to.
+struct DecideAcc {
+  Acc acc;             // newEggs and bad
+  uint32_t l1, dmin, dmax, devoob;
+};
+__device__ __forceinline__ void clear_acc(DecideAcc& d) {
+  d.acc = Acc{0, 0, 0, 0, 0, 0};
+  d.l1 = d.dmax = d.devoob = 0;
+  d.dmin = 0xffffffffu;
+}
+// A range's decisions (state RG, and NX for those that moved there) into the warp's sums.
+template <int RG, int NX>
+__device__ __forceinline__ void add_decided(const DecideAcc& d, WarpSum& t) {
+  constexpr bool larvae = RG <= LARVA || NX == LARVA, lays = RG == GRAVID || NX == GRAVID;
+  const uint32_t ne = lays ? __reduce_add_sync(0xffffffffu, d.acc.newEggs) : 0u;
+  const uint32_t l1 = larvae ? __reduce_add_sync(0xffffffffu, d.l1) : 0u;
+  const uint32_t mn = larvae ? __reduce_min_sync(0xffffffffu, d.dmin) : 0xffffffffu, mx = larvae ? __reduce_max_sync(0xffffffffu, d.dmax) : 0u;
+  const uint32_t bad = larvae ? __reduce_or_sync(0xffffffffu, (d.acc.bad ? SAMPO_DEV_ERR_LARVATABLE : 0u) |
+                                                                (d.devoob ? SAMPO_DEV_ERR_DEVRATES : 0u)) : 0u;
+  if ((threadIdx.x & 31) == 0) {
+    t.dec.newEggs += ne;
+    t.dec.L1de += l1;
+    t.dec.dmin = min(t.dec.dmin, mn);
+    t.dec.dmax = max(t.dec.dmax, mx);
+    t.error |= bad;
+  }
+}
+// The decision about the agent a at slot g of range RG (a: its fields of
+// decide_cols; changed). Adds the larva it leaves to the next pool's
+// statistics (kernel/calcL1de.cl:28-30).
+template <int RG, bool WIDE>
+__device__ __forceinline__ uint32_t decide(const StepCtx& c, const KillConst& kc, uint32_t g, Rec& a, DecideAcc& d) {
+  if (RG == LARVA) d.devoob |= c.devOOB;
+  const uint32_t code = decision_code(RG, update_agent<false, true, true, false, !WIDE>(c, kc, RG, g, a, d.acc));
+  if (RG == EGG && code == DEC_MOVES) {  // hatched: 24 hours old
+    d.l1 += 1u;
+    d.dmin = min(d.dmin, 1u); d.dmax = max(d.dmax, 1u);
+  }
+  if (RG == LARVA && code == DEC_STAYS) {
+    const uint32_t dd = age_days<!WIDE>(a.age);
+    d.l1 += age_days_uncapped<!WIDE>(a.age);
+    d.dmin = min(d.dmin, dd); d.dmax = max(d.dmax, dd);
+  }
+  return code;
+}
+
+// The count pass over slots [lo, hi) of range RG: each agent's decision into
+// its flags (bits 4-5), or into dec where the pool belongs to the caller, and
+// the survivors by next state into cs.
+template <int I, bool WIDE, int RG>
+__device__ __forceinline__ void count_range(const WarpRep& w, const KillConst& kc, uint8_t* ring, uint32_t lo, uint32_t hi, uint4& cs,
+                                            WarpSum& sum) {
+  constexpr uint32_t COLS = decide_cols(RG, WIDE);
+  using RING = Ring<COLS, 1, I>;
+  const uint32_t lane = threadIdx.x & 31u;
+  const DevPool src = w.src;
+  uint8_t* const dec = WIDE ? w.dec : nullptr;
+  const StepCtx& c = w.c;
+  DecideAcc da;
+  clear_acc(da);
+  uint32_t ns_stay = 0, ns_move = 0;
+  stream_range<RING, COLS>(ring, src, src.flags, nullptr, lo, hi, [&](const uint8_t* st, uint32_t g0) {
+#pragma unroll kRowUnroll
+    for (uint32_t k = 0; k < RING::kSlots / 32; k++) {
+      const uint32_t i = 32u * k + lane, g = g0 + i;
+      uint32_t code = DEC_DIES;
+      if (g >= lo && g < hi) {
+        Rec a;
+        read_chunk<RING, COLS>(st, i, a);
+        const uint32_t fl = st[RING::kByteOffset + i];
+        implied_fields<RG, WIDE>(a);
+        a.female = (fl >> 3) & 1u;
+        code = decide<RG, WIDE>(c, kc, g, a, da);
+        if (WIDE && dec) put(dec + g, code);
+        else put(src.flags + g, (fl & 15u) | (code << 4));
+      }
+      ns_stay += __popc(__ballot_sync(0xffffffffu, code == DEC_STAYS));
+      ns_move += __popc(__ballot_sync(0xffffffffu, code == DEC_MOVES));
+    }
+  });
+  add_decided<RG, RG>(da, sum);
+  add_count<RG>(cs, ns_stay);
+  add_count<next_state(RG)>(cs, ns_move);
+}
+
+// Calls f<RG>(lo, hi) for the part of every range that lies in [u0, u1), in
+// slot order.
+template <int RG = 0, class F>
+__device__ __forceinline__ void for_ranges(const sampo_population& pop, uint32_t u0, uint32_t u1, F&& f) {
+  if constexpr (RG < NSTATE) {
+    const uint32_t lo = max(pop.r[RG].start, u0), hi = min(pop.r[RG].end, u1);
+    if (lo < hi) f.template operator()<RG>(lo, hi);
+    for_ranges<RG + 1>(pop, u0, u1, f);
   }
 }
 
-// The count pass. Its warps share no barrier once the tiles flow: each warp
-// takes the stages' tiles in turn (stage it & 1 for its it-th tile, behind
-// the stage's mbarrier), and the LAST warp to finish a tile does the tile's
-// bookkeeping while the others go on with the tile in the other stage: it
-// builds the tile's prefix table from the warps' chunk counts, adds the
-// tile's totals to the stage's counts, claims the next ticket and starts
-// that tile's copies into the stage it has just emptied. A warp's stall is
-// then the wait for a tile's data, never the wait for the slowest warp.
-template <int I>
-__global__ void __launch_bounds__(kBlock, 5) k_count(KParams p) {
-  SAMPO_TILE_CONSTANTS(I);
-  extern __shared__ __align__(128) uint8_t dsm[];
-  __shared__ CountStage s_cs[2];
+template <int I, bool WIDE>
+struct CountRanges {
+  const WarpRep& w;
+  const KillConst& kc;
+  uint8_t* ring;
+  uint4& cs;
+  WarpSum& sum;
+  template <int RG>
+  __device__ __forceinline__ void operator()(uint32_t lo, uint32_t hi) {
+    count_range<I, WIDE, RG>(w, kc, ring, lo, hi, cs, sum);
+  }
+};
+
+// The count pass: decisions, the survivors by next state of every span and
+// super, and (by the warp that finishes the replicate's last span) the
+// supers' prefixes and the replicate's totals. Spans are taken from the last
+// one down, so that the update/scatter pass starts on those this pass
+// touched last.
+template <int I, bool WIDE>
+__global__ void __launch_bounds__(kBlock, 4) k_count(KParams p) {
+  extern __shared__ __align__(16) uint8_t dsm[];  // the warps' rings, then the batch's unit prefix
+  uint32_t* s_pre = reinterpret_cast<uint32_t*>(dsm + kWarps * kRingBytes);
+  uint8_t* ring = dsm + (threadIdx.x >> 5) * kRingBytes;
+  __shared__ WarpRep s_wr[kWarps];
   __shared__ KillConst s_mc;
   __shared__ uint32_t s_w[33];
-  uint32_t* s_pre = reinterpret_cast<uint32_t*>(dsm + kCountSmem);
-  __shared__ __align__(8) uint64_t bars[2];
-  __shared__ uint32_t s_tnext;                // the next ticket, drawn one claim ahead
-  __shared__ uint2 s_ent[2][kChunks];         // per stage, per (round, warp): survivors by state, 8-bit fields (states 0-3 | 4-7)
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   load_model_const(&p.mc->kill, s_mc);
   plan_tickets(p.nrep, s_pre, s_w, [&](uint32_t r) -> uint32_t {
     const SimDev* sim = p.reps[r].sim;
-    return sim->active ? (sim->pop.r[GRAVID].end + kTile - 1) / kTile : 0u;
+    return sim->active ? span_count(sim->pop.r[GRAVID].end) : 0u;
   });
-  const uint32_t total = s_pre[p.nrep];
-  // a step with no more tiles than CTAs gives CTA b tile b (no CTA queues a
-  // second tile while others have none)
-  const bool one_each = total <= gridDim.x;
-
-  // the whole warp: add the stage's counts to their replicate's totals
-  auto flush_stage = [&](CountStage& cs) {
-    if (cs.crep != kNoRep && lane < 8 && cs.cnt[lane]) atomicAdd(&p.reps[cs.crep].sim->cnt[lane], cs.cnt[lane]);
-    __syncwarp();
-    if (lane < 8) cs.cnt[lane] = 0;
-    if (lane == 0) cs.crep = kNoRep;
-    __syncwarp();
-  };
-  // the whole warp: take the next ticket into stage sidx (emptied by every
-  // warp), describe its tile and start its copies. The description is
-  // written before the arrival on bars[sidx] that the waiting warps acquire.
-  // Tickets run from the last tile down: the scatter pass then starts on the
-  // tiles whose decision columns and prefix tables this pass touched last,
-  // while they are still in L2.
-  auto claim = [&](uint32_t sidx) {
-    CountStage& cs = s_cs[sidx];
-    uint32_t t = 0;
-    if (lane == 0) t = s_tnext;
-    t = __shfl_sync(0xffffffffu, t, 0);
-    const uint32_t tile = total - 1u - t;
-    const uint32_t r = t < total ? find_rep(s_pre, p.nrep, tile) : kNoRep;
-    const uint32_t cur = cs.rep;
-    __syncwarp();
-    if (cur != r) {  // uniform: the stage moves on to another replicate
-      flush_stage(cs);
-      if (r != kNoRep) {
-        const RepParams& rp = p.reps[r];
-        const SimDev* sim = rp.sim;
-        copy16(&cs.c, &sim->ctx, (int)sizeof(StepCtx), lane, 32);
-        if (lane == 0) {
-          cs.pop = sim->pop;
-          cs.end = cs.pop.r[GRAVID].end;
-          cs.src = rp.pool[sim->cur];
-          cs.tileAgg = rp.tileAgg;
-          cs.tilePre = rp.tilePre;
-          cs.larv = sim->ctx.env.larvacideValue > 0.0f;
-          cs.crep = r;
-        }
-      }
-      if (lane == 0) cs.rep = r;
-      __syncwarp();
-    }
-    if (lane == 0) {
-      cs.tick = t;
-      cs.left = kWarps;
-      if (t >= total) {
-        mbar_arrive(&bars[sidx]);  // no copy: the waiting warps see the end
-      } else {
-        cs.lt = tile - s_pre[r];
-        const uint32_t lo = cs.lt * kTile, n = min((uint32_t)kTile, cs.end - lo);
-        const int u = range_of(cs.pop, lo);
-        cs.urg = (u >= 0 && lo + n <= cs.pop.r[u].end) ? u : -1;
-        fence_proxy_async();  // the stage was last read through the generic proxy
-        issue_count_tile<I>(cs.src, dsm + sidx * kCountStage, &bars[sidx], cs.pop, lo, n, cs.larv != 0);
-        // the ticket of the claim after this one, drawn once the copies are
-        // on their way (its round trip stays off the stage's refill)
-        s_tnext = one_each ? 0xffffffffu : atomicAdd(&p.bat->ticket1, 1u);
-      }
-    }
-  };
-
-  if (tid == 0) {
-    mbar_init(&bars[0]);
-    mbar_init(&bars[1]);
-    fence_mbar_init();
-    s_tnext = one_each ? blockIdx.x : atomicAdd(&p.bat->ticket1, 1u);
-  }
-  if (tid < 2) {
-    s_cs[tid].rep = kNoRep;
-    s_cs[tid].crep = kNoRep;
-  }
-  if (tid < 16) s_cs[tid >> 3].cnt[tid & 7] = 0;
   __syncthreads();
-  if (warp == 0) {
-    claim(0);
-    claim(1);
-  }
-  __syncthreads();
-
-  Acc acc = {0, 0, 0, 0, 0, 0};
-  uint32_t devoob = 0, w_rep = kNoRep;
-  // the warp's own accumulators into replicate r's totals
-  auto flush_warp = [&](uint32_t r) {
-    const uint32_t ne = __reduce_add_sync(0xffffffffu, acc.newEggs);
-    if (lane == 0 && ne) atomicAdd(&p.reps[r].sim->newEggs, ne);
-    const uint32_t bad = __reduce_or_sync(0xffffffffu, (acc.bad ? SAMPO_DEV_ERR_LARVATABLE : 0u) | (devoob ? SAMPO_DEV_ERR_DEVRATES : 0u));
-    if (lane == 0 && bad) atomicOr(&p.reps[r].sim->error, bad);
-    acc.newEggs = 0; acc.bad = 0; devoob = 0;
-  };
-
-  uint32_t it = 0;
-  bool failed = false;
-  for (;; it++) {
-    const uint32_t sidx = it & 1u;
-    CountStage& cs = s_cs[sidx];
-    if (!__all_sync(0xffffffffu, mbar_wait(&bars[sidx], (it >> 1) & 1u))) {  // bounded; acquires the description
-      failed = true;
-      break;
-    }
-    const uint32_t t = cs.tick;
-    if (t >= total) break;
-    const uint32_t rep = cs.rep;
-    if (rep != w_rep) {
-      if (w_rep != kNoRep) flush_warp(w_rep);
-      w_rep = rep;
-    }
-    const uint8_t* st = dsm + sidx * kCountStage;
-    const uint32_t end = cs.end, lo = cs.lt * kTile;
-    uint2* ent = s_ent[sidx];
-    switch (cs.urg) {  // CTA-uniform: a tile inside one range runs that state's code only
-      case EGG: count_items<I, EGG>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-      case LARVA: count_items<I, LARVA>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-      case PUPA: count_items<I, PUPA>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-      case IMMATURE: count_items<I, IMMATURE>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-      case MATESEEKING: count_items<I, MATESEEKING>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-      case BMS: count_items<I, BMS>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-      case BMD: count_items<I, BMD>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-      case GRAVID: count_items<I, GRAVID>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-      default: count_items<I, -1>(cs, st, s_mc, lo, end, tid, ent, acc, devoob); break;
-    }
-    // this warp is done with the stage: the last warp out does the tile's bookkeeping
+  const uint32_t total = s_pre[p.nrep], stride = gridDim.x * kWarps;
+  WarpRep& w = s_wr[warp];
+  __shared__ WarpSum s_sum[kWarps];
+  WarpSum& sum = s_sum[warp];
+  if (lane == 0) clear_sum(sum);
+  uint32_t cur_rep = kNoRep, done = 0;
+  // the warp's counters into its replicate's totals; the warp that brings
+  // the last spans scans the supers
+  auto flush = [&]() {
+    if (cur_rep == kNoRep) return;
+    const RepParams& rp = p.reps[cur_rep];
+    SimDev* sim = rp.sim;
     uint32_t last = 0;
-    __syncwarp();
     if (lane == 0) {
-      __threadfence_block();  // this warp's entries and its reads of the stage come first
-      last = atomicSub(&cs.left, 1u) == 1u;
-      __threadfence_block();  // and the other warps' before the last warp's work
+      flush_sum(sum, sim, &sim->dec);
+      __threadfence();  // this warp's adds to the supers come before its arrival
+      last = atomicAdd(&sim->spans_done, done) + done == w.nspans;
+      __threadfence();
     }
-    if (!__shfl_sync(0xffffffffu, last, 0)) continue;
-    {
-      // the tile's prefix table: exclusive prefix of the 32 (round, warp)
-      // chunks, 16-bit packed, and the tile's totals (the update/scatter pass
-      // reads both; the totals also feed the look-back)
-      const uint2 e = lane < kChunks ? s_ent[sidx][lane] : make_uint2(0u, 0u);
-      uint32_t w[5], x[5];
-      w[0] = (e.x & 0xffu) | ((e.x & 0xff00u) << 8);
-      w[1] = ((e.x >> 16) & 0xffu) | ((e.x >> 8) & 0xff0000u);
-      w[2] = (e.y & 0xffu) | ((e.y & 0xff00u) << 8);
-      w[3] = ((e.y >> 16) & 0xffu) | ((e.y >> 8) & 0xff0000u);
-      w[4] = ((e.x * 0x01010101u) >> 24) + ((e.y * 0x01010101u) >> 24);  // byte sums <= 32 cannot carry
-#pragma unroll
-      for (int q = 0; q < 5; q++) x[q] = w[q];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-        for (int q = 0; q < 5; q++) {
-          const uint32_t y = __shfl_up_sync(0xffffffffu, x[q], o);
-          if (lane >= o) x[q] += y;
-        }
+    last = __shfl_sync(0xffffffffu, last, 0);
+    __syncwarp();
+    if (last) {
+      scan_supers_warp(rp, w.nspans, sim->cnt);
+      if (lane == 0) {
+        sim->spans_done = 0;
+        sim->dirty[sim->rot] = max(sim->dirty[sim->rot], w.nspans);
       }
-      uint32_t* pre = cs.tilePre + (size_t)cs.lt * kPreWords;
-      if (lane < kChunks) {
-#pragma unroll
-        for (int q = 0; q < 5; q++) pre[lane * kPreEntryWords + q] = x[q] - w[q];
-      }
-      if (lane == kChunks - 1) {
-#pragma unroll
-        for (int q = 0; q < 5; q++) pre[kChunks * kPreEntryWords + q] = x[q];
-      }
-      uint32_t tw = 0;  // lanes 0..7: the tile's survivors of next state `lane`
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint32_t tq = __shfl_sync(0xffffffffu, x[q], kChunks - 1);
-        if ((lane >> 1) == q) tw = (tq >> (16 * (lane & 1))) & 0xffffu;
-      }
-      if (lane < 8) {
-        cs.tileAgg[(size_t)cs.lt * 8 + lane] = tw;
-        cs.cnt[lane] += tw;
-      }
-      __syncwarp();
     }
-    claim(sidx);  // the next tile into the stage this tile emptied
+    done = 0;
+  };
+  for (uint32_t u = blockIdx.x * kWarps + warp; u < total; u += stride) {
+    const uint32_t t = total - 1u - u;
+    const uint32_t r = find_rep(s_pre, p.nrep, t);
+    if (r != cur_rep) {  // uniform
+      flush();
+      load_warp_rep<false, false>(p.reps[r], w);
+      cur_rep = r;
+    }
+    const uint32_t sp = t - s_pre[r], end = w.pop.r[GRAVID].end, u0 = sp << w.shift;
+    const uint32_t u1 = end - u0 > (1u << w.shift) ? u0 + (1u << w.shift) : end;
+    uint4 cs = make_uint4(0u, 0u, 0u, 0u);
+    for_ranges(w.pop, u0, u1, CountRanges<I, WIDE>{w, s_mc, ring, cs, sum});
+    if (lane == 0) {
+      w.spans[sp] = cs;
+      add_super(w.supers + (sp >> 5), cs);
+    }
+    done++;
   }
-  // (each stage's counts were added to their totals by the claim that found
-  // no more tickets for it: the claims alternate stages in iteration order)
-  if (w_rep != kNoRep) flush_warp(w_rep);
-  if (failed && lane == 0) {
-    const uint32_t r = s_cs[it & 1u].rep;
-    atomicOr(&p.reps[r != kNoRep ? r : 0u].sim->error, SAMPO_DEV_ERR_TMA);
-    // let copies still in flight land before the warp exits (bounded waits)
-    (void)mbar_wait(&bars[it & 1u], (it >> 1) & 1u);
-    (void)mbar_wait(&bars[(it + 1) & 1u], ((it + 1) >> 1) & 1u);
-  }
+  flush();
 }
 
 // ------------------------------------------------------------------------
 // Publishing the start of a step
 // ------------------------------------------------------------------------
-// warp 0 publishes; warps 1-4 fill the 100 entries of the larval table at once
-constexpr int kPublishThreads = 160;
-
-// A replicate's state read through L2 (ld.global.cg): in the one-launch step
-// other CTAs of the same kernel wrote it, and this SM's L1 may hold older
-// copies of the same lines.
-template <class T>
-__device__ __forceinline__ T ld_l2(const T* p) {
-  static_assert(sizeof(T) % 4 == 0, "whole words");
-  T v;
-  uint32_t* d = reinterpret_cast<uint32_t*>(&v);
-  const uint32_t* q = reinterpret_cast<const uint32_t*>(p);
-#pragma unroll
-  for (int k = 0; k < (int)(sizeof(T) / 4); k++) d[k] = __ldcg(q + k);
-  return v;
-}
+// warp 0 publishes; the other warps fill the 100 entries of the larval table
+constexpr int kPublishThreads = 256;
+// Supers that warp 0 scans alone (four per lane), while the others fill the
+// table; more are scanned by the CTA first.
+constexpr uint32_t kScanByWarp = 128;
 
 // The larval hourly mortality of larvae d days old in a pool of L1de l1
-// (kernel/killAgents.cl:117-125); NaN outside the ages [dmin, dmax] present.
-__device__ __forceinline__ float larva_hmr_entry(uint32_t d, uint32_t dmin, uint32_t dmax, uint32_t l1, float cc) {
-  if (d < dmin || d > dmax) return SAMPO_NAN_F;
+// (kernel/killAgents.cl:117-125), as a kill_threshold; 0 outside the ages
+// [dmin, dmax] present.
+__device__ __forceinline__ uint32_t larva_kill_entry(uint32_t d, uint32_t dmin, uint32_t dmax, uint32_t l1, float cc) {
+  if (d < dmin || d > dmax) return 0u;
   float dmr = 0.1f * sampo_expf((float)l1 / ((float)d * cc * 1.0f));
   dmr = sampo_fminf(dmr, 0.8f);
   const float dsr = 1.0f - dmr;
   const float hsr = sampo_powf(dsr, 1.0f / 24.0f);
-  return 1.0f - hsr;
+  return kill_threshold(1.0f - hsr);
 }
 
-// The publish of replicate r by the calling CTA (at least kPublishThreads
-// threads; all of them call it): after a step, the next layout from the
-// survivor counts (kernel/oldToNewAgents.cl:57-95); then the pool's L1de,
-// female and infective counts (calcStats, src/abms.c:230-310), the stats
-// row, the next step's constants and the larval hourly mortality for every
-// larva age present (kernel/killAgents.cl:117-133 depends on the age and
-// L1de only). Reads and clears the acc_* accumulators. Mode PUB_REFRESH only
-// recomputes the input-dependent step constants (the inputs of the coming
-// step may have been written after its publish). When the next layout does
-// not fit the replicate's capacity (the scatter pass then flagged
-// SAMPO_DEV_ERR_CAPACITY and wrote nothing), the replicate pauses instead:
-// it becomes inactive at the same step with the same pool, constants and
-// larval table, and only the step's counters are cleared, so that the step
-// runs again, with the same result, once its pool has been moved into a
-// larger one (sampo_batch_grow). Returns the end of the replicate's pool
-// after the publish (0 when it is inactive) to every thread.
-__device__ uint32_t publish_rep(const KParams& p, uint32_t r, int mode) {
-  __shared__ uint32_t s_go, s_l1, s_dmin, s_dmax, s_end, s_pause;
-  __shared__ float s_cc;
+// A replicate whose decided step does not fit: inactive, the step's counters cleared.
+__device__ __forceinline__ void pause_rep(SimDev* sim) {
+#pragma unroll
+  for (int k = 0; k < 8; k++) sim->cnt[k] = 0;
+  sim->dec = Decided{0u, 0u, 0xffffffffu, 0u};
+  sim->ahead_dec = Decided{0u, 0u, 0xffffffffu, 0u};
+  sim->acc_fem = 0; sim->acc_inf = 0;
+  sim->acc_bnc[0] = sim->acc_bnc[1] = sim->acc_bnc[2] = sim->acc_bnc[3] = 0;
+  sim->ahead = 0;
+  sim->active = 0;
+}
+
+// The publish of replicate r by the calling CTA (kPublishThreads threads; all
+// of them call it). Step s is the one the replicate is at.
+//  PUB_AFTER_STEP  ends step s: the next layout from its survivor counts
+//    (kernel/oldToNewAgents.cl:57-95), the pool's L1de, female and infective
+//    counts (calcStats, src/abms.c:230-310) and the stats row of s + 1. When
+//    the pass decided s + 1 as well, the counts of s + 1 are scanned and
+//    become the decided ones.
+//  PUB_DECIDED     follows the count pass of step s.
+//  PUB_INITIAL     the statistics and row of a pool put in place by the host.
+//  PUB_REFRESH     recomputes the input-dependent constants of step s only
+//    (its inputs may have been written after its publish).
+// Every mode prepares the constants and the larval mortality table
+// (kernel/killAgents.cl:117-133 depends on the age and L1de only) of the next
+// step somebody decides: the coming step, or with PUB_AHEAD, for a replicate
+// that does not stop there, the one after, whose pool's size and L1de the
+// decisions already give.
+// When the decided step's layout does not fit the replicate's capacity, the
+// replicate pauses: it becomes inactive at that step with its pool, constants
+// and larval table as they are, and only the step's counters are cleared, so
+// that the step runs again, with the same result, once its pool has been
+// moved into a larger one (sampo_batch_grow).
+__device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
+  __shared__ uint32_t s_cnt[8], s_part[32][8], s_pause;
+  const int mode = mode_bits & PUB_MODE;
   const RepParams& rp = p.reps[r];
   SimDev* sim = rp.sim;
-  if (threadIdx.x < 32) {
-    // a device seed stream draws the coming step's seeds once, before thread 0 reads them
-    const uint32_t coming = __ldcg(&sim->step) + (mode == PUB_AFTER_STEP ? 1u : 0u);
-    if (__ldcg(&sim->active) && __ldcg(&sim->rnd.next) == coming && coming < __ldcg(&sim->stop_step))
-      draw_step_seeds(rp, coming);
+  const uint32_t tid = threadIdx.x;
+  if (!sim->active) return;
+  const uint32_t s = sim->step, stop = sim->stop_step;
+  const bool after = mode == PUB_AFTER_STEP;
+  const bool decided = mode == PUB_DECIDED || (after && sim->ahead);  // step sd's decisions are there
+  const uint32_t sd = after ? s + 1u : s;                              // the step the replicate is at after this publish
+  const bool ahead = decided && (mode_bits & PUB_AHEAD) && sd + 1u < stop;
+  const bool prepare = !decided || ahead;      // constants and table of step x
+  const uint32_t x = decided ? sd + 1u : sd;
+  if (tid < 32 && prepare) {
+    // a device seed stream draws a step's seeds once, before thread 0 reads them
+    if (sim->rnd.next == x && x < stop) draw_step_seeds(rp, x);
     __syncwarp();
   }
   if (mode == PUB_REFRESH) {
-    if (threadIdx.x == 0 && sim->active) {
+    if (tid == 0) {
       CtxInputs in;
-      load_ctx_inputs(rp, sim->step, in);
+      load_ctx_inputs(rp, s, in);
       StepCtx c;
-      make_ctx(in, sim->larvaHMR, sim->pop, c);
-      sim->ctx = c;
+      make_ctx(in, sim->larvaKill[s & 1u], sim->pop, c);
+      sim->ctx[s & 1u] = c;
     }
-    return 0u;
+    return;
   }
-  const bool after_step = mode == PUB_AFTER_STEP;
+  // the decisions whose totals describe the larvae of pool x, and the supers to scan
+  const Decided* from = after && decided ? &sim->ahead_dec : &sim->dec;
+  const uint32_t l1 = from->L1de, dmin = from->dmin, dmax = from->dmax;
+  const float cc = sim->cc;
   // Thread 0 reads all it needs before its first store (a store that may
   // alias a later load would hold that load back until the store is issued,
-  // turning the reads into a chain), hands the larval table's inputs to the
-  // other warps and does its writes while they fill the table.
-  sampo_population np;
+  // turning the reads into a chain).
+  sampo_population np;   // the pool of step sd
   sampo_bites_cycles bnc;
+  Decided dec;           // of the step that ends (after), then of step sd
   CtxInputs in;
-  uint32_t step = 0, stop = 0, epoch = 0, cur = 0, warn = 0;
-  bool relayout = false, shared_end_warn = false, pause = false;
-  if (threadIdx.x == 0) {
-    const uint32_t active = __ldcg(&sim->active);
-    np = ld_l2(&sim->pop);
-    bnc = ld_l2(&sim->bnc);
-    uint32_t cnt[8], abnc[4];
+  uint32_t cnt[8], cur = 0, rot = 0, warn = 0, capacity = 0, nspans = 0, dirty = 0;
+  bool shared_end_warn = false, pause = false;
+  if (tid == 0) {
+    np = sim->pop;
+    bnc = sim->bnc;
+    dec = sim->dec;
 #pragma unroll
-    for (int k = 0; k < 8; k++) cnt[k] = __ldcg(&sim->cnt[k]);
+    for (int k = 0; k < 8; k++) cnt[k] = sim->cnt[k];
+    capacity = sim->capacity;
+    cur = sim->cur;
+    rot = sim->rot;
+    warn = sim->warn;
+    const uint32_t fem = sim->acc_fem, inf = sim->acc_inf;
+    uint32_t abnc[4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) abnc[q] = __ldcg(&sim->acc_bnc[q]);
-    const uint32_t ne = __ldcg(&sim->newEggs), capacity = __ldcg(&sim->capacity);
-    const uint32_t aL1 = __ldcg(&sim->acc_L1de), afem = __ldcg(&sim->acc_fem), ainf = __ldcg(&sim->acc_inf);
-    const uint32_t dmin = __ldcg(&sim->acc_dmin), dmax = __ldcg(&sim->acc_dmax);
-    const float cc = __ldcg(&sim->cc);
-    step = __ldcg(&sim->step);
-    stop = __ldcg(&sim->stop_step);
-    epoch = __ldcg(&sim->epoch);
-    cur = __ldcg(&sim->cur);
-    warn = __ldcg(&sim->warn);
-    if (after_step) {
+    for (int q = 0; q < 4; q++) abnc[q] = sim->acc_bnc[q];
+    if (prepare) load_ctx_inputs(rp, x, in);
+    if (after) {
       // the reference's shared empty initial ranges (src/abms.c:204-219) make
       // oldToNewAgents read one prefix-sum entry for several range ends
       bool shared_end = false;
@@ -744,580 +923,452 @@ __device__ uint32_t publish_rep(const KParams& p, uint32_t r, int mode) {
         moved += cnt[k];
       }
       shared_end_warn = shared_end && moved;
-      if (layout_fits(cnt, ne, capacity)) {
+      pause = !layout_fits(cnt, dec.newEggs, capacity);  // the scatter pass flagged the capacity error and wrote nothing
+      if (!pause) {
+        nspans = span_count(np.r[GRAVID].end);  // (of the pool that the step left)
         uint32_t base[8];
-        next_layout(cnt, ne, np, base);
-        relayout = true;
-      } else {
-        pause = true;  // the scatter pass flagged the capacity error and wrote nothing
+        next_layout(cnt, dec.newEggs, np, base);
       }
-      step += 1u;
       bnc.numCyclesReported = abnc[0];
       bnc.sumCyclesReported = abnc[1];
       bnc.numBitesReported = abnc[2];
       bnc.numInfectBitesReported = abnc[3];
     }
-    np.numLarvae1DayEquiv = (np.r[LARVA].end > np.r[LARVA].start) ? aL1 : 0u;  // kernel/calcL1de.cl:259-280
-    np.numFemale = afem;
-    np.numPotentiallyInfective = ainf;
-    if (active) load_ctx_inputs(rp, step, in);
-    s_go = active;
+    if (mode != PUB_DECIDED) {
+      np.numLarvae1DayEquiv = (np.r[LARVA].end > np.r[LARVA].start) ? dec.L1de : 0u;  // kernel/calcL1de.cl:259-280
+      np.numFemale = fem;
+      np.numPotentiallyInfective = inf;
+    }
+    if (after && decided) {
+      const uint32_t units = nspans + dec.newEggs;  // (the pass cleared the oldest span counts if it had any unit)
+      dirty = units ? 0u : sim->dirty[rot == 0u ? 2u : rot - 1u];
+      s_part[0][0] = span_count(np.r[GRAVID].end);
+    }
     s_pause = pause;
-    s_end = active ? np.r[GRAVID].end : 0u;
-    s_l1 = np.numLarvae1DayEquiv;
-    s_dmin = dmin;
-    s_dmax = dmax;
-    s_cc = cc;
   }
   __syncthreads();
-  const uint32_t pool_end = s_end;
-  if (!s_go) return pool_end;
   if (s_pause) {
-    if (threadIdx.x == 0) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) sim->cnt[k] = 0;
-      sim->newEggs = 0;
-      sim->acc_L1de = 0; sim->acc_fem = 0; sim->acc_inf = 0;
-      sim->acc_dmin = 0xffffffffu; sim->acc_dmax = 0;
-      sim->acc_bnc[0] = sim->acc_bnc[1] = sim->acc_bnc[2] = sim->acc_bnc[3] = 0;
-      sim->active = 0;
+    if (tid == 0) {
+      pause_rep(sim);
     }
-    return 0u;
+    return;
   }
-  if (threadIdx.x == 0) {
-    if (shared_end_warn) sim->warn = warn | SAMPO_DEV_WARN_REF_LAYOUT;
-    if (after_step) {
-      if (relayout) sim->cur = cur ^ 1u;
-      sim->step = step;
-      sim->epoch = epoch + 1u;
-#pragma unroll
-      for (int k = 0; k < 8; k++) sim->cnt[k] = 0;
-      sim->newEggs = 0;
+  if (after && decided) {  // the counts of step sd, made while step s was applied
+    const uint32_t n = s_part[0][0];
+    __syncthreads();
+    if ((n + 31u) / 32u > kScanByWarp) scan_supers_block(rp, n, s_cnt, s_part);
+    else if (tid < 32) scan_supers_warp(rp, n, s_cnt);
+    __syncwarp();
+  }
+  if (tid == 0) {
+    if (after) {
+      if (shared_end_warn) sim->warn = warn | SAMPO_DEV_WARN_REF_LAYOUT;
+      sim->cur = cur ^ 1u;
+      sim->step = sd;
       sim->bnc = bnc;
+      if (sd >= stop) sim->active = 0;
     }
-    sim->pop = np;
-    sampo_stats_row row;
-    row.pop = np;
-    row.bnc = bnc;
-    rp.rows[step % rp.ring] = row;
-    sim->acc_L1de = 0; sim->acc_fem = 0; sim->acc_inf = 0;
-    sim->acc_dmin = 0xffffffffu; sim->acc_dmax = 0;
-    sim->acc_bnc[0] = sim->acc_bnc[1] = sim->acc_bnc[2] = sim->acc_bnc[3] = 0;
-    StepCtx c;
-    make_ctx(in, sim->larvaHMR, np, c);
-    sim->ctx = c;
-    if (step >= stop) sim->active = 0;
-  } else if (threadIdx.x >= 32) {
-    for (int d = threadIdx.x - 32; d < 100; d += blockDim.x - 32) {
-      sim->larvaHMR[d] = larva_hmr_entry((uint32_t)d, s_dmin, s_dmax, s_l1, s_cc);
+    if (mode != PUB_DECIDED) {
+      sim->pop = np;
+      sampo_stats_row row;
+      row.pop = np;
+      row.bnc = bnc;
+      rp.rows[sd % rp.ring] = row;
+      sim->acc_fem = 0; sim->acc_inf = 0;
+      sim->acc_bnc[0] = sim->acc_bnc[1] = sim->acc_bnc[2] = sim->acc_bnc[3] = 0;
     }
+    sampo_population px = np;  // the pool of step x
+    if (after && decided) {
+      const uint32_t old = rot == 0u ? 2u : rot - 1u, now = rot == 2u ? 0u : rot + 1u;
+      sim->rot = now;
+      sim->dirty[old] = dirty;
+      sim->dirty[now] = max(sim->dirty[now], span_count(np.r[GRAVID].end));
+      dec = sim->ahead_dec;
+      sim->dec = dec;
+#pragma unroll
+      for (int k = 0; k < 8; k++) sim->cnt[k] = cnt[k] = s_cnt[k];
+    } else if (mode != PUB_DECIDED) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) sim->cnt[k] = 0;
+      sim->dec = Decided{0u, 0u, 0xffffffffu, 0u};
+    }
+    if (after) sim->ahead_dec = Decided{0u, 0u, 0xffffffffu, 0u};
+    if (decided) {
+      if (!layout_fits(cnt, dec.newEggs, capacity)) {
+        atomicOr(&sim->error, SAMPO_DEV_ERR_CAPACITY);
+        pause_rep(sim);
+        pause = true;
+      } else if (ahead) {
+        uint32_t base[8];
+        next_layout(cnt, dec.newEggs, px, base);
+        px.numLarvae1DayEquiv = (px.r[LARVA].end > px.r[LARVA].start) ? dec.L1de : 0u;
+      }
+    }
+    sim->ahead = ahead && !pause ? 1u : 0u;
+    if (prepare && !pause) {
+      StepCtx c;
+      make_ctx(in, sim->larvaKill[x & 1u], px, c);
+      sim->ctx[x & 1u] = c;
+    }
+  } else if (tid >= 32 && prepare) {
+    // (a replicate that pauses keeps the table of its step: x is the step after)
+    for (uint32_t d = tid - 32; d < 100; d += blockDim.x - 32) sim->larvaKill[x & 1u][d] = larva_kill_entry(d, dmin, dmax, l1, cc);
   }
-  return pool_end;
 }
 
-// Publishing the start of a step for every replicate of p (one CTA each);
-// block 0 rearms the tickets.
-__global__ void __launch_bounds__(kPublishThreads) k_publish(KParams p, int mode) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    p.bat->ticket1 = 0u;
-    p.bat->ticket2 = 0u;
-  }
-  (void)publish_rep(p, blockIdx.x, mode);
-}
+// Publishing the start of a step for every replicate of p (one CTA each).
+__global__ void __launch_bounds__(kPublishThreads) k_publish(KParams p, int mode) { publish_rep(p, blockIdx.x, mode); }
 
 // ------------------------------------------------------------------------
 // Update + scatter pass
 // ------------------------------------------------------------------------
-template <int I>
-__device__ void issue_scatter_tile(const DevPool& src, const uint32_t* pre, uint8_t* st, uint64_t* bar, uint32_t lo, uint32_t n) {
-  SAMPO_TILE_CONSTANTS(I);
-  const uint32_t b4 = (n * 4 + 15) & ~15u, b1 = (n + 15) & ~15u;
-  mbar_arrive_tx(bar, 9 * b4 + b1 + kPreWords * 4);
-  bulk_load(st + kPreOff, pre, kPreWords * 4, bar);
-  bulk_load(st + 0 * kColBytes, src.age + lo, b4, bar);
-  bulk_load(st + 1 * kColBytes, src.his + lo, b4, bar);
-  bulk_load(st + 2 * kColBytes, src.delay + lo, b4, bar);
-  bulk_load(st + 3 * kColBytes, src.sporo + lo, b4, bar);
-  bulk_load(st + 4 * kColBytes, src.uni + lo, b4, bar);
-  bulk_load(st + 5 * kColBytes, src.avail + lo, b4, bar);
-  bulk_load(st + 6 * kColBytes, src.cycle + lo, b4, bar);
-  bulk_load(st + 7 * kColBytes, src.hbc + lo, b4, bar);
-  bulk_load(st + 8 * kColBytes, src.batches + lo, b4, bar);
-  bulk_load(st + 9 * kColBytes, src.flags + lo, b1, bar);
-}
+// A survivor that moves on out of a state whose transition draws a normal
+// number (include/gpuRand.h:56-63): its record is finished after the chunk,
+// densely over the lanes. Those of a chunk take consecutive slots. gid: its
+// slot in the current buffer (the generator's); kind: BM_* | isFemale << 2.
+struct MovedEntry { uint32_t gid, kind; };
+struct MovedExtra { float age; uint32_t avail, batches; };  // BMD only
+constexpr uint32_t kMovedExtra = 32;
 
-// Decoupled look-back for tile t of one replicate by one warp over the count
-// pass's tile aggregates: sums earlier tiles' aggregates back to the nearest
-// published inclusive prefix (no waiting). A published prefix is eight 64-bit
-// words, each holding a state's inclusive prefix and the step's epoch: every
-// word is written and read whole (single-copy atomic), so a reader validates
-// each by its epoch and no fence or flag is needed on either side. Lane 0
-// publishes t's words. Every lane returns the exclusive prefix ex[] and t's
-// counts cnt[].
-struct LookbackArrays {
-  uint32_t* agg;             // count pass tile aggregates
-  unsigned long long* incl;  // inclusive prefixes: value | epoch << 32
-};
-
-__device__ __forceinline__ void ld_relaxed_v2u64(const unsigned long long* p, unsigned long long& a, unsigned long long& b) {
-  asm volatile("ld.relaxed.gpu.global.v2.u64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-}
-__device__ __forceinline__ void st_relaxed_v2u64(unsigned long long* p, unsigned long long a, unsigned long long b) {
-  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1,%2};" ::"l"(p), "l"(a), "l"(b) : "memory");
-}
-
-__device__ void tile_lookback(const LookbackArrays& rp, uint32_t t, uint32_t epoch, int lane, uint32_t ex[8], uint32_t cnt[8]) {
-#pragma unroll
-  for (int b = 0; b < 8; b++) ex[b] = 0;
-  int64_t pos = (int64_t)t - 1;
-  while (pos >= 0) {
-    const int64_t idx = pos - lane;
-    const bool valid = idx >= 0;
-    uint32_t v[8];
-    bool pub = false;
-#pragma unroll
-    for (int b = 0; b < 8; b++) v[b] = 0;
-    if (valid) {
-      const uint4 a0 = ld_cg_v4(rp.agg + (size_t)idx * 8), a1 = ld_cg_v4(rp.agg + (size_t)idx * 8 + 4);
-      unsigned long long w[8];
-#pragma unroll
-      for (int q = 0; q < 4; q++) ld_relaxed_v2u64(rp.incl + (size_t)idx * 8 + 2 * q, w[2 * q], w[2 * q + 1]);
-      pub = true;
-#pragma unroll
-      for (int b = 0; b < 8; b++) pub = pub && (uint32_t)(w[b] >> 32) == epoch;
-      const uint32_t ag[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-#pragma unroll
-      for (int b = 0; b < 8; b++) v[b] = pub ? (uint32_t)w[b] : ag[b];
-    }
-    const uint32_t m = __ballot_sync(0xffffffffu, !valid || pub);
-    const int stop = m ? __ffs(m) - 1 : 32;
-    if (lane > stop) {  // beyond the nearest published tile (or the first tile)
-#pragma unroll
-      for (int b = 0; b < 8; b++) v[b] = 0;
-    }
-#pragma unroll
-    for (int b = 0; b < 8; b++) ex[b] += __reduce_add_sync(0xffffffffu, v[b]);
-    if (m) break;
-    pos -= 32;
+// Deciding ahead: the decisions about survivors that a warp has put into
+// consecutive slots of state ST, gathered per span of the next pool.
+struct Tally { uint32_t end, stay, move; };  // first slot past the span being counted; its counts so far
+template <int ST>
+__device__ __forceinline__ void flush_tally(const WarpRep& w, Tally& t) {
+  if ((t.stay | t.move) && (threadIdx.x & 31) == 0) {
+    const uint32_t span = (t.end - 1u) >> w.shift1;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    add_count<ST>(v, t.stay);
+    add_count<next_state(ST)>(v, t.move);
+    add_super(w.spans1 + span, v);
+    add_super(w.supers + (span >> 5), v);
   }
-  const uint32_t* ag = rp.agg + (size_t)t * 8;
-  const uint4 a0 = ld_cg_v4(ag), a1 = ld_cg_v4(ag + 4);
-  cnt[0] = a0.x; cnt[1] = a0.y; cnt[2] = a0.z; cnt[3] = a0.w; cnt[4] = a1.x; cnt[5] = a1.y; cnt[6] = a1.z; cnt[7] = a1.w;
-  if (lane == 0) {
-    const unsigned long long e = (unsigned long long)epoch << 32;
-    unsigned long long* q = rp.incl + (size_t)t * 8;
-#pragma unroll
-    for (int b = 0; b < 8; b += 2) st_relaxed_v2u64(q + b, e | (ex[b] + cnt[b]), e | (ex[b + 1] + cnt[b + 1]));
-  }
+  t.stay = t.move = 0;
 }
-
-
-constexpr int kScatterThreads = kBlock + 32;  // eight consumer warps and one producer warp
-static_assert(kChunks <= 32, "one (round, warp) chunk per lane");
-// resident CTAs per SM the registers of the update/scatter pass are sized for
-__host__ __device__ constexpr int scatter_min_blocks(int items) { return items >= 4 ? 2 : 3; }
-enum : uint32_t { TK_OLD = 0, TK_EGG = 1, TK_END = 2 };
-
-// What the producer warp hands the consumers with a tile. The replicate's
-// part (c .. base) is reloaded only when the slot changes replicate.
-struct alignas(16) ScatterStage {
-  StepCtx c;                 // the replicate's step constants
-  sampo_population pop;      // its current ranges
-  DevPool dst, src;          // its next and current buffers
-  LookbackArrays lb;         // its look-back arrays
-  const uint32_t* pre;       // its prefix tables
-  uint32_t rep, end, newEggs, nold, epoch;  // replicate, pool end, eggs laid, old tiles, look-back epoch
-  uint32_t base[8];          // first slot of each next-state range
-  uint32_t kind, lo;         // TK_*, first slot (old tile) or first egg id (egg tile)
-  int urg;                   // old tile: the range that holds every slot of the tile, or -1
-  uint32_t d0[8], cnt[8];    // per next state: the tile's first slot in it, survivors
-};
-constexpr int kAhead = 3;                 // the producer describes tiles this far ahead of the consumers
-constexpr int kDescSlots = kAhead + 1;    // tile descriptions in flight
-// Each pass of the loop issues tile seq + 2; with kAhead >= 3 it was described
-// by an earlier pass, with kAhead == 2 the pass describes it first.
-static_assert(kAhead >= 2 && kDescSlots <= 16, "issue() needs tile seq + 2 described; 2 kind bits per slot");
-
-// A survivor's owed normal draw (include/gpuRand.h:56-63): its slot in the
-// next buffer, its slot in the current one (the generator's gid), its
-// numEggBatches after the step, BM_*.
-struct BmEntry { uint32_t d, gid, batches, kind; };
-
-// Phase A of the update/scatter pass for one warp's items of an old tile in
-// stage memory st: the full update of each slot, and each survivor's slot in
-// the next buffer (dk; 0xffffffff for none): the tile's first slot of its
-// next state + the survivors of that state in earlier (round, warp) chunks
-// (the count pass's prefix table) + its rank within its chunk. nb gets the
-// next state (8: none) | female << 4 | owed draw << 5. RG >= 0: every slot
-// of the tile lies in range RG, so only that state's code is compiled in;
-// RG = -1: a tile that spans ranges.
-template <int I, int RG>
-__device__ __forceinline__ void scatter_phase_a(const ScatterStage& si, const uint8_t* st, const KillConst& kc, int tid,
-                                                Rec (&a)[I], uint32_t (&nb)[I], uint32_t (&dk)[I], Acc& acc,
-                                                uint32_t& tilebad) {
-  SAMPO_TILE_CONSTANTS(I);
-  const int warp = tid >> 5;
-  const float* c_age = (const float*)(st + 0 * kColBytes);
-  const float* c_his = (const float*)(st + 1 * kColBytes);
-  const float* c_delay = (const float*)(st + 2 * kColBytes);
-  const float* c_sporo = (const float*)(st + 3 * kColBytes);
-  const uint32_t* c_uni = (const uint32_t*)(st + 4 * kColBytes);
-  const uint32_t* c_avail = (const uint32_t*)(st + 5 * kColBytes);
-  const uint32_t* c_cycle = (const uint32_t*)(st + 6 * kColBytes);
-  const uint32_t* c_hbc = (const uint32_t*)(st + 7 * kColBytes);
-  const uint32_t* c_batches = (const uint32_t*)(st + 8 * kColBytes);
-  const uint8_t* c_flags = st + 9 * kColBytes;
-  const uint32_t* c_pre = (const uint32_t*)(st + kPreOff);
-  const StepCtx& c = si.c;
-  const uint32_t lo = si.lo, end = si.end;
-#pragma unroll
-  for (int k = 0; k < kItems; k++) {
-    const uint32_t i = k * kBlock + tid;
-    const uint32_t g = lo + i;
-    int rg;
-    bool valid;
-    if (RG >= 0) {
-      rg = RG;
-      valid = g < end;
+// The slots [first, first + n) of a row; ks, km: the lanes that hold one
+// whose agent stays / moves on; d: a lane's slot. A row fills at most two spans.
+template <int ST>
+__device__ __forceinline__ void add_tally(const WarpRep& w, Tally& t, uint32_t first, uint32_t n, uint32_t ks, uint32_t km, uint32_t d) {
+  if (first + n > t.end) {  // (and at the start, with t.end = 0)
+    const uint32_t in = __ballot_sync(0xffffffffu, d < t.end);  // (lanes that hold none are in neither mask)
+    t.stay += __popc(ks & in);
+    t.move += __popc(km & in);
+    flush_tally<ST>(w, t);
+    if (first >= t.end) {
+      t.end = ((first >> w.shift1) + 1u) << w.shift1;
+      if (first + n > t.end) {  // the first row of a run that starts near a span's end
+        const uint32_t in0 = __ballot_sync(0xffffffffu, d < t.end);
+        t.stay = __popc(ks & in0);
+        t.move = __popc(km & in0);
+        flush_tally<ST>(w, t);
+        ks &= ~in0;
+        km &= ~in0;
+        t.end += 1u << w.shift1;
+      }
     } else {
-      rg = g < end ? range_of(si.pop, g) : -1;
-      valid = rg >= 0;
+      ks &= ~in;
+      km &= ~in;
+      t.end += 1u << w.shift1;
     }
-    nb[k] = 8;
-    a[k].bm = BM_NONE;
-    a[k].female = 0u;
-    if (valid) {
-      a[k].age = c_age[i]; a[k].his = c_his[i]; a[k].delay = c_delay[i]; a[k].sporo = c_sporo[i];
-      a[k].uni = c_uni[i]; a[k].avail = c_avail[i]; a[k].cycle = c_cycle[i]; a[k].hbc = c_hbc[i];
-      a[k].batches = c_batches[i];
-      a[k].female = (c_flags[i] >> 3) & 1u;
-      const int ns = update_agent<true>(c, kc, rg, g, a[k], acc);
-      if (ns >= 0) nb[k] = ns;
-    }
-    const uint32_t peers = __match_any_sync(0xffffffffu, nb[k]);
-    const uint32_t rk = __popc(peers & lanemask_lt());
-    const uint32_t* e0 = c_pre + (k * kWarps + warp) * kPreEntryWords;  // this chunk's entry
-    const uint32_t* e1 = e0 + kPreEntryWords;                         // the next one
-    const int b = nb[k];
-    dk[k] = 0xffffffffu;
-    if (b < 8) {
-      const uint32_t sh = 16 * (b & 1);
-      const uint32_t j = ((e0[b >> 1] >> sh) & 0xffffu) + rk;
-      // the two passes disagree when a survivor falls outside its chunk's run
-      if (j < ((e1[b >> 1] >> sh) & 0xffffu)) dk[k] = si.d0[b] + j;
-      else tilebad = 1;
-    }
-    // ... or when the chunk's survivors are not the count pass's
-    const uint32_t ns = __popc(__ballot_sync(0xffffffffu, b < 8));
-    if (ns != e1[4] - e0[4]) tilebad = 1;
-    nb[k] = (uint32_t)b | (a[k].female << 4) | (a[k].bm << 5);
   }
+  t.stay += __popc(ks);
+  t.move += __popc(km);
 }
 
-// The producer warp describes tiles three ahead (ticket, replicate data,
-// look-back, layout) and hands each to the consumers in a free stage with
-// its TMA loads (full[s]: the expect-tx arrival + the arrival that publishes
-// the description). A stage carries the tile's columns and the count pass's
-// prefix table of its (round, warp) chunks, so every consumer warp knows
-// where its survivors go without the other warps: the consumer warps share
-// no barrier. Each releases a stage (empty[s], 256 arrivals) as soon as it
-// has read its inputs, then writes every survivor straight to its slot in the
-// next buffer: the survivors of one next state are contiguous within a warp,
-// so the stores coalesce.
-template <int I>
-__global__ void __launch_bounds__(kScatterThreads, scatter_min_blocks(I)) k_scatter(KParams p) {
-  SAMPO_TILE_CONSTANTS(I);
-  extern __shared__ __align__(128) uint8_t dsm[];
-  __shared__ ScatterStage s_si[kDescSlots];
+// The update/scatter pass over slots [lo, hi) of range RG. base (lanes 0-7):
+// the next slot of next state `lane` for this warp's survivors; advanced past
+// the range's. A survivor's slot is that plus its rank among the survivors
+// of its state in the row (two ballots: an agent stays or moves on to one
+// other state). The survivors of a state are consecutive, so the stores of a
+// row coalesce.
+// AHEAD: each survivor's decision of the step after is taken here as well,
+// while its record is in registers: its slot in the next pool, that step's
+// inputs and (from this step's decisions) that pool's L1de and size are all
+// known. The decisions go into the flags, their counts to the next pool's
+// spans and supers, and no count pass is needed before the next step.
+template <int I, bool WIDE, bool AHEAD, int RG>
+__device__ __forceinline__ void scatter_range(const WarpRep& w, const ModelConst& mc, uint8_t* ring, uint32_t lo, uint32_t hi,
+                                              uint32_t& base, MovedEntry* mq, MovedExtra* mx, WarpSum& sum) {
+  constexpr int NX = next_state(RG);
+  constexpr uint32_t CS = state_cols(RG, WIDE), CM = state_cols(NX, WIDE);
+  using RING = Ring<CS, WIDE ? 2 : 1, I>;
+#ifdef SAMPO_USER_SPECIES
+  constexpr uint32_t OWED = 0;  // the header's draws are made at the transition
+#else
+  constexpr uint32_t OWED = RG == EGG ? (uint32_t)C_DELAY : RG == BMD ? (uint32_t)C_AVAIL : 0u;
+#endif
+  static_assert(RG != BMD || RING::kSlots <= kMovedExtra, "the moved females of a chunk have room");
+  const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
+  const DevPool src = w.src, dst = w.dst;
+  const uint8_t* const dec = WIDE ? w.dec : nullptr;
+  const StepCtx &c = w.c, &c1 = w.c1;
+  const bool ahead = AHEAD && w.ahead;
+  Acc acc = {0, 0, 0, 0, 0, 0};
+  uint32_t fem = 0, inf = 0, bad = 0;
+  DecideAcc da;
+  clear_acc(da);
+  uint32_t bs = __shfl_sync(0xffffffffu, base, RG), bm = __shfl_sync(0xffffffffu, base, NX);
+  const uint32_t es = w.next.r[RG].end, em = w.next.r[NX].end;
+  Tally ts = {0, 0, 0}, tm = {0, 0, 0};
+  stream_range<RING, CS>(ring, src, src.flags, dec, lo, hi, [&](const uint8_t* st, uint32_t g0) {
+    uint32_t nq = 0;
+    const uint32_t bm0 = bm;
+#pragma unroll kRowUnroll
+    for (uint32_t k = 0; k < RING::kSlots / 32; k++) {
+      const uint32_t i = 32u * k + lane, g = g0 + i;
+      const uint32_t fl = st[RING::kByteOffset + i];
+      uint32_t code = WIDE && dec ? st[RING::kByteOffset + RING::kSlots + i] : (fl >> 4) & 3u;
+      if (g < lo || g >= hi) code = DEC_DIES;
+      uint32_t ms = __ballot_sync(0xffffffffu, code == DEC_STAYS), mm = __ballot_sync(0xffffffffu, code == DEC_MOVES);
+      uint32_t n = __popc(ms);
+      if (bs + n > es) {  // no store leaves the state's run
+        bad = SAMPO_DEV_ERR_TILECOUNT;
+        ms = n = 0;
+      }
+      {  // those that stay
+        const uint32_t d = bs + __popc(ms & lt);
+        uint32_t code1 = DEC_DIES;
+        if ((ms >> lane) & 1u) {
+          Rec a;
+          read_chunk<RING, CS>(st, i, a);
+          implied_fields<RG, WIDE>(a);
+          a.female = (fl >> 3) & 1u;
+          (void)update_agent<true, false, true, true, !WIDE>(c, mc.kill, RG, g, a, acc, DEC_STAYS);
+          store_cols<CS>(dst, d, a);
+          // statistics of the next pool (kernel/calcGender.cl:24-37)
+          if (RG >= IMMATURE && a.female) {
+            fem += 1u;
+            inf += a.sporo >= 1.0f ? 1u : 0u;
+          }
+          if (ahead) code1 = decide<RG, WIDE>(c1, mc.kill, d, a, da);
+          put(dst.flags + d, (fl & 15u) | (code1 << 4));
+        }
+        if (ahead) {
+          const uint32_t ks = __ballot_sync(0xffffffffu, code1 == DEC_STAYS), km = __ballot_sync(0xffffffffu, code1 == DEC_MOVES);
+          add_tally<RG>(w, ts, bs, n, ks, km, d);
+        }
+        bs += n;
+      }
+      if (mm) {  // those that move on
+        n = __popc(mm);
+        if (bm + n > em) {
+          bad = SAMPO_DEV_ERR_TILECOUNT;
+          mm = n = 0;
+        }
+        const uint32_t d = bm + __popc(mm & lt);
+        uint32_t code1 = DEC_DIES;
+        if ((mm >> lane) & 1u) {
+          Rec a;
+          read_chunk<RING, CS>(st, i, a);
+          implied_fields<RG, WIDE>(a);
+          a.female = (fl >> 3) & 1u;
+          (void)update_agent<true, false, true, true, !WIDE>(c, mc.kill, RG, g, a, acc, DEC_MOVES);
+          store_cols<(CM & ~OWED)>(dst, d, a);
+          if (RG >= PUPA && a.female) {
+            fem += 1u;
+            inf += a.sporo >= 1.0f ? 1u : 0u;
+          }
+          if (OWED) {
+            const uint32_t j = nq + __popc(mm & lt);
+            mq[j] = MovedEntry{g, a.bm | (a.female << 2)};
+            if (RG == BMD) mx[j] = MovedExtra{a.age, a.avail, a.batches};
+          } else {
+            if (ahead) code1 = decide<NX, WIDE>(c1, mc.kill, d, a, da);
+            put(dst.flags + d, (fl & 8u) | NX | (code1 << 4));
+          }
+        }
+        if (!OWED && ahead) {
+          const uint32_t ks = __ballot_sync(0xffffffffu, code1 == DEC_STAYS), km = __ballot_sync(0xffffffffu, code1 == DEC_MOVES);
+          add_tally<NX>(w, tm, bm, n, ks, km, d);
+        }
+        bm += n;
+        nq += n;
+      }
+      if (RG == GRAVID && code == DEC_TRAPPED) {  // her last hour counts (kernel/updateAgents.cl:247-255)
+        acc.cycles += 1u;
+        acc.sumCycles += reinterpret_cast<const uint32_t*>(st)[RING::offset(C_CYCLE) / 4 + i] + 1u;
+      }
+    }
+    if (OWED && nq) {  // the moved agents' owed draws, decisions and flags, dense over the lanes
+      __syncwarp();
+#pragma unroll 1
+      for (uint32_t j0 = 0; j0 < nq; j0 += 32u) {
+        const uint32_t j = j0 + lane, d = bm0 + j;
+        uint32_t code1 = DEC_DIES;
+        if (j < nq) {
+          const MovedEntry q = mq[j];
+          const uint32_t kind = q.kind & 3u, female = q.kind >> 2;
+          Rec b = Rec{};
+          if (RG == EGG) {
+            b.age = 24.0f;
+            b.delay = __uint_as_float(finish_box_muller(c, mc, q.gid, BM_LARVA_DELAY, 0u));
+            put(dst.delay + d, b.delay);
+          } else {
+            const MovedExtra x = mx[j];
+            b.age = x.age;
+            b.avail = kind != BM_NONE ? finish_box_muller(c, mc, q.gid, kind, x.batches) : x.avail;
+            put(dst.avail + d, b.avail);
+          }
+          b.female = female;
+          if (ahead) code1 = decide<NX, WIDE>(c1, mc.kill, d, b, da);
+          put(dst.flags + d, NX | (female << 3) | (code1 << 4));
+        }
+        if (ahead) {
+          const uint32_t ks = __ballot_sync(0xffffffffu, code1 == DEC_STAYS), km = __ballot_sync(0xffffffffu, code1 == DEC_MOVES);
+          add_tally<NX>(w, tm, bm0 + j0, min(nq - j0, 32u), ks, km, d);
+        }
+      }
+    }
+  });
+  if (ahead) {
+    flush_tally<RG>(w, ts);
+    flush_tally<NX>(w, tm);
+  }
+  if (AHEAD) add_decided<RG, NX>(da, sum);
+  if (RG >= PUPA) {
+    uint32_t v[6] = {fem, inf, acc.cycles, acc.sumCycles, acc.bites, acc.infectBites};
+#pragma unroll
+    for (int j = 0; j < 6; j++) v[j] = (j < 2 || RG >= BMS) ? __reduce_add_sync(0xffffffffu, v[j]) : 0u;
+    if (lane == 0) {
+      sum.fem += v[0];
+      sum.inf += v[1];
+#pragma unroll
+      for (int j = 0; j < 4; j++) sum.bnc[j] += v[2 + j];
+    }
+  }
+  if (bad && lane == 0) sum.error |= bad;
+  if (lane == (uint32_t)RG) base = bs;
+  if (lane == (uint32_t)NX) base = bm;
+}
+
+template <int I, bool WIDE, bool AHEAD>
+struct ScatterRanges {
+  const WarpRep& w;
+  const ModelConst& mc;
+  uint8_t* ring;
+  uint32_t& base;
+  MovedEntry* mq;
+  MovedExtra* mx;
+  WarpSum& sum;
+  template <int RG>
+  __device__ __forceinline__ void operator()(uint32_t lo, uint32_t hi) {
+    scatter_range<I, WIDE, AHEAD, RG>(w, mc, ring, lo, hi, base, mq, mx, sum);
+  }
+};
+
+// The update/scatter pass: units 0 .. nspans-1 of a replicate are its spans,
+// the rest its new eggs. A span's first slot in every next-state range comes
+// from the decisions' counts: its super's prefix plus the spans before it in
+// the super (one 16-byte word per lane). No warp waits for another.
+template <int I, bool WIDE, bool AHEAD>
+__global__ void __launch_bounds__(kBlock, 3) k_scatter(KParams p) {
+  extern __shared__ __align__(16) uint8_t dsm[];  // the warps' rings, then the batch's unit prefix
+  uint32_t* s_pre = reinterpret_cast<uint32_t*>(dsm + kWarps * kRingBytes);
+  uint8_t* ring = dsm + (threadIdx.x >> 5) * kRingBytes;
+  __shared__ WarpRep s_wr[kWarps];
   __shared__ ModelConst s_mc;
   __shared__ uint32_t s_w[33];
-  uint32_t* s_pre = reinterpret_cast<uint32_t*>(dsm + kScatterSmem);
-  __shared__ __align__(8) uint64_t full[2], empty[2];
-  __shared__ BmEntry s_bmq[kWarps][kItems * 32];    // per warp: owed draws of the tile
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  __shared__ MovedEntry s_mq[kWarps][I * 32];
+  __shared__ MovedExtra s_mx[kWarps][kMovedExtra];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   load_model_const(p.mc, s_mc);
   plan_tickets(p.nrep, s_pre, s_w, [&](uint32_t r) -> uint32_t {
     SimDev* sim = p.reps[r].sim;
     if (!sim->active) return 0u;
     uint32_t cnt[8];
     for (int k = 0; k < 8; k++) cnt[k] = sim->cnt[k];
-    const uint32_t ne = sim->newEggs;
+    const uint32_t ne = sim->dec.newEggs;
     if (!layout_fits(cnt, ne, sim->capacity)) {
       if (blockIdx.x == 0) atomicOr(&sim->error, SAMPO_DEV_ERR_CAPACITY);
       return 0u;
     }
-    return (sim->pop.r[GRAVID].end + kTile - 1) / kTile + (ne + kTile - 1) / kTile;
+    const uint32_t end = sim->pop.r[GRAVID].end;
+    return span_count(end) + units_of(ne, span_shift(end));
   });
-  const uint32_t total = s_pre[p.nrep];
-  if (tid == 0) {
-    mbar_init_count(&full[0], 2);
-    mbar_init_count(&full[1], 2);
-    mbar_init_count(&empty[0], kBlock);
-    mbar_init_count(&empty[1], kBlock);
-    fence_mbar_init();
-    for (int k = 0; k < kDescSlots; k++) s_si[k].rep = 0xffffffffu;
-  }
   __syncthreads();
-
-  uint32_t fail = 0, fail_rep = 0;
-  if (warp == kWarps) {
-    // ================= producer warp =================
-    // describe tile `seq` (slot seq % kDescSlots): take a ticket, load the
-    // replicate's data when the slot changes replicate, run the look-back,
-    // lay out the tile's runs. Touches no stage.
-    // lane 0 draws each ticket one description ahead, so the atomic's round
-    // trip overlaps a tile; a step with no more tiles than CTAs gives CTA b
-    // tile b (no CTA queues several tiles while others have none)
-    const bool one_each = total <= gridDim.x;
-    uint32_t t_next = 0;
-    if (lane == 0) t_next = one_each ? blockIdx.x : atomicAdd(&p.bat->ticket2, 1u);
-    auto describe = [&](uint32_t seq) -> uint32_t {
-      uint32_t t = 0;
-      if (lane == 0) {
-        t = t_next;
-        t_next = one_each ? 0xffffffffu : atomicAdd(&p.bat->ticket2, 1u);
-      }
-      t = __shfl_sync(0xffffffffu, t, 0);
-      ScatterStage& si = s_si[seq % kDescSlots];
-      if (t >= total) {
-        if (lane == 0) si.kind = TK_END;
-        __syncwarp();
-        return TK_END;
-      }
-      const uint32_t r = find_rep(s_pre, p.nrep, t);
-      const uint32_t j = t - s_pre[r];
-      if (si.rep != r) {  // uniform: the slot's replicate data, once per replicate
-        const RepParams& rp = p.reps[r];
-        SimDev* sim = rp.sim;
-        copy16(&si.c, &sim->ctx, (int)sizeof(StepCtx), lane, 32);
-        if (lane == 0) {
-          const uint32_t cur = sim->cur, ne = sim->newEggs;
-          si.pop = sim->pop;
-          si.end = si.pop.r[GRAVID].end;
-          si.nold = (si.end + kTile - 1) / kTile;
-          si.newEggs = ne;
-          si.epoch = sim->epoch;
-          si.src = rp.pool[cur];
-          si.dst = rp.pool[cur ^ 1u];
-          si.lb.agg = rp.tileAgg;
-          si.lb.incl = rp.tileIncl;
-          si.pre = rp.tilePre;
-          uint32_t tc[8], base[8];
-          for (int k = 0; k < 8; k++) tc[k] = sim->cnt[k];
-          sampo_population np;
-          next_layout(tc, ne, np, base);
-          for (int k = 0; k < 8; k++) si.base[k] = base[k];
-        }
-        __syncwarp();
-        if (lane == 0) si.rep = r;
-        __syncwarp();
-      }
-      if (j < si.nold) {
-        uint32_t ex[8], cnt[8];
-        tile_lookback(si.lb, j, si.epoch, lane, ex, cnt);
-        if (lane == 0) {
-#pragma unroll
-          for (int b = 0; b < 8; b++) {
-            si.d0[b] = si.base[b] + ex[b];
-            si.cnt[b] = cnt[b];
-          }
-          si.kind = TK_OLD;
-          si.lo = j * kTile;
-          const uint32_t n = min((uint32_t)kTile, si.end - si.lo);
-          const int u = range_of(si.pop, si.lo);
-          si.urg = (u >= 0 && si.lo + n <= si.pop.r[u].end) ? u : -1;
-        }
-        __syncwarp();
-        return TK_OLD;
-      }
-      if (lane == 0) {
-        si.kind = TK_EGG;
-        si.lo = (j - si.nold) * kTile;
-      }
-      __syncwarp();
-      return TK_EGG;
-    };
-    // hand tile `seq` to the consumers in stage seq & 1 (free): its loads
-    // (expect-tx arrival) and the arrival that publishes its description
-    auto issue = [&](uint32_t seq) {
-      const uint32_t s = seq & 1u;
-      const ScatterStage& si = s_si[seq % kDescSlots];
-      if (lane == 0) {
-        if (si.kind == TK_OLD) {
-          fence_proxy_async();  // the stage was last read through the generic proxy
-          issue_scatter_tile<I>(si.src, si.pre + (size_t)(si.lo / kTile) * kPreWords, dsm + s * kScatterStage, &full[s], si.lo,
-                             min((uint32_t)kTile, si.end - si.lo));
-        } else {
-          mbar_arrive(&full[s]);
-        }
-        mbar_arrive(&full[s]);  // description written (release)
-      }
-    };
-    uint32_t kinds = 0, ph = 0;  // 2 bits per described tile, slot seq % kDescSlots
-    auto kind_of = [&](uint32_t seq) { return (kinds >> (2 * (seq % kDescSlots))) & 3u; };
-    auto set_kind = [&](uint32_t seq, uint32_t k) {
-      const uint32_t sh = 2 * (seq % kDescSlots);
-      kinds = (kinds & ~(3u << sh)) | (k << sh);
-    };
-    set_kind(0, describe(0));
-    issue(0);
-    set_kind(1, describe(1));
-    issue(1);
-    for (uint32_t seq = 2; seq < (uint32_t)kAhead; seq++) set_kind(seq, describe(seq));
-    for (uint32_t seq = 0;; seq++) {
-      const uint32_t s = seq & 1u;
-      if (kind_of(seq) == TK_END) break;
-      uint32_t ok = 1;
-      if (lane == 0) ok = mbar_wait(&empty[s], (ph >> s) & 1u) ? 1u : 0u;  // tile seq's inputs are read
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (!ok) { fail = 1; fail_rep = s_si[seq % kDescSlots].rep; break; }
-      ph ^= 1u << s;
-      // slot (seq + kAhead) % kDescSlots held tile seq - 1, whose consumers
-      // are done: they released tile seq's inputs after finishing it
-      if (kAhead == 2) {
-        set_kind(seq + 2, describe(seq + 2));
-        issue(seq + 2);
-      } else {
-        issue(seq + 2);
-        set_kind(seq + kAhead, describe(seq + kAhead));
-      }
+  const uint32_t total = s_pre[p.nrep], stride = gridDim.x * kWarps;
+  WarpRep& w = s_wr[warp];
+  MovedEntry* mq = s_mq[warp];
+  MovedExtra* mx = s_mx[warp];
+  uint32_t cur_rep = kNoRep;
+  __shared__ WarpSum s_sum[kWarps];
+  WarpSum& sum = s_sum[warp];
+  if (lane == 0) clear_sum(sum);
+  // this warp's sums into its replicate's
+  auto flush = [&]() {
+    if (cur_rep != kNoRep && lane == 0) {
+      SimDev* sim = p.reps[cur_rep].sim;
+      flush_sum(sum, sim, &sim->ahead_dec);
     }
-  } else {
-    // ================= consumer warps =================
-    const ModelConst& mc = s_mc;
-    Acc acc = {0, 0, 0, 0, 0, 0};
-    uint32_t l1 = 0, fem = 0, inf = 0, dmin = 0xffffffffu, dmax = 0, tilebad = 0;
-    uint32_t cur_rep = 0xffffffffu;
-    // this warp's statistics of replicate r into its totals
-    auto flush = [&](uint32_t r) {
-      SimDev* sim = p.reps[r].sim;
-      uint32_t v[8] = {l1, fem, inf, acc.cycles, acc.sumCycles, acc.bites, acc.infectBites,
-                       (acc.bad ? SAMPO_DEV_ERR_LARVATABLE : 0u) | (tilebad ? SAMPO_DEV_ERR_TILECOUNT : 0u)};
-#pragma unroll
-      for (int j = 0; j < 8; j++) v[j] = j == 7 ? __reduce_or_sync(0xffffffffu, v[j]) : __reduce_add_sync(0xffffffffu, v[j]);
-      const uint32_t mn = __reduce_min_sync(0xffffffffu, dmin), mx = __reduce_max_sync(0xffffffffu, dmax);
-      if (lane == 0) {
-        if (v[0]) atomicAdd(&sim->acc_L1de, v[0]);
-        if (v[1]) atomicAdd(&sim->acc_fem, v[1]);
-        if (v[2]) atomicAdd(&sim->acc_inf, v[2]);
-        if (v[3]) atomicAdd(&sim->acc_bnc[0], v[3]);
-        if (v[4]) atomicAdd(&sim->acc_bnc[1], v[4]);
-        if (v[5]) atomicAdd(&sim->acc_bnc[2], v[5]);
-        if (v[6]) atomicAdd(&sim->acc_bnc[3], v[6]);
-        if (v[7]) atomicOr(&sim->error, v[7]);
-        if (mn != 0xffffffffu) { atomicMin(&sim->acc_dmin, mn); atomicMax(&sim->acc_dmax, mx); }
-      }
-      acc = Acc{0, 0, 0, 0, 0, 0};
-      l1 = fem = inf = dmax = tilebad = 0;
-      dmin = 0xffffffffu;
-    };
-    uint32_t ph = 0;
-    for (uint32_t it = 0;; it++) {
-      const uint32_t s = it & 1u;
-      const uint8_t* st = dsm + s * kScatterStage;
-      const bool ok = __all_sync(0xffffffffu, mbar_wait(&full[s], (ph >> s) & 1u));  // bounded; acquires the stage
-      if (ok) ph ^= 1u << s;  // else the phase is still owed: the exit path waits for it again
-      const ScatterStage& si = s_si[it % kDescSlots];
-      const uint32_t kind = ok ? si.kind : TK_END;
-      if (kind != TK_END && si.rep != cur_rep) {
-        if (cur_rep != 0xffffffffu) flush(cur_rep);
-        cur_rep = si.rep;
-      }
-      // ---- phase A (old tiles): recompute the step for the tile's agents and
-      //      find each survivor's slot: the tile's first slot of its next
-      //      state + the survivors of that state in earlier (round, warp)
-      //      chunks (prefix table) + its rank within its chunk ----
-      Rec a[kItems];
-      uint32_t nb[kItems];  // after phase A: next state (8: none) | female << 4 | owed draw << 5
-      uint32_t dk[kItems];
-      if (kind == TK_OLD) {
-        switch (si.urg) {  // CTA-uniform: a tile inside one range runs that state's code only
-          case EGG: scatter_phase_a<I, EGG>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-          case LARVA: scatter_phase_a<I, LARVA>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-          case PUPA: scatter_phase_a<I, PUPA>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-          case IMMATURE: scatter_phase_a<I, IMMATURE>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-          case MATESEEKING: scatter_phase_a<I, MATESEEKING>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-          case BMS: scatter_phase_a<I, BMS>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-          case BMD: scatter_phase_a<I, BMD>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-          case GRAVID: scatter_phase_a<I, GRAVID>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-          default: scatter_phase_a<I, -1>(si, st, mc.kill, tid, a, nb, dk, acc, tilebad); break;
-        }
-      }
-      if (kind != TK_END) mbar_arrive(&empty[s]);  // this thread is done with the stage's inputs
-      if (!ok) { fail = 1; fail_rep = cur_rep == 0xffffffffu ? 0u : cur_rep; break; }
-      if (kind == TK_END) break;
-      const StepCtx& c = si.c;
-      const DevPool& dst = si.dst;
-      if (kind == TK_OLD) {
-        BmEntry* bmq = s_bmq[warp];
-        uint32_t nq = 0;
-        // ---- phase B: every survivor to its slot in the next buffer ----
-#pragma unroll
-        for (int k = 0; k < kItems; k++) {
-          const int b = (int)(nb[k] & 15u);
-          const uint32_t female = (nb[k] >> 4) & 1u;
-          const uint32_t d = dk[k];
-          // queue this warp's owed draws; their column is written after the draw
-          const uint32_t owed = d != 0xffffffffu ? nb[k] >> 5 : BM_NONE;
-          const uint32_t om = __ballot_sync(0xffffffffu, owed != BM_NONE);
-          if (owed != BM_NONE) {
-            BmEntry q;
-            q.d = d; q.gid = si.lo + k * kBlock + tid; q.batches = a[k].batches; q.kind = owed;
-            bmq[nq + __popc(om & lanemask_lt())] = q;
-          }
-          nq += __popc(om);
-          if (d != 0xffffffffu) {
-            dst.age[d] = a[k].age; dst.his[d] = a[k].his; dst.sporo[d] = a[k].sporo; dst.uni[d] = a[k].uni;
-            dst.cycle[d] = a[k].cycle; dst.hbc[d] = a[k].hbc; dst.batches[d] = a[k].batches;
-            dst.flags[d] = (uint8_t)(b | (female << 3));
-            if (owed != BM_LARVA_DELAY) dst.delay[d] = a[k].delay;
-            if (owed != BM_EGG_BATCH) dst.avail[d] = a[k].avail;
-            // statistics of the next pool (kernel/calcL1de.cl:28-30, kernel/calcGender.cl:24-37)
-            if (b == LARVA) {
-              l1 += age_days_uncapped(a[k].age);
-              const uint32_t dd = age_days(a[k].age);
-              dmin = min(dmin, dd); dmax = max(dmax, dd);
-            } else if (b >= IMMATURE && female) {
-              fem += 1u;
-              inf += a[k].sporo >= 1.0f ? 1u : 0u;
-            }
-          }
-        }
-        // ---- the warp's owed draws, dense over its lanes ----
-        if (nq) {
-          __syncwarp();
-          for (uint32_t jq = lane; jq < nq; jq += 32) {
-            const BmEntry q = bmq[jq];
-            const uint32_t v = finish_box_muller(c, mc, q.gid, q.kind, q.batches);
-            if (q.kind == BM_LARVA_DELAY) dst.delay[q.d] = __uint_as_float(v);
-            else dst.avail[q.d] = v;
-          }
-          __syncwarp();  // the queue is rewritten by the next tile
-        }
-      } else {
-        // ---- new eggs at [0, newEggs) of the next buffer ----
-        const uint32_t e0 = si.lo, ne = si.newEggs;
-#pragma unroll
-        for (int k = 0; k < kItems; k++) {
-          const uint32_t id = e0 + k * kBlock + tid;
-          if (id < ne) {
-            Rec a;
-            new_egg(c, id, a);
-            dst.age[id] = a.age; dst.his[id] = a.his; dst.delay[id] = a.delay; dst.sporo[id] = a.sporo;
-            dst.uni[id] = a.uni; dst.avail[id] = a.avail; dst.cycle[id] = a.cycle; dst.hbc[id] = a.hbc;
-            dst.batches[id] = a.batches;
-            dst.flags[id] = (uint8_t)(EGG | (a.female << 3));
-          }
-        }
-      }
+  };
+  for (uint32_t t = blockIdx.x * kWarps + warp; t < total; t += stride) {
+    const uint32_t r = find_rep(s_pre, p.nrep, t);
+    if (r != cur_rep) {  // uniform
+      flush();
+      load_warp_rep<true, AHEAD>(p.reps[r], w);
+      cur_rep = r;
     }
-    if (cur_rep != 0xffffffffu) flush(cur_rep);
-    if (fail && lane == 0) {
-      // let loads still in flight land before the CTA exits (bounded waits)
-      for (int s = 0; s < 2; s++) (void)mbar_wait(&full[s], (ph >> s) & 1u);
+    const uint32_t sp = t - s_pre[r];
+    if (AHEAD) {  // this unit's share of the span counts that the pass after the next adds to
+      const uint32_t z1 = min((sp + 1u) * w.clearPer, w.clear);
+      for (uint32_t z = sp * w.clearPer + lane; z < z1; z += 32u) w.spans2[z] = make_uint4(0u, 0u, 0u, 0u);
+    }
+    if (sp < w.nspans) {
+      const uint32_t i = (sp & ~31u) + lane;
+      uint4 v = make_uint4(0u, 0u, 0u, 0u);
+      if (i <= sp) v = __ldg(w.spans + i);
+      const uint32_t pre = lane < 8 ? __ldg(w.superPre + (size_t)(sp >> 5) * 8 + lane) : 0u;
+      uint4 own, before;
+      own.x = __shfl_sync(0xffffffffu, v.x, sp & 31u);
+      own.y = __shfl_sync(0xffffffffu, v.y, sp & 31u);
+      own.z = __shfl_sync(0xffffffffu, v.z, sp & 31u);
+      own.w = __shfl_sync(0xffffffffu, v.w, sp & 31u);
+      before.x = __reduce_add_sync(0xffffffffu, v.x) - own.x;
+      before.y = __reduce_add_sync(0xffffffffu, v.y) - own.y;
+      before.z = __reduce_add_sync(0xffffffffu, v.z) - own.z;
+      before.w = __reduce_add_sync(0xffffffffu, v.w) - own.w;
+      const uint32_t b = lane & 7;
+      const uint32_t base0 = (b == EGG ? w.newEggs : w.next.r[b].start) + pre + state_count(before, b);
+      uint32_t base = base0;
+      const uint32_t end = w.pop.r[GRAVID].end, u0 = sp << w.shift;
+      const uint32_t u1 = end - u0 > (1u << w.shift) ? u0 + (1u << w.shift) : end;
+      for_ranges(w.pop, u0, u1, ScatterRanges<I, WIDE, AHEAD>{w, s_mc, ring, base, mq, mx, sum});
+      // the decisions and their counts must agree on the span's survivors
+      const bool differ = __any_sync(0xffffffffu, lane < 8 && base - base0 != state_count(own, b));
+      if (differ && lane == 0) sum.error |= SAMPO_DEV_ERR_TILECOUNT;
+    } else {
+      // ---- new eggs at [0, newEggs) of the next buffer ----
+      const uint32_t e0 = (sp - w.nspans) << w.shift, ne = w.newEggs;
+      const uint32_t e1 = ne - e0 > (1u << w.shift) ? e0 + (1u << w.shift) : ne;
+      const DevPool dst = w.dst;
+      const bool ahead = AHEAD && w.ahead;
+      Tally ts = {0, 0, 0};
+      DecideAcc da;
+      clear_acc(da);
+      for (uint32_t r0 = e0; r0 < e1; r0 += 32u) {
+        const uint32_t id = r0 + lane;
+        const bool in = id < e1;
+        uint32_t code1 = DEC_DIES;
+        if (in) {
+          Rec a;
+          new_egg(w.c, id, a);
+          store_cols<state_cols(EGG, WIDE)>(dst, id, a);
+          const uint32_t female = a.female;
+          if (ahead) code1 = decide<EGG, WIDE>(w.c1, s_mc.kill, id, a, da);
+          put(dst.flags + id, EGG | (female << 3) | (code1 << 4));
+        }
+        if (ahead) {
+          const uint32_t ks = __ballot_sync(0xffffffffu, code1 == DEC_STAYS), km = __ballot_sync(0xffffffffu, code1 == DEC_MOVES);
+          add_tally<EGG>(w, ts, r0, min(e1 - r0, 32u), ks, km, id);
+        }
+      }
+      if (ahead) {
+        flush_tally<EGG>(w, ts);
+        add_decided<EGG, EGG>(da, sum);
+      }
     }
   }
-  if (fail && (lane == 0)) atomicOr(&p.reps[fail_rep].sim->error, SAMPO_DEV_ERR_TMA);
+  flush();
 }
 
 // ------------------------------------------------------------------------
@@ -1338,7 +1389,7 @@ __global__ void k_init_eggs(KParams p, uint32_t n, float T0, const sampo_seeds* 
     for (int k = 0; k < 4; k++) {
       c.rng_c13[k] = taus_step(seeds[k].z1 + 128u, 13, 19, 12, 4294967294u) ^ taus_step(seeds[k].z3 + 128u, 3, 11, 17, 4294967280u);
       c.rng_z2[k] = seeds[k].z2 + 128u;
-      c.rng_z4[k] = seeds[k].z4;
+      c.rng_k4[k] = 1664525u * seeds[k].z4;
     }
     species_step(T0, 0u, c);  // eggsIncubation(temperature[0]) (kernel/initAgents.cl:57)
   }
@@ -1354,58 +1405,80 @@ __global__ void k_init_eggs(KParams p, uint32_t n, float T0, const sampo_seeds* 
       float h = 24.0f * (float)(uint32_t)((z >> 32) % ((uint64_t)age_days_max + 1));
       a.age = h; a.his = h;
     }
-    dst.age[id] = a.age; dst.his[id] = a.his; dst.delay[id] = a.delay; dst.sporo[id] = a.sporo;
-    dst.uni[id] = a.uni; dst.avail[id] = a.avail; dst.cycle[id] = a.cycle; dst.hbc[id] = a.hbc;
-    dst.batches[id] = a.batches;
+    if (p.wide) store_cols<C_ALL>(dst, id, a);
+    else store_cols<state_cols(EGG, false)>(dst, id, a);
     dst.flags[id] = (uint8_t)(EGG | (a.female << 3));
   }
 }
 
 // Before and after a timing trial of the step kernels: zero what they add to
-// (survivor counts, eggs laid, next-pool statistics, tickets). Their other
-// writes - the next buffer, and tile counts and prefixes equal to the ones
-// the real step computes at the same tile size (k_clear_lookback clears the
-// prefixes between tile sizes) - leave the simulation's course unchanged.
+// (eggs laid, next-pool statistics) and the survivor counts. Their other
+// writes - the next buffer, and decisions and span counts equal to the ones
+// the real step computes - leave the simulation's course unchanged.
 __global__ void k_trial_reset(KParams p) {
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < p.nrep; r += gridDim.x * blockDim.x) {
     SimDev* sim = p.reps[r].sim;
     for (int k = 0; k < 8; k++) sim->cnt[k] = 0;
-    sim->newEggs = 0;
-    sim->acc_L1de = sim->acc_fem = sim->acc_inf = 0;
-    sim->acc_dmin = 0xffffffffu;
-    sim->acc_dmax = 0;
+    sim->dec = Decided{0u, 0u, 0xffffffffu, 0u};
+    sim->acc_fem = sim->acc_inf = 0;
     for (int k = 0; k < 4; k++) sim->acc_bnc[k] = 0;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    p.bat->ticket1 = 0;
-    p.bat->ticket2 = 0;
-  }
 }
 
-// Between timing trials of different tile sizes, and after them: every
-// replicate's inclusive prefixes to zero. A trial leaves prefixes tagged with
-// the coming step's epoch; at another tile size they sum other slots, and the
-// look-back would take them as published. Zero epochs match no step (epochs
-// start at 1).
-__global__ void k_clear_lookback(KParams p) {
-  const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+// The columns a narrow record implies (state_cols), written out, the decision
+// bits taken out of the flags, and zeros into the slots between the ranges,
+// for every replicate of p: what a reader of the pool's columns expects.
+__global__ void k_widen(KParams p) {
   for (uint32_t r = 0; r < p.nrep; r++) {
-    unsigned long long* incl = p.reps[r].tileIncl;
-    const size_t n = (size_t)p.reps[r].maxTiles * 8;
-    for (size_t i = i0; i < n; i += stride) incl[i] = 0ull;
+    const SimDev* sim = p.reps[r].sim;
+    const sampo_population pop = sim->pop;
+    const DevPool d = p.reps[r].pool[sim->cur];
+    if (!d.age) continue;  // an empty slot of a batch
+    const uint32_t end = pop.r[GRAVID].end;
+    for (uint64_t g64 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g64 < end; g64 += (uint64_t)gridDim.x * blockDim.x) {
+      const uint32_t g = (uint32_t)g64;
+      const int rg = range_of(pop, g);
+      if (rg < 0) {  // a slot between two ranges
+        store_cols<C_ALL>(d, g, Rec{});
+        d.flags[g] = 0;
+        continue;
+      }
+      d.flags[g] &= 15u;
+      if (p.wide || rg >= BMS) continue;
+      if (rg == EGG) { d.his[g] = d.age[g]; d.uni[g] = 0u; }
+      if (rg == LARVA) d.his[g] = d.age[g] - 24.0f;
+      d.sporo[g] = 0.0f; d.avail[g] = 0u; d.cycle[g] = 0u; d.hbc[g] = 0u; d.batches[g] = 0u;
+    }
   }
 }
 
-// Statistics of p.reps[0]'s current pool (grid-stride), accumulated into acc_*.
-__global__ void k_pool_stats(KParams p) {
+// Whether an agent's record holds anything its state does not imply (see
+// state_cols), or an age that is not a whole number of hours below 2^20 (the
+// narrow passes take days from whole hours, and a larva's hoursInState from
+// its age; no agent lives another 2^20 hours).
+__device__ __forceinline__ bool wide_record(const DevPool& s, uint32_t g, int rg) {
+  const float age = s.age[g], his = s.his[g];
+  if (!(age >= 0.0f && age < 1048576.0f) || age != floorf(age)) return true;
+  if (rg >= BMS) return false;
+  bool w = __float_as_uint(s.sporo[g]) != 0u || s.avail[g] || s.cycle[g] || s.hbc[g] || s.batches[g];
+  if (rg == EGG) w |= __float_as_uint(his) != __float_as_uint(age) || s.uni[g];
+  if (rg == LARVA) w |= __float_as_uint(his) != __float_as_uint(age - 24.0f);
+  return w;
+}
+
+// Statistics of p.reps[0]'s current pool (grid-stride), accumulated into
+// acc_*; with `check`, also whether its records are wide.
+__global__ void k_pool_stats(KParams p, int check) {
   SimDev* sim = p.reps[0].sim;
   const sampo_population pop = sim->pop;
   const DevPool src = p.reps[0].pool[sim->cur];
   uint32_t l1 = 0, fem = 0, inf = 0, dmin = 0xffffffffu, dmax = 0;
+  bool wide = false;
   const uint32_t end = pop.r[GRAVID].end;
   for (uint64_t g64 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g64 < end; g64 += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t g = (uint32_t)g64;
     int rg = range_of(pop, g);
+    if (check && rg >= 0) wide |= wide_record(src, g, rg);
     if (rg == LARVA) {
       float age = src.age[g];
       l1 += age_days_uncapped(age);
@@ -1415,16 +1488,18 @@ __global__ void k_pool_stats(KParams p) {
       if ((src.flags[g] >> 3) & 1u) { fem++; inf += src.sporo[g] >= 1.0f ? 1u : 0u; }
     }
   }
+  wide = __any_sync(0xffffffffu, wide);
   l1 = __reduce_add_sync(0xffffffffu, l1);
   fem = __reduce_add_sync(0xffffffffu, fem);
   inf = __reduce_add_sync(0xffffffffu, inf);
   dmin = __reduce_min_sync(0xffffffffu, dmin);
   dmax = __reduce_max_sync(0xffffffffu, dmax);
   if ((threadIdx.x & 31) == 0) {
-    if (l1) atomicAdd(&sim->acc_L1de, l1);
+    if (l1) atomicAdd(&sim->dec.L1de, l1);
     if (fem) atomicAdd(&sim->acc_fem, fem);
     if (inf) atomicAdd(&sim->acc_inf, inf);
-    if (dmin != 0xffffffffu) { atomicMin(&sim->acc_dmin, dmin); atomicMax(&sim->acc_dmax, dmax); }
+    if (dmin != 0xffffffffu) { atomicMin(&sim->dec.dmin, dmin); atomicMax(&sim->dec.dmax, dmax); }
+    if (wide) sim->wide = 1u;
   }
 }
 
