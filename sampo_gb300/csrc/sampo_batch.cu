@@ -76,6 +76,7 @@ struct sampo_batch {
   std::vector<uint32_t> wt_staging;
   int grid_count = 0, grid_scatter = 0;
   int items = kItems;                // slots per thread of the count and update/scatter passes (2 or 4)
+  uint32_t min_span = 0;             // BatchDev::minSpan as last set
   bool wide = false;                 // every slot's pool holds whole records (state_cols): set by the first loaded one that has to
   cudaGraphExec_t day_graph[2] = {nullptr, nullptr};  // three kernels every hour, and deciding ahead
   uint32_t day_graph_kernels[2] = {0, 0};             // kernel nodes of each
@@ -414,7 +415,7 @@ extern "C" int sampo_batch_init_population(sampo_batch* b, uint32_t slot, uint32
   BCK(cudaMemcpyAsync(b->init_seeds_dev + (size_t)slot * 4, init_seeds, 4 * sizeof(sampo_seeds), cudaMemcpyHostToDevice, b->stream),
       "seeds");
   const KParams p = slot_params(b, slot);
-  BCK(launch_init_eggs(p, n, r->T_host[0], b->init_seeds_dev + (size_t)slot * 4, age_days_max, age_seed, b->stream), "initAgents");
+  BCK(launch_init_eggs(p, n, r->T_host[0], b->init_seeds_dev + (size_t)slot * 4, age_days_max, age_seed, b->wide, b->stream), "initAgents");
   BCK(launch_publish_start(p, false, b->stream), "initial statistics");
   r->have_pop = true;
   r->known_end = pop.r[7].end;
@@ -558,11 +559,23 @@ static cudaError_t launch_hours(sampo_batch* b, const KParams& p, uint32_t nstep
 // more than kAheadSlots slots. Below that a step is three launches' latency
 // either way.
 constexpr uint64_t kAheadSlots = 65536;
-static bool decides_ahead(const sampo_batch* b) {
+static uint64_t known_slots(const sampo_batch* b) {
   uint64_t slots = 0;
   for (const Replicate& r : b->reps)
     if (r.used && r.have_pop && r.active) slots += r.known_end;
-  return slots > kAheadSlots;
+  return slots;
+}
+static bool decides_ahead(const sampo_batch* b) { return known_slots(b) > kAheadSlots; }
+
+// The smallest span of the run's passes: what the warps' share of all the
+// replicates' slots comes to (the spans of a replicate alone would be sized
+// for it to occupy every warp).
+static cudaError_t set_min_span(sampo_batch* b) {
+  const uint64_t share = known_slots(b) / kSpanWarps;
+  const uint32_t span = share > kSpanMax ? kSpanMax : (uint32_t)share;
+  if (span == b->min_span) return cudaSuccess;
+  b->min_span = span;
+  return cudaMemcpyAsync(&b->bat_dev->minSpan, &b->min_span, sizeof(uint32_t), cudaMemcpyHostToDevice, b->stream);
 }
 
 static int build_batch_graph(sampo_batch* b, bool ahead) {
@@ -611,6 +624,7 @@ extern "C" int sampo_batch_run(sampo_batch* b, uint32_t nsteps, int wait) {
   cudaSetDevice(b->device);
   const KParams p = all_params(b);
   BCK(cudaEventRecord(b->ev0, b->stream), "event");
+  BCK(set_min_span(b), "span size");
   BCK(launch_publish(p, PUB_REFRESH, b->stream), "step constants");  // inputs may postdate the last publish
   b->launches += 1;
   const bool ahead = decides_ahead(b);

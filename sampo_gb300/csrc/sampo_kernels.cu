@@ -100,7 +100,7 @@ cudaError_t launch_steps(const KParams& p, uint32_t nsteps, bool ahead, int grid
     // one count pass; every pass but the last decides the hour after its own
     bool ok = run(launch_count(p, grid_count, st, items)) && run(launch_publish(p, PUB_DECIDED | PUB_AHEAD, st));
     for (uint32_t i = 0; i < nsteps && ok; i++)
-      ok = run(launch_scatter(p, grid_scatter, st, items, true)) &&
+      ok = run(launch_scatter(p, grid_scatter, st, items, i + 1 < nsteps)) &&
            run(launch_publish(p, PUB_AFTER_STEP | (i + 2 < nsteps ? PUB_AHEAD : 0), st));
   } else {
     for (uint32_t i = 0; i < nsteps; i++)
@@ -117,9 +117,10 @@ cudaError_t launch_publish(const KParams& p, int mode, cudaStream_t st) {
   return launch(p, KID_PUBLISH, (const void*)k_publish, p.nrep, mode == PUB_REFRESH ? 32 : kPublishThreads, 0, st, args);
 }
 cudaError_t launch_init_eggs(const KParams& p, uint32_t n, float T0, const sampo_seeds* seeds_dev, int age_days_max,
-                             uint64_t age_seed, cudaStream_t st) {
+                             uint64_t age_seed, bool full, cudaStream_t st) {
   KParams q = p;
-  void* args[] = {&q, &n, &T0, &seeds_dev, &age_days_max, &age_seed};
+  int fc = full ? 1 : 0;
+  void* args[] = {&q, &n, &T0, &seeds_dev, &age_days_max, &age_seed, &fc};
   return launch(p, KID_INIT_EGGS, (const void*)k_init_eggs, sm_count() * 4, 256, 0, st, args);
 }
 cudaError_t launch_publish_start(const KParams& p, bool check, cudaStream_t st) {

@@ -74,29 +74,36 @@ struct SimDev {
   uint32_t larvaKill[2][100]; // larval mortality of step s by age in days (kill_threshold), at s % 2
 };
 
-// Batch-wide counters.
+// Batch-wide state.
 struct BatchDev {
+  uint32_t minSpan;           // smallest span (slots), see span_size; set by the host between runs
   uint32_t bar;               // one-launch step: CTAs past the decision phase (reset by its last CTA)
   uint32_t done;              // one-launch step: CTAs finished (reset by its last CTA)
 };
 
-// Spans: the slots a warp of the two passes takes at once, 2^span_shift(end)
-// of a pool that ends at `end`. Small enough that every warp of the largest
-// grid (4,864) gets several, so that the last round is a small part of the
-// pass; large enough that a span's fixed work (its prefix, about a hundred
-// instructions) stays a small part of its own.
-constexpr uint32_t kSpanMinShift = 7, kSpanMaxShift = 10, kSpanTarget = 16384;
-__host__ __device__ constexpr uint32_t units_of(uint32_t n, uint32_t shift) { return (n >> shift) + ((n & ((1u << shift) - 1u)) ? 1u : 0u); }
-__host__ __device__ constexpr uint32_t span_shift(uint32_t end) {
-  uint32_t s = kSpanMinShift;
-  while (s < kSpanMaxShift && units_of(end, s) > kSpanTarget) s++;
-  return s;
+// Spans: the slots a warp of the two passes takes at once, a multiple of 32.
+// A span costs a warp about a thousand instructions besides its rows (its
+// prefix, the start and end of its range, the agents that move on in a
+// partly filled warp), a row of 32 agents 60 to 150, so a pool is cut into as
+// few spans as keep every warp of the resident grid (kSpanWarps on 152 SMs)
+// equally busy: the smallest multiple of kSpanWarps that keeps them at
+// kSpanMax slots. A batch sets a larger smallest span (BatchDev::minSpan),
+// since its replicates share the warps.
+constexpr uint32_t kSpanMin = 128, kSpanMax = 1024, kSpanWarps = 3648;
+__host__ __device__ constexpr uint32_t units_of(uint32_t n, uint32_t size) { return n / size + (n % size ? 1u : 0u); }
+__host__ __device__ constexpr uint32_t span_size(uint32_t end, uint32_t min_span) {
+  const uint32_t warps = kSpanWarps * (end / (kSpanWarps * kSpanMax) + 1u);
+  uint32_t s = units_of(end, warps);
+  s = s < kSpanMin ? kSpanMin : s;
+  s = s < min_span ? min_span : s;
+  s = (s + 31u) / 32u * 32u;
+  return s < kSpanMax ? s : kSpanMax;
 }
-__host__ __device__ constexpr uint32_t span_count(uint32_t end) { return units_of(end, span_shift(end)); }
+__host__ __device__ constexpr uint32_t span_count(uint32_t end, uint32_t min_span) { return units_of(end, span_size(end, min_span)); }
 // The most spans any pool of up to `capacity` slots has.
 __host__ __device__ constexpr uint32_t max_spans(uint32_t capacity) {
-  const uint32_t most = units_of(capacity, kSpanMaxShift), small = units_of(capacity, kSpanMinShift);
-  return small <= kSpanTarget ? small : most > kSpanTarget ? most : kSpanTarget;
+  const uint32_t a = capacity / kSpanMin + 1u, b = capacity / kSpanMax + kSpanWarps + 1u;
+  return a < b ? a : b;
 }
 // The span arrays of a pool of `capacity` slots, in 16-byte words: a span's
 // survivors by next state (one word, for each of three steps), a super's (32
@@ -232,8 +239,9 @@ cudaError_t launch_steps(const KParams& p, uint32_t nsteps, bool ahead, int grid
                          uint32_t* launches);
 // k_publish over every replicate of p (modes PUB_*, above).
 cudaError_t launch_publish(const KParams& p, int mode, cudaStream_t st);
+// (`full`: every column, else those that hold an egg's record in a narrow pool)
 cudaError_t launch_init_eggs(const KParams& p, uint32_t n, float T0, const sampo_seeds* seeds_dev,
-                             int age_days_max, uint64_t age_seed, cudaStream_t st);
+                             int age_days_max, uint64_t age_seed, bool full, cudaStream_t st);
 // statistics of p.reps[0]'s current pool, then its publish (PUB_INITIAL);
 // `check` also finds out whether the pool is a wide one (SimDev::wide)
 cudaError_t launch_publish_start(const KParams& p, bool check, cudaStream_t st);

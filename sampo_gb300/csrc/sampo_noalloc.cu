@@ -125,7 +125,7 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
 
   // The array keeps the previous call's contents: reset the state and clear
   // the supers this step adds to.
-  const uint32_t nsup = (span_count(pop_in->r[7].end) + 31u) / 32u;
+  const uint32_t nsup = (span_count(pop_in->r[7].end, 0) + 31u) / 32u;
   RepParams rp;
   rp.sim = &sc->sim;
   rp.pool[0] = to_dev(in);

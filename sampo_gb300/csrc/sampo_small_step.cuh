@@ -28,6 +28,9 @@
 // takes tiles b + G, b + 2G, ... (G CTAs); their decisions are counted in
 // phase 1 and the tile is loaded and updated again in phase 2.
 //
+// It reads and writes whole records: a narrow pool (state_cols) that the other
+// passes wrote last has its implied columns written out first (k_widen).
+//
 // Built into the library for the built-in species only (a user species keeps
 // the three-kernel step).
 #pragma once
@@ -108,7 +111,7 @@ struct SmallAcc {
 // counters and the next pool's statistics go to sa (a tile updated twice
 // counts its eggs the first time and the rest the second).
 template <int I, bool KEEP, bool EGGS, bool STATS>
-__device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelConst& mc, const sampo_population& pop, bool wide,
+__device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelConst& mc, const sampo_population& pop,
                                                   uint8_t* st, uint32_t lo, uint32_t end, uint2* s_ent, SmallAcc& sa) {
   SAMPO_TILE_CONSTANTS(I);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -137,12 +140,6 @@ __device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelC
       a.batches = c_batches[i];
       a.female = (c_flags[i] >> 3) & 1u;
       a.bm = BM_NONE;
-      if (!wide && rg < BMS) {  // a narrow record's implied fields (state_cols): the columns hold anything
-        a.sporo = 0.0f;
-        a.avail = a.cycle = a.hbc = a.batches = 0u;
-        if (rg == EGG) { a.his = a.age; a.uni = 0u; }
-        if (rg == LARVA) a.his = a.age - 24.0f;
-      }
       sa.devoob |= (rg == LARVA) & c.devOOB;
       const int ns = update_agent<true, true, false>(c, mc.kill, rg, g, a, t);
       if (ns >= 0) {
@@ -435,7 +432,6 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
   const uint32_t G = gridDim.x, b = blockIdx.x;
   uint32_t phase = 0, barriers = 0;
   bool met = true, ok = true;
-  const bool wide = p.wide != 0;
   const uint32_t stride = rp.smallStride;  // >= the tiles of any pool that fits, at 256-slot tiles
   uint32_t* rows = rp.smallRows;  // [kSmallRows + kSmallStats][stride]
 
@@ -491,7 +487,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           if (!ok) break;
         }
         const uint32_t eggs_before = sa.acc.newEggs;
-        small_update_tile<I, false, true, true>(s_c, s_mc, s_pop, wide, stage, t * kTile, end, s_ent, sa);
+        small_update_tile<I, false, true, true>(s_c, s_mc, s_pop, stage, t * kTile, end, s_ent, sa);
         const uint32_t ne = __reduce_add_sync(0xffffffffu, sa.acc.newEggs - eggs_before);
         if (lane == 0) s_ne[warp] = ne;
         __syncthreads();
@@ -511,7 +507,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
         }
         ok = small_wait_stage(&s_mbar, phase);
         if (ok) {
-          small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, wide, stage, b * kTile, end, s_ent, sa);  // counted above
+          small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, stage, b * kTile, end, s_ent, sa);  // counted above
           small_stats_warps(sa, s_red);
           __syncthreads();
           if (warp == 0) (void)small_build_table<I>(s_ent, s_tab);
@@ -522,7 +518,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
       ok = small_wait_stage(&s_mbar, phase);
       if (ok) {
         const uint32_t eggs_before = sa.acc.newEggs;
-        small_update_tile<I, true, true, true>(s_c, s_mc, s_pop, wide, stage, b * kTile, end, s_ent, sa);
+        small_update_tile<I, true, true, true>(s_c, s_mc, s_pop, stage, b * kTile, end, s_ent, sa);
         const uint32_t ne = __reduce_add_sync(0xffffffffu, sa.acc.newEggs - eggs_before);
         if (lane == 0) s_ne[warp] = ne;
         small_stats_warps(sa, s_red);
@@ -567,7 +563,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           small_issue_tile<I>(rp.pool[s_cur], stage, &s_mbar, t * kTile, min((uint32_t)kTile, end - t * kTile));
         }
         if (!small_wait_stage(&s_mbar, phase)) { ok = false; break; }
-        small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, wide, stage, t * kTile, end, s_ent, sa);
+        small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, stage, t * kTile, end, s_ent, sa);
         small_sum_rows(rows, stride, nold, t, false, s_ex, s_tot, s_part);
         if (warp == 0) {
           const uint32_t tw = small_build_table<I>(s_ent, s_tab);

@@ -258,7 +258,7 @@ static_assert(sizeof(StepCtx) % 16 == 0, "StepCtx is copied in 16-byte words");
 // The two passes of a step
 // ------------------------------------------------------------------------
 // Both passes cut every active replicate's pool into spans of
-// 2^span_shift(end) slots and give the spans of the batch to the warps of a
+// span_size(end) slots and give the spans of the batch to the warps of a
 // grid of resident CTAs in turn (warp w takes units w, w + W, ...). A warp
 // walks its span range by range, 32 slots of one state at a time, with code
 // specialised for the state, and shares nothing with the other warps but the
@@ -311,13 +311,7 @@ __host__ __device__ constexpr uint32_t num_cols(uint32_t cols) {
 // 57 % of its cycles). The chunk is the largest of 32 * I, 64 or 32 slots of
 // which at least two fit (I = 4 or 2, the "slots per thread").
 constexpr int kRowUnroll = 2;  // rows of a chunk unrolled together
-constexpr uint32_t kRingBytes = 4096;
-// Dynamic shared memory of the two passes: the rings and the batch's unit
-// prefix (nrep + 1 words), sized at launch so that a single simulation pays 8
-// bytes for it.
-__host__ __device__ constexpr size_t pass_smem(uint32_t nrep) {
-  return kWarps * (size_t)kRingBytes + (((size_t)(nrep + 1) * 4 + 15) & ~(size_t)15);
-}
+constexpr uint32_t kRingBytes = 5120;
 template <uint32_t COLS, uint32_t BYTE_COLS, int I>
 struct Ring {
   static constexpr uint32_t kSlotBytes = 4 * num_cols(COLS) + BYTE_COLS;
@@ -399,6 +393,21 @@ __device__ __forceinline__ void stream_range(uint8_t* ring, const DevPool& s, co
     wr = wr + 1 == N ? 0 : wr + 1;
   }
   cp_async_wait<0>();
+}
+// The same columns of one slot, from the pool itself.
+template <uint32_t COLS>
+__device__ __forceinline__ void load_cols(const DevPool& s, uint32_t g, Rec& a) {
+  a.age = (COLS & C_AGE) ? __ldg(s.age + g) : 0.0f;
+  a.his = (COLS & C_HIS) ? __ldg(s.his + g) : 0.0f;
+  a.delay = (COLS & C_DELAY) ? __ldg(s.delay + g) : 0.0f;
+  a.sporo = (COLS & C_SPORO) ? __ldg(s.sporo + g) : 0.0f;
+  a.uni = (COLS & C_UNI) ? __ldg(s.uni + g) : 0u;
+  a.avail = (COLS & C_AVAIL) ? __ldg(s.avail + g) : 0u;
+  a.cycle = (COLS & C_CYCLE) ? __ldg(s.cycle + g) : 0u;
+  a.hbc = (COLS & C_HBC) ? __ldg(s.hbc + g) : 0u;
+  a.batches = (COLS & C_BATCHES) ? __ldg(s.batches + g) : 0u;
+  a.female = 0u;
+  a.bm = BM_NONE;
 }
 // The fields a narrow record implies.
 template <int RG, bool WIDE>
@@ -539,15 +548,16 @@ __device__ void scan_supers_block(const RepParams& rp, uint32_t nspans, uint32_t
 // its next unit belongs to another one.
 struct alignas(16) WarpRep {
   StepCtx c;                    // constants of the step
-  StepCtx c1;                   // and of the step after, while deciding ahead
+  StepCtx c1;                   // and of the step after, in a pass that decides ahead
+  uint32_t larvaKill1[100];     // its larval mortality
   sampo_population pop, next;   // current ranges; the next pool's (update/scatter pass)
   DevPool src, dst;
   uint8_t* dec;                 // decisions of caller-owned pools, or null: in the flags
   uint4 *spans, *spans1, *spans2;  // span counts of the step, of the step after, and the ones to clear
   uint4* supers;
   const uint32_t* superPre;
-  uint32_t shift, nspans, newEggs, ahead;
-  uint32_t shift1, clear, clearPer;  // span size of the next pool; spans to clear, and of them per unit
+  uint32_t span, nspans, newEggs, ahead;  // slots per span, spans, eggs laid, whether it decides ahead
+  uint32_t span1, clear, clearPer;        // slots per span of the next pool; spans to clear, and of them per unit
 };
 // Words of src to dst by the lanes of a warp.
 template <class T>
@@ -559,12 +569,18 @@ __device__ __forceinline__ void warp_copy(T* dst, const T* src) {
 }
 // (PASS2: also what the update/scatter pass needs)
 template <bool PASS2, bool AHEAD>
-__device__ __forceinline__ void load_warp_rep(const RepParams& rp, WarpRep& w) {
+__device__ __forceinline__ void load_warp_rep(const RepParams& rp, uint32_t min_span, WarpRep& w) {
   const SimDev* sim = rp.sim;
   const uint32_t cur = sim->cur, par = sim->step & 1u;
   __syncwarp();  // every lane is past its reads of the last replicate's
   warp_copy(&w.c, &sim->ctx[par]);
-  if (AHEAD) warp_copy(&w.c1, &sim->ctx[par ^ 1u]);
+  if (AHEAD) {
+    // a replicate that stops after this step decides nothing ahead: it runs
+    // through the same code with this step's constants, and nothing is kept
+    const uint32_t q = sim->ahead ? par ^ 1u : par;
+    warp_copy(&w.c1, &sim->ctx[q]);
+    for (uint32_t k = threadIdx.x & 31; k < 100; k += 32) w.larvaKill1[k] = sim->larvaKill[q][k];
+  }
   warp_copy(&w.pop, &sim->pop);
   warp_copy(&w.src, &rp.pool[cur]);
   if (PASS2) warp_copy(&w.dst, &rp.pool[cur ^ 1u]);
@@ -574,8 +590,8 @@ __device__ __forceinline__ void load_warp_rep(const RepParams& rp, WarpRep& w) {
     w.spans = rp.spans + (size_t)rot * rp.spanStride;
     w.supers = rp.supers;
     w.superPre = rp.superPre;
-    w.shift = span_shift(end);
-    w.nspans = span_count(end);
+    w.span = span_size(end, min_span);
+    w.nspans = units_of(end, w.span);
     w.newEggs = sim->dec.newEggs;
     if (PASS2) {
       uint32_t tc[8], base[8];
@@ -585,9 +601,9 @@ __device__ __forceinline__ void load_warp_rep(const RepParams& rp, WarpRep& w) {
       w.next = np;
       if (AHEAD) {
         w.ahead = sim->ahead;
-        w.shift1 = span_shift(np.r[GRAVID].end);
+        w.span1 = span_size(np.r[GRAVID].end, min_span);
         w.spans1 = rp.spans + (size_t)(rot == 2u ? 0u : rot + 1u) * rp.spanStride;
-        const uint32_t old = rot == 0u ? 2u : rot - 1u, units = w.nspans + units_of(w.newEggs, w.shift);
+        const uint32_t old = rot == 0u ? 2u : rot - 1u, units = w.nspans + units_of(w.newEggs, w.span);
         w.spans2 = rp.spans + (size_t)old * rp.spanStride;
         w.clear = w.ahead ? sim->dirty[old] : 0u;
         w.clearPer = units ? (w.clear + units - 1u) / units : 0u;
@@ -596,6 +612,13 @@ __device__ __forceinline__ void load_warp_rep(const RepParams& rp, WarpRep& w) {
   }
   __syncwarp();
 }
+
+// Slots whose agents move on to another state this hour wait here until 32
+// are there (or the range ends) and are then written out by 32 lanes at once:
+// in a row of 32 agents one moves every few hours, and its transition (for a
+// hatching egg a normal draw) would occupy the warp for a single lane. A
+// power of two above 31 + a chunk's slots.
+constexpr uint32_t kMoved = 256;
 
 // What a warp adds to its replicate, gathered range by range in shared memory
 // (written by lane 0).
@@ -620,6 +643,25 @@ __device__ __forceinline__ void flush_sum(WarpSum& t, SimDev* sim, Decided* to) 
     if (t.bnc[j]) atomicAdd(&sim->acc_bnc[j], t.bnc[j]);
   if (t.error) atomicOr(&sim->error, t.error);
   clear_sum(t);
+}
+
+// The dynamic shared memory of the two passes, followed by the batch's unit
+// prefix (nrep + 1 words, sized at launch so that a single simulation pays 8
+// bytes for it). The code of a range is a function of its own, so that its
+// registers are its own (inlined together, the eight ranges' code spilled in
+// its loops); it finds its warp's state here.
+struct alignas(128) PassShared {
+  uint8_t ring[kWarps][kRingBytes];
+  WarpRep rep[kWarps];
+  ModelConst mc;
+  uint32_t moved[kWarps][kMoved];
+  WarpSum sum[kWarps];
+  uint32_t scan[36];
+};
+extern __shared__ __align__(128) uint8_t pass_shared_memory[];
+__device__ __forceinline__ PassShared& pass_shared() { return *reinterpret_cast<PassShared*>(pass_shared_memory); }
+__host__ __device__ constexpr size_t pass_smem(uint32_t nrep) {
+  return sizeof(PassShared) + (((size_t)(nrep + 1) * 4 + 15) & ~(size_t)15);
 }
 
 // What a lane's decisions in one range add up to.
@@ -649,6 +691,19 @@ __device__ __forceinline__ void add_decided(const DecideAcc& d, WarpSum& t) {
     t.error |= bad;
   }
 }
+// A range's (or its moves') females and counters into the warp's sums.
+template <int RG>
+__device__ __forceinline__ void add_moved(uint32_t fem, uint32_t inf, const Acc& acc, WarpSum& t) {
+  uint32_t v[6] = {fem, inf, acc.cycles, acc.sumCycles, acc.bites, acc.infectBites};
+#pragma unroll
+  for (int j = 0; j < 6; j++) v[j] = (j < 2 || RG >= BMS) ? __reduce_add_sync(0xffffffffu, v[j]) : 0u;
+  if ((threadIdx.x & 31) == 0) {
+    t.fem += v[0];
+    t.inf += v[1];
+#pragma unroll
+    for (int j = 0; j < 4; j++) t.bnc[j] += v[2 + j];
+  }
+}
 // The decision about the agent a at slot g of range RG (a: its fields of
 // decide_cols; changed). Adds the larva it leaves to the next pool's
 // statistics (kernel/calcL1de.cl:28-30).
@@ -669,11 +724,15 @@ __device__ __forceinline__ uint32_t decide(const StepCtx& c, const KillConst& kc
 }
 
 // The count pass over slots [lo, hi) of range RG: each agent's decision into
-// its flags (bits 4-5), or into dec where the pool belongs to the caller, and
-// the survivors by next state into cs.
+// its flags (bits 4-5), or into dec where the pool belongs to the caller.
+// Returns the agents that stay | those that move on << 16 (a span has at most
+// 2^10).
 template <int I, bool WIDE, int RG>
-__device__ __forceinline__ void count_range(const WarpRep& w, const KillConst& kc, uint8_t* ring, uint32_t lo, uint32_t hi, uint4& cs,
-                                            WarpSum& sum) {
+__device__ __noinline__ uint32_t count_range(uint32_t lo, uint32_t hi) {
+  PassShared& ps = pass_shared();
+  const uint32_t warp = threadIdx.x >> 5;
+  const WarpRep& w = ps.rep[warp];
+  const KillConst& kc = ps.mc.kill;
   constexpr uint32_t COLS = decide_cols(RG, WIDE);
   using RING = Ring<COLS, 1, I>;
   const uint32_t lane = threadIdx.x & 31u;
@@ -683,7 +742,7 @@ __device__ __forceinline__ void count_range(const WarpRep& w, const KillConst& k
   DecideAcc da;
   clear_acc(da);
   uint32_t ns_stay = 0, ns_move = 0;
-  stream_range<RING, COLS>(ring, src, src.flags, nullptr, lo, hi, [&](const uint8_t* st, uint32_t g0) {
+  stream_range<RING, COLS>(ps.ring[warp], src, src.flags, nullptr, lo, hi, [&](const uint8_t* st, uint32_t g0) {
 #pragma unroll kRowUnroll
     for (uint32_t k = 0; k < RING::kSlots / 32; k++) {
       const uint32_t i = 32u * k + lane, g = g0 + i;
@@ -702,9 +761,8 @@ __device__ __forceinline__ void count_range(const WarpRep& w, const KillConst& k
       ns_move += __popc(__ballot_sync(0xffffffffu, code == DEC_MOVES));
     }
   });
-  add_decided<RG, RG>(da, sum);
-  add_count<RG>(cs, ns_stay);
-  add_count<next_state(RG)>(cs, ns_move);
+  add_decided<RG, RG>(da, ps.sum[warp]);
+  return ns_stay | (ns_move << 16);
 }
 
 // Calls f<RG>(lo, hi) for the part of every range that lies in [u0, u1), in
@@ -720,14 +778,12 @@ __device__ __forceinline__ void for_ranges(const sampo_population& pop, uint32_t
 
 template <int I, bool WIDE>
 struct CountRanges {
-  const WarpRep& w;
-  const KillConst& kc;
-  uint8_t* ring;
   uint4& cs;
-  WarpSum& sum;
   template <int RG>
   __device__ __forceinline__ void operator()(uint32_t lo, uint32_t hi) {
-    count_range<I, WIDE, RG>(w, kc, ring, lo, hi, cs, sum);
+    const uint32_t n = count_range<I, WIDE, RG>(lo, hi);
+    add_count<RG>(cs, n & 0xffffu);
+    add_count<next_state(RG)>(cs, n >> 16);
   }
 };
 
@@ -737,24 +793,20 @@ struct CountRanges {
 // one down, so that the update/scatter pass starts on those this pass
 // touched last.
 template <int I, bool WIDE>
-__global__ void __launch_bounds__(kBlock, 4) k_count(KParams p) {
-  extern __shared__ __align__(16) uint8_t dsm[];  // the warps' rings, then the batch's unit prefix
-  uint32_t* s_pre = reinterpret_cast<uint32_t*>(dsm + kWarps * kRingBytes);
-  uint8_t* ring = dsm + (threadIdx.x >> 5) * kRingBytes;
-  __shared__ WarpRep s_wr[kWarps];
-  __shared__ KillConst s_mc;
-  __shared__ uint32_t s_w[33];
+__global__ void __launch_bounds__(kBlock, 3) k_count(KParams p) {
+  PassShared& ps = pass_shared();
+  uint32_t* s_pre = reinterpret_cast<uint32_t*>(pass_shared_memory + sizeof(PassShared));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  load_model_const(&p.mc->kill, s_mc);
-  plan_tickets(p.nrep, s_pre, s_w, [&](uint32_t r) -> uint32_t {
+  load_model_const(&p.mc->kill, ps.mc.kill);
+  const uint32_t min_span = p.bat->minSpan;
+  plan_tickets(p.nrep, s_pre, ps.scan, [&](uint32_t r) -> uint32_t {
     const SimDev* sim = p.reps[r].sim;
-    return sim->active ? span_count(sim->pop.r[GRAVID].end) : 0u;
+    return sim->active ? span_count(sim->pop.r[GRAVID].end, min_span) : 0u;
   });
   __syncthreads();
   const uint32_t total = s_pre[p.nrep], stride = gridDim.x * kWarps;
-  WarpRep& w = s_wr[warp];
-  __shared__ WarpSum s_sum[kWarps];
-  WarpSum& sum = s_sum[warp];
+  WarpRep& w = ps.rep[warp];
+  WarpSum& sum = ps.sum[warp];
   if (lane == 0) clear_sum(sum);
   uint32_t cur_rep = kNoRep, done = 0;
   // the warp's counters into its replicate's totals; the warp that brings
@@ -786,13 +838,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_count(KParams p) {
     const uint32_t r = find_rep(s_pre, p.nrep, t);
     if (r != cur_rep) {  // uniform
       flush();
-      load_warp_rep<false, false>(p.reps[r], w);
+      load_warp_rep<false, false>(p.reps[r], min_span, w);
       cur_rep = r;
     }
-    const uint32_t sp = t - s_pre[r], end = w.pop.r[GRAVID].end, u0 = sp << w.shift;
-    const uint32_t u1 = end - u0 > (1u << w.shift) ? u0 + (1u << w.shift) : end;
+    const uint32_t sp = t - s_pre[r], end = w.pop.r[GRAVID].end, u0 = sp * w.span;
+    const uint32_t u1 = end - u0 > w.span ? u0 + w.span : end;
     uint4 cs = make_uint4(0u, 0u, 0u, 0u);
-    for_ranges(w.pop, u0, u1, CountRanges<I, WIDE>{w, s_mc, ring, cs, sum});
+    for_ranges(w.pop, u0, u1, CountRanges<I, WIDE>{cs});
     if (lane == 0) {
       w.spans[sp] = cs;
       add_super(w.supers + (sp >> 5), cs);
@@ -885,6 +937,7 @@ __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
     }
     return;
   }
+  const uint32_t min_span = p.bat->minSpan;
   // the decisions whose totals describe the larvae of pool x, and the supers to scan
   const Decided* from = after && decided ? &sim->ahead_dec : &sim->dec;
   const uint32_t l1 = from->L1de, dmin = from->dmin, dmax = from->dmax;
@@ -925,7 +978,7 @@ __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
       shared_end_warn = shared_end && moved;
       pause = !layout_fits(cnt, dec.newEggs, capacity);  // the scatter pass flagged the capacity error and wrote nothing
       if (!pause) {
-        nspans = span_count(np.r[GRAVID].end);  // (of the pool that the step left)
+        nspans = span_count(np.r[GRAVID].end, min_span);  // (of the pool that the step left)
         uint32_t base[8];
         next_layout(cnt, dec.newEggs, np, base);
       }
@@ -942,7 +995,7 @@ __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
     if (after && decided) {
       const uint32_t units = nspans + dec.newEggs;  // (the pass cleared the oldest span counts if it had any unit)
       dirty = units ? 0u : sim->dirty[rot == 0u ? 2u : rot - 1u];
-      s_part[0][0] = span_count(np.r[GRAVID].end);
+      s_part[0][0] = span_count(np.r[GRAVID].end, min_span);
     }
     s_pause = pause;
   }
@@ -982,7 +1035,7 @@ __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
       const uint32_t old = rot == 0u ? 2u : rot - 1u, now = rot == 2u ? 0u : rot + 1u;
       sim->rot = now;
       sim->dirty[old] = dirty;
-      sim->dirty[now] = max(sim->dirty[now], span_count(np.r[GRAVID].end));
+      sim->dirty[now] = max(sim->dirty[now], span_count(np.r[GRAVID].end, min_span));
       dec = sim->ahead_dec;
       sim->dec = dec;
 #pragma unroll
@@ -1022,61 +1075,116 @@ __global__ void __launch_bounds__(kPublishThreads) k_publish(KParams p, int mode
 // ------------------------------------------------------------------------
 // Update + scatter pass
 // ------------------------------------------------------------------------
-// A survivor that moves on out of a state whose transition draws a normal
-// number (include/gpuRand.h:56-63): its record is finished after the chunk,
-// densely over the lanes. Those of a chunk take consecutive slots. gid: its
-// slot in the current buffer (the generator's); kind: BM_* | isFemale << 2.
-struct MovedEntry { uint32_t gid, kind; };
-struct MovedExtra { float age; uint32_t avail, batches; };  // BMD only
-constexpr uint32_t kMovedExtra = 32;
-
 // Deciding ahead: the decisions about survivors that a warp has put into
-// consecutive slots of state ST, gathered per span of the next pool.
-struct Tally { uint32_t end, stay, move; };  // first slot past the span being counted; its counts so far
+// consecutive slots of state ST, gathered per span of the next pool: the span
+// being counted, the first slot past it, and each lane's counts so far
+// (stays | moves on << 16).
+struct Tally { uint32_t span, end, cnt; };
+__device__ __forceinline__ uint32_t tally_count(uint32_t code) {
+  return code == DEC_STAYS ? 1u : code == DEC_MOVES ? 1u << 16 : 0u;
+}
 template <int ST>
 __device__ __forceinline__ void flush_tally(const WarpRep& w, Tally& t) {
-  if ((t.stay | t.move) && (threadIdx.x & 31) == 0) {
-    const uint32_t span = (t.end - 1u) >> w.shift1;
+  const uint32_t n = __reduce_add_sync(0xffffffffu, t.cnt);
+  if (w.ahead && n && (threadIdx.x & 31) == 0) {
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    add_count<ST>(v, t.stay);
-    add_count<next_state(ST)>(v, t.move);
-    add_super(w.spans1 + span, v);
-    add_super(w.supers + (span >> 5), v);
+    add_count<ST>(v, n & 0xffffu);
+    add_count<next_state(ST)>(v, n >> 16);
+    add_super(w.spans1 + t.span, v);
+    add_super(w.supers + (t.span >> 5), v);
   }
-  t.stay = t.move = 0;
+  t.cnt = 0;
 }
-// The slots [first, first + n) of a row; ks, km: the lanes that hold one
-// whose agent stays / moves on; d: a lane's slot. A row fills at most two spans.
+// Starts (slots from `first` on) or continues past t.end.
 template <int ST>
-__device__ __forceinline__ void add_tally(const WarpRep& w, Tally& t, uint32_t first, uint32_t n, uint32_t ks, uint32_t km, uint32_t d) {
-  if (first + n > t.end) {  // (and at the start, with t.end = 0)
-    const uint32_t in = __ballot_sync(0xffffffffu, d < t.end);  // (lanes that hold none are in neither mask)
-    t.stay += __popc(ks & in);
-    t.move += __popc(km & in);
-    flush_tally<ST>(w, t);
-    if (first >= t.end) {
-      t.end = ((first >> w.shift1) + 1u) << w.shift1;
-      if (first + n > t.end) {  // the first row of a run that starts near a span's end
-        const uint32_t in0 = __ballot_sync(0xffffffffu, d < t.end);
-        t.stay = __popc(ks & in0);
-        t.move = __popc(km & in0);
-        flush_tally<ST>(w, t);
-        ks &= ~in0;
-        km &= ~in0;
-        t.end += 1u << w.shift1;
-      }
-    } else {
-      ks &= ~in;
-      km &= ~in;
-      t.end += 1u << w.shift1;
-    }
+__device__ __forceinline__ void next_tally(const WarpRep& w, Tally& t, uint32_t first) {
+  if (t.end) flush_tally<ST>(w, t);
+  t.span = first / w.span1;
+  t.end = (t.span + 1u) * w.span1;
+}
+// The slots [first, first + n) of a row (n <= 32, so at most two spans); d: a
+// lane's slot, c: its tally_count (0 on lanes that hold none).
+template <int ST>
+__device__ __forceinline__ void add_tally(const WarpRep& w, Tally& t, uint32_t first, uint32_t n, uint32_t d, uint32_t c) {
+  if (first >= t.end) next_tally<ST>(w, t, first);
+  if (first + n > t.end) {
+    const bool here = d < t.end;
+    t.cnt += here ? c : 0u;
+    next_tally<ST>(w, t, t.end);
+    c = here ? 0u : c;
   }
-  t.stay += __popc(ks);
-  t.move += __popc(km);
+  t.cnt += c;
+}
+
+// Lanes where `on` holds store their survivor's narrow egg or larva record.
+template <int RG>
+__device__ __forceinline__ void put_if(bool on, const DevPool& p, uint32_t d, float age, float delay, float cld, uint32_t flags) {
+  if (RG == EGG)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %6, 0;\n\t@p st.global.f32 [%0], %3;\n\t@p st.global.f32 [%1], %4;\n\t@p st.global.u8 [%2], %5;\n\t}"
+                 ::"l"(p.age + d), "l"(p.delay + d), "l"(p.flags + d), "f"(age), "f"(delay), "r"(flags), "r"((uint32_t)on));
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %8, 0;\n\t@p st.global.f32 [%0], %4;\n\t@p st.global.f32 [%1], %5;\n\t@p st.global.f32 [%2], %6;\n\t@p st.global.u8 [%3], %7;\n\t}"
+                 ::"l"(p.age + d), "l"(p.delay + d), "l"(p.uni + d), "l"(p.flags + d), "f"(age), "f"(delay), "f"(cld), "r"(flags), "r"((uint32_t)on));
+}
+
+// The first n of the warp's waiting slots (moved), whose agents of range RG
+// move on to the next state: 32 at a time to the slots from bm on. Returns
+// the slot after the last. (A function of its own: called once in a span or
+// two, it would otherwise take the registers of the rows' loop.)
+template <bool WIDE, bool AHEAD, int RG>
+__device__ __noinline__ uint32_t move_on(uint32_t n, uint32_t bm) {
+  constexpr int NX = next_state(RG);
+  constexpr uint32_t CS = state_cols(RG, WIDE), CM = state_cols(NX, WIDE);
+  PassShared& ps = pass_shared();
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  const WarpRep& w = ps.rep[warp];
+  const ModelConst& mc = ps.mc;
+  WarpSum& sum = ps.sum[warp];
+  if (bm + n > w.next.r[NX].end) {  // no store leaves the state's run
+    if (lane == 0) sum.error |= SAMPO_DEV_ERR_TILECOUNT;
+    return bm;
+  }
+  Acc acc = {0, 0, 0, 0, 0, 0};
+  DecideAcc da;
+  clear_acc(da);
+  Tally t = {0, 0, 0};
+  uint32_t fem = 0, inf = 0;
+#pragma unroll 1
+  for (uint32_t j0 = 0; j0 < n; j0 += 32u) {
+    const uint32_t d = bm + j0 + lane;
+    uint32_t code1 = DEC_DIES;
+    if (j0 + lane < n) {
+      const uint32_t g = ps.moved[warp][j0 + lane];
+      Rec a;
+      load_cols<CS>(w.src, g, a);
+      const uint32_t female = (__ldg(w.src.flags + g) >> 3) & 1u;
+      implied_fields<RG, WIDE>(a);
+      a.female = female;
+      (void)update_agent<true, false, true, true, !WIDE>(w.c, mc.kill, RG, g, a, acc, DEC_MOVES);
+      if (RG == EGG || RG == BMD) {  // the owed normal draw (include/gpuRand.h:56-63)
+        if (a.bm == BM_LARVA_DELAY) a.delay = __uint_as_float(finish_box_muller(w.c, mc, g, BM_LARVA_DELAY, 0u));
+        else if (a.bm == BM_EGG_BATCH) a.avail = finish_box_muller(w.c, mc, g, BM_EGG_BATCH, a.batches);
+      }
+      store_cols<CM>(w.dst, d, a);
+      if (RG >= PUPA && female) {  // statistics of the next pool (kernel/calcGender.cl:24-37)
+        fem += 1u;
+        inf += a.sporo >= 1.0f ? 1u : 0u;
+      }
+      if (AHEAD) code1 = decide<NX, WIDE>(w.c1, mc.kill, d, a, da);
+      put(w.dst.flags + d, NX | (female << 3) | (code1 << 4));
+    }
+    if (AHEAD) add_tally<NX>(w, t, bm + j0, min(n - j0, 32u), d, tally_count(code1));
+  }
+  if (AHEAD) {
+    flush_tally<NX>(w, t);
+    add_decided<NX, NX>(da, sum);
+  }
+  if (RG >= PUPA) add_moved<RG>(fem, inf, acc, sum);
+  return bm + n;
 }
 
 // The update/scatter pass over slots [lo, hi) of range RG. base (lanes 0-7):
-// the next slot of next state `lane` for this warp's survivors; advanced past
+// the next slot of next state `lane` for this warp's survivors; returned past
 // the range's. A survivor's slot is that plus its rank among the survivors
 // of its state in the row (two ballots: an agent stays or moves on to one
 // other state). The survivors of a state are consecutive, so the stores of a
@@ -1086,46 +1194,157 @@ __device__ __forceinline__ void add_tally(const WarpRep& w, Tally& t, uint32_t f
 // inputs and (from this step's decisions) that pool's L1de and size are all
 // known. The decisions go into the flags, their counts to the next pool's
 // spans and supers, and no count pass is needed before the next step.
+template <bool B>
+struct Flag { static constexpr bool value = B; };
 template <int I, bool WIDE, bool AHEAD, int RG>
-__device__ __forceinline__ void scatter_range(const WarpRep& w, const ModelConst& mc, uint8_t* ring, uint32_t lo, uint32_t hi,
-                                              uint32_t& base, MovedEntry* mq, MovedExtra* mx, WarpSum& sum) {
+__device__ __noinline__ uint32_t scatter_range(uint32_t lo, uint32_t hi, uint32_t base) {
   constexpr int NX = next_state(RG);
-  constexpr uint32_t CS = state_cols(RG, WIDE), CM = state_cols(NX, WIDE);
+  constexpr uint32_t CS = state_cols(RG, WIDE);
   using RING = Ring<CS, WIDE ? 2 : 1, I>;
-#ifdef SAMPO_USER_SPECIES
-  constexpr uint32_t OWED = 0;  // the header's draws are made at the transition
-#else
-  constexpr uint32_t OWED = RG == EGG ? (uint32_t)C_DELAY : RG == BMD ? (uint32_t)C_AVAIL : 0u;
-#endif
-  static_assert(RG != BMD || RING::kSlots <= kMovedExtra, "the moved females of a chunk have room");
-  const uint32_t lane = threadIdx.x & 31u, lt = lanemask_lt();
-  const DevPool src = w.src, dst = w.dst;
-  const uint8_t* const dec = WIDE ? w.dec : nullptr;
-  const StepCtx &c = w.c, &c1 = w.c1;
-  const bool ahead = AHEAD && w.ahead;
-  Acc acc = {0, 0, 0, 0, 0, 0};
-  uint32_t fem = 0, inf = 0, bad = 0;
+  constexpr uint32_t ROWS = RING::kSlots / 32;
+  static_assert(RING::kSlots + 31 < kMoved && RING::kSlots <= kSpanMin, "a chunk's moves fit behind the ones that wait; a chunk fills at most two spans");
+  PassShared& ps = pass_shared();
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, lt = lanemask_lt();
+  const WarpRep& w = ps.rep[warp];
+  const ModelConst& mc = ps.mc;
+  uint32_t* const moved = ps.moved[warp];
+  WarpSum& sum = ps.sum[warp];
+  uint32_t bs = __shfl_sync(0xffffffffu, base, RG), bm = __shfl_sync(0xffffffffu, base, NX);
+  const uint32_t es = w.next.r[RG].end, span = hi - lo;
+  Tally ts = {0, 0, 0};
   DecideAcc da;
   clear_acc(da);
-  uint32_t bs = __shfl_sync(0xffffffffu, base, RG), bm = __shfl_sync(0xffffffffu, base, NX);
-  const uint32_t es = w.next.r[RG].end, em = w.next.r[NX].end;
-  Tally ts = {0, 0, 0}, tm = {0, 0, 0};
-  stream_range<RING, CS>(ring, src, src.flags, dec, lo, hi, [&](const uint8_t* st, uint32_t g0) {
-    uint32_t nq = 0;
-    const uint32_t bm0 = bm;
-#pragma unroll kRowUnroll
-    for (uint32_t k = 0; k < RING::kSlots / 32; k++) {
-      const uint32_t i = 32u * k + lane, g = g0 + i;
-      const uint32_t fl = st[RING::kByteOffset + i];
-      uint32_t code = WIDE && dec ? st[RING::kByteOffset + RING::kSlots + i] : (fl >> 4) & 3u;
-      if (g < lo || g >= hi) code = DEC_DIES;
-      uint32_t ms = __ballot_sync(0xffffffffu, code == DEC_STAYS), mm = __ballot_sync(0xffffffffu, code == DEC_MOVES);
-      uint32_t n = __popc(ms);
+  uint32_t bad = 0, qn = 0;  // qn: slots that wait to be moved on
+  // the rows' moves (mm: a row's lanes; g: the lane's slot) into the queue, and out of it
+  auto queue_moves = [&](uint32_t mm, uint32_t g) {
+    if ((mm >> lane) & 1u) moved[qn + __popc(mm & lt)] = g;
+    qn += __popc(mm);
+  };
+  auto move_waiting = [&](bool last) {
+    if (qn >= (last ? 1u : 32u)) {
+      const uint32_t n = last ? qn : qn & ~31u;
+      __syncwarp();
+      bm = move_on<WIDE, AHEAD, RG>(n, bm);
+      qn -= n;
+      __syncwarp();
+      const uint32_t rest = lane < qn ? moved[n + lane] : 0u;
+      __syncwarp();
+      if (lane < qn) moved[lane] = rest;
+    }
+  };
+  if constexpr (AHEAD && !WIDE && RG <= LARVA) {
+    // Eggs and larvae that stay: nearly all of every pool. The same update
+    // and decision as update_agent's, laid out without branches (every lane
+    // computes, the survivors store), a chunk's bookkeeping done once. What
+    // bounds it is the instructions of a row (about 45 and 70).
+    const DevPool src = w.src, dst = w.dst;
+    const uint32_t h13 = w.c1.rng_c13[0], hz2 = w.c1.rng_z2[0], hk4 = w.c1.rng_k4[0], hkill = mc.kill.aquatic;
+    const float hdev = w.c.larvaDev, hdev1 = w.c1.larvaDev;
+    const bool htt = w.c1.tt & (RG == EGG ? TT_EGG : TT_LARVA), hcide = RG == LARVA && w.c1.env.larvacideValue > 0.0f;
+    uint32_t youngest = 0xffffffffu, oldest = 0, hatched = 0, seen = 0;
+    stream_range<RING, CS>(ps.ring[warp], src, src.flags, nullptr, lo, hi, [&](const uint8_t* st, uint32_t g0) {
+      const uint8_t* const stf = st + RING::kByteOffset + lane;
+      const bool whole = g0 >= lo && hi - g0 >= RING::kSlots;
+      auto code_of = [&](uint32_t k) {
+        const uint32_t code = stf[32 * k] & 0x30u;
+        return whole || g0 + 32u * k + lane - lo < span ? code : 0u;
+      };
+      uint32_t ms[ROWS], n = 0, any = 0;
+#pragma unroll
+      for (uint32_t k = 0; k < ROWS; k++) {
+        const uint32_t code = code_of(k);
+        ms[k] = __ballot_sync(0xffffffffu, code == DEC_STAYS << 4);
+        any |= code;
+        n += __popc(ms[k]);
+      }
       if (bs + n > es) {  // no store leaves the state's run
         bad = SAMPO_DEV_ERR_TILECOUNT;
-        ms = n = 0;
+        return;
       }
-      {  // those that stay
+      if (bs >= ts.end) {
+        hatched += ts.cnt >> 16;
+        next_tally<RG>(w, ts, bs);
+      }
+      seen |= n;
+      auto rows = [&](auto crosses) {  // crosses: the chunk's survivors reach past the span's end
+        uint32_t past = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < ROWS; k++) {
+          const uint32_t fl = stf[32 * k];
+          const float* f = reinterpret_cast<const float*>(st) + 32u * k + lane;
+          const float delay = f[RING::offset(C_DELAY) / 4], age = f[RING::offset(C_AGE) / 4] + 1.0f;
+          const float cld = RG == LARVA ? f[RING::offset(C_UNI) / 4] + hdev : 0.0f;
+          const uint32_t d = bs + __popc(ms[k] & lt);
+          const bool live = (ms[k] >> lane) & 1u;
+          bs += __popc(ms[k]);
+          // the step after: mortality, then the transition (update_agent<false>)
+          uint32_t kill = hkill;
+          float q = 0.0f;  // (age + 1/2) / 24: whole_age_days before truncation
+          if (RG == LARVA) {
+            q = __fmul_rn(__fadd_rn(live ? age : 24.0f, 0.5f), 1.0f / 24.0f);
+            const uint32_t days = __float_as_uint(__fadd_rz(q, 8388608.0f)) - 0x4B000000u;
+            kill = w.larvaKill1[days < 99u ? days : 99u];
+            if (live && kill == 0u) da.acc.bad = 1u;
+          }
+          bool lives = live && rng_bits(h13, hz2, hk4, d) >= kill;
+          if (RG == LARVA && hcide) lives = lives && !(age - 23.0f == 1.0f && rng(w.c1, 2, d) <= w.c1.env.larvacideValue);
+          const bool due = htt && (RG == EGG ? age + 1.0f >= delay : cld + hdev1 >= delay);
+          const uint32_t c = lives ? (due ? 1u << 16 : 1u) : 0u;
+          ts.cnt += c;
+          if (crosses.value && d >= ts.end) past += c;
+          if (RG == LARVA && lives && !due) {  // its whole days an hour on (the margin of whole_age_days covers this sum too)
+            const uint32_t days = __float_as_uint(__fadd_rz(__fadd_rn(q, 1.0f / 24.0f), 8388608.0f)) - 0x4B000000u;
+            da.l1 += days;
+            youngest = min(youngest, days);
+            oldest = max(oldest, days);
+          }
+          put_if<RG>(live, dst, d, age, delay, cld, (fl & 15u) | (lives ? (due ? DEC_MOVES << 4 : DEC_STAYS << 4) : 0u));
+        }
+        if (crosses.value) {
+          ts.cnt -= past;
+          hatched += ts.cnt >> 16;
+          next_tally<RG>(w, ts, ts.end);
+          ts.cnt = past;
+        }
+      };
+      if (bs + n > ts.end) rows(Flag<true>{});
+      else rows(Flag<false>{});
+      if (__any_sync(0xffffffffu, any & (DEC_MOVES << 4))) {
+#pragma unroll 1
+        for (uint32_t k = 0; k < ROWS; k++) queue_moves(__ballot_sync(0xffffffffu, code_of(k) == DEC_MOVES << 4), g0 + 32u * k + lane);
+      }
+      move_waiting(hi - g0 <= RING::kSlots);
+    });
+    hatched += ts.cnt >> 16;
+    if (RG == EGG) {  // hatched: 24 hours old
+      da.l1 = hatched;
+      if (hatched) da.dmin = da.dmax = 1u;
+    } else {
+      da.devoob = seen ? w.c1.devOOB : 0u;
+      if (oldest) {
+        da.dmin = min(youngest, 99u);
+        da.dmax = min(oldest, 99u);
+      }
+    }
+  } else {
+    const DevPool &src = w.src, &dst = w.dst;
+    const uint8_t* const dec = WIDE ? w.dec : nullptr;
+    Acc acc = {0, 0, 0, 0, 0, 0};
+    uint32_t fem = 0, inf = 0;
+    stream_range<RING, CS>(ps.ring[warp], src, src.flags, dec, lo, hi, [&](const uint8_t* st, uint32_t g0) {
+#pragma unroll kRowUnroll
+      for (uint32_t k = 0; k < ROWS; k++) {
+        const uint32_t i = 32u * k + lane, g = g0 + i;
+        const uint32_t fl = st[RING::kByteOffset + i];
+        uint32_t code = WIDE && dec ? st[RING::kByteOffset + RING::kSlots + i] : (fl >> 4) & 3u;
+        if (g - lo >= span) code = DEC_DIES;
+        uint32_t ms = __ballot_sync(0xffffffffu, code == DEC_STAYS);
+        const uint32_t mm = __ballot_sync(0xffffffffu, code == DEC_MOVES);
+        uint32_t n = __popc(ms);
+        if (bs + n > es) {  // no store leaves the state's run
+          bad = SAMPO_DEV_ERR_TILECOUNT;
+          ms = n = 0;
+        }
         const uint32_t d = bs + __popc(ms & lt);
         uint32_t code1 = DEC_DIES;
         if ((ms >> lane) & 1u) {
@@ -1133,126 +1352,41 @@ __device__ __forceinline__ void scatter_range(const WarpRep& w, const ModelConst
           read_chunk<RING, CS>(st, i, a);
           implied_fields<RG, WIDE>(a);
           a.female = (fl >> 3) & 1u;
-          (void)update_agent<true, false, true, true, !WIDE>(c, mc.kill, RG, g, a, acc, DEC_STAYS);
+          (void)update_agent<true, false, true, true, !WIDE>(w.c, mc.kill, RG, g, a, acc, DEC_STAYS);
           store_cols<CS>(dst, d, a);
-          // statistics of the next pool (kernel/calcGender.cl:24-37)
-          if (RG >= IMMATURE && a.female) {
+          if (RG >= IMMATURE && a.female) {  // statistics of the next pool (kernel/calcGender.cl:24-37)
             fem += 1u;
             inf += a.sporo >= 1.0f ? 1u : 0u;
           }
-          if (ahead) code1 = decide<RG, WIDE>(c1, mc.kill, d, a, da);
+          if (AHEAD) code1 = decide<RG, WIDE>(w.c1, mc.kill, d, a, da);
           put(dst.flags + d, (fl & 15u) | (code1 << 4));
         }
-        if (ahead) {
-          const uint32_t ks = __ballot_sync(0xffffffffu, code1 == DEC_STAYS), km = __ballot_sync(0xffffffffu, code1 == DEC_MOVES);
-          add_tally<RG>(w, ts, bs, n, ks, km, d);
-        }
+        if (AHEAD) add_tally<RG>(w, ts, bs, n, d, tally_count(code1));
         bs += n;
-      }
-      if (mm) {  // those that move on
-        n = __popc(mm);
-        if (bm + n > em) {
-          bad = SAMPO_DEV_ERR_TILECOUNT;
-          mm = n = 0;
-        }
-        const uint32_t d = bm + __popc(mm & lt);
-        uint32_t code1 = DEC_DIES;
-        if ((mm >> lane) & 1u) {
-          Rec a;
-          read_chunk<RING, CS>(st, i, a);
-          implied_fields<RG, WIDE>(a);
-          a.female = (fl >> 3) & 1u;
-          (void)update_agent<true, false, true, true, !WIDE>(c, mc.kill, RG, g, a, acc, DEC_MOVES);
-          store_cols<(CM & ~OWED)>(dst, d, a);
-          if (RG >= PUPA && a.female) {
-            fem += 1u;
-            inf += a.sporo >= 1.0f ? 1u : 0u;
-          }
-          if (OWED) {
-            const uint32_t j = nq + __popc(mm & lt);
-            mq[j] = MovedEntry{g, a.bm | (a.female << 2)};
-            if (RG == BMD) mx[j] = MovedExtra{a.age, a.avail, a.batches};
-          } else {
-            if (ahead) code1 = decide<NX, WIDE>(c1, mc.kill, d, a, da);
-            put(dst.flags + d, (fl & 8u) | NX | (code1 << 4));
-          }
-        }
-        if (!OWED && ahead) {
-          const uint32_t ks = __ballot_sync(0xffffffffu, code1 == DEC_STAYS), km = __ballot_sync(0xffffffffu, code1 == DEC_MOVES);
-          add_tally<NX>(w, tm, bm, n, ks, km, d);
-        }
-        bm += n;
-        nq += n;
-      }
-      if (RG == GRAVID && code == DEC_TRAPPED) {  // her last hour counts (kernel/updateAgents.cl:247-255)
-        acc.cycles += 1u;
-        acc.sumCycles += reinterpret_cast<const uint32_t*>(st)[RING::offset(C_CYCLE) / 4 + i] + 1u;
-      }
-    }
-    if (OWED && nq) {  // the moved agents' owed draws, decisions and flags, dense over the lanes
-      __syncwarp();
-#pragma unroll 1
-      for (uint32_t j0 = 0; j0 < nq; j0 += 32u) {
-        const uint32_t j = j0 + lane, d = bm0 + j;
-        uint32_t code1 = DEC_DIES;
-        if (j < nq) {
-          const MovedEntry q = mq[j];
-          const uint32_t kind = q.kind & 3u, female = q.kind >> 2;
-          Rec b = Rec{};
-          if (RG == EGG) {
-            b.age = 24.0f;
-            b.delay = __uint_as_float(finish_box_muller(c, mc, q.gid, BM_LARVA_DELAY, 0u));
-            put(dst.delay + d, b.delay);
-          } else {
-            const MovedExtra x = mx[j];
-            b.age = x.age;
-            b.avail = kind != BM_NONE ? finish_box_muller(c, mc, q.gid, kind, x.batches) : x.avail;
-            put(dst.avail + d, b.avail);
-          }
-          b.female = female;
-          if (ahead) code1 = decide<NX, WIDE>(c1, mc.kill, d, b, da);
-          put(dst.flags + d, NX | (female << 3) | (code1 << 4));
-        }
-        if (ahead) {
-          const uint32_t ks = __ballot_sync(0xffffffffu, code1 == DEC_STAYS), km = __ballot_sync(0xffffffffu, code1 == DEC_MOVES);
-          add_tally<NX>(w, tm, bm0 + j0, min(nq - j0, 32u), ks, km, d);
+        if (mm) queue_moves(mm, g);
+        if (RG == GRAVID && code == DEC_TRAPPED) {  // her last hour counts (kernel/updateAgents.cl:247-255)
+          acc.cycles += 1u;
+          acc.sumCycles += reinterpret_cast<const uint32_t*>(st)[RING::offset(C_CYCLE) / 4 + i] + 1u;
         }
       }
-    }
-  });
-  if (ahead) {
-    flush_tally<RG>(w, ts);
-    flush_tally<NX>(w, tm);
+      move_waiting(hi - g0 <= RING::kSlots);
+    });
+    if (RG >= IMMATURE) add_moved<RG>(fem, inf, acc, sum);
   }
-  if (AHEAD) add_decided<RG, NX>(da, sum);
-  if (RG >= PUPA) {
-    uint32_t v[6] = {fem, inf, acc.cycles, acc.sumCycles, acc.bites, acc.infectBites};
-#pragma unroll
-    for (int j = 0; j < 6; j++) v[j] = (j < 2 || RG >= BMS) ? __reduce_add_sync(0xffffffffu, v[j]) : 0u;
-    if (lane == 0) {
-      sum.fem += v[0];
-      sum.inf += v[1];
-#pragma unroll
-      for (int j = 0; j < 4; j++) sum.bnc[j] += v[2 + j];
-    }
+  if (AHEAD) {
+    if (ts.end) flush_tally<RG>(w, ts);
+    add_decided<RG, RG>(da, sum);
   }
   if (bad && lane == 0) sum.error |= bad;
-  if (lane == (uint32_t)RG) base = bs;
-  if (lane == (uint32_t)NX) base = bm;
+  return lane == (uint32_t)RG ? bs : lane == (uint32_t)NX ? bm : base;
 }
 
 template <int I, bool WIDE, bool AHEAD>
 struct ScatterRanges {
-  const WarpRep& w;
-  const ModelConst& mc;
-  uint8_t* ring;
   uint32_t& base;
-  MovedEntry* mq;
-  MovedExtra* mx;
-  WarpSum& sum;
   template <int RG>
   __device__ __forceinline__ void operator()(uint32_t lo, uint32_t hi) {
-    scatter_range<I, WIDE, AHEAD, RG>(w, mc, ring, lo, hi, base, mq, mx, sum);
+    base = scatter_range<I, WIDE, AHEAD, RG>(lo, hi, base);
   }
 };
 
@@ -1262,17 +1396,12 @@ struct ScatterRanges {
 // the super (one 16-byte word per lane). No warp waits for another.
 template <int I, bool WIDE, bool AHEAD>
 __global__ void __launch_bounds__(kBlock, 3) k_scatter(KParams p) {
-  extern __shared__ __align__(16) uint8_t dsm[];  // the warps' rings, then the batch's unit prefix
-  uint32_t* s_pre = reinterpret_cast<uint32_t*>(dsm + kWarps * kRingBytes);
-  uint8_t* ring = dsm + (threadIdx.x >> 5) * kRingBytes;
-  __shared__ WarpRep s_wr[kWarps];
-  __shared__ ModelConst s_mc;
-  __shared__ uint32_t s_w[33];
-  __shared__ MovedEntry s_mq[kWarps][I * 32];
-  __shared__ MovedExtra s_mx[kWarps][kMovedExtra];
+  PassShared& ps = pass_shared();
+  uint32_t* s_pre = reinterpret_cast<uint32_t*>(pass_shared_memory + sizeof(PassShared));
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  load_model_const(p.mc, s_mc);
-  plan_tickets(p.nrep, s_pre, s_w, [&](uint32_t r) -> uint32_t {
+  load_model_const(p.mc, ps.mc);
+  const uint32_t min_span = p.bat->minSpan;
+  plan_tickets(p.nrep, s_pre, ps.scan, [&](uint32_t r) -> uint32_t {
     SimDev* sim = p.reps[r].sim;
     if (!sim->active) return 0u;
     uint32_t cnt[8];
@@ -1283,21 +1412,23 @@ __global__ void __launch_bounds__(kBlock, 3) k_scatter(KParams p) {
       return 0u;
     }
     const uint32_t end = sim->pop.r[GRAVID].end;
-    return span_count(end) + units_of(ne, span_shift(end));
+    const uint32_t span = span_size(end, min_span);
+    return units_of(end, span) + units_of(ne, span);
   });
   __syncthreads();
   const uint32_t total = s_pre[p.nrep], stride = gridDim.x * kWarps;
-  WarpRep& w = s_wr[warp];
-  MovedEntry* mq = s_mq[warp];
-  MovedExtra* mx = s_mx[warp];
+  WarpRep& w = ps.rep[warp];
   uint32_t cur_rep = kNoRep;
-  __shared__ WarpSum s_sum[kWarps];
-  WarpSum& sum = s_sum[warp];
+  WarpSum& sum = ps.sum[warp];
   if (lane == 0) clear_sum(sum);
   // this warp's sums into its replicate's
   auto flush = [&]() {
     if (cur_rep != kNoRep && lane == 0) {
       SimDev* sim = p.reps[cur_rep].sim;
+      if (AHEAD && !w.ahead) {  // (its decisions were taken for nothing)
+        sum.dec = Decided{0u, 0u, 0xffffffffu, 0u};
+        sum.error &= SAMPO_DEV_ERR_TILECOUNT;
+      }
       flush_sum(sum, sim, &sim->ahead_dec);
     }
   };
@@ -1305,7 +1436,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_scatter(KParams p) {
     const uint32_t r = find_rep(s_pre, p.nrep, t);
     if (r != cur_rep) {  // uniform
       flush();
-      load_warp_rep<true, AHEAD>(p.reps[r], w);
+      load_warp_rep<true, AHEAD>(p.reps[r], min_span, w);
       cur_rep = r;
     }
     const uint32_t sp = t - s_pre[r];
@@ -1330,18 +1461,18 @@ __global__ void __launch_bounds__(kBlock, 3) k_scatter(KParams p) {
       const uint32_t b = lane & 7;
       const uint32_t base0 = (b == EGG ? w.newEggs : w.next.r[b].start) + pre + state_count(before, b);
       uint32_t base = base0;
-      const uint32_t end = w.pop.r[GRAVID].end, u0 = sp << w.shift;
-      const uint32_t u1 = end - u0 > (1u << w.shift) ? u0 + (1u << w.shift) : end;
-      for_ranges(w.pop, u0, u1, ScatterRanges<I, WIDE, AHEAD>{w, s_mc, ring, base, mq, mx, sum});
+      const uint32_t end = w.pop.r[GRAVID].end, u0 = sp * w.span;
+      const uint32_t u1 = end - u0 > w.span ? u0 + w.span : end;
+      for_ranges(w.pop, u0, u1, ScatterRanges<I, WIDE, AHEAD>{base});
       // the decisions and their counts must agree on the span's survivors
       const bool differ = __any_sync(0xffffffffu, lane < 8 && base - base0 != state_count(own, b));
       if (differ && lane == 0) sum.error |= SAMPO_DEV_ERR_TILECOUNT;
     } else {
       // ---- new eggs at [0, newEggs) of the next buffer ----
-      const uint32_t e0 = (sp - w.nspans) << w.shift, ne = w.newEggs;
-      const uint32_t e1 = ne - e0 > (1u << w.shift) ? e0 + (1u << w.shift) : ne;
+      const uint32_t e0 = (sp - w.nspans) * w.span, ne = w.newEggs;
+      const uint32_t e1 = ne - e0 > w.span ? e0 + w.span : ne;
       const DevPool dst = w.dst;
-      const bool ahead = AHEAD && w.ahead;
+      constexpr bool ahead = AHEAD;
       Tally ts = {0, 0, 0};
       DecideAcc da;
       clear_acc(da);
@@ -1354,13 +1485,10 @@ __global__ void __launch_bounds__(kBlock, 3) k_scatter(KParams p) {
           new_egg(w.c, id, a);
           store_cols<state_cols(EGG, WIDE)>(dst, id, a);
           const uint32_t female = a.female;
-          if (ahead) code1 = decide<EGG, WIDE>(w.c1, s_mc.kill, id, a, da);
+          if (ahead) code1 = decide<EGG, WIDE>(w.c1, ps.mc.kill, id, a, da);
           put(dst.flags + id, EGG | (female << 3) | (code1 << 4));
         }
-        if (ahead) {
-          const uint32_t ks = __ballot_sync(0xffffffffu, code1 == DEC_STAYS), km = __ballot_sync(0xffffffffu, code1 == DEC_MOVES);
-          add_tally<EGG>(w, ts, r0, min(e1 - r0, 32u), ks, km, id);
-        }
+        if (ahead) add_tally<EGG>(w, ts, r0, min(e1 - r0, 32u), id, tally_count(code1));
       }
       if (ahead) {
         flush_tally<EGG>(w, ts);
@@ -1383,7 +1511,7 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
   return z ^ (z >> 31);
 }
 
-__global__ void k_init_eggs(KParams p, uint32_t n, float T0, const sampo_seeds* seeds, int age_days_max, uint64_t age_seed) {
+__global__ void k_init_eggs(KParams p, uint32_t n, float T0, const sampo_seeds* seeds, int age_days_max, uint64_t age_seed, int full) {
   __shared__ StepCtx c;
   if (threadIdx.x == 0) {
     for (int k = 0; k < 4; k++) {
@@ -1405,7 +1533,7 @@ __global__ void k_init_eggs(KParams p, uint32_t n, float T0, const sampo_seeds* 
       float h = 24.0f * (float)(uint32_t)((z >> 32) % ((uint64_t)age_days_max + 1));
       a.age = h; a.his = h;
     }
-    if (p.wide) store_cols<C_ALL>(dst, id, a);
+    if (full) store_cols<C_ALL>(dst, id, a);
     else store_cols<state_cols(EGG, false)>(dst, id, a);
     dst.flags[id] = (uint8_t)(EGG | (a.female << 3));
   }
