@@ -1,5 +1,6 @@
 """Generate sampo_fast_tables.h: the breakpoint tables of the binary32 fast
-paths in sampo_math_fast.h (log on (0, 1], sin on [0, 2*pi]).
+paths in sampo_math_fast.h (log on (0, 1], sin on [0, 2*pi], exp on
+[-3/32, 71/32)).
 
 Every entry is computed with mpmath at 300 bits and rounded once to binary32
 (round to nearest even), so the header is the same wherever it is made.
@@ -12,6 +13,8 @@ Every entry is computed with mpmath at 300 bits and rounded once to binary32
   sin table, 513 entries for k = 0..512, x_k = k * pi / 256:
       Ph + Pm + Pl = x_k as an unevaluated binary32 triple
       Sh + Sl = sin(x_k),  Ch + Cl = cos(x_k)  (exact 0 and +-1 where they are)
+  exp table, 75 entries for i = -3..71, x_i = i / 32:
+      Eh + El = exp(x_i) (exactly 1 for i = 0)
   constants: ln 2 = LN2_A + LN2_B + LN2_C with A and B of 16 significant
       bits (k * A and k * B are exact for |k| < 256); 256/pi.
 
@@ -105,6 +108,10 @@ def sin_table():
     return rows
 
 
+def exp_table():
+    return [split2(mp.exp(mp.mpf(i) / 32)) for i in range(-3, 72)]
+
+
 def main():
     out = os.path.join(os.path.dirname(os.path.abspath(__file__)), "sampo_fast_tables.h")
     lines = [
@@ -125,6 +132,9 @@ def main():
               "#define SAMPO_SIN_TABLE_INIT { \\"]
     for a, b in sin_table():
         lines.append("  {{" + ", ".join(lit(v) for v in a) + "}, {" + ", ".join(lit(v) for v in b) + "}}, \\")
+    lines += ["}", "", "/* {Eh, El} = exp(i / 32), i = -3..71 */", "#define SAMPO_EXP_TABLE_INIT { \\"]
+    for r in exp_table():
+        lines.append("  {" + ", ".join(lit(v) for v in r) + "}, \\")
     lines += ["}", "", "#endif", ""]
     with open(out, "w") as f:
         f.write("\n".join(lines))

@@ -1,11 +1,13 @@
 /*
- * sampo_math_fast.h - binary32-only evaluations of three binary64 results
- * of the SAMPO model, for the GPU, where binary64 instructions issue at a
- * small fraction of the binary32 rate.
+ * sampo_math_fast.h - binary32-only evaluations of binary64 results of the
+ * SAMPO model, for the GPU, where binary64 instructions issue at a small
+ * fraction of the binary32 rate.
  *
  *   sampo_logf_bm(x)  = sampo_logf(x)   for the normal draw's log
  *   sampo_sinf_bm(x)  = sampo_sinf(x)   for the normal draw's sin
  *                                       (include/gpuRand.h:56-63)
+ *   sampo_larva_hmr() = the larvae's hourly mortality, an expf and a powf
+ *                       (kernel/killAgents.cl:117-125)
  *   sampo_sporo_add() = (float)((double)s + d), the sporogonic development
  *                       update done in double (kernel/updateAgents.cl:69-70)
  *
@@ -20,8 +22,10 @@
  * also the definition's result. Otherwise the binary64 definition itself is
  * evaluated. The error bounds were measured over every input of the domains
  * the model produces (log: x in {0} and [2^-32, 1]; sin: x = fl(2*pi_f * u)
- * for those u), and tests/fastmath_check.c checks that the results equal the
- * binary64 definitions bit for bit on those domains.
+ * for those u; the mortality: its exp for every float in [0, 2.2), its pow for
+ * every float in [0.15, 1)). tests/fastmath_check.c and tests/mortality_check.c
+ * check that the results equal the binary64 definitions bit for bit on those
+ * domains.
  *
  * Compile with FP contraction off (-ffp-contract=off / --fmad=false): the
  * transformations rely on every + and * rounding separately.
@@ -35,19 +39,24 @@
 #if defined(__CUDACC__)
 static __device__ __align__(16) const float sampo_log_tab_d[128][4] = SAMPO_LOG_TABLE_INIT;
 static __device__ __align__(16) const float sampo_sin_tab_d[513][2][4] = SAMPO_SIN_TABLE_INIT;
+static __device__ __align__(16) const float sampo_exp_tab_d[75][2] = SAMPO_EXP_TABLE_INIT;
 #endif
 #if !defined(__CUDA_ARCH__)
 static const float sampo_log_tab_h[128][4] __attribute__((aligned(16))) = SAMPO_LOG_TABLE_INIT;
 static const float sampo_sin_tab_h[513][2][4] __attribute__((aligned(16))) = SAMPO_SIN_TABLE_INIT;
+static const float sampo_exp_tab_h[75][2] __attribute__((aligned(16))) = SAMPO_EXP_TABLE_INIT;
 #endif
 
 /* Relative error bounds of H + L, each at least 4 times the largest error
- * measured over the whole domain (log 2^-40.12, sin 2^-38.75) plus 2^-48 for
- * the binary64 definition; the add's bound follows from its two roundings
- * (below 2^-45) and the double rounding of the definition (2^-52). */
+ * measured over the whole domain (log 2^-40.12, sin 2^-38.75, exp 2^-42.11,
+ * pow 2^-40.24) plus 2^-48 for the binary64 definition; the add's bound
+ * follows from its two roundings (below 2^-45) and the double rounding of the
+ * definition (2^-52). */
 #define SAMPO_FAST_LOG_EPS 0x1p-38f
 #define SAMPO_FAST_SIN_EPS 0x1p-36f
 #define SAMPO_FAST_ADD_EPS 0x1p-40f
+#define SAMPO_FAST_EXP_EPS 0x1p-40f
+#define SAMPO_FAST_POW_EPS 0x1p-38f
 
 SAMPO_HD float sampo_fmaf(float a, float b, float c) {
 #if defined(__CUDA_ARCH__)
@@ -163,6 +172,62 @@ SAMPO_HD int sampo_sin_pair(float x, float* H, float* L) {
   const float lo = ((e1 + e2) + p1e) + ((small - t4) + (t5 + t6));
   sampo_two_sum(s2, lo, H, L);
   return 1;
+}
+
+/* exp(x + xl) as H + L for x in [-3/32, 71/32), |xl| < 2^-24; 0 for other x. */
+SAMPO_HD int sampo_exp_pair(float x, float xl, float* H, float* L) {
+  if (!(x >= -0.09375f && x < 2.21875f)) return 0;      /* also NaN */
+  /* i = nearest integer to 32 x; r = x - i/32 exactly, |r| <= 2^-6 */
+  const float fi = (x * 32.0f + 12582912.0f) - 12582912.0f;
+  const uint32_t i = (uint32_t)((int32_t)fi + 3);
+  const float r = x - fi * 0.03125f;
+  float eh, el;
+#if defined(__CUDA_ARCH__)
+  const float2 e = __ldg(reinterpret_cast<const float2*>(sampo_exp_tab_d[i]));
+  eh = e.x; el = e.y;
+#else
+  eh = sampo_exp_tab_h[i][0]; el = sampo_exp_tab_h[i][1];
+#endif
+  /* exp(r) - 1 = r + r^2/2 + r^3 (1/6 + r/24 + r^2/120 + r^3/720) */
+  const float zh = r * r;
+  const float ze = sampo_fmaf(r, r, -zh);
+  const float tail = (r * zh) * (0x1.555556p-3f + r * (0x1.555556p-5f + r * (0x1.111112p-7f + r * 0x1.6c16c2p-10f)));
+  float uh, ul;
+  sampo_two_sum(r, 0.5f * zh, &uh, &ul);
+  ul = ul + ((0.5f * ze + tail) + (xl + xl * r));
+  /* E (1 + u) */
+  const float p = eh * uh;
+  const float pe = sampo_fmaf(eh, uh, -p);
+  float s, e1;
+  sampo_two_sum(eh, p, &s, &e1);
+  const float lo = (e1 + pe) + ((el + el * uh) + eh * ul);
+  sampo_two_sum(s, lo, H, L);
+  return 1;
+}
+
+/* sampo_powf(x, y) for the mortality's x in [0.15, 1) and y = 1/24. */
+SAMPO_HD float sampo_powf_hourly(float x) {
+  const float y = 1.0f / 24.0f;
+  float h, l, H, L, f;
+  if (x >= 0.15f && x < 1.0f && sampo_log_pair(x, &h, &l)) {
+    const float zh = y * h;
+    const float zl = sampo_fmaf(y, h, -zh) + y * l;
+    if (sampo_exp_pair(zh, zl, &H, &L) && sampo_round_test(H, L, SAMPO_FAST_POW_EPS, &f)) return f;
+  }
+  return sampo_powf(x, y);
+}
+SAMPO_HD float sampo_expf_hourly(float x) {
+  float H, L, f;
+  if (x >= 0.0f && sampo_exp_pair(x, 0.0f, &H, &L) && sampo_round_test(H, L, SAMPO_FAST_EXP_EPS, &f)) return f;
+  return sampo_expf(x);
+}
+
+/* The hourly mortality of larvae whose daily one is 0.1 exp(x), at most 0.8:
+ *   dmr = fminf(0.1f * expf(x), 0.8f); 1 - powf(1 - dmr, 1/24)
+ * (past x = 2.2 the daily mortality is 0.8, and for a NaN, as in fminf). */
+SAMPO_HD float sampo_larva_hmr(float x) {
+  const float dmr = x < 2.2f ? sampo_fminf(0.1f * sampo_expf_hourly(x), 0.8f) : 0.8f;
+  return 1.0f - sampo_powf_hourly(1.0f - dmr);
 }
 
 SAMPO_HD float sampo_logf_bm(float x) {

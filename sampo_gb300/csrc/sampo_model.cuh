@@ -161,8 +161,11 @@ __host__ __device__ __forceinline__ uint32_t kill_threshold(float hmr) {
   if (!(h < 4294967040.0f)) return 0xffffffffu;
   const uint32_t n = (uint32_t)h;
   if (h < 16777216.0f) return n + 1u;
-  uint32_t half = 1u;  // half a unit in the last place of h
-  for (uint32_t m = n >> 25; m; m >>= 1) half <<= 1;
+#if defined(__CUDA_ARCH__)
+  const uint32_t half = 1u << (7 - __clz(n));  // half a unit in the last place of h
+#else
+  const uint32_t half = 1u << (7 - __builtin_clz(n));
+#endif
   return n + half + ((n / (2u * half)) & 1u ? 0u : 1u);
 }
 
