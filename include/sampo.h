@@ -201,8 +201,7 @@ int sampo_items_per_thread(sampo_sim* s, uint32_t* items);
  * hour. Both give the same results at any size. SAMPO_SMALL_STEP_DEFAULT:
  * the largest co-resident grid of the one-launch kernel, one tile per CTA
  * (the default); 0: never. sampo_run_async picks by the size seen at its
- * call; sampo_step, runs with timing on and a run-time species
- * (sampo_set_species) always take the three-kernel step. */
+ * call; sampo_step and runs with timing on always take the three-kernel step. */
 #define SAMPO_SMALL_STEP_DEFAULT 0xffffffffu
 int sampo_set_small_step(sampo_sim* s, uint32_t max_tiles);
 /* Slots per thread of the one-launch step: 0 (the default) takes the

@@ -26,7 +26,8 @@ NVFLAGS = ARCH + ["-O3", "--fmad=false", "-prec-div=true", "-prec-sqrt=true", "-
 SOURCES = ["sampo_kernels.cu", "sampo_api.cu", "sampo_batch.cu", "sampo_host.cpp", "sampo_noalloc.cu", "sampo_species.cu"]
 # the device sources a user species is compiled with at run time, under the
 # names their #include lines use (embedded as text by jit_sources())
-JIT_HEADERS = [("sampo_step_kernels.cuh", "sampo_step_kernels.cuh"), ("sampo_kernels.cuh", "sampo_kernels.cuh"),
+JIT_HEADERS = [("sampo_step_kernels.cuh", "sampo_step_kernels.cuh"), ("sampo_small_step.cuh", "sampo_small_step.cuh"),
+               ("sampo_kernels.cuh", "sampo_kernels.cuh"),
                ("sampo_model.cuh", "sampo_model.cuh"), ("sampo_species.cuh", "sampo_species.cuh"),
                ("sampo_species_prelude.h", "sampo_species_prelude.h"), ("sampo_math.h", "sampo_math.h"),
                ("sampo_math_fast.h", "sampo_math_fast.h"), ("sampo_fast_tables.h", "sampo_fast_tables.h"),

@@ -6,6 +6,7 @@
 // the process; errors come back as status codes with a message in
 // sampo_last_error.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <string.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -63,6 +64,7 @@ struct sampo_sim {
   // per day from the pool end the host last saw (known_end).
   int small_grid = 0;                  // largest grid of the one-launch step (0: it cannot run on this device)
   uint32_t small_tiles = 0;            // largest pool in 1024-slot tiles that takes the one-launch step (0: never)
+  bool small_default = true;           // small_tiles follows small_grid
   int small_items = 0;                 // its slots per thread: 1, 2, 4, or 0 (by pool size)
   cudaGraphExec_t small_graph[3][8] = {};  // [256-, 512-, 1024-slot tiles][grid bucket]
   int small_graph_kind[3][8] = {};     // DG_* of each
@@ -91,6 +93,13 @@ constexpr uint32_t kSmallGrowth = 2;
 static uint32_t small_bucket_grid(const sampo_sim* s, int b) {
   const uint32_t g = 8u << b;
   return (b == kSmallBuckets - 1 || g >= (uint32_t)s->small_grid) ? (uint32_t)s->small_grid : g;
+}
+
+// The one-launch step's largest grid with the simulation's species, and by
+// default one tile per CTA of it as the largest pool that takes it.
+static void size_small_step(sampo_sim* s) {
+  s->small_grid = std::min({grid_blocks_small(1, s->species), grid_blocks_small(2, s->species), grid_blocks_small(4, s->species)});
+  if (s->small_default) s->small_tiles = s->small_grid > 0 ? (uint32_t)s->small_grid : 0u;
 }
 
 static int fail(sampo_sim* s, int code, const std::string& msg) {
@@ -246,8 +255,7 @@ extern "C" int sampo_create(const sampo_config* cfg, sampo_sim** out) {
     }
     s->grid_count = grid_blocks_count(1);
     s->grid_scatter = grid_blocks_scatter(1);
-    s->small_grid = std::min(grid_blocks_small(1), std::min(grid_blocks_small(2), grid_blocks_small(4)));
-    s->small_tiles = s->small_grid > 0 ? (uint32_t)s->small_grid : 0u;  // one tile per CTA
+    size_small_step(s);
     if ((e = cudaMallocHost(&s->end_pinned, 2 * sizeof(uint32_t))) != cudaSuccess) { rc = cuda_fail(s, e, "pinned"); break; }
     for (auto& ev : s->ev_day) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     for (auto& ev : s->ev) cudaEventCreate(&ev);
@@ -535,7 +543,7 @@ static cudaError_t build_small_graph(sampo_sim* s, int items, int b) {
 static int day_graph_for(sampo_sim* s, cudaGraphExec_t* gx, uint32_t* kernels, int* kind) {
   const uint32_t end = s->known_end;
   const uint32_t t4 = (end + kTile - 1) / kTile;
-  if (!s->species && s->small_grid > 0 && s->small_tiles > 0 && t4 <= s->small_tiles) {
+  if (s->small_grid > 0 && s->small_tiles > 0 && t4 <= s->small_tiles) {
     auto tiles_of = [&](int items) { const uint32_t t = (end + kBlock * items - 1) / (kBlock * items); return t ? t : 1u; };
     int items = s->small_items;
     if (items == 0) {
@@ -565,7 +573,8 @@ static int day_graph_for(sampo_sim* s, cudaGraphExec_t* gx, uint32_t* kernels, i
 extern "C" int sampo_set_small_step(sampo_sim* s, uint32_t max_tiles) {
   if (!s) return SAMPO_ERR_ARG;
   SETTLE(s);
-  if (max_tiles == SAMPO_SMALL_STEP_DEFAULT) max_tiles = s->small_grid > 0 ? (uint32_t)s->small_grid : 0u;
+  s->small_default = max_tiles == SAMPO_SMALL_STEP_DEFAULT;
+  if (s->small_default) max_tiles = s->small_grid > 0 ? (uint32_t)s->small_grid : 0u;
   s->small_tiles = max_tiles;
   return SAMPO_OK;
 }
@@ -652,7 +661,7 @@ static int queue_run(sampo_sim* s, uint32_t nsteps, sampo_stats_row* rows, bool 
       // with the one-launch step available, a waiting run learns the pool end
       // after each day one day behind the queue (the GPU keeps the next day
       // queued meanwhile) and picks each day's graph from it
-      const bool track = wait && !s->species && s->small_grid > 0 && s->small_tiles > 0;
+      const bool track = wait && s->small_grid > 0 && s->small_tiles > 0;
       for (uint32_t day = 0; i + 24 <= n; i += 24, day++) {
         cudaGraphExec_t gx = nullptr;
         uint32_t kernels = 0;
@@ -956,6 +965,8 @@ extern "C" int sampo_set_species(sampo_sim* s, const sampo_species* sp) {
   s->grid_count = grid_blocks_count(1, sp, s->items, s->wide);
   s->grid_scatter = grid_blocks_scatter(1, sp, s->items, s->wide);
   drop_day_graph(s);  // captured with the other kernels
+  drop_small_graphs(s);
+  size_small_step(s);
   return SAMPO_OK;
 }
 

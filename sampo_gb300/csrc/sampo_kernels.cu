@@ -249,11 +249,13 @@ cudaError_t tune_grids(const KParams& p, cudaStream_t st, int* grid_count, int* 
   if (best_ms) *best_ms = best;
   return e;
 }
+static int small_kid(int items) { return items == 1 ? KID_SMALL1 : items == 2 ? KID_SMALL2 : KID_SMALL4; }
 static const void* small_fn(int items) {
   return items == 1 ? (const void*)k_step_small<1> : items == 2 ? (const void*)k_step_small<2> : (const void*)k_step_small<4>;
 }
-int grid_blocks_small(int items) {
+int grid_blocks_small(int items, const void* ks) {
   int per = 0;
+  if (ks) return sm_count() * species_occupancy(ks, small_kid(items), kSmallThreads, small_stage(items));
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, small_fn(items), kSmallThreads, small_stage(items)) != cudaSuccess) {
     (void)cudaGetLastError();
     return 0;
@@ -279,6 +281,8 @@ cudaError_t graph_kernel_nodes(cudaGraph_t g, uint32_t* kernels) {
 cudaError_t launch_small(const KParams& p, int grid, bool cooperative, uint32_t nsteps, cudaStream_t st, int items) {
   KParams q = p;
   void* args[] = {&q, &nsteps};
+  if (p.ks)
+    return species_launch(p.ks, small_kid(items), dim3(grid), dim3(kSmallThreads), small_stage(items), st, args, cooperative);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kSmallThreads);

@@ -81,6 +81,9 @@ struct BatchDev {
   uint32_t done;              // one-launch step: CTAs finished (reset by its last CTA)
 };
 
+// Words of the one-launch step's rows per tile (sampo_small_step.cuh).
+constexpr uint32_t kSmallRowWords = 18;
+
 // Spans: the slots a warp of the two passes takes at once, a multiple of 32.
 // A span costs a warp about a thousand instructions besides its rows (its
 // prefix, the start and end of its range, the agents that move on in a
@@ -219,9 +222,10 @@ int grid_blocks_scatter(uint32_t nrep, const void* ks = nullptr, int items = kIt
 // resident CTAs per SM.
 enum : int {
   KID_COUNT, KID_SCATTER, KID_COUNT_WIDE, KID_SCATTER_WIDE, KID_PUBLISH, KID_INIT_EGGS, KID_POOL_STATS, KID_HISTOGRAM,
-  KID_TRIAL_RESET, KID_WIDEN, KID_N
+  KID_TRIAL_RESET, KID_WIDEN, KID_SMALL1, KID_SMALL2, KID_SMALL4, KID_N
 };
-cudaError_t species_launch(const void* ks, int kid, dim3 grid, dim3 block, size_t smem, cudaStream_t st, void** args);
+cudaError_t species_launch(const void* ks, int kid, dim3 grid, dim3 block, size_t smem, cudaStream_t st, void** args,
+                           bool cooperative = false);
 int species_occupancy(const void* ks, int kid, int threads, size_t smem);
 // dynamic shared memory the two passes may request
 size_t pass_smem_max();
@@ -252,13 +256,11 @@ cudaError_t launch_histogram(const KParams& p, uint32_t* hist_dev, cudaStream_t 
 cudaError_t launch_eval_math(int fn, const float* x, const float* y, float* out, uint32_t n, cudaStream_t st);
 // Kernel nodes in a captured graph (the launches one replay makes).
 cudaError_t graph_kernel_nodes(cudaGraph_t g, uint32_t* kernels);
-// Words of the one-launch step's rows per tile (sampo_small_step.cuh).
-constexpr uint32_t kSmallRowWords = 18;
 // The one-launch steps of a single simulation (sampo_small_step.cuh) with
-// tiles of kBlock * items slots (items 1, 2 or 4): the largest grid (CTAs
-// resident on all SMs, 0 if it cannot run) and a launch of `nsteps` hourly
+// tiles of kBlock * items slots (items 1, 2 or 4), built in or of ks: the
+// largest grid (CTAs resident on all SMs, 0 if it cannot run) and a launch of `nsteps` hourly
 // steps (a cooperative launch when `cooperative`) on `grid` CTAs.
-int grid_blocks_small(int items = kItems);
+int grid_blocks_small(int items = kItems, const void* ks = nullptr);
 cudaError_t launch_small(const KParams& p, int grid, bool cooperative, uint32_t nsteps, cudaStream_t st,
                          int items = kItems);
 // Times count + scatter of the coming step for each number of rows at once

@@ -321,7 +321,11 @@ __device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& m
       }
       return BMD;
     default: {  // GRAVID
+#ifdef SAMPO_USER_SPECIES
+      a.cycle += 1u;  // (the header's layEggs may read it)
+#else
       if (FULL) a.cycle += 1u;
+#endif
       // a trapped gravid loses her eggs and dies, so a decided one was not trapped
       if (DECIDED && moves) {  // she has laid her last eggs
         if (FULL) {
