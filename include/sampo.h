@@ -201,7 +201,8 @@ int sampo_items_per_thread(sampo_sim* s, uint32_t* items);
  * hour. Both give the same results at any size. SAMPO_SMALL_STEP_DEFAULT:
  * the largest co-resident grid of the one-launch kernel, one tile per CTA
  * (the default); 0: never. sampo_run_async picks by the size seen at its
- * call; sampo_step and runs with timing on always take the three-kernel step. */
+ * call, sampo_step by the size at its hour (one launch of one hourly step);
+ * with timing on both always take the three-kernel step. */
 #define SAMPO_SMALL_STEP_DEFAULT 0xffffffffu
 int sampo_set_small_step(sampo_sim* s, uint32_t max_tiles);
 /* Slots per thread of the one-launch step: 0 (the default) takes the
@@ -288,10 +289,10 @@ int sampo_read_environment_file(const char* path, sampo_environment* out, uint32
  * code running where allocation is forbidden or unsafe (inside another
  * framework's memory pool or arena, a host that must not grow device memory
  * after start-up, a memory-capped sandbox). They bring their own pool
- * buffers; the step's scratch (step state, per-tile prefix tables and
- * look-back counts, one step of inputs and stats) lives in a fixed array
+ * buffers; the step's scratch (step state, decisions and span counts or a small
+ * pool's rows, one step of inputs and stats) lives in a fixed array
  * inside the library, sized for pools of up to SAMPO_NOALLOC_MAX_SLOTS slots
- * (about 15 MB, held by every GPU that loads the library until the process
+ * (about 18 MB, held by every GPU that loads the library until the process
  * exits).
  *
  * in/out: device columns of two pool buffers; each column 16-byte aligned

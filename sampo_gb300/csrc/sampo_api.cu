@@ -70,6 +70,7 @@ struct sampo_sim {
   int small_graph_kind[3][8] = {};     // DG_* of each
   uint32_t known_end = 0;              // pool end at the start of the coming day, as last seen by the host
   uint32_t* end_pinned = nullptr;      // pool end after a day, copied back one day behind the queue
+  SimDev* status = nullptr;            // page-locked: the state's head (kStatusBytes), as check_device last read it
   cudaEvent_t ev_day[2] = {nullptr, nullptr};
   int last_day_kind = 0;               // DG_* of the last day launched
   uint64_t days_small = 0, days_three = 0;
@@ -98,7 +99,7 @@ static uint32_t small_bucket_grid(const sampo_sim* s, int b) {
 // The one-launch step's largest grid with the simulation's species, and by
 // default one tile per CTA of it as the largest pool that takes it.
 static void size_small_step(sampo_sim* s) {
-  s->small_grid = std::min({grid_blocks_small(1, s->species), grid_blocks_small(2, s->species), grid_blocks_small(4, s->species)});
+  s->small_grid = grid_blocks_small_all(s->species);
   if (s->small_default) s->small_tiles = s->small_grid > 0 ? (uint32_t)s->small_grid : 0u;
 }
 
@@ -170,6 +171,7 @@ extern "C" int sampo_destroy(sampo_sim* s) {
     for (auto& g : row) if (g) cudaGraphExecDestroy(g);
   for (auto& e : s->ev_day) if (e) cudaEventDestroy(e);
   if (s->end_pinned) cudaFreeHost(s->end_pinned);
+  if (s->status) cudaFreeHost(s->status);
   for (auto& e : s->ev) if (e) cudaEventDestroy(e);
   cudaFree(s->pool_mem[0]); cudaFree(s->pool_mem[1]);
   cudaFree(s->sim_dev); cudaFree(s->span_mem); cudaFree(s->small_mem);
@@ -256,7 +258,8 @@ extern "C" int sampo_create(const sampo_config* cfg, sampo_sim** out) {
     s->grid_count = grid_blocks_count(1);
     s->grid_scatter = grid_blocks_scatter(1);
     size_small_step(s);
-    if ((e = cudaMallocHost(&s->end_pinned, 2 * sizeof(uint32_t))) != cudaSuccess) { rc = cuda_fail(s, e, "pinned"); break; }
+    if ((e = cudaMallocHost(&s->end_pinned, 2 * sizeof(uint32_t))) != cudaSuccess ||
+        (e = cudaMallocHost(&s->status, sizeof(SimDev))) != cudaSuccess) { rc = cuda_fail(s, e, "pinned"); break; }
     for (auto& ev : s->ev_day) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     for (auto& ev : s->ev) cudaEventCreate(&ev);
     if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) { rc = cuda_fail(s, e, "create"); break; }
@@ -354,11 +357,11 @@ static void set_wide(sampo_sim* s, bool wide) {
   drop_small_graphs(s);
 }
 
-// Statistics and publish of the pool the caller has just put in buffer 0;
+// Statistics and publish of the pool, of that end, that the caller has just put in buffer 0;
 // `loaded`: its records come from outside and may be wide.
-static int publish_initial(sampo_sim* s, bool loaded) {
+static int publish_initial(sampo_sim* s, uint32_t end, bool loaded) {
   KParams p = make_params(s);
-  CK(launch_publish_start(p, loaded, s->stream), "initial statistics");
+  CK(launch_publish_start(p, loaded ? (uint32_t)PS_CHECK : 0u, end, s->stream), "initial statistics");
   CK(cudaMemcpyAsync(s->end_pinned, &s->sim_dev->pop.r[GRAVID].end, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream),
      "initial statistics");
   CK(cudaMemcpyAsync(s->end_pinned + 1, &s->sim_dev->wide, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream),
@@ -396,7 +399,7 @@ extern "C" int sampo_init_population(sampo_sim* s, uint32_t n, const sampo_seeds
   // the one-launch step reads whole records: a pool it will step gets them at once
   s->full_cols = n <= s->small_tiles * (uint64_t)kTile;
   CK(launch_init_eggs(p, n, s->T_host[0], s->init_seeds_dev, age_days_max, age_seed, s->full_cols, s->stream), "initAgents");
-  return publish_initial(s, false);
+  return publish_initial(s, pop.r[7].end, false);
 }
 
 extern "C" int sampo_load_pool(sampo_sim* s, const sampo_population* pop, const sampo_pool_view* v) {
@@ -425,24 +428,29 @@ extern "C" int sampo_load_pool(sampo_sim* s, const sampo_population* pop, const 
   CK(cudaMemcpyAsync(P.flags, flags.data(), n, cudaMemcpyHostToDevice, s->stream), "pool upload");
   CK(cudaStreamSynchronize(s->stream), "pool upload");
   s->full_cols = true;
-  return publish_initial(s, true);
+  return publish_initial(s, n, true);
 }
 
+constexpr size_t kStatusBytes = offsetof(SimDev, capacity);
 static int check_device(sampo_sim* s) {
-  uint32_t st[2];
-  CK(cudaMemcpyAsync(st, &s->sim_dev->error, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream), "status");
-  CK(cudaMemcpyAsync(s->end_pinned, &s->sim_dev->pop.r[GRAVID].end, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream), "status");
+  CK(cudaMemcpyAsync(s->status, s->sim_dev, kStatusBytes, cudaMemcpyDeviceToHost, s->stream), "status");
   CK(cudaStreamSynchronize(s->stream), "status");
-  s->known_end = s->end_pinned[0];  // the pool end the coming day's graph is picked by
-  if (st[0] & SAMPO_DEV_ERR_CAPACITY) return fail(s, SAMPO_ERR_CAPACITY, "not enough capacity for the next layout");
-  if (st[0] & SAMPO_DEV_ERR_DEVRATES) return fail(s, SAMPO_ERR_TEMPERATURE, "temperature >= 44 C: the reference reads past devRates");
-  if (st[0]) return fail(s, SAMPO_ERR_INTERNAL, "device consistency check failed (bits " + std::to_string(st[0]) + ")");
+  s->known_end = s->status->pop.r[GRAVID].end;  // the pool end the coming day's graph is picked by
+  const uint32_t error = s->status->error;
+  if (error & SAMPO_DEV_ERR_CAPACITY) return fail(s, SAMPO_ERR_CAPACITY, "not enough capacity for the next layout");
+  if (error & SAMPO_DEV_ERR_DEVRATES) return fail(s, SAMPO_ERR_TEMPERATURE, "temperature >= 44 C: the reference reads past devRates");
+  if (error) return fail(s, SAMPO_ERR_INTERNAL, "device consistency check failed (bits " + std::to_string(error) + ")");
   return SAMPO_OK;
 }
 
 static cudaError_t launch_hours(sampo_sim* s, const KParams& p, uint32_t nsteps, uint32_t* launches) {
   s->full_cols = false;
   return launch_steps(p, nsteps, true, s->grid_count, s->grid_scatter, s->items, s->stream, launches);
+}
+
+// Whether the pool the host last saw is of a size the one-launch step takes.
+static bool takes_small_step(const sampo_sim* s) {
+  return s->small_grid > 0 && s->small_tiles > 0 && units_of(s->known_end, (uint32_t)kTile) <= s->small_tiles;
 }
 
 extern "C" int sampo_step(sampo_sim* s, const sampo_environment* env, float temperature, uint32_t world_time,
@@ -453,22 +461,33 @@ extern "C" int sampo_step(sampo_sim* s, const sampo_environment* env, float temp
   if (env->carryingCapacity != s->cc) return fail(s, SAMPO_ERR_ARG, "environment carryingCapacity differs from the configured carrying capacity");
   cudaSetDevice(s->device);
   const uint32_t slot = s->step % s->ring;
-  CK(cudaMemcpyAsync(s->T_dev + slot, &temperature, sizeof(float), cudaMemcpyHostToDevice, s->stream), "step inputs");
-  CK(cudaMemcpyAsync(s->env_dev + slot, env, sizeof(sampo_environment), cudaMemcpyHostToDevice, s->stream), "step inputs");
-  CK(cudaMemcpyAsync(s->wt_dev + slot, &world_time, sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream), "step inputs");
-  CK(cudaMemcpyAsync(s->seeds_dev + (size_t)slot * 4, seeds, 4 * sizeof(sampo_seeds), cudaMemcpyHostToDevice, s->stream), "step inputs");
+  CtxInputs in;
+  memcpy(in.sd, seeds, sizeof(in.sd));
+  in.env = *env;
+  in.T = temperature;
+  in.wt = world_time;
   s->T_host[slot] = temperature;
   s->have_inputs[slot] = 1;
   s->input_step[slot] = s->step;
   s->seed_step[slot] = s->step;
-  if (row) CK(cudaMemcpyAsync(row, s->rows_dev + slot, sizeof(sampo_stats_row), cudaMemcpyDeviceToHost, s->stream), "row");
   KParams p = make_params(s);
-  CK(launch_publish(p, PUB_REFRESH, s->stream), "step constants");  // this step's inputs were just written
-  uint32_t n = 1;  // the refresh
-  CK(launch_hours(s, p, 1, &n), "step kernels");
+  uint32_t n = 1;
+  if (!s->timing && takes_small_step(s)) {
+    // (the pool's end is exact here: the tiles need no room to grow)
+    CK(widen(s), "whole records");
+    CK(launch_begin_step(p, in, slot, s->stream), "step inputs");
+    const int items = s->small_items ? s->small_items : small_items_for(s->known_end, 1, s->small_grid);
+    CK(launch_small_hour(p, s->known_end, items, s->small_grid, s->stream), "one-launch step");
+    n++;
+  } else {
+    CK(launch_begin_step(p, in, slot, s->stream), "step inputs");
+    CK(launch_hours(s, p, 1, &n), "step kernels");
+  }
   s->launches += n;
   s->step++;
-  return check_device(s);
+  const int rc = check_device(s);
+  if (row) *row = s->status->begun;
+  return rc;
 }
 
 static int build_day_graph(sampo_sim* s) {
@@ -542,16 +561,9 @@ static cudaError_t build_small_graph(sampo_sim* s, int items, int b) {
 // extra-tile route.
 static int day_graph_for(sampo_sim* s, cudaGraphExec_t* gx, uint32_t* kernels, int* kind) {
   const uint32_t end = s->known_end;
-  const uint32_t t4 = (end + kTile - 1) / kTile;
-  if (s->small_grid > 0 && s->small_tiles > 0 && t4 <= s->small_tiles) {
-    auto tiles_of = [&](int items) { const uint32_t t = (end + kBlock * items - 1) / (kBlock * items); return t ? t : 1u; };
-    int items = s->small_items;
-    if (items == 0) {
-      items = 4;
-      for (int i : {2, 1})
-        if ((uint64_t)tiles_of(i) * kSmallGrowth <= (uint64_t)s->small_grid) items = i;
-    }
-    const uint64_t want = (uint64_t)tiles_of(items) * kSmallGrowth;
+  if (takes_small_step(s)) {
+    const int items = s->small_items ? s->small_items : small_items_for(end, kSmallGrowth, s->small_grid);
+    const uint64_t want = (uint64_t)std::max(units_of(end, (uint32_t)(kBlock * items)), 1u) * kSmallGrowth;
     const int ti = items == 1 ? 0 : items == 2 ? 1 : 2;
     int b = 0;
     while (b + 1 < kSmallBuckets && small_bucket_grid(s, b) < want) b++;
@@ -915,7 +927,7 @@ extern "C" int sampo_checkpoint_load(sampo_sim* s, const char* path) {
   CK(cudaMemcpyAsync(s->sim_dev, &h, sizeof(SimDev), cudaMemcpyHostToDevice, s->stream), "state");
   s->step = hd.step;
   s->full_cols = true;
-  const int rc = publish_initial(s, true);
+  const int rc = publish_initial(s, hd.pop.r[7].end, true);
   if (rc) return rc;
   sampo_population p;
   SimDev back;

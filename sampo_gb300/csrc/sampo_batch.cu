@@ -236,10 +236,10 @@ static RepParams carve(const RepLayout& L, void* mem, SimDev* sim, uint64_t capa
   char* q = m + 2 * L.pool;
   set_span_arrays(rp, q, (uint32_t)capacity);
   q += L.spans;
-  rp.T = (const float*)q; q += L.T;
-  rp.env = (const sampo_environment*)q; q += L.env;
+  rp.T = (float*)q; q += L.T;
+  rp.env = (sampo_environment*)q; q += L.env;
   rp.seeds = (sampo_seeds*)q; q += L.seeds;
-  rp.wt = (const uint32_t*)q; q += L.wt;
+  rp.wt = (uint32_t*)q; q += L.wt;
   rp.rows = (sampo_stats_row*)q;
   rp.ring = ring;
   return rp;
@@ -416,7 +416,7 @@ extern "C" int sampo_batch_init_population(sampo_batch* b, uint32_t slot, uint32
       "seeds");
   const KParams p = slot_params(b, slot);
   BCK(launch_init_eggs(p, n, r->T_host[0], b->init_seeds_dev + (size_t)slot * 4, age_days_max, age_seed, b->wide, b->stream), "initAgents");
-  BCK(launch_publish_start(p, false, b->stream), "initial statistics");
+  BCK(launch_publish_start(p, 0, pop.r[7].end, b->stream), "initial statistics");
   r->have_pop = true;
   r->known_end = pop.r[7].end;
   r->step = 0;
@@ -517,7 +517,7 @@ extern "C" int sampo_batch_checkpoint_load(sampo_batch* b, uint32_t slot, const 
   const int st = upload_slot(b, slot, h);
   if (st) return st;
   BCK(cudaMemsetAsync(r->rp.supers, 0, span_array_bytes((uint32_t)r->capacity), b->stream), "span arrays");
-  BCK(launch_publish_start(slot_params(b, slot), true, b->stream), "checkpoint statistics");
+  BCK(launch_publish_start(slot_params(b, slot), PS_CHECK, h.pop.r[7].end, b->stream), "checkpoint statistics");
   SimDev back;
   BCK(cudaMemcpyAsync(&back, b->sims_dev + slot, sizeof(SimDev), cudaMemcpyDeviceToHost, b->stream), "state");
   BCK(cudaStreamSynchronize(b->stream), "state");

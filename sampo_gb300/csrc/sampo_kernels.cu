@@ -123,11 +123,18 @@ cudaError_t launch_init_eggs(const KParams& p, uint32_t n, float T0, const sampo
   void* args[] = {&q, &n, &T0, &seeds_dev, &age_days_max, &age_seed, &fc};
   return launch(p, KID_INIT_EGGS, (const void*)k_init_eggs, sm_count() * 4, 256, 0, st, args);
 }
-cudaError_t launch_publish_start(const KParams& p, bool check, cudaStream_t st) {
+cudaError_t launch_begin_step(const KParams& p, const CtxInputs& in, uint32_t slot, cudaStream_t st) {
   KParams q = p;
-  int ck = check ? 1 : 0;
-  void* args[] = {&q, &ck};
-  cudaError_t e = launch(p, KID_POOL_STATS, (const void*)k_pool_stats, sm_count() * 4, 256, 0, st, args);
+  CtxInputs x = in;
+  void* args[] = {&q, &x, &slot};
+  return launch(p, KID_BEGIN_STEP, (const void*)k_begin_step, 1, 32, 0, st, args);
+}
+cudaError_t launch_publish_start(const KParams& p, uint32_t flags, uint32_t end, cudaStream_t st) {
+  KParams q = p;
+  void* args[] = {&q, &flags};
+  // (a pool that needs fewer CTAs than are resident gets no more: their start is most of its time)
+  const int grid = (int)std::min((uint64_t)sm_count() * 8, std::max<uint64_t>(units_of(end, 256), 1));
+  cudaError_t e = launch(p, KID_POOL_STATS, (const void*)k_pool_stats, grid, 256, 0, st, args);
   if (e != cudaSuccess) return e;
   int mode = PUB_INITIAL;
   void* args2[] = {&q, &mode};
@@ -261,6 +268,14 @@ int grid_blocks_small(int items, const void* ks) {
     return 0;
   }
   return sm_count() * per;
+}
+
+int grid_blocks_small_all(const void* ks) {
+  return std::min({grid_blocks_small(1, ks), grid_blocks_small(2, ks), grid_blocks_small(4, ks)});
+}
+cudaError_t launch_small_hour(const KParams& p, uint32_t end, int items, int max_grid, cudaStream_t st) {
+  const uint64_t want = (uint64_t)units_of(end, (uint32_t)(kBlock * items)) + 1u;
+  return launch_small(p, (int)std::min(want, (uint64_t)max_grid), true, 1u, st, items);
 }
 
 cudaError_t graph_kernel_nodes(cudaGraph_t g, uint32_t* kernels) {

@@ -9,6 +9,7 @@
 #include <stdint.h>
 #ifndef __CUDACC_RTC__
 #include <string.h>
+#include <algorithm>
 #endif
 #include "../../include/sampo.h"
 #include "sampo_math.h"
@@ -49,6 +50,7 @@ struct Decided {
 struct SimDev {
   sampo_population pop;       // ranges + stats of the current pool (reference pop[0] at step start)
   sampo_bites_cycles bnc;     // counters of the last update (printed with the next row)
+  sampo_stats_row begun;      // the row of the step that k_begin_step began
   uint32_t step;              // index of the next step
   uint32_t cur;               // current pool buffer (0/1)
   // The decided step: what its decisions (count pass, or the update/scatter
@@ -79,6 +81,14 @@ struct BatchDev {
   uint32_t minSpan;           // smallest span (slots), see span_size; set by the host between runs
   uint32_t bar;               // one-launch step: CTAs past the decision phase (reset by its last CTA)
   uint32_t done;              // one-launch step: CTAs finished (reset by its last CTA)
+};
+
+// The inputs of one step.
+struct CtxInputs {
+  sampo_seeds sd[4];
+  sampo_environment env;
+  float T;
+  uint32_t wt;
 };
 
 // Words of the one-launch step's rows per tile (sampo_small_step.cuh).
@@ -128,10 +138,10 @@ struct RepParams {
   uint32_t spanStride;
   uint32_t* smallRows;        // one-launch step: [kSmallRows + kSmallStats][smallStride], or null
   uint32_t smallStride;
-  const float* T;             // [ring] temperature per step
-  const sampo_environment* env;  // [ring]
+  float* T;                   // [ring] temperature per step
+  sampo_environment* env;     // [ring]
   sampo_seeds* seeds;         // [ring][4] (written by the device for a device seed stream)
-  const uint32_t* wt;         // [ring] world time per step
+  uint32_t* wt;               // [ring] world time per step
   sampo_stats_row* rows;      // [ring] stats at the start of each step
   uint32_t ring;
 };
@@ -151,6 +161,8 @@ struct KParams {
 // after writing that step's inputs); PUB_DECIDED follows a count pass whose
 // update/scatter pass decides ahead. PUB_DECIDED and PUB_AFTER_STEP take
 // PUB_AHEAD when the update/scatter pass that comes next decides ahead.
+// Flags of k_pool_stats.
+enum : uint32_t { PS_CHECK = 1, PS_CLEAR = 2 };
 enum : int { PUB_INITIAL = 0, PUB_AFTER_STEP = 1, PUB_REFRESH = 2, PUB_DECIDED = 3, PUB_MODE = 3, PUB_AHEAD = 4 };
 
 #ifndef __CUDACC_RTC__  // host side (the run-time compiler sees the device part only)
@@ -222,7 +234,7 @@ int grid_blocks_scatter(uint32_t nrep, const void* ks = nullptr, int items = kIt
 // resident CTAs per SM.
 enum : int {
   KID_COUNT, KID_SCATTER, KID_COUNT_WIDE, KID_SCATTER_WIDE, KID_PUBLISH, KID_INIT_EGGS, KID_POOL_STATS, KID_HISTOGRAM,
-  KID_TRIAL_RESET, KID_WIDEN, KID_SMALL1, KID_SMALL2, KID_SMALL4, KID_N
+  KID_TRIAL_RESET, KID_WIDEN, KID_SMALL1, KID_SMALL2, KID_SMALL4, KID_BEGIN_STEP, KID_N
 };
 cudaError_t species_launch(const void* ks, int kid, dim3 grid, dim3 block, size_t smem, cudaStream_t st, void** args,
                            bool cooperative = false);
@@ -248,7 +260,10 @@ cudaError_t launch_init_eggs(const KParams& p, uint32_t n, float T0, const sampo
                              int age_days_max, uint64_t age_seed, bool full, cudaStream_t st);
 // statistics of p.reps[0]'s current pool, then its publish (PUB_INITIAL);
 // `check` also finds out whether the pool is a wide one (SimDev::wide)
-cudaError_t launch_publish_start(const KParams& p, bool check, cudaStream_t st);
+// (flags: PS_CHECK | PS_CLEAR; end: the pool's end, which sizes the grid)
+cudaError_t launch_publish_start(const KParams& p, uint32_t flags, uint32_t end, cudaStream_t st);
+// The coming step's inputs into ring slot `slot`, and its constants.
+cudaError_t launch_begin_step(const KParams& p, const CtxInputs& in, uint32_t slot, cudaStream_t st);
 // the columns that the records of p's narrow pools imply, written out, and
 // the decisions taken out of the flags (before a pool is read back)
 cudaError_t launch_widen(const KParams& p, cudaStream_t st);
@@ -261,6 +276,18 @@ cudaError_t graph_kernel_nodes(cudaGraph_t g, uint32_t* kernels);
 // largest grid (CTAs resident on all SMs, 0 if it cannot run) and a launch of `nsteps` hourly
 // steps (a cooperative launch when `cooperative`) on `grid` CTAs.
 int grid_blocks_small(int items = kItems, const void* ks = nullptr);
+// The largest grid all three tile sizes can take.
+int grid_blocks_small_all(const void* ks);
+// A step or day on a pool that ends at `end`: the smallest tiles (the shortest
+// chain of updates per thread) of which `growth` times the pool's fit `grid`
+// CTAs, as slots per thread.
+inline int small_items_for(uint32_t end, uint32_t growth, int grid) {
+  for (int i : {1, 2})
+    if ((uint64_t)std::max(units_of(end, (uint32_t)(kBlock * i)), 1u) * growth <= (uint64_t)grid) return i;
+  return 4;
+}
+// One hour now: every tile its CTA and one more, which prepares the next hour.
+cudaError_t launch_small_hour(const KParams& p, uint32_t end, int items, int max_grid, cudaStream_t st);
 cudaError_t launch_small(const KParams& p, int grid, bool cooperative, uint32_t nsteps, cudaStream_t st,
                          int items = kItems);
 // Times count + scatter of the coming step for each number of rows at once

@@ -2,15 +2,18 @@
 // memory (see sampo_step_noalloc in include/sampo.h).
 //
 // The caller owns both pool buffers. Everything else the step needs - the
-// device step state, the per-tile survivor counts and look-back prefixes,
-// one step of inputs and two stats rows - lives in g_noalloc_scratch, a
-// fixed file-scope device array sized for pools of up to
+// device step state, the count pass's decisions and span counts (or a small
+// pool's rows), one step of inputs and two stats rows - lives in
+// g_noalloc_scratch, a fixed file-scope device array sized for pools of up to
 // SAMPO_NOALLOC_MAX_SLOTS slots. The kernels are the ones sampo_step runs;
-// only where their scratch lives differs. Nothing here calls cudaMalloc,
+// only where their scratch lives differs. The call's state goes up in one copy
+// and its results come down in one: each copy from or to pageable memory costs
+// about as much as a kernel of a small pool. Nothing here calls cudaMalloc,
 // cudaFree or any routine that allocates device memory.
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <string.h>
+#include <algorithm>
 #include <mutex>
 #include "sampo_model.cuh"
 #include "sampo_kernels.cuh"
@@ -28,16 +31,41 @@ struct InputBlock {
   sampo_seeds seeds[8];
 };
 
-struct Scratch {
-  __align__(16) uint4 spans[span_array_words(SAMPO_NOALLOC_MAX_SLOTS)];
-  uint8_t dec[SAMPO_NOALLOC_MAX_SLOTS];  // the count pass's decisions (the caller's pool is only read)
+// What a call sends up, in one copy ...
+struct CallState {
   SimDev sim;
   RepParams rep;
   BatchDev bat;
   ModelConst mc;
-  sampo_stats_row rows[2];
   InputBlock in;
 };
+// ... and what it brings back: the rows and the head of the state after them.
+struct Results {
+  sampo_stats_row rows[2];
+  alignas(16) unsigned char sim[offsetof(SimDev, capacity)];
+};
+
+// Largest pool, in 1024-slot tiles, that takes the one-launch step here: its
+// rows lie in the scratch. (Grids of up to 512 CTAs; a GB300 has 456.)
+constexpr uint32_t kSmallTiles = 512, kSmallStride = kSmallTiles * 4;
+
+struct Scratch {
+  __align__(16) uint4 spans[span_array_words(SAMPO_NOALLOC_MAX_SLOTS)];
+  uint8_t dec[SAMPO_NOALLOC_MAX_SLOTS];  // the count pass's decisions (the caller's pool is only read)
+  uint32_t small[kSmallRowWords * kSmallStride];
+  sampo_stats_row rows[2];
+  alignas(16) CallState call;
+};
+static_assert(offsetof(Scratch, call) - offsetof(Scratch, rows) == offsetof(Results, sim), "the rows and the state are copied at once");
+
+// The one-launch step's largest grid on the current device, asked for once.
+int small_grid(int device) {
+  constexpr int kMaxDevices = 64;
+  static std::once_flag once[kMaxDevices];
+  static int grid[kMaxDevices];
+  std::call_once(once[device], [&] { grid[device] = grid_blocks_small_all(nullptr); });
+  return grid[device];
+}
 
 }  // namespace
 
@@ -108,66 +136,67 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
   if (scratch_address(device, &base) != cudaSuccess) return SAMPO_ERR_CUDA;
   Scratch* sc = (Scratch*)base;
 
-  SimDev h = initial_sim_state(out_capacity, cc);
+  CallState up;
+  memset(&up, 0, sizeof(up));
+  SimDev& h = up.sim;
+  h = initial_sim_state(out_capacity, cc);
   h.pop = *pop_in;
   h.pop.numLarvae1DayEquiv = h.pop.numFemale = h.pop.numPotentiallyInfective = 0;
   h.active = 1;
-  ModelConst mc;
-  fill_constant_tables(mc);
-  BatchDev bat;
-  memset(&bat, 0, sizeof(bat));
-  InputBlock ib;
-  memset(&ib, 0, sizeof(ib));
+  fill_constant_tables(up.mc);
+  InputBlock& ib = up.in;
   ib.T[0] = temperature;
   ib.wt[0] = world_time;
   ib.env[0] = *env;
   for (int k = 0; k < 4; k++) ib.seeds[k] = seeds[k];
 
-  // The array keeps the previous call's contents: reset the state and clear
-  // the supers this step adds to.
-  const uint32_t nsup = (span_count(pop_in->r[7].end, 0) + 31u) / 32u;
-  RepParams rp;
-  rp.sim = &sc->sim;
+  RepParams& rp = up.rep;
+  rp.sim = &sc->call.sim;
   rp.pool[0] = to_dev(in);
   rp.pool[1] = to_dev(out);
   rp.dec = sc->dec;
   set_span_arrays(rp, sc->spans, SAMPO_NOALLOC_MAX_SLOTS);
-  rp.smallRows = nullptr;
-  rp.smallStride = 0;
-  rp.T = sc->in.T;
-  rp.env = sc->in.env;
-  rp.seeds = sc->in.seeds;
-  rp.wt = sc->in.wt;
+  rp.smallRows = sc->small;
+  rp.smallStride = kSmallStride;
+  rp.T = sc->call.in.T;
+  rp.env = sc->call.in.env;
+  rp.seeds = sc->call.in.seeds;
+  rp.wt = sc->call.in.wt;
   rp.rows = sc->rows;
   rp.ring = 2;
-  if (cudaMemcpyAsync(&sc->sim, &h, sizeof(h), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(&sc->rep, &rp, sizeof(rp), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(&sc->bat, &bat, sizeof(bat), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(&sc->mc, &mc, sizeof(mc), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-      cudaMemcpyAsync(&sc->in, &ib, sizeof(ib), cudaMemcpyHostToDevice, st) != cudaSuccess)
-    return SAMPO_ERR_CUDA;
-  if (nsup && cudaMemsetAsync(rp.supers, 0, (size_t)nsup * sizeof(uint4), st) != cudaSuccess)
-    return SAMPO_ERR_CUDA;
+  if (cudaMemcpyAsync(&sc->call, &up, sizeof(up), cudaMemcpyHostToDevice, st) != cudaSuccess) return SAMPO_ERR_CUDA;
 
   KParams p;
-  p.reps = &sc->rep;
+  p.reps = &sc->call.rep;
   p.nrep = 1;
-  p.bat = &sc->bat;
-  p.mc = &sc->mc;
+  p.bat = &sc->call.bat;
+  p.mc = &sc->call.mc;
   p.ks = nullptr;  // the built-in species
   p.wide = 1u;     // the caller's columns hold whole records
-  if (launch_publish_start(p, false, st) != cudaSuccess) return SAMPO_ERR_CUDA;
-  if (launch_count(p, grid_blocks_count(1, nullptr, kItems, true), st) != cudaSuccess) return SAMPO_ERR_CUDA;
-  if (launch_scatter(p, grid_blocks_scatter(1, nullptr, kItems, true), st) != cudaSuccess) return SAMPO_ERR_CUDA;
-  if (launch_publish(p, PUB_AFTER_STEP, st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  // The one-launch step for a pool of at most one 1024-slot tile per CTA (as
+  // in sampo_step), else the passes. (5,000 agents: 104 us with the passes and
+  // ten copies, 57 with one launch and two copies.) The array keeps the
+  // previous call's contents: the supers the passes add to are cleared.
+  const uint32_t end = pop_in->r[7].end;
+  const int grid = small_grid(device);
+  const bool small = units_of(end, (uint32_t)kTile) <= std::min((uint32_t)grid, kSmallTiles);
+  if (launch_publish_start(p, small ? 0u : (uint32_t)PS_CLEAR, end, st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  if (small) {
+    if (launch_small_hour(p, end, small_items_for(end, 1, grid), grid, st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  } else {
+    if (launch_count(p, grid_blocks_count(1, nullptr, kItems, true), st) != cudaSuccess) return SAMPO_ERR_CUDA;
+    if (launch_scatter(p, grid_blocks_scatter(1, nullptr, kItems, true), st) != cudaSuccess) return SAMPO_ERR_CUDA;
+    if (launch_publish(p, PUB_AFTER_STEP, st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  }
 
-  uint32_t err = 0;
-  if (cudaMemcpyAsync(row, &sc->rows[0], sizeof(*row), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaMemcpyAsync(pop_out, &sc->sim.pop, sizeof(*pop_out), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaMemcpyAsync(bnc_out, &sc->sim.bnc, sizeof(*bnc_out), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaMemcpyAsync(&err, &sc->sim.error, sizeof(err), cudaMemcpyDeviceToHost, st) != cudaSuccess)
-    return SAMPO_ERR_CUDA;
+  Results down;
+  if (cudaMemcpyAsync(&down, sc->rows, sizeof(down), cudaMemcpyDeviceToHost, st) != cudaSuccess) return SAMPO_ERR_CUDA;
   if (cudaStreamSynchronize(st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  uint32_t err;
+  memcpy(&err, down.sim + offsetof(SimDev, error), sizeof(err));
+  *row = down.rows[0];
+  memcpy(pop_out, down.sim + offsetof(SimDev, pop), sizeof(*pop_out));
+  memcpy(bnc_out, down.sim + offsetof(SimDev, bnc), sizeof(*bnc_out));
   if (err & SAMPO_DEV_ERR_CAPACITY) return SAMPO_ERR_CAPACITY;
   if (err & SAMPO_DEV_ERR_DEVRATES) return SAMPO_ERR_TEMPERATURE;
   if (err) return SAMPO_ERR_INTERNAL;

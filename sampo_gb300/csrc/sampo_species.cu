@@ -123,7 +123,7 @@ const char* const kKernelNames[KID_N] = {"&sampo::k_count<4, false>", "&sampo::k
                                          "&sampo::k_pool_stats",      "&sampo::k_histogram",
                                          "&sampo::k_trial_reset",     "&sampo::k_widen",
                                          "&sampo::k_step_small<1>",   "&sampo::k_step_small<2>",
-                                         "&sampo::k_step_small<4>"};
+                                         "&sampo::k_step_small<4>",   "&sampo::k_begin_step"};
 
 // standard headers the kernel sources include, reduced to what NVRTC lacks,
 // and the reference's headers a species header includes (the prelude defines

@@ -103,12 +103,6 @@ __device__ __forceinline__ bool layout_fits(const uint32_t cnt[8], uint32_t newE
 }
 
 // The inputs of step `step` of one replicate (its ring slot).
-struct CtxInputs {
-  sampo_seeds sd[4];
-  sampo_environment env;
-  float T;
-  uint32_t wt;
-};
 __device__ __forceinline__ void load_ctx_inputs(const RepParams& rp, uint32_t step, CtxInputs& in) {
   const uint32_t i = step % rp.ring;
 #pragma unroll
@@ -1068,6 +1062,27 @@ __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
   }
 }
 
+// The start of one hour called on its own: its inputs, which come with the
+// launch (no copies ahead of it in the stream), into their ring slots, and the
+// step's constants; the step's row goes beside the status words, so that one
+// copy brings both to the host. One thread: what it does is a chain anyway.
+__global__ void k_begin_step(KParams p, CtxInputs in, uint32_t slot) {
+  if (threadIdx.x != 0) return;
+  const RepParams& rp = p.reps[0];
+  SimDev* sim = rp.sim;
+  rp.T[slot] = in.T;
+  rp.env[slot] = in.env;
+  rp.wt[slot] = in.wt;
+#pragma unroll
+  for (int k = 0; k < 4; k++) rp.seeds[(size_t)slot * 4 + k] = in.sd[k];
+  sim->begun = rp.rows[slot];
+  if (!sim->active) return;
+  const uint32_t s = sim->step;
+  StepCtx c;
+  make_ctx(in, sim->larvaKill[s & 1u], sim->pop, c);
+  sim->ctx[s & 1u] = c;
+}
+
 // Publishing the start of a step for every replicate of p (one CTA each).
 __global__ void __launch_bounds__(kPublishThreads) k_publish(KParams p, int mode) { publish_rep(p, blockIdx.x, mode); }
 
@@ -1593,28 +1608,59 @@ __device__ __forceinline__ bool wide_record(const DevPool& s, uint32_t g, int rg
   return w;
 }
 
-// Statistics of p.reps[0]'s current pool (grid-stride), accumulated into
-// acc_*; with `check`, also whether its records are wide.
-__global__ void k_pool_stats(KParams p, int check) {
-  SimDev* sim = p.reps[0].sim;
-  const sampo_population pop = sim->pop;
-  const DevPool src = p.reps[0].pool[sim->cur];
-  uint32_t l1 = 0, fem = 0, inf = 0, dmin = 0xffffffffu, dmax = 0;
-  bool wide = false;
-  const uint32_t end = pop.r[GRAVID].end;
-  for (uint64_t g64 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; g64 < end; g64 += (uint64_t)gridDim.x * blockDim.x) {
+// Statistics of p.reps[0]'s current pool, accumulated into acc_*; PS_CHECK:
+// also whether its records are wide, PS_CLEAR: also clears the supers. Only
+// the ranges that the statistics come from are read (larvae and adults; with
+// PS_CHECK all), each by the whole grid.
+template <int RG>
+struct Stage {
+  __device__ constexpr int operator()() const { return RG; }
+};
+template <int RG>
+__device__ __forceinline__ void stats_range(const DevPool& s, uint32_t lo, uint32_t hi, bool check, uint32_t& l1, uint32_t& dmin,
+                                            uint32_t& dmax, uint32_t& fem, uint32_t& inf, bool& wide) {
+  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (uint64_t g64 = (uint64_t)lo + blockIdx.x * blockDim.x + threadIdx.x; g64 < hi; g64 += step) {
     const uint32_t g = (uint32_t)g64;
-    int rg = range_of(pop, g);
-    if (check && rg >= 0) wide |= wide_record(src, g, rg);
-    if (rg == LARVA) {
-      float age = src.age[g];
+    if (check) wide |= wide_record(s, g, RG);
+    if (RG == LARVA) {
+      const float age = s.age[g];
+      const uint32_t dd = age_days(age);
       l1 += age_days_uncapped(age);
-      uint32_t dd = age_days(age);
       dmin = min(dmin, dd); dmax = max(dmax, dd);
-    } else if (rg >= IMMATURE) {
-      if ((src.flags[g] >> 3) & 1u) { fem++; inf += src.sporo[g] >= 1.0f ? 1u : 0u; }
+    } else if (RG >= IMMATURE) {
+      const uint32_t female = (s.flags[g] >> 3) & 1u;
+      fem += female;
+      inf += s.sporo[g] >= 1.0f ? female : 0u;
     }
   }
+}
+__global__ void __launch_bounds__(256) k_pool_stats(KParams p, uint32_t flags) {
+  const RepParams& rp = p.reps[0];
+  SimDev* sim = rp.sim;
+  const sampo_population pop = sim->pop;
+  const DevPool src = rp.pool[sim->cur];
+  const bool check = flags & PS_CHECK;
+  uint32_t l1 = 0, fem = 0, inf = 0, dmin = 0xffffffffu, dmax = 0;
+  bool wide = false;
+  if (flags & PS_CLEAR) {
+    const uint32_t n = units_of(span_count(pop.r[GRAVID].end, 0), 32);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) rp.supers[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  auto range = [&](auto rg) {
+    stats_range<rg()>(src, pop.r[rg()].start, pop.r[rg()].end, check, l1, dmin, dmax, fem, inf, wide);
+  };
+  if (check) {
+    range(Stage<EGG>());
+    range(Stage<PUPA>());
+  }
+  range(Stage<LARVA>());
+  range(Stage<IMMATURE>());
+  range(Stage<MATESEEKING>());
+  range(Stage<BMS>());
+  range(Stage<BMD>());
+  range(Stage<GRAVID>());
   wide = __any_sync(0xffffffffu, wide);
   l1 = __reduce_add_sync(0xffffffffu, l1);
   fem = __reduce_add_sync(0xffffffffu, fem);

@@ -89,3 +89,26 @@ def test_species_one_launch_day(gpu_ready, sizes):
         assert r.tobytes() == rows.tobytes(), key
         assert np.array_equal(p["ranges"], pop["ranges"]), key
         _same_pools(pop["ranges"], a, pool)
+
+
+@pytest.mark.parametrize("sizes", [(1, 0, 0, 0), (255, 1, 128, 130), (257, 256, 255, 1025), (60000, 40001, 9000, 20000)])
+def test_single_hours_match_oracle(gpu_ready, oracle_mod, sizes):
+    """sampo_step, one launch an hour and three, with a pool read between."""
+    from oracle import OracleSim
+    from sampo_gb300.sim import Simulation
+    n, cc, cap = 6, 30000.0, 1 << 20
+    ranges, arrays, T, env, seeds = _workload(sizes, n, cc, seed=9)
+    for tiles in (None, 0):
+        orc = OracleSim(cap)
+        orc.load_pool(ranges, arrays)
+        with Simulation(capacity=cap, carrying_capacity=cc, max_steps=n + 1) as sim:
+            sim.set_inputs(T, env)
+            sim.set_small_step(tiles)
+            sim.load_pool(ranges, arrays)
+            for i in range(n):
+                row = sim.step(env[i], T[i], (18 + i) % 24, seeds[i])
+                assert row.tobytes() == orc.step(env[i], T[i], (18 + i) % 24, seeds[i]).tobytes(), (tiles, i)
+                if i in (2, n - 1):
+                    ro, ao = orc.read_pool()
+                    _same_pools(ro, sim.read_pool()[1], ao)
+            assert sim.device_status() & 0xFF == 0
