@@ -132,8 +132,8 @@ cudaError_t launch_begin_step(const KParams& p, const CtxInputs& in, uint32_t sl
 cudaError_t launch_publish_start(const KParams& p, uint32_t flags, uint32_t end, cudaStream_t st) {
   KParams q = p;
   void* args[] = {&q, &flags};
-  // (a pool that needs fewer CTAs than are resident gets no more: their start is most of its time)
-  const int grid = (int)std::min((uint64_t)sm_count() * 8, std::max<uint64_t>(units_of(end, 256), 1));
+  // four slots a thread and turn; a small pool gets no more CTAs than that takes (their start is most of its time)
+  const int grid = (int)std::min((uint64_t)sm_count() * 4, std::max<uint64_t>(units_of(end, 1024), 1));
   cudaError_t e = launch(p, KID_POOL_STATS, (const void*)k_pool_stats, grid, 256, 0, st, args);
   if (e != cudaSuccess) return e;
   int mode = PUB_INITIAL;

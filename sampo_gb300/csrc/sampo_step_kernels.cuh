@@ -26,6 +26,9 @@
 // updateAgents, initAgents, 3 x preScan + 3 x Bolt scan-by-key,
 // oldToNewAgents, calcL1de x2, calcFemales x2) and its blocking transfers.
 #pragma once
+#ifndef __CUDACC_RTC__
+#include <stddef.h>
+#endif
 #include "sampo_kernels.cuh"
 
 namespace sampo {
@@ -620,6 +623,7 @@ struct WarpSum {
   Decided dec;                 // of the step being decided
   uint32_t fem, inf, bnc[4];   // of the pool being written
   uint32_t error;
+  uint32_t rep, spans;         // the replicate they belong to; count pass: spans counted
 };
 __device__ __forceinline__ void clear_sum(WarpSum& t) {
   t.dec = Decided{0u, 0u, 0xffffffffu, 0u};
@@ -637,6 +641,53 @@ __device__ __forceinline__ void flush_sum(WarpSum& t, SimDev* sim, Decided* to) 
     if (t.bnc[j]) atomicAdd(&sim->acc_bnc[j], t.bnc[j]);
   if (t.error) atomicOr(&sim->error, t.error);
   clear_sum(t);
+}
+
+// The end of a pass (every thread of the CTA): the sums that its warps hold
+// (WarpSum::rep) into their replicates', the CTA's warps of one replicate
+// together (the adds of 3,648 warps to the same few words, all at the end,
+// queued up: k_scatter 113 -> 109 us at 5e6 caller-owned agents). Returns, on the lanes of the first warp of a
+// replicate, the spans its warps have counted (0 on other warps).
+__device__ __forceinline__ uint32_t flush_sums(const RepParams* reps, WarpSum* sums, bool dec_ahead) {
+  constexpr uint32_t kMin = 2, kMax = 3, kFem = 4, kBnc = 6, kError = 10, kSpans = 12;  // a WarpSum's words
+#ifndef __CUDACC_RTC__  // (it has no offsetof)
+  static_assert(offsetof(WarpSum, dec.dmin) == 4 * kMin && offsetof(WarpSum, dec.dmax) == 4 * kMax && offsetof(WarpSum, fem) == 4 * kFem &&
+                offsetof(WarpSum, bnc) == 4 * kBnc && offsetof(WarpSum, error) == 4 * kError && offsetof(WarpSum, spans) == 4 * kSpans &&
+                offsetof(SimDev, acc_inf) == offsetof(SimDev, acc_fem) + 4, "words of the sums");
+#endif
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  __syncthreads();
+  const uint32_t rep = sums[warp].rep;
+  for (uint32_t j = 0; j < warp; j++)
+    if (sums[j].rep == rep) return 0u;
+  if (rep == kNoRep) return 0u;
+  const uint32_t k = min(lane, kSpans);
+  uint32_t sum = 0, lo = 0xffffffffu, hi = 0, any = 0;
+#pragma unroll
+  for (uint32_t j = 0; j < kWarps; j++) {
+    if (sums[j].rep != rep) continue;
+    const uint32_t x = reinterpret_cast<const uint32_t*>(&sums[j])[k];
+    sum += x;
+    lo = min(lo, x);
+    hi = max(hi, x);
+    any |= x;
+  }
+  SimDev* sim = reps[rep].sim;
+  uint32_t* dec = reinterpret_cast<uint32_t*>(dec_ahead ? &sim->ahead_dec : &sim->dec);
+  if (lane == kMin) {
+    if (lo != 0xffffffffu) atomicMin(dec + kMin, lo);
+  } else if (lane == kMax) {
+    if (hi) atomicMax(dec + kMax, hi);
+  } else if (lane < kFem) {
+    if (sum) atomicAdd(dec + lane, sum);
+  } else if (lane < kBnc) {
+    if (sum) atomicAdd(&sim->acc_fem + (lane - kFem), sum);
+  } else if (lane < kError) {
+    if (sum) atomicAdd(&sim->acc_bnc[lane - kBnc], sum);
+  } else if (lane == kError) {
+    if (any) atomicOr(&sim->error, any);
+  }
+  return __shfl_sync(0xffffffffu, sum, kSpans);
 }
 
 // The dynamic shared memory of the two passes, followed by the batch's unit
@@ -803,17 +854,14 @@ __global__ void __launch_bounds__(kBlock, 3) k_count(KParams p) {
   WarpSum& sum = ps.sum[warp];
   if (lane == 0) clear_sum(sum);
   uint32_t cur_rep = kNoRep, done = 0;
-  // the warp's counters into its replicate's totals; the warp that brings
-  // the last spans scans the supers
-  auto flush = [&]() {
-    if (cur_rep == kNoRep) return;
+  // `n` counted spans into the replicate's: the warp that brings the last ones scans the supers
+  auto arrive = [&](uint32_t n) {
     const RepParams& rp = p.reps[cur_rep];
     SimDev* sim = rp.sim;
     uint32_t last = 0;
     if (lane == 0) {
-      flush_sum(sum, sim, &sim->dec);
-      __threadfence();  // this warp's adds to the supers come before its arrival
-      last = atomicAdd(&sim->spans_done, done) + done == w.nspans;
+      __threadfence();  // the adds to the supers come before the arrival
+      last = atomicAdd(&sim->spans_done, n) + n == w.nspans;
       __threadfence();
     }
     last = __shfl_sync(0xffffffffu, last, 0);
@@ -825,13 +873,16 @@ __global__ void __launch_bounds__(kBlock, 3) k_count(KParams p) {
         sim->dirty[sim->rot] = max(sim->dirty[sim->rot], w.nspans);
       }
     }
-    done = 0;
   };
   for (uint32_t u = blockIdx.x * kWarps + warp; u < total; u += stride) {
     const uint32_t t = total - 1u - u;
     const uint32_t r = find_rep(s_pre, p.nrep, t);
     if (r != cur_rep) {  // uniform
-      flush();
+      if (cur_rep != kNoRep) {
+        if (lane == 0) flush_sum(sum, p.reps[cur_rep].sim, &p.reps[cur_rep].sim->dec);
+        arrive(done);
+        done = 0;
+      }
       load_warp_rep<false, false>(p.reps[r], min_span, w);
       cur_rep = r;
     }
@@ -845,7 +896,13 @@ __global__ void __launch_bounds__(kBlock, 3) k_count(KParams p) {
     }
     done++;
   }
-  flush();
+  if (lane == 0) {
+    sum.rep = cur_rep;
+    sum.spans = done;
+    __threadfence();  // (the first warp of the replicate arrives for this one)
+  }
+  const uint32_t n = flush_sums(p.reps, ps.sum, false);
+  if (n) arrive(n);
 }
 
 // ------------------------------------------------------------------------
@@ -1435,21 +1492,20 @@ __global__ void __launch_bounds__(kBlock, 3) k_scatter(KParams p) {
   uint32_t cur_rep = kNoRep;
   WarpSum& sum = ps.sum[warp];
   if (lane == 0) clear_sum(sum);
-  // this warp's sums into its replicate's
-  auto flush = [&]() {
-    if (cur_rep != kNoRep && lane == 0) {
-      SimDev* sim = p.reps[cur_rep].sim;
-      if (AHEAD && !w.ahead) {  // (its decisions were taken for nothing)
-        sum.dec = Decided{0u, 0u, 0xffffffffu, 0u};
-        sum.error &= SAMPO_DEV_ERR_TILECOUNT;
-      }
-      flush_sum(sum, sim, &sim->ahead_dec);
+  // lane 0, before this warp's sums go into its replicate's
+  auto end_rep = [&]() {
+    if (AHEAD && cur_rep != kNoRep && !w.ahead) {  // (its decisions were taken for nothing)
+      sum.dec = Decided{0u, 0u, 0xffffffffu, 0u};
+      sum.error &= SAMPO_DEV_ERR_TILECOUNT;
     }
   };
   for (uint32_t t = blockIdx.x * kWarps + warp; t < total; t += stride) {
     const uint32_t r = find_rep(s_pre, p.nrep, t);
     if (r != cur_rep) {  // uniform
-      flush();
+      if (cur_rep != kNoRep && lane == 0) {
+        end_rep();
+        flush_sum(sum, p.reps[cur_rep].sim, &p.reps[cur_rep].sim->ahead_dec);
+      }
       load_warp_rep<true, AHEAD>(p.reps[r], min_span, w);
       cur_rep = r;
     }
@@ -1510,7 +1566,12 @@ __global__ void __launch_bounds__(kBlock, 3) k_scatter(KParams p) {
       }
     }
   }
-  flush();
+  if (lane == 0) {
+    end_rep();
+    sum.rep = cur_rep;
+    sum.spans = 0;
+  }
+  (void)flush_sums(p.reps, ps.sum, true);
 }
 
 // ------------------------------------------------------------------------
@@ -1611,69 +1672,88 @@ __device__ __forceinline__ bool wide_record(const DevPool& s, uint32_t g, int rg
 // Statistics of p.reps[0]'s current pool, accumulated into acc_*; PS_CHECK:
 // also whether its records are wide, PS_CLEAR: also clears the supers. Only
 // the ranges that the statistics come from are read (larvae and adults; with
-// PS_CHECK all), each by the whole grid.
-template <int RG>
-struct Stage {
-  __device__ constexpr int operator()() const { return RG; }
-};
-template <int RG>
-__device__ __forceinline__ void stats_range(const DevPool& s, uint32_t lo, uint32_t hi, bool check, uint32_t& l1, uint32_t& dmin,
-                                            uint32_t& dmax, uint32_t& fem, uint32_t& inf, bool& wide) {
-  const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-#pragma unroll 4
-  for (uint64_t g64 = (uint64_t)lo + blockIdx.x * blockDim.x + threadIdx.x; g64 < hi; g64 += step) {
-    const uint32_t g = (uint32_t)g64;
-    if (check) wide |= wide_record(s, g, RG);
-    if (RG == LARVA) {
-      const float age = s.age[g];
-      const uint32_t dd = age_days(age);
-      l1 += age_days_uncapped(age);
-      dmin = min(dmin, dd); dmax = max(dmax, dd);
-    } else if (RG >= IMMATURE) {
-      const uint32_t female = (s.flags[g] >> 3) & 1u;
-      fem += female;
-      inf += s.sporo[g] >= 1.0f ? female : 0u;
-    }
-  }
-}
+// PS_CHECK all), as one sequence of four-slot groups (16-byte loads), so that
+// a thread has few turns of a load latency each; a loop over all slots that
+// looked its range up, and an add per warp to the same words, took 32 us at
+// 5e6 agents where this takes 14.
 __global__ void __launch_bounds__(256) k_pool_stats(KParams p, uint32_t flags) {
+  __shared__ WarpSum sums[kWarps];
   const RepParams& rp = p.reps[0];
   SimDev* sim = rp.sim;
   const sampo_population pop = sim->pop;
   const DevPool src = rp.pool[sim->cur];
   const bool check = flags & PS_CHECK;
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
   uint32_t l1 = 0, fem = 0, inf = 0, dmin = 0xffffffffu, dmax = 0;
   bool wide = false;
   if (flags & PS_CLEAR) {
     const uint32_t n = units_of(span_count(pop.r[GRAVID].end, 0), 32);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) rp.supers[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (uint32_t i = tid; i < n; i += threads) rp.supers[i] = make_uint4(0u, 0u, 0u, 0u);
   }
-  auto range = [&](auto rg) {
-    stats_range<rg()>(src, pop.r[rg()].start, pop.r[rg()].end, check, l1, dmin, dmax, fem, inf, wide);
-  };
-  if (check) {
-    range(Stage<EGG>());
-    range(Stage<PUPA>());
+  uint32_t upto[8], groups = 0;  // groups of the ranges up to each
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const bool read = (check || k == LARVA || k >= IMMATURE) && pop.r[k].end > pop.r[k].start;
+    groups += read ? (pop.r[k].end - (pop.r[k].start & ~3u) + 3u) / 4u : 0u;
+    upto[k] = groups;
   }
-  range(Stage<LARVA>());
-  range(Stage<IMMATURE>());
-  range(Stage<MATESEEKING>());
-  range(Stage<BMS>());
-  range(Stage<BMD>());
-  range(Stage<GRAVID>());
+#pragma unroll 2
+  for (uint32_t q = tid; q < groups; q += threads) {
+    int rg = 0;
+    uint32_t before = 0, lo = pop.r[0].start, hi = pop.r[0].end;
+#pragma unroll
+    for (int k = 1; k < 8; k++)
+      if (q >= upto[k - 1]) {
+        rg = k;
+        before = upto[k - 1];
+        lo = pop.r[k].start;
+        hi = pop.r[k].end;
+      }
+    const uint32_t g = (lo & ~3u) + 4u * (q - before);
+    if (check)
+      for (uint32_t i = max(g, lo); i < min(g + 4u, hi); i++) wide |= wide_record(src, i, rg);
+    if (rg == LARVA) {
+      const float4 v = *reinterpret_cast<const float4*>(src.age + g);
+      const float age[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (uint32_t i = 0; i < 4; i++) {
+        if (g + i < lo || g + i >= hi) continue;
+        const uint32_t dd = age_days(age[i]);
+        l1 += age_days_uncapped(age[i]);
+        dmin = min(dmin, dd);
+        dmax = max(dmax, dd);
+      }
+    } else if (rg >= IMMATURE) {
+      const uint32_t fl = *reinterpret_cast<const uint32_t*>(src.flags + g);
+      const float4 v = *reinterpret_cast<const float4*>(src.sporo + g);
+      const float sporo[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (uint32_t i = 0; i < 4; i++) {
+        const uint32_t female = g + i >= lo && g + i < hi ? (fl >> (8 * i + 3)) & 1u : 0u;
+        fem += female;
+        inf += sporo[i] >= 1.0f ? female : 0u;
+      }
+    }
+  }
   wide = __any_sync(0xffffffffu, wide);
   l1 = __reduce_add_sync(0xffffffffu, l1);
   fem = __reduce_add_sync(0xffffffffu, fem);
   inf = __reduce_add_sync(0xffffffffu, inf);
   dmin = __reduce_min_sync(0xffffffffu, dmin);
   dmax = __reduce_max_sync(0xffffffffu, dmax);
+  // one add per CTA and word
   if ((threadIdx.x & 31) == 0) {
-    if (l1) atomicAdd(&sim->dec.L1de, l1);
-    if (fem) atomicAdd(&sim->acc_fem, fem);
-    if (inf) atomicAdd(&sim->acc_inf, inf);
-    if (dmin != 0xffffffffu) { atomicMin(&sim->dec.dmin, dmin); atomicMax(&sim->dec.dmax, dmax); }
+    WarpSum& t = sums[threadIdx.x >> 5];
+    clear_sum(t);
+    t.dec.L1de = l1;
+    t.dec.dmin = dmin;
+    t.dec.dmax = dmax;
+    t.fem = fem;
+    t.inf = inf;
+    t.rep = t.spans = 0;
     if (wide) sim->wide = 1u;
   }
+  (void)flush_sums(p.reps, sums, false);
 }
 
 // ageHistogram (kernel/ageHistogram.cl:13-35) of p.reps[0] with
