@@ -19,6 +19,8 @@ from ._lib import ENV_DTYPE, ROW_DTYPE, BatchConfig, Population, RandState, Repl
 from .sim import make_pool_arrays, pool_view, pop_to_numpy, rand_state, seed_stream
 
 NEVER = 0xFFFFFFFF
+# sampo_slot_state, as the library writes it
+SLOT_STATE = np.dtype([("step", "u4"), ("active", "u4"), ("status", "u4"), ("end", "u4"), ("capacity", "u8")])
 
 
 class Batch:
@@ -124,12 +126,8 @@ class Batch:
 
     def states(self) -> np.ndarray:
         """sampo_batch_states: step, active, status, end and capacity of every slot."""
-        out = (_lib.SlotState * self.max_replicates)()
-        self._check(self.lib.sampo_batch_states(self.h, C.addressof(out), self.max_replicates))
-        a = np.zeros(self.max_replicates, dtype=[("step", "u4"), ("active", "u4"), ("status", "u4"), ("end", "u4"),
-                                                 ("capacity", "u8")])
-        for i, o in enumerate(out):
-            a[i] = (o.step, o.active, o.status, o.end, o.capacity)
+        a = np.zeros(self.max_replicates, dtype=SLOT_STATE)
+        self._check(self.lib.sampo_batch_states(self.h, ptr(a), self.max_replicates))
         return a
 
     def histogram(self, slot: int) -> np.ndarray:
