@@ -88,9 +88,12 @@ enum : int { DG_PLAIN = 1, DG_SMALL_COOP = 2, DG_SMALL = 3 };
 // Grid sizes of the one-launch day graphs (the last one is the largest
 // co-resident grid), and the growth a pool is allowed between the day whose
 // end the host saw and the end of the day it picks for (one day behind, one
-// day of growth): a grid of at least kSmallGrowth CTAs per tile seen.
+// day of growth): a grid of at least kSmallGrowth / 2 CTAs per tile seen. (A
+// year from 1e4 eggs took 13.54 us per hour with room for twice the pool, 13.23
+// for 3/2, which keeps smaller tiles longer, 13.17 for 5/4 and 13.43 for none;
+// a month from 1e3 eggs 7.85, 7.86, 8.30 and 8.42.)
 constexpr int kSmallBuckets = 8;
-constexpr uint32_t kSmallGrowth = 2;
+constexpr uint32_t kSmallGrowth = 3;
 static uint32_t small_bucket_grid(const sampo_sim* s, int b) {
   const uint32_t g = 8u << b;
   return (b == kSmallBuckets - 1 || g >= (uint32_t)s->small_grid) ? (uint32_t)s->small_grid : g;
@@ -552,7 +555,7 @@ static cudaError_t build_small_graph(sampo_sim* s, int items, int b) {
 }
 
 // The graph of the coming day and its kernel launches: the one-launch step
-// (grid of at least kSmallGrowth CTAs per tile of the pool end last seen)
+// (a grid with room to grow over the pool end last seen, kSmallGrowth)
 // when that pool has at most small_tiles 1024-slot tiles, else the
 // three-kernel step. The one-launch step takes the smallest tiles (the
 // shortest chain of updates per thread: 256, then 512, then 1024 slots) the
@@ -562,8 +565,8 @@ static cudaError_t build_small_graph(sampo_sim* s, int items, int b) {
 static int day_graph_for(sampo_sim* s, cudaGraphExec_t* gx, uint32_t* kernels, int* kind) {
   const uint32_t end = s->known_end;
   if (takes_small_step(s)) {
-    const int items = s->small_items ? s->small_items : small_items_for(end, kSmallGrowth, s->small_grid);
-    const uint64_t want = (uint64_t)std::max(units_of(end, (uint32_t)(kBlock * items)), 1u) * kSmallGrowth;
+    const int items = s->small_items ? s->small_items : small_items_for(end, kSmallGrowth, 2 * s->small_grid);
+    const uint64_t want = ((uint64_t)std::max(units_of(end, (uint32_t)(kBlock * items)), 1u) * kSmallGrowth + 1u) / 2u;
     const int ti = items == 1 ? 0 : items == 2 ? 1 : 2;
     int b = 0;
     while (b + 1 < kSmallBuckets && small_bucket_grid(s, b) < want) b++;
