@@ -69,7 +69,7 @@ struct sampo_sim {
   cudaGraphExec_t small_graph[3][8] = {};  // [256-, 512-, 1024-slot tiles][grid bucket]
   int small_graph_kind[3][8] = {};     // DG_* of each
   uint32_t known_end = 0;              // pool end at the start of the coming day, as last seen by the host
-  uint32_t* end_pinned = nullptr;      // pool end after a day, copied back one day behind the queue
+  uint32_t* end_pinned = nullptr;      // behind it: pool ends after a day, copied back one day behind the queue
   SimDev* status = nullptr;            // page-locked: the state's head (kStatusBytes), as check_device last read it
   cudaEvent_t ev_day[2] = {nullptr, nullptr};
   int last_day_kind = 0;               // DG_* of the last day launched
@@ -140,7 +140,7 @@ static RepParams make_rep(sampo_sim* s) {
   r.dec = nullptr;
   set_span_arrays(r, s->span_mem, (uint32_t)s->capacity);
   r.smallRows = s->small_mem;
-  r.smallStride = units_of((uint32_t)s->capacity, 256);  // the tiles of any pool that fits, at 256 slots
+  r.smallTiles = units_of((uint32_t)s->capacity, 256);  // the tiles of any pool that fits, at 256 slots
   r.T = s->T_dev;
   r.env = s->env_dev;
   r.seeds = s->seeds_dev;
@@ -173,7 +173,6 @@ extern "C" int sampo_destroy(sampo_sim* s) {
   for (auto& row : s->small_graph)
     for (auto& g : row) if (g) cudaGraphExecDestroy(g);
   for (auto& e : s->ev_day) if (e) cudaEventDestroy(e);
-  if (s->end_pinned) cudaFreeHost(s->end_pinned);
   if (s->status) cudaFreeHost(s->status);
   for (auto& e : s->ev) if (e) cudaEventDestroy(e);
   cudaFree(s->pool_mem[0]); cudaFree(s->pool_mem[1]);
@@ -218,7 +217,8 @@ extern "C" int sampo_create(const sampo_config* cfg, sampo_sim** out) {
     }
     if (rc) break;
     if ((e = cudaMalloc(&s->span_mem, span_array_bytes((uint32_t)C))) != cudaSuccess ||
-        (e = cudaMalloc(&s->small_mem, (size_t)units_of((uint32_t)C, 256) * kSmallRowWords * 4)) != cudaSuccess) {
+        (e = cudaMalloc(&s->small_mem, small_row_words(units_of((uint32_t)C, 256)) * 4)) != cudaSuccess ||
+        (e = cudaMemsetAsync(s->small_mem, 0, small_row_words(units_of((uint32_t)C, 256)) * 4, s->stream)) != cudaSuccess) {
       rc = cuda_fail(s, e, "span arrays");
       break;
     }
@@ -261,8 +261,9 @@ extern "C" int sampo_create(const sampo_config* cfg, sampo_sim** out) {
     s->grid_count = grid_blocks_count(1);
     s->grid_scatter = grid_blocks_scatter(1);
     size_small_step(s);
-    if ((e = cudaMallocHost(&s->end_pinned, 2 * sizeof(uint32_t))) != cudaSuccess ||
-        (e = cudaMallocHost(&s->status, sizeof(SimDev))) != cudaSuccess) { rc = cuda_fail(s, e, "pinned"); break; }
+    if ((e = cudaMallocHost(&s->status, sizeof(SimDev) + 2 * sizeof(uint32_t))) != cudaSuccess) { rc = cuda_fail(s, e, "pinned"); break; }
+    memset(s->status, 0, sizeof(SimDev));
+    s->end_pinned = reinterpret_cast<uint32_t*>(s->status + 1);  // (one page-locked allocation)
     for (auto& ev : s->ev_day) cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     for (auto& ev : s->ev) cudaEventCreate(&ev);
     if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) { rc = cuda_fail(s, e, "create"); break; }
@@ -331,7 +332,10 @@ static int reset_state(sampo_sim* s, const sampo_population& pop) {
   h.step = 0;
   h.cur = 0;
   CK(cudaMemsetAsync(s->span_mem, 0, span_array_bytes((uint32_t)s->capacity), s->stream), "span reset");
-  // the one-launch step's grid barrier and exit counters start from zero
+  // the one-launch step's grid barrier and exit counters start from zero, and
+  // its rows, unless a launch gave up at a barrier, are as it left them
+  if (s->status->error & (SAMPO_DEV_ERR_BARRIER | SAMPO_DEV_ERR_TMA))
+    CK(cudaMemsetAsync(s->small_mem, 0, small_row_words(units_of((uint32_t)s->capacity, 256)) * 4, s->stream), "row reset");
   CK(cudaMemsetAsync(&s->bat_dev->bar, 0, 2 * sizeof(uint32_t), s->stream), "barrier reset");
   CK(cudaMemcpyAsync(s->sim_dev, &h, sizeof(SimDev), cudaMemcpyHostToDevice, s->stream), "state reset");
   s->step = 0;

@@ -83,6 +83,8 @@ struct BatchDev {
   uint32_t done;              // one-launch step: CTAs finished (reset by its last CTA)
 };
 
+__host__ __device__ constexpr uint32_t units_of(uint32_t n, uint32_t size) { return n / size + (n % size ? 1u : 0u); }
+
 // The inputs of one step.
 struct CtxInputs {
   sampo_seeds sd[4];
@@ -91,8 +93,13 @@ struct CtxInputs {
   uint32_t wt;
 };
 
-// Words of the one-launch step's rows per tile (sampo_small_step.cuh).
-constexpr uint32_t kSmallRowWords = 18;
+// The one-launch step's rows for pools of up to `tiles` 256-slot tiles
+// (sampo_small_step.cuh): three sets of group records, a 16-byte word per
+// tile, four words of state. The records and the state start from zero.
+constexpr uint32_t kSmallGroupTiles = 16, kSmallGroupWords = 16;
+__host__ __device__ constexpr size_t small_row_words(uint32_t tiles) {
+  return 3 * (size_t)units_of(tiles, kSmallGroupTiles) * kSmallGroupWords + 4 * (size_t)tiles + 4;
+}
 
 // Spans: the slots a warp of the two passes takes at once, a multiple of 32.
 // A span costs a warp about a thousand instructions besides its rows (its
@@ -103,7 +110,6 @@ constexpr uint32_t kSmallRowWords = 18;
 // kSpanMax slots. A batch sets a larger smallest span (BatchDev::minSpan),
 // since its replicates share the warps.
 constexpr uint32_t kSpanMin = 128, kSpanMax = 1024, kSpanWarps = 3648;
-__host__ __device__ constexpr uint32_t units_of(uint32_t n, uint32_t size) { return n / size + (n % size ? 1u : 0u); }
 __host__ __device__ constexpr uint32_t span_size(uint32_t end, uint32_t min_span) {
   const uint32_t warps = kSpanWarps * (end / (kSpanWarps * kSpanMax) + 1u);
   uint32_t s = units_of(end, warps);
@@ -136,8 +142,8 @@ struct RepParams {
   uint4* supers;              // [max_supers] the same of 32 spans, while they are being counted; zero otherwise
   uint32_t* superPre;         // [max_supers][8] survivors of the supers before, of the decided step
   uint32_t spanStride;
-  uint32_t* smallRows;        // one-launch step: [kSmallRows + kSmallStats][smallStride], or null
-  uint32_t smallStride;
+  uint32_t* smallRows;        // one-launch step: small_row_words(smallTiles) words (16-byte aligned), or null
+  uint32_t smallTiles;
   float* T;                   // [ring] temperature per step
   sampo_environment* env;     // [ring]
   sampo_seeds* seeds;         // [ring][4] (written by the device for a device seed stream)

@@ -211,18 +211,19 @@ __device__ __forceinline__ uint32_t age_days_uncapped(float age) {
 // Returns the next state (0..7), or a negative value when the agent dies
 // this step (-2: a gravid caught by an oviposition trap, whose cycle is
 // still reported).
-template <bool FULL, bool EGGS = !FULL, bool LDG = true, bool DECIDED = false, bool WHOLE = false>
+// DAYS: the caller gives the agent's age in days (age_days).
+template <bool FULL, bool EGGS = !FULL, bool LDG = true, bool DECIDED = false, bool WHOLE = false, bool DAYS = false>
 __device__ __forceinline__ int update_agent(const StepCtx& c, const KillConst& mc, int rg, uint32_t gid, Rec& a, Acc& acc,
-                                            uint32_t code = DEC_STAYS) {
+                                            uint32_t code = DEC_STAYS, uint32_t days = 0u) {
   const bool moves = code == DEC_MOVES;  // DECIDED only
   // ---- killAgents (kernel/killAgents.cl:52-147) ----
   if (!DECIDED) {
     const uint32_t v = rng_bits(c.rng_c13[0], c.rng_z2[0], c.rng_k4[0], gid);
     uint32_t kill;
     if (rg >= IMMATURE) {
-      kill = mc.adult[age_days<WHOLE>(a.age)];
+      kill = mc.adult[DAYS ? days : age_days<WHOLE>(a.age)];
     } else if (rg == LARVA) {
-      const uint32_t d = age_days<WHOLE>(a.age);
+      const uint32_t d = DAYS ? days : age_days<WHOLE>(a.age);
       kill = LDG ? __ldg(c.larvaKill + d) : c.larvaKill[d];
       if (kill == 0u) acc.bad = 1;  // table entry not prepared
     } else {

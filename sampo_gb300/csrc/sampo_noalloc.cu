@@ -47,12 +47,12 @@ struct Results {
 
 // Largest pool, in 1024-slot tiles, that takes the one-launch step here: its
 // rows lie in the scratch. (Grids of up to 512 CTAs; a GB300 has 456.)
-constexpr uint32_t kSmallTiles = 512, kSmallStride = kSmallTiles * 4;
+constexpr uint32_t kSmallTiles = 512;
 
 struct Scratch {
   __align__(16) uint4 spans[span_array_words(SAMPO_NOALLOC_MAX_SLOTS)];
   uint8_t dec[SAMPO_NOALLOC_MAX_SLOTS];  // the count pass's decisions (the caller's pool is only read)
-  uint32_t small[kSmallRowWords * kSmallStride];
+  __align__(16) uint32_t small[small_row_words(kSmallTiles * 4)];  // (256-slot tiles; zero when the library is loaded)
   sampo_stats_row rows[2];
   alignas(16) CallState call;
 };
@@ -157,7 +157,7 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
   rp.dec = sc->dec;
   set_span_arrays(rp, sc->spans, SAMPO_NOALLOC_MAX_SLOTS);
   rp.smallRows = sc->small;
-  rp.smallStride = kSmallStride;
+  rp.smallTiles = kSmallTiles * 4;
   rp.T = sc->call.in.T;
   rp.env = sc->call.in.env;
   rp.seeds = sc->call.in.seeds;
@@ -197,6 +197,9 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
   *row = down.rows[0];
   memcpy(pop_out, down.sim + offsetof(SimDev, pop), sizeof(*pop_out));
   memcpy(bnc_out, down.sim + offsetof(SimDev, bnc), sizeof(*bnc_out));
+  // a launch that gave up at a barrier leaves its rows in no defined state
+  if ((err & (SAMPO_DEV_ERR_BARRIER | SAMPO_DEV_ERR_TMA)) && cudaMemsetAsync(sc->small, 0, sizeof(sc->small), st) != cudaSuccess)
+    return SAMPO_ERR_CUDA;
   if (err & SAMPO_DEV_ERR_CAPACITY) return SAMPO_ERR_CAPACITY;
   if (err & SAMPO_DEV_ERR_DEVRATES) return SAMPO_ERR_TEMPERATURE;
   if (err) return SAMPO_ERR_INTERNAL;

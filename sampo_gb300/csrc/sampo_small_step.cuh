@@ -43,12 +43,12 @@ constexpr int kSmallMinBlocks = 3;         // resident CTAs per SM the registers
 __host__ __device__ constexpr uint32_t small_stage(int items) { return 9 * kBlock * items * 4 + kBlock * items; }  // ten columns
 constexpr uint32_t kSmallRows = 9;         // per-tile counts: survivors by next state, eggs laid
 constexpr uint8_t kGone = 0xffu;           // flag byte of a slot without a survivor
-constexpr uint32_t kSmallHours = 24;       // hours whose inputs a CTA holds in shared memory
+constexpr uint32_t kSmallHours = 24;       // most hours of a launch, whose constants a CTA holds in shared memory
 // Per-CTA statistics of the next pool (CTA b's column, b < the tiles):
 // L1de, females, infective, cycles, sum of cycles, bites, infective bites
 // (sums) and the min and max larva age in days.
 enum : uint32_t { SA_L1 = 0, SA_FEM, SA_INF, SA_CYC, SA_SUMCYC, SA_BITES, SA_IBITES, SA_DMIN, SA_DMAX, kSmallStats };
-static_assert(kSmallRows + kSmallStats == kSmallRowWords, "the rows' array has a word per row and tile");
+static_assert(kSmallRows == 9 && SA_DMIN == 7 && kSmallStats == SA_DMAX + 1 && kSmallStats == 9, "a group's record, by fours");
 // The sizes of a kernel built for I slots per thread. A tile's prefix table
 // has, for each (round, warp) chunk of 32 slots (slot k * kBlock + tid is
 // round k of warp tid / 32) and for the whole tile, the survivors of the
@@ -112,7 +112,7 @@ struct SmallAcc {
 // counts its eggs the first time and the rest the second).
 template <int I, bool KEEP, bool EGGS, bool STATS>
 __device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelConst& mc, const sampo_population& pop,
-                                                  uint8_t* st, uint32_t lo, uint32_t end, uint2* s_ent, SmallAcc& sa) {
+                                                  bool whole, uint8_t* st, uint32_t lo, uint32_t end, uint2* s_ent, SmallAcc& sa) {
   SAMPO_TILE_CONSTANTS(I);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float* c_age = (float*)(st + 0 * kColBytes);
@@ -141,7 +141,9 @@ __device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelC
       a.female = (c_flags[i] >> 3) & 1u;
       a.bm = BM_NONE;
       sa.devoob |= (rg == LARVA) & c.devOOB;
-      const int ns = update_agent<true, true, false>(c, mc.kill, rg, g, a, t);
+      // (days from whole hours without the division: a uniform choice)
+      const uint32_t days = rg != LARVA && rg < IMMATURE ? 0u : whole ? age_days<true>(a.age) : age_days(a.age);
+      const int ns = update_agent<true, true, false, false, false, true>(c, mc.kill, rg, g, a, t, DEC_STAYS, days);
       if (ns >= 0) {
         if (a.bm != BM_NONE) {  // the owed normal draw (include/gpuRand.h:56-63)
           const uint32_t v = finish_box_muller(c, mc, g, a.bm, a.batches);
@@ -153,8 +155,9 @@ __device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelC
         fb = (uint8_t)(ns | (a.female << 3));
         if (STATS) {  // kernel/calcL1de.cl:28-30, kernel/calcGender.cl:24-37
           if (ns == LARVA) {
-            sa.l1 += age_days_uncapped(a.age);
-            const uint32_t dd = age_days(a.age);
+            const uint32_t du = whole ? whole_age_days(a.age) : age_days_uncapped(a.age);
+            const uint32_t dd = whole ? min(du, 99u) : age_days(a.age);
+            sa.l1 += du;
             sa.dmin = min(sa.dmin, dd); sa.dmax = max(sa.dmax, dd);
           } else if (ns >= IMMATURE && a.female) {
             sa.fem += 1u;
@@ -267,87 +270,117 @@ __device__ __forceinline__ void small_scatter_tile(const uint8_t* st, const uint
   }
 }
 
-// Phase 2, all threads: over the per-tile counts (rows 0..8), the sums of
-// tiles [0, t) into s_ex and, with `totals`, of all nold tiles into s_tot,
-// followed by the statistics rows over the columns of the CTAs that held
-// tiles (min(nold, G); sums, min and max) into s_tot[kSmallRows ..]. Thread
-// i takes columns i, i + blockDim.x, ...: every row of a column is loaded at
-// once, so one round trip to L2 serves them all. Rows are state-major:
-// rows[row * stride + column], read through L2. Ends synchronised.
-constexpr uint32_t kSumWords = 2 * kSmallRows + kSmallStats;  // ex, tot, statistics
-__device__ __forceinline__ void small_sum_rows(const uint32_t* rows, uint32_t stride, uint32_t nold, uint32_t t,
-                                               bool totals, uint32_t* s_ex, uint32_t* s_tot,
-                                               uint32_t (*s_part)[kSumWords]) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t ex[kSmallRows], tot[kSmallRows], st[kSmallStats];
+// What the CTAs tell each other of an hour (RepParams::smallRows): per tile its
+// survivors by next state (16 bits each, 16 bytes), and per group of 16 tiles
+// a record of 16 words that the CTAs of its tiles add to:
+//   0-3  survivors by next state, 16 bits each   4  eggs laid
+//   5 on  statistics of the next pool (SA_*; the youngest larva as the largest
+//         SA_YOUNG - days, so that zero is the identity of every word)
+// A CTA reads the groups' records and the tiles of its own group. (Every CTA
+// reading 18 words of every tile took 2.3 us of an hour with three tiles,
+// where its 27 reductions on every warp bound it, and 4 us with 300, where
+// the L2 slices that hold the rows did; the hour went from 7.7 to 6.7 us and
+// from 13.3 to 11.8 us.) Three sets of records rotate through the hours: the
+// one in use, and the next, cleared meanwhile.
+struct SmallRows {
+  uint4* tiles;
+  uint32_t* groups;    // [3][stride][16]
+  uint32_t* state;     // the set the next launch starts with (all zero); records of the next one and of the one after that
+                       // that may not be
+  uint32_t stride;     // records of a set
+};
+constexpr uint32_t kGroupTiles = kSmallGroupTiles, kGroupWords = kSmallGroupWords, SA_YOUNG = 128;
+__device__ __forceinline__ SmallRows small_rows(const RepParams& rp) {
+  SmallRows r;
+  r.stride = units_of(rp.smallTiles, kGroupTiles);
+  r.groups = rp.smallRows;
+  r.tiles = reinterpret_cast<uint4*>(r.groups + 3 * (size_t)r.stride * kGroupWords);
+  r.state = reinterpret_cast<uint32_t*>(r.tiles + rp.smallTiles);
+  return r;
+}
+// Phase 2, all threads: the survivors of tiles [0, t) into s_ex (two parts:
+// the groups before t's, and the tiles before t in its own) and, with
+// `totals`, those of all nold tiles, their eggs and the statistics into
+// s_tot. Warp 0 reads the groups' records once, four lanes each (all CTAs read
+// the same few lines, and the L2 slices that hold them serve them one after
+// the other), warp 1 the tiles of t's group. Ends synchronised.
+__device__ __forceinline__ void small_sum_rows(const SmallRows& rows, uint32_t set, uint32_t nold, uint32_t t, bool totals,
+                                               uint32_t (*s_ex)[8], uint32_t* s_tot) {
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, gt = t / kGroupTiles, q = lane & 3u;
+  auto unpack = [](const uint4& c, uint32_t (&v)[8]) {
+    v[0] = c.x & 0xffffu; v[1] = c.x >> 16; v[2] = c.y & 0xffffu; v[3] = c.y >> 16;
+    v[4] = c.z & 0xffffu; v[5] = c.z >> 16; v[6] = c.w & 0xffffu; v[7] = c.w >> 16;
+  };
+  if (warp == 0) {
+    const uint4* g = reinterpret_cast<const uint4*>(rows.groups + (size_t)set * rows.stride * kGroupWords);
+    const uint32_t lim = totals ? units_of(nold, kGroupTiles) : gt;
+    uint32_t sum[8] = {0, 0, 0, 0, 0, 0, 0, 0}, ex[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // q = 0: survivors; else the record's words 4q on
+    const bool widest = q == 3u;  // the youngest and oldest larva
+#pragma unroll 1
+    for (uint32_t j = lane >> 2; j < lim; j += 8u) {
+      const uint4 c = __ldcg(g + (size_t)j * (kGroupWords / 4) + q);
+      uint32_t v[8] = {c.x, c.y, c.z, c.w, 0u, 0u, 0u, 0u};
+      if (q == 0u) unpack(c, v);
 #pragma unroll
-  for (int r = 0; r < (int)kSmallRows; r++) ex[r] = tot[r] = 0;
-#pragma unroll
-  for (int k = 0; k < (int)kSmallStats; k++) st[k] = k == (int)SA_DMIN ? 0xffffffffu : 0u;
-  const uint32_t lim = totals ? nold : t;
-  for (uint32_t j = tid; j < lim; j += blockDim.x) {
-    uint32_t v[kSmallRows];
-#pragma unroll
-    for (int r = 0; r < (int)kSmallRows; r++) v[r] = __ldcg(rows + (size_t)r * stride + j);
-#pragma unroll
-    for (int r = 0; r < (int)kSmallRows; r++) {
-      tot[r] += v[r];
-      ex[r] += j < t ? v[r] : 0u;
+      for (int k = 0; k < 8; k++) {
+        sum[k] = widest ? max(sum[k], v[k]) : sum[k] + v[k];
+        ex[k] += j < gt ? v[k] : 0u;
+      }
     }
-  }
-  if (totals) {
-    const uint32_t cols = min(nold, gridDim.x);  // one column per CTA with tiles
-    for (uint32_t j = tid; j < cols; j += blockDim.x) {
-      uint32_t v[kSmallStats];
 #pragma unroll
-      for (int k = 0; k < (int)kSmallStats; k++) v[k] = __ldcg(rows + (size_t)(kSmallRows + k) * stride + j);
+    for (int o = 4; o < 32; o <<= 1) {
 #pragma unroll
-      for (int k = 0; k < (int)kSmallStats; k++)
-        st[k] = k == (int)SA_DMIN ? min(st[k], v[k]) : k == (int)SA_DMAX ? max(st[k], v[k]) : st[k] + v[k];
+      for (int k = 0; k < 8; k++) {
+        const uint32_t x = __shfl_xor_sync(0xffffffffu, sum[k], o);
+        sum[k] = widest ? max(sum[k], x) : sum[k] + x;
+        ex[k] += __shfl_xor_sync(0xffffffffu, ex[k], o);
+      }
     }
-  }
+    if (lane == 0u) {
 #pragma unroll
-  for (int r = 0; r < (int)kSmallRows; r++) {
-    ex[r] = __reduce_add_sync(0xffffffffu, ex[r]);
-    tot[r] = __reduce_add_sync(0xffffffffu, tot[r]);
-  }
-#pragma unroll
-  for (int k = 0; k < (int)kSmallStats; k++)
-    st[k] = k == (int)SA_DMIN ? __reduce_min_sync(0xffffffffu, st[k])
-          : k == (int)SA_DMAX ? __reduce_max_sync(0xffffffffu, st[k]) : __reduce_add_sync(0xffffffffu, st[k]);
-  if (lane == 0) {
-#pragma unroll
-    for (int r = 0; r < (int)kSmallRows; r++) {
-      s_part[warp][r] = ex[r];
-      s_part[warp][kSmallRows + r] = tot[r];
+      for (int k = 0; k < 8; k++) s_ex[0][k] = ex[k];
     }
+    if (totals && lane < 4u) {
+      if (widest) sum[0] = sum[0] ? SA_YOUNG - sum[0] : 0xffffffffu;
+      // eggs laid and the statistics follow the survivors, as in the record
+      uint32_t* to = s_tot + (q ? 4u + 4u * q : 0u);
 #pragma unroll
-    for (int k = 0; k < (int)kSmallStats; k++) s_part[warp][2 * kSmallRows + k] = st[k];
-  }
-  __syncthreads();
-  if (tid < (int)kSumWords) {
-    const int k = tid - 2 * (int)kSmallRows;  // statistic, for the last kSmallStats words
-    uint32_t x = s_part[0][tid];
-    for (int w = 1; w < kWarps; w++) {
-      const uint32_t y = s_part[w][tid];
-      x = k == (int)SA_DMIN ? min(x, y) : k == (int)SA_DMAX ? max(x, y) : x + y;
+      for (uint32_t k = 0; k < 8; k++)
+        if (q == 0u || k < (widest ? 2u : 4u)) to[k] = sum[k];
     }
-    if (tid < (int)kSmallRows) s_ex[tid] = x;
-    else if (totals) s_tot[tid - kSmallRows] = x;
+  } else if (warp == 1) {
+    uint32_t v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (lane < t - gt * kGroupTiles) unpack(__ldcg(rows.tiles + gt * kGroupTiles + lane), v);
+#pragma unroll
+    for (int o = 1; o < (int)kGroupTiles; o <<= 1) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+    if (lane == 0u) {
+#pragma unroll
+      for (int k = 0; k < 8; k++) s_ex[1][k] = v[k];
+    }
   }
   __syncthreads();
 }
 
 // Phase 1's end: the CTA's statistics of the next pool (its tiles) to its
-// column of the statistics rows, in two halves around a CTA barrier: each
-// warp's totals into s_red (every thread), then the CTA's totals out by the
-// threads of warp `w` (the other warps may do other work meanwhile).
+// row, in two halves around a CTA barrier: each warp's totals into s_red
+// (every thread), then the CTA's totals out by the threads of warp `w` (the
+// other warps may do other work meanwhile). ONE: the CTA has one tile, so that
+// a warp's counts fit in 8 bits each (32 * I agents).
+template <bool ONE>
 __device__ __forceinline__ void small_stats_warps(const SmallAcc& sa, uint32_t (*s_red)[kSmallStats]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t v[kSmallStats] = {sa.l1, sa.fem, sa.inf, sa.acc.cycles, sa.acc.sumCycles, sa.acc.bites, sa.acc.infectBites,
                              sa.dmin, sa.dmax};
+  if (ONE) {
+    const uint32_t x = __reduce_add_sync(0xffffffffu, v[SA_FEM] | (v[SA_INF] << 8) | (v[SA_CYC] << 16) | (v[SA_BITES] << 24));
+    v[SA_FEM] = x & 0xffu; v[SA_INF] = (x >> 8) & 0xffu; v[SA_CYC] = (x >> 16) & 0xffu; v[SA_BITES] = x >> 24;
+  }
 #pragma unroll
-  for (int j = 0; j < (int)SA_DMIN; j++) v[j] = __reduce_add_sync(0xffffffffu, v[j]);
+  for (int j = 0; j < (int)SA_DMIN; j++)
+    if (!ONE || j == (int)SA_L1 || j == (int)SA_SUMCYC || j == (int)SA_IBITES) v[j] = __reduce_add_sync(0xffffffffu, v[j]);
   v[SA_DMIN] = __reduce_min_sync(0xffffffffu, v[SA_DMIN]);
   v[SA_DMAX] = __reduce_max_sync(0xffffffffu, v[SA_DMAX]);
   if (lane == 0) {
@@ -355,17 +388,30 @@ __device__ __forceinline__ void small_stats_warps(const SmallAcc& sa, uint32_t (
     for (int j = 0; j < (int)kSmallStats; j++) s_red[warp][j] = v[j];
   }
 }
-__device__ __forceinline__ void small_stats_store(uint32_t* rows, uint32_t stride, uint32_t b,
-                                                  const uint32_t (*s_red)[kSmallStats], int w) {
-  const int k = (int)threadIdx.x - 32 * w;
-  if (k >= 0 && k < (int)kSmallStats) {
+__device__ __forceinline__ void small_stats_store(const SmallRows& rows, uint32_t set, uint32_t b, const uint32_t (*s_red)[kSmallStats], int w) {
+  const uint32_t k = threadIdx.x - 32u * (uint32_t)w;
+  if (k < kSmallStats) {
     uint32_t x = s_red[0][k];
+#pragma unroll
     for (int i = 1; i < kWarps; i++) {
       const uint32_t y = s_red[i][k];
-      x = k == (int)SA_DMIN ? min(x, y) : k == (int)SA_DMAX ? max(x, y) : x + y;
+      x = k == SA_DMIN ? min(x, y) : k == SA_DMAX ? max(x, y) : x + y;
     }
-    __stcg(rows + (size_t)(kSmallRows + k) * stride + b, x);
+    uint32_t* to = rows.groups + ((size_t)set * rows.stride + b / kGroupTiles) * kGroupWords + 5 + k;
+    if (k == SA_DMIN) x = x == 0xffffffffu ? 0u : SA_YOUNG - x;
+    if (x) {
+      if (k >= SA_DMIN) atomicMax(to, x);
+      else atomicAdd(to, x);
+    }
   }
+}
+// Warp 0: tile t's survivors (tw: of next state `lane`, on lanes 0..7) and eggs.
+__device__ __forceinline__ void small_counts_store(const SmallRows& rows, uint32_t set, uint32_t t, uint32_t tw, uint32_t eggs) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t lo = __shfl_sync(0xffffffffu, tw, (2u * lane) & 7u), hi = __shfl_sync(0xffffffffu, tw, (2u * lane + 1u) & 7u);
+  const uint32_t x = lane < 4u ? lo | (hi << 16) : eggs;
+  if (lane < 4u) __stcg(reinterpret_cast<uint32_t*>(rows.tiles + t) + lane, x);
+  if (lane < 5u && x) atomicAdd(rows.groups + ((size_t)set * rows.stride + t / kGroupTiles) * kGroupWords + lane, x);
 }
 
 // Every thread waits (bounded) for the bulk copies of the stage's tile;
@@ -404,10 +450,11 @@ __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence
 // statistics row, step constants and larval table itself from the same
 // totals (the k_publish arithmetic; the last CTA, the one least likely to
 // hold a tile, also writes them to the replicate's state for the host) before
-// it waits there; then the next hour's tile copies go out. The step inputs of
-// the launch's hours are read into shared memory at its start (the host
-// writes them before the launch). The rows (smallRows: kSmallRows +
-// kSmallStats words per column) are read through L2. The pool the scatter wrote with ordinary stores is
+// it waits there; then the next hour's tile copies go out. The constants
+// of the launch's hours are prepared in shared memory at its start, one hour
+// per thread (the host writes their inputs before the launch); only the
+// biomass and the larval table wait for the hour's pool. The rows (SmallRows)
+// are read through L2. The pool the scatter wrote with ordinary stores is
 // read by the next hour's bulk copies after proxy fences.
 template <int I>
 __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(KParams p, uint32_t nsteps) {
@@ -417,12 +464,12 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
   __shared__ ModelConst s_mc;
   __shared__ uint32_t s_kill[100];
   __shared__ sampo_population s_pop;
-  __shared__ CtxInputs s_in[kSmallHours];
+  __shared__ StepCtx s_ctx[kSmallHours];
   __shared__ __align__(8) uint64_t s_mbar;
   __shared__ uint2 s_ent[kChunks];
   __shared__ __align__(16) uint32_t s_tab[(kChunks + 1) * kPreEntryWords];
-  __shared__ uint32_t s_ex[kSmallRows], s_tot[kSmallRows + kSmallStats], s_d0[8], s_ne[kWarps];
-  __shared__ uint32_t s_red[kWarps][kSmallStats], s_part[kWarps][kSumWords];
+  __shared__ uint32_t s_ex[2][8], s_tot[kSmallRows + kSmallStats], s_d0[8], s_ne[kWarps];
+  __shared__ uint32_t s_red[kWarps][kSmallStats];
   __shared__ uint32_t s_flag, s_ok, s_last;
   __shared__ uint32_t s_active, s_end, s_nold, s_cur, s_cap, s_step, s_stop;
   __shared__ float s_cc;
@@ -432,14 +479,19 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
   const uint32_t G = gridDim.x, b = blockIdx.x;
   uint32_t phase = 0, barriers = 0;
   bool met = true, ok = true;
-  const uint32_t stride = rp.smallStride;  // >= the tiles of any pool that fits, at 256-slot tiles
-  uint32_t* rows = rp.smallRows;  // [kSmallRows + kSmallStats][stride]
+  __shared__ SmallRows rows;            // (in shared memory: registers are short)
+  __shared__ uint32_t s_set, s_dirty[3];  // the set in use; records of the next one (1) and the one after (2) that may not be zero
+  const bool whole = !p.wide;     // ages are whole hours (state_cols)
 
   // ---- the replicate's state at the launch (the previous kernel wrote it) ----
   if (tid == 0) {
     mbar_init(&s_mbar);
     fence_mbar_init();
     const uint32_t active = sim->active;
+    rows = small_rows(rp);
+    s_set = __ldcg(rows.state);
+    s_dirty[1] = __ldcg(rows.state + 1);
+    s_dirty[2] = __ldcg(rows.state + 2);
     s_pop = sim->pop;
     s_active = active;
     s_end = active ? s_pop.r[GRAVID].end : 0u;
@@ -459,8 +511,15 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
   load_model_const(p.mc, s_mc);
   __syncthreads();
   if (tid == 0) s_c.larvaKill = s_kill;
-  // the inputs of the steps that follow the launch's hours
-  for (uint32_t j = tid; j < min(nsteps, kSmallHours); j += blockDim.x) load_ctx_inputs(rp, s_step + 1u + j, s_in[j]);
+  // the constants of the steps that follow the launch's hours, but for their pool's biomass
+  nsteps = min(nsteps, kSmallHours);
+  for (uint32_t j = tid; j < nsteps; j += blockDim.x) {
+    CtxInputs in;
+    load_ctx_inputs(rp, s_step + 1u + j, in);
+    StepCtx c;
+    make_ctx(in, s_kill, s_pop, c);
+    s_ctx[j] = c;
+  }
   __syncthreads();
 
   for (uint32_t hour = 0; hour < nsteps; hour++) {
@@ -470,6 +529,8 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     sa.acc = Acc{0, 0, 0, 0, 0, 0};
     sa.l1 = sa.fem = sa.inf = sa.dmax = sa.devoob = sa.tilebad = 0;
     sa.dmin = 0xffffffffu;
+
+    const uint32_t set = s_set, stale = s_dirty[1];
 
     // ---- phase 1: decide (and, for tile b, finish) every tile of this CTA ----
     if (nold > G && b < nold) {
@@ -487,16 +548,15 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           if (!ok) break;
         }
         const uint32_t eggs_before = sa.acc.newEggs;
-        small_update_tile<I, false, true, true>(s_c, s_mc, s_pop, stage, t * kTile, end, s_ent, sa);
+        small_update_tile<I, false, true, true>(s_c, s_mc, s_pop, whole, stage, t * kTile, end, s_ent, sa);
         const uint32_t ne = __reduce_add_sync(0xffffffffu, sa.acc.newEggs - eggs_before);
         if (lane == 0) s_ne[warp] = ne;
         __syncthreads();
         if (warp == 0) {
           const uint32_t tw = small_build_table<I>(s_ent, s_tab);
-          if (lane < 8) __stcg(rows + (size_t)lane * stride + t, tw);
           uint32_t e = lane < kWarps ? s_ne[lane] : 0u;
           e = __reduce_add_sync(0xffffffffu, e);
-          if (lane == 0) __stcg(rows + (size_t)8 * stride + t, e);
+          small_counts_store(rows, set, t, tw, e);
         }
         __syncthreads();  // the stage is read before the next copy overwrites it
       }
@@ -507,30 +567,29 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
         }
         ok = small_wait_stage(&s_mbar, phase);
         if (ok) {
-          small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, stage, b * kTile, end, s_ent, sa);  // counted above
-          small_stats_warps(sa, s_red);
+          small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, whole, stage, b * kTile, end, s_ent, sa);  // counted above
+          small_stats_warps<false>(sa, s_red);
           __syncthreads();
           if (warp == 0) (void)small_build_table<I>(s_ent, s_tab);
-          else if (warp == 1) small_stats_store(rows, stride, b, s_red, 1);
+          else if (warp == 1) small_stats_store(rows, set, b, s_red, 1);
         }
       }
     } else if (b < nold) {
       ok = small_wait_stage(&s_mbar, phase);
       if (ok) {
         const uint32_t eggs_before = sa.acc.newEggs;
-        small_update_tile<I, true, true, true>(s_c, s_mc, s_pop, stage, b * kTile, end, s_ent, sa);
+        small_update_tile<I, true, true, true>(s_c, s_mc, s_pop, whole, stage, b * kTile, end, s_ent, sa);
         const uint32_t ne = __reduce_add_sync(0xffffffffu, sa.acc.newEggs - eggs_before);
         if (lane == 0) s_ne[warp] = ne;
-        small_stats_warps(sa, s_red);
+        small_stats_warps<true>(sa, s_red);
         __syncthreads();
         if (warp == 0) {  // the tile's table and counts
           const uint32_t tw = small_build_table<I>(s_ent, s_tab);
-          if (lane < 8) __stcg(rows + (size_t)lane * stride + b, tw);
           uint32_t e = lane < kWarps ? s_ne[lane] : 0u;
           e = __reduce_add_sync(0xffffffffu, e);
-          if (lane == 0) __stcg(rows + (size_t)8 * stride + b, e);
+          small_counts_store(rows, set, b, tw, e);
         } else if (warp == 1) {  // meanwhile the CTA's statistics
-          small_stats_store(rows, stride, b, s_red, 1);
+          small_stats_store(rows, set, b, s_red, 1);
         }
       }
     }
@@ -541,7 +600,17 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     ok = s_ok != 0;  // this CTA's copies all landed
 
     // ---- phase 2: totals, next layout, this tile's first slots; scatter ----
-    small_sum_rows(rows, stride, nold, b < nold ? b : nold, true, s_ex, s_tot, s_part);
+    small_sum_rows(rows, set, nold, b < nold ? b : nold, true, s_ex, s_tot);
+    {  // the next hour's records (nobody has read them since the hour before the last)
+      const uint32_t n = set == 2u ? 0u : set + 1u;
+      uint32_t* next = rows.groups + (size_t)n * rows.stride * kGroupWords;
+      for (uint32_t i = b * blockDim.x + tid; i < stale * kGroupWords; i += G * blockDim.x) __stcg(next + i, 0u);
+      if (tid == 0) {  // (read again past the next CTA barrier at the earliest)
+        s_set = n;
+        s_dirty[1] = s_dirty[2];
+        s_dirty[2] = units_of(nold, kGroupTiles);
+      }
+    }
     uint32_t tot[8], base[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) tot[k] = s_tot[k];
@@ -552,7 +621,11 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     const bool write = ok && met && fits;
     const DevPool dst = rp.pool[s_cur ^ 1u];
     if (write && b < nold) {
-      if (tid < 8) s_d0[tid] = base[tid] + s_ex[tid];
+      // (by constant indexes: base stays in registers)
+      uint32_t mine = base[0];
+#pragma unroll
+      for (int k = 1; k < 8; k++) mine = tid == k ? base[k] : mine;
+      if (tid < 8) s_d0[tid] = mine + s_ex[0][tid] + s_ex[1][tid];
       __syncthreads();
       small_scatter_tile<I>(stage, s_tab, s_d0, dst, sa.tilebad);
       // more tiles than CTAs: the other tiles of this CTA, loaded and updated again
@@ -563,13 +636,17 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           small_issue_tile<I>(rp.pool[s_cur], stage, &s_mbar, t * kTile, min((uint32_t)kTile, end - t * kTile));
         }
         if (!small_wait_stage(&s_mbar, phase)) { ok = false; break; }
-        small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, stage, t * kTile, end, s_ent, sa);
-        small_sum_rows(rows, stride, nold, t, false, s_ex, s_tot, s_part);
+        small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, whole, stage, t * kTile, end, s_ent, sa);
+        small_sum_rows(rows, set, nold, t, false, s_ex, s_tot);
         if (warp == 0) {
           const uint32_t tw = small_build_table<I>(s_ent, s_tab);
           // the update again must give the counts of phase 1
-          if (lane < 8 && tw != __ldcg(rows + (size_t)lane * stride + t)) sa.tilebad = 1;
-          if (lane < 8) s_d0[lane] = base[lane] + s_ex[lane];
+          if (lane < 8 && tw != ((__ldcg(reinterpret_cast<const uint32_t*>(rows.tiles + t) + lane / 2) >> (16 * (lane & 1))) & 0xffffu))
+            sa.tilebad = 1;
+          uint32_t mine = base[0];
+#pragma unroll
+          for (int k = 1; k < 8; k++) mine = lane == k ? base[k] : mine;
+          if (lane < 8) s_d0[lane] = mine + s_ex[0][lane] + s_ex[1][lane];
         }
         if (__syncthreads_or(sa.tilebad)) break;
         small_scatter_tile<I>(stage, s_tab, s_d0, dst, sa.tilebad);
@@ -627,10 +704,8 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     np.numPotentiallyInfective = st[SA_INF];
     __syncthreads();  // every thread is past its last read of s_c, s_kill and s_pop
     if (tid == 0) {
-      CtxInputs& in = s_in[hour % kSmallHours];
-      if (hour >= kSmallHours) load_ctx_inputs(rp, step, in);  // (its slot's hour is done)
-      StepCtx c;
-      make_ctx(in, sim->larvaKill[step & 1u], np, c);  // the global table: the last CTA stores this one
+      const uint32_t biomass = np.numLarvae1DayEquiv + np.r[EGG].end + (np.r[PUPA].end - np.r[PUPA].start);
+      s_c.totalBiomass = biomass;
       if (b == G - 1u) {
         // the replicate's state and the coming step's row for the host
         sampo_bites_cycles nbnc;
@@ -646,7 +721,8 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           moved += s_tot[k];
         }
         if (shared_end && moved) sim->warn = __ldcg(&sim->warn) | SAMPO_DEV_WARN_REF_LAYOUT;
-        sim->ctx[step & 1u] = c;
+        sim->ctx[step & 1u].totalBiomass = biomass;
+        sim->ctx[step & 1u].larvaKill = sim->larvaKill[step & 1u];
         sim->pop = np;
         sim->bnc = nbnc;
         sim->step = step;
@@ -657,8 +733,6 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
         rp.rows[step % rp.ring] = row;
         if (!active) sim->active = 0;
       }
-      c.larvaKill = s_kill;
-      s_c = c;
       s_pop = np;
       s_step = step;
       s_cur ^= 1u;
@@ -666,9 +740,20 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
       s_nold = next_nold;
       s_active = active;
     }
-    {  // the next hour's larval table (every CTA; the last one also stores it)
+    if (warp == kWarps - 1) {  // the next hour's constants (the last CTA also stores them)
+      const StepCtx& c = s_ctx[hour];
+      const uint32_t* from = reinterpret_cast<const uint32_t*>(&c);
+      const uint32_t bio = (uint32_t)(&c.totalBiomass - from), tab = (uint32_t)(reinterpret_cast<const uint32_t*>(&c.larvaKill) - from);
+      uint32_t* const to = reinterpret_cast<uint32_t*>(&s_c);
+      uint32_t* const out = reinterpret_cast<uint32_t*>(&sim->ctx[step & 1u]);
+      for (uint32_t k = lane; k < sizeof(StepCtx) / 4; k += 32u) {
+        if (k == bio) continue;
+        to[k] = from[k];
+        if (b == G - 1u && k != tab && k != tab + 1u) out[k] = from[k];
+      }
+    } else {  // the next hour's larval table (every CTA; the last one also stores it)
       const uint32_t dmin = st[SA_DMIN], dmax = st[SA_DMAX], l1 = np.numLarvae1DayEquiv;
-      for (int d = tid - 32; d >= 0 && d < 100; d += blockDim.x - 32) {
+      for (int d = tid - 32; d >= 0 && d < 100; d += blockDim.x - 64) {
         const uint32_t k = larva_kill_entry((uint32_t)d, dmin, dmax, l1, s_cc);
         s_kill[d] = k;
         if (b == G - 1u) sim->larvaKill[step & 1u][d] = k;
@@ -698,6 +783,9 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     if (s_last) {
       p.bat->bar = 0u;
       p.bat->done = 0u;
+      rows.state[0] = s_set;
+      rows.state[1] = s_dirty[1];
+      rows.state[2] = s_dirty[2];
     }
   }
 }
