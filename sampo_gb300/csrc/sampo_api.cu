@@ -34,7 +34,6 @@ struct sampo_sim {
   void* span_mem = nullptr;            // span arrays (set_span_arrays)
   uint32_t* small_mem = nullptr;       // the one-launch step's rows
   bool wide = false;                   // the pool holds whole records (state_cols)
-  bool full_cols = false;              // a narrow pool's implied columns are written out
   float* T_dev = nullptr;
   sampo_environment* env_dev = nullptr;
   sampo_seeds* seeds_dev = nullptr;
@@ -342,15 +341,6 @@ static int reset_state(sampo_sim* s, const sampo_population& pop) {
   return SAMPO_OK;
 }
 
-// The implied columns of a narrow pool, for readers of whole records.
-static cudaError_t widen(sampo_sim* s) {
-  if (s->wide || s->full_cols) return cudaSuccess;
-  const cudaError_t e = launch_widen(make_params(s), s->stream);
-  s->launches += 1;
-  s->full_cols = e == cudaSuccess;
-  return e;
-}
-
 static void drop_day_graph(sampo_sim* s);
 static void drop_small_graphs(sampo_sim* s);
 
@@ -403,9 +393,7 @@ extern "C" int sampo_init_population(sampo_sim* s, uint32_t n, const sampo_seeds
   if (rc) return rc;
   CK(cudaMemcpyAsync(s->init_seeds_dev, init_seeds, 4 * sizeof(sampo_seeds), cudaMemcpyHostToDevice, s->stream), "seeds");
   KParams p = make_params(s);
-  // the one-launch step reads whole records: a pool it will step gets them at once
-  s->full_cols = n <= s->small_tiles * (uint64_t)kTile;
-  CK(launch_init_eggs(p, n, s->T_host[0], s->init_seeds_dev, age_days_max, age_seed, s->full_cols, s->stream), "initAgents");
+  CK(launch_init_eggs(p, n, s->T_host[0], s->init_seeds_dev, age_days_max, age_seed, false, s->stream), "initAgents");
   return publish_initial(s, pop.r[7].end, false);
 }
 
@@ -434,7 +422,6 @@ extern "C" int sampo_load_pool(sampo_sim* s, const sampo_population* pop, const 
   for (uint32_t i = 0; i < n; i++) flags[i] = (uint8_t)((v->state[i] & 7u) | ((v->isFemale[i] ? 1u : 0u) << 3));
   CK(cudaMemcpyAsync(P.flags, flags.data(), n, cudaMemcpyHostToDevice, s->stream), "pool upload");
   CK(cudaStreamSynchronize(s->stream), "pool upload");
-  s->full_cols = true;
   return publish_initial(s, n, true);
 }
 
@@ -451,7 +438,6 @@ static int check_device(sampo_sim* s) {
 }
 
 static cudaError_t launch_hours(sampo_sim* s, const KParams& p, uint32_t nsteps, uint32_t* launches) {
-  s->full_cols = false;
   return launch_steps(p, nsteps, true, s->grid_count, s->grid_scatter, s->items, s->stream, launches);
 }
 
@@ -481,7 +467,6 @@ extern "C" int sampo_step(sampo_sim* s, const sampo_environment* env, float temp
   uint32_t n = 1;
   if (!s->timing && takes_small_step(s)) {
     // (the pool's end is exact here: the tiles need no room to grow)
-    CK(widen(s), "whole records");
     CK(launch_begin_step(p, in, slot, s->stream), "step inputs");
     const int items = s->small_items ? s->small_items : small_items_for(s->known_end, 1, s->small_grid);
     CK(launch_small_hour(p, s->known_end, items, s->small_grid, s->stream), "one-launch step");
@@ -659,7 +644,6 @@ static int queue_run(sampo_sim* s, uint32_t nsteps, sampo_stats_row* rows, bool 
     const uint32_t first = s->step;
     if (s->timing) {
       for (uint32_t i = 0; i < n; i++) {
-        s->full_cols = false;
         CK(cudaEventRecord(s->ev[0], s->stream), "event");
         CK(launch_count(p, s->grid_count, s->stream, s->items), "count kernel");
         CK(cudaEventRecord(s->ev[1], s->stream), "event");
@@ -687,8 +671,6 @@ static int queue_run(sampo_sim* s, uint32_t nsteps, sampo_stats_row* rows, bool 
         int kind = 0;
         int rc = day_graph_for(s, &gx, &kernels, &kind);
         if (rc) return rc;
-        if (kind == DG_PLAIN) s->full_cols = false;
-        else CK(widen(s), "whole records");
         CK(cudaGraphLaunch(gx, s->stream), "day graph");
         s->launches += kernels;
         s->last_day_kind = kind;
@@ -933,7 +915,6 @@ extern "C" int sampo_checkpoint_load(sampo_sim* s, const char* path) {
   CK(cudaMemsetAsync(s->span_mem, 0, span_array_bytes((uint32_t)s->capacity), s->stream), "span reset");
   CK(cudaMemcpyAsync(s->sim_dev, &h, sizeof(SimDev), cudaMemcpyHostToDevice, s->stream), "state");
   s->step = hd.step;
-  s->full_cols = true;
   const int rc = publish_initial(s, hd.pop.r[7].end, true);
   if (rc) return rc;
   sampo_population p;

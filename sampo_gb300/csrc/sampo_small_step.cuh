@@ -28,9 +28,9 @@
 // takes tiles b + G, b + 2G, ... (G CTAs); their decisions are counted in
 // phase 1 and the tile is loaded and updated again in phase 2.
 //
-// It reads and writes whole records: a narrow pool (state_cols) that the other
-// passes wrote last has its implied columns written out first (k_widen).
-//
+// A narrow pool's records are read and written by the columns of their state
+// (state_cols), as in the other passes (a year from 1e4 eggs: 11.9 us an hour
+// with whole records, 11.0 so).
 // A species compiled at run time has it too (20,000 eggs for a month: 21.7 ms
 // with three kernels an hour, 13.2 ms with one launch a day).
 #pragma once
@@ -135,9 +135,14 @@ __device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelC
     uint8_t fb = kGone;
     if (rg >= 0) {
       Rec a;
-      a.age = c_age[i]; a.his = c_his[i]; a.delay = c_delay[i]; a.sporo = c_sporo[i];
-      a.uni = c_uni[i]; a.avail = c_avail[i]; a.cycle = c_cycle[i]; a.hbc = c_hbc[i];
-      a.batches = c_batches[i];
+      // (state_cols: what a narrow record's state implies is not there)
+      a.age = c_age[i]; a.delay = c_delay[i];
+      a.uni = !whole || rg != EGG ? c_uni[i] : 0u;
+      a.his = !whole || rg >= PUPA ? c_his[i] : rg == EGG ? a.age : a.age - 24.0f;
+      a.sporo = 0.0f; a.avail = a.cycle = a.hbc = a.batches = 0u;
+      if (!whole || rg >= BMS) {
+        a.sporo = c_sporo[i]; a.avail = c_avail[i]; a.cycle = c_cycle[i]; a.hbc = c_hbc[i]; a.batches = c_batches[i];
+      }
       a.female = (c_flags[i] >> 3) & 1u;
       a.bm = BM_NONE;
       sa.devoob |= (rg == LARVA) & c.devOOB;
@@ -165,9 +170,12 @@ __device__ __forceinline__ void small_update_tile(const StepCtx& c, const ModelC
           }
         }
         if (KEEP) {
-          c_age[i] = a.age; c_his[i] = a.his; c_delay[i] = a.delay; c_sporo[i] = a.sporo;
-          c_uni[i] = a.uni; c_avail[i] = a.avail; c_cycle[i] = a.cycle; c_hbc[i] = a.hbc;
-          c_batches[i] = a.batches;
+          c_age[i] = a.age; c_delay[i] = a.delay;
+          if (!whole || ns != EGG) c_uni[i] = a.uni;
+          if (!whole || ns >= PUPA) c_his[i] = a.his;
+          if (!whole || ns >= BMS) {
+            c_sporo[i] = a.sporo; c_avail[i] = a.avail; c_cycle[i] = a.cycle; c_hbc[i] = a.hbc; c_batches[i] = a.batches;
+          }
         }
       }
     }
@@ -231,7 +239,7 @@ __device__ __forceinline__ uint32_t small_build_table(const uint2* s_ent, uint32
 // state in earlier chunks (s_tab) + the rank within the chunk. A survivor
 // whose slot falls outside its chunk's run sets tilebad and is not stored.
 template <int I>
-__device__ __forceinline__ void small_scatter_tile(const uint8_t* st, const uint32_t* s_tab, const uint32_t* s_d0,
+__device__ __forceinline__ void small_scatter_tile(bool whole, const uint8_t* st, const uint32_t* s_tab, const uint32_t* s_d0,
                                                    const DevPool& dst, uint32_t& tilebad) {
   SAMPO_TILE_CONSTANTS(I);
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -259,10 +267,14 @@ __device__ __forceinline__ void small_scatter_tile(const uint8_t* st, const uint
       const uint32_t j = ((e0[b >> 1] >> sh) & 0xffffu) + rk;
       if (j < ((e1[b >> 1] >> sh) & 0xffffu)) {
         const uint32_t d = s_d0[b] + j;
-        dst.age[d] = c_age[i]; dst.his[d] = c_his[i]; dst.delay[d] = c_delay[i]; dst.sporo[d] = c_sporo[i];
-        dst.uni[d] = c_uni[i]; dst.avail[d] = c_avail[i]; dst.cycle[d] = c_cycle[i]; dst.hbc[d] = c_hbc[i];
-        dst.batches[d] = c_batches[i];
+        dst.age[d] = c_age[i]; dst.delay[d] = c_delay[i];
         dst.flags[d] = fb;
+        if (!whole || b != EGG) dst.uni[d] = c_uni[i];
+        if (!whole || b >= PUPA) dst.his[d] = c_his[i];
+        if (!whole || b >= BMS) {
+          dst.sporo[d] = c_sporo[i]; dst.avail[d] = c_avail[i]; dst.cycle[d] = c_cycle[i]; dst.hbc[d] = c_hbc[i];
+          dst.batches[d] = c_batches[i];
+        }
       } else {
         tilebad = 1;
       }
@@ -422,21 +434,28 @@ __device__ __forceinline__ bool small_wait_stage(uint64_t* bar, uint32_t& phase)
   return __syncthreads_and(ok) != 0;
 }
 
+// One thread: the copies of slots [lo, lo + n) of the pool to the stage, the
+// columns that hold a record of a state in them (whole: a narrow pool's).
 template <int I>
-__device__ __forceinline__ void small_issue_tile(const DevPool& src, uint8_t* st, uint64_t* bar, uint32_t lo, uint32_t n) {
+__device__ __forceinline__ void small_issue_tile(const DevPool& src, const sampo_population& pop, bool whole, uint8_t* st, uint64_t* bar,
+                                                 uint32_t lo, uint32_t n) {
   SAMPO_TILE_CONSTANTS(I);
   const uint32_t b4 = (n * 4 + 15) & ~15u, b1 = (n + 15) & ~15u;
-  mbar_arrive_tx(bar, 9 * b4 + b1);
+  const bool uni = !whole || lo + n > pop.r[LARVA].start, his = !whole || lo + n > pop.r[PUPA].start,
+             rest = !whole || lo + n > pop.r[BMS].start;
+  mbar_arrive_tx(bar, (2u + (uni ? 1u : 0u) + (his ? 1u : 0u) + (rest ? 5u : 0u)) * b4 + b1);
   bulk_load(st + 0 * kColBytes, src.age + lo, b4, bar);
-  bulk_load(st + 1 * kColBytes, src.his + lo, b4, bar);
   bulk_load(st + 2 * kColBytes, src.delay + lo, b4, bar);
-  bulk_load(st + 3 * kColBytes, src.sporo + lo, b4, bar);
-  bulk_load(st + 4 * kColBytes, src.uni + lo, b4, bar);
-  bulk_load(st + 5 * kColBytes, src.avail + lo, b4, bar);
-  bulk_load(st + 6 * kColBytes, src.cycle + lo, b4, bar);
-  bulk_load(st + 7 * kColBytes, src.hbc + lo, b4, bar);
-  bulk_load(st + 8 * kColBytes, src.batches + lo, b4, bar);
   bulk_load(st + 9 * kColBytes, src.flags + lo, b1, bar);
+  if (uni) bulk_load(st + 4 * kColBytes, src.uni + lo, b4, bar);
+  if (his) bulk_load(st + 1 * kColBytes, src.his + lo, b4, bar);
+  if (rest) {
+    bulk_load(st + 3 * kColBytes, src.sporo + lo, b4, bar);
+    bulk_load(st + 5 * kColBytes, src.avail + lo, b4, bar);
+    bulk_load(st + 6 * kColBytes, src.cycle + lo, b4, bar);
+    bulk_load(st + 7 * kColBytes, src.hbc + lo, b4, bar);
+    bulk_load(st + 8 * kColBytes, src.batches + lo, b4, bar);
+  }
 }
 
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
@@ -503,7 +522,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     s_cc = sim->cc;
     if (b < s_nold) {
       const uint32_t lo = b * kTile;
-      small_issue_tile<I>(rp.pool[s_cur], stage, &s_mbar, lo, min((uint32_t)kTile, s_end - lo));
+      small_issue_tile<I>(rp.pool[s_cur], s_pop, whole, stage, &s_mbar, lo, min((uint32_t)kTile, s_end - lo));
     }
   }
   copy16(&s_c, &sim->ctx[sim->step & 1u], (int)sizeof(StepCtx), tid, blockDim.x);
@@ -542,7 +561,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
         if (t != b) {
           if (tid == 0) {
             fence_proxy_async();
-            small_issue_tile<I>(rp.pool[s_cur], stage, &s_mbar, t * kTile, min((uint32_t)kTile, end - t * kTile));
+            small_issue_tile<I>(rp.pool[s_cur], s_pop, whole, stage, &s_mbar, t * kTile, min((uint32_t)kTile, end - t * kTile));
           }
           ok = small_wait_stage(&s_mbar, phase);
           if (!ok) break;
@@ -563,7 +582,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
       if (ok) {
         if (tid == 0) {
           fence_proxy_async();
-          small_issue_tile<I>(rp.pool[s_cur], stage, &s_mbar, b * kTile, min((uint32_t)kTile, end - b * kTile));
+          small_issue_tile<I>(rp.pool[s_cur], s_pop, whole, stage, &s_mbar, b * kTile, min((uint32_t)kTile, end - b * kTile));
         }
         ok = small_wait_stage(&s_mbar, phase);
         if (ok) {
@@ -627,13 +646,13 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
       for (int k = 1; k < 8; k++) mine = tid == k ? base[k] : mine;
       if (tid < 8) s_d0[tid] = mine + s_ex[0][tid] + s_ex[1][tid];
       __syncthreads();
-      small_scatter_tile<I>(stage, s_tab, s_d0, dst, sa.tilebad);
+      small_scatter_tile<I>(whole, stage, s_tab, s_d0, dst, sa.tilebad);
       // more tiles than CTAs: the other tiles of this CTA, loaded and updated again
       for (uint32_t t = b + G; t < nold; t += G) {
         __syncthreads();  // the stage is read
         if (tid == 0) {
           fence_proxy_async();
-          small_issue_tile<I>(rp.pool[s_cur], stage, &s_mbar, t * kTile, min((uint32_t)kTile, end - t * kTile));
+          small_issue_tile<I>(rp.pool[s_cur], s_pop, whole, stage, &s_mbar, t * kTile, min((uint32_t)kTile, end - t * kTile));
         }
         if (!small_wait_stage(&s_mbar, phase)) { ok = false; break; }
         small_update_tile<I, true, false, false>(s_c, s_mc, s_pop, whole, stage, t * kTile, end, s_ent, sa);
@@ -649,7 +668,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           if (lane < 8) s_d0[lane] = mine + s_ex[0][lane] + s_ex[1][lane];
         }
         if (__syncthreads_or(sa.tilebad)) break;
-        small_scatter_tile<I>(stage, s_tab, s_d0, dst, sa.tilebad);
+        small_scatter_tile<I>(whole, stage, s_tab, s_d0, dst, sa.tilebad);
       }
     }
     if (write) {
@@ -662,9 +681,11 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
           if (id < ne) {
             Rec a;
             new_egg(s_c, id, a);
-            dst.age[id] = a.age; dst.his[id] = a.his; dst.delay[id] = a.delay; dst.sporo[id] = a.sporo;
-            dst.uni[id] = a.uni; dst.avail[id] = a.avail; dst.cycle[id] = a.cycle; dst.hbc[id] = a.hbc;
-            dst.batches[id] = a.batches;
+            dst.age[id] = a.age; dst.delay[id] = a.delay;
+            if (!whole) {
+              dst.his[id] = a.his; dst.sporo[id] = a.sporo; dst.uni[id] = a.uni; dst.avail[id] = a.avail;
+              dst.cycle[id] = a.cycle; dst.hbc[id] = a.hbc; dst.batches[id] = a.batches;
+            }
             dst.flags[id] = (uint8_t)(EGG | (a.female << 3));
           }
         }
@@ -767,7 +788,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     if (tid == 0 && b < next_nold) {
       fence_proxy_async_global();
       fence_proxy_async();
-      small_issue_tile<I>(dst, stage, &s_mbar, b * kTile, min((uint32_t)kTile, next_end - b * kTile));
+      small_issue_tile<I>(dst, s_pop, whole, stage, &s_mbar, b * kTile, min((uint32_t)kTile, next_end - b * kTile));
     }
   }
   if (!met && tid == 0) atomicOr(&sim->error, SAMPO_DEV_ERR_BARRIER);
