@@ -45,10 +45,12 @@ sys.path.insert(0, REPO)
 
 from sampo_gb300.workloads import WORKLOADS, build_workload  # noqa: E402
 
-# algorithmic bytes per live agent read by the count pass, by state of its range
-# (the fields that decide survival, the next state and eggs laid)
-COUNT_BYTES = np.array([8, 12, 8, 12, 13, 12, 12, 12], dtype=np.float64)
-RECORD_BYTES = 37.0   # 9 x 4-byte fields + 1 flag byte
+# algorithmic bytes per live agent of the count pass, by state of its range: the
+# fields that decide survival, the next state and eggs laid, and the flags that
+# take the decision (read and written)
+COUNT_BYTES = np.array([10, 14, 10, 14, 14, 14, 14, 14], dtype=np.float64)
+# ... and of a record: the 4-byte fields that its state does not imply, and the flags
+RECORD_BYTES = np.array([9, 13, 17, 17, 17, 37, 37, 37], dtype=np.float64)
 
 
 def peaks():
@@ -207,8 +209,8 @@ def gpu_arm(args, wl, rank, world, device):
     if not np.array_equal(live2, live):
         raise RuntimeError("timing-mode rerun diverged from the graph run")
     tot = live2.sum(axis=1).astype(np.float64)
-    nxt = np.append(tot[1:], tot[-1])  # agents written = pool size at the next step's start
-    scatter_bytes = RECORD_BYTES * (tot + nxt)
+    record = (live2 * RECORD_BYTES).sum(axis=1)
+    scatter_bytes = record + np.append(record[1:], record[-1])  # agents written: the pool at the next step's start
     count_bytes = (live2 * COUNT_BYTES).sum(axis=1)
     n_launch = len(tot)
     scatter_ms, count_ms = times[1] / n_launch, times[0] / n_launch
@@ -250,15 +252,15 @@ def gpu_arm(args, wl, rank, world, device):
     sim.close()
     # each pass against the peak, and the whole step as the day graphs run it
     step_ms_graph = ms / (24 * args.steps)
-    step_bytes = float(count_bytes.mean() + scatter_bytes.mean())
+    step_bytes = float(count_bytes.mean() / 24 + scatter_bytes.mean())
 
     def pass_line(nbytes, t_ms):
         gbs = nbytes / (t_ms * 1e-3) / 1e9
         return {"bytes_per_launch": nbytes, "ms_per_launch": t_ms, "gbs": gbs, "frac": gbs / peak}
     passes = {
-        "k_count: decisions + in-tile scan (8-13 B read per live agent)": pass_line(float(count_bytes.mean()), count_ms),
-        "k_scatter: update + cross-tile scan + compaction (37 B read + 37 B written per agent)": pass_line(float(scatter_bytes.mean()), scatter_ms),
-        "hourly step in the day graphs (both passes + k_publish)": pass_line(step_bytes, step_ms_graph),
+        "k_count: decisions (10-14 B per live agent; once a day in the day graphs)": pass_line(float(count_bytes.mean()), count_ms),
+        "k_scatter: update + compaction (9-37 B read and written per agent, by its state)": pass_line(float(scatter_bytes.mean()), scatter_ms),
+        "hourly step in the day graphs (the update/scatter pass, which decides the next hour too, and k_publish)": pass_line(step_bytes, step_ms_graph),
     }
     return dict(agent_days=agent_days, ms=ms, wall=wall, live=live, rows=rows, clocks=clk.summary(), passes=passes,
                 gpu_launches=gpu_launches, scatter_ms=scatter_ms, count_ms=count_ms, publish_ms=publish_ms, achieved=achieved, peak=peak,
@@ -649,7 +651,7 @@ def main():
         return
     cpu = cpu_reference(wl, args.cpu_seconds) if world == 1 else None
     live_tot = r["live"].sum(axis=1)
-    pool_bytes = live_tot * RECORD_BYTES
+    pool_bytes = (r["live"] * RECORD_BYTES).sum(axis=1)  # of records as the passes move them
     details = {"live_agents_min": int(live_tot.min()), "live_agents_max": int(live_tot.max()),
                "pool_bytes": [float(pool_bytes.min()), float(pool_bytes.max())], "parallelism": f"replicas x{world}",
                "ctas_per_sm": {"count": r["tuned"][0], "scatter": r["tuned"][1],
@@ -659,7 +661,7 @@ def main():
                               "timed_days_one_launch": r["small"]["days_one_launch"] - r["small0"]["days_one_launch"],
                               "timed_days_three_kernel": r["small"]["days_three_kernel"] - r["small0"]["days_three_kernel"],
                               "one_launch_kind": {0: "-", 1: "-", 2: "cooperative launch", 3: "plain launch of a co-resident grid"}[r["small"]["last_day"]],
-                              "slots_per_thread": args.small_items or "by pool size (the smallest tiles, of 256, 512 or 1024 slots, that fit two per CTA of the largest grid)"}}
+                              "slots_per_thread": args.small_items or "by pool size (the smallest tiles, of 256, 512 or 1024 slots, that fit the largest grid with room to grow by half)"}}
     line = {
         "metric": "agent-days/s", "value": job_rate(tot_days, tmax), "unit": "agent-days/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": tmax * 1e3 / args.steps,
@@ -668,12 +670,13 @@ def main():
         "roofline": {"bound": "hbm", "achieved": r["achieved"], "peak": r["peak"], "unit": "GB/s",
                      "frac": r["achieved"] / r["peak"], "traffic": r["traffic"], "kernel": "k_scatter (update + stable scatter)",
                      "traffic_from": "scaled: DRAM bytes per live agent of a single-pass ncu capture of k_scatter on the "
-                                     "roofline workload at 5.7e7 live agents (profiles/k_scatter_dram.json: 0.998 of the "
+                                     "roofline workload at 5.7e7 live agents (profiles/k_scatter_dram.json: 1.10 of the "
                                      "algorithmic bytes) x this run's mean live pool",
                      "peak_kind": r["peak_kind"], "scatter_ms_per_launch": r["scatter_ms"], "count_ms_per_launch": r["count_ms"],
                      "publish_and_gaps_ms_per_step": r["publish_ms"],
                      "count_pass_gbs": r["count_gbs"],
-                     "algorithmic_bytes": "k_scatter: 37 B read per live agent + 37 B written per agent of the next pool",
+                     "algorithmic_bytes": "k_scatter: the fields that an agent's state does not imply and its flags (9-37 B), read per live "
+                                          "agent and written per agent of the next pool",
                      "passes": r["passes"]},
         "e2e": {"value": e2e_days / e2e_max, "unit": "agent-days/s", "h2d_bytes_per_step": 24 * (4 + 24 + 4 + 64),
                 "d2h_bytes_per_step": 24 * 92},

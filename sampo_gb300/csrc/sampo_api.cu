@@ -1,7 +1,7 @@
 // sampo_api.cu - host side of the C ABI declared in include/sampo.h.
 //
 // One handle owns one simulation on one GPU: two pool buffers, the device
-// step state, the per-tile look-back arrays and rings of per-step inputs and
+// step state, the span arrays and rings of per-step inputs and
 // stats rows; the kernels see it as a batch of one replicate. No call exits
 // the process; errors come back as status codes with a message in
 // sampo_last_error.

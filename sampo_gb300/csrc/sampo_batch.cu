@@ -5,7 +5,7 @@
 //   * a SimDev per slot and the RepParams array the kernels walk (fixed
 //     addresses, so a captured day graph stays valid while slots change);
 //   * per used slot, one stream-ordered allocation from the batch's memory
-//     pool holding the two pool buffers, the look-back tile arrays and the
+//     pool holding the two pool buffers, the span arrays and the
 //     rings of inputs and stats rows.
 // A slot's replicate is bit-identical to the same simulation run alone: the
 // kernels index its RNG by its own slots and its own step.

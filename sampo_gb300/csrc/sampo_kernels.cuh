@@ -1,10 +1,9 @@
 // sampo_kernels.cuh - device state shared by the kernels and the host API.
 //
 // The kernels step a batch of independent simulations ("replicates") at
-// once: every replicate has its own pool buffers, state, look-back arrays and
-// input rings (RepParams), and the persistent kernels hand out tiles of all
-// active replicates from one ticket counter. A single simulation is a batch
-// of one.
+// once: every replicate has its own pool buffers, state, span arrays and
+// input rings (RepParams), and the persistent kernels' warps take the spans of
+// all active replicates in turn. A single simulation is a batch of one.
 #pragma once
 #include <stdint.h>
 #ifndef __CUDACC_RTC__

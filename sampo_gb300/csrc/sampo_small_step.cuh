@@ -14,7 +14,7 @@
 //           state, its eggs laid and its share of the next pool's statistics
 //           (calcL1de.cl, calcGender.cl) to global memory.
 //  barrier  a grid barrier with a bounded wait.
-//  phase 2  every CTA sums the per-tile counts: the totals give the next
+//  phase 2  every CTA sums the counts (SmallRows): the totals give the next
 //           layout (kernel/oldToNewAgents.cl:57-95), the tiles before its own
 //           the tile's first slot in each next-state range. It writes its
 //           survivors from shared memory to their slots in the next buffer
