@@ -188,7 +188,11 @@ extern "C" int sampo_batch_create(const sampo_batch_config* cfg, sampo_batch** o
       rc = bfail(b, SAMPO_ERR_CUDA, std::string("batch state: ") + cudaGetErrorString(e));
       break;
     }
-    std::vector<SimDev> sims(n, initial_sim_state(0, 1.0f));
+    // every slot's state up to its step constants, which a replicate brings with it
+    constexpr size_t kHead = offsetof(SimDev, ctx);
+    const SimDev empty = initial_sim_state(0, 1.0f);
+    std::vector<uint8_t> heads(n * kHead);
+    for (size_t i = 0; i < n; i++) memcpy(heads.data() + i * kHead, &empty, kHead);
     std::vector<RepParams> rps(n);
     memset(rps.data(), 0, n * sizeof(RepParams));
     for (size_t i = 0; i < n; i++) {
@@ -198,7 +202,8 @@ extern "C" int sampo_batch_create(const sampo_batch_config* cfg, sampo_batch** o
     }
     ModelConst mc;
     fill_constant_tables(mc);
-    if ((e = cudaMemcpyAsync(b->sims_dev, sims.data(), n * sizeof(SimDev), cudaMemcpyHostToDevice, b->stream)) != cudaSuccess ||
+    if ((e = cudaMemsetAsync(b->sims_dev, 0, n * sizeof(SimDev), b->stream)) != cudaSuccess ||
+        (e = cudaMemcpy2DAsync(b->sims_dev, sizeof(SimDev), heads.data(), kHead, kHead, n, cudaMemcpyHostToDevice, b->stream)) != cudaSuccess ||
         (e = cudaMemcpyAsync(b->reps_dev, rps.data(), n * sizeof(RepParams), cudaMemcpyHostToDevice, b->stream)) != cudaSuccess ||
         (e = cudaMemcpyAsync(b->mc_dev, &mc, sizeof(mc), cudaMemcpyHostToDevice, b->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(b->bat_dev, 0, sizeof(BatchDev), b->stream)) != cudaSuccess ||
