@@ -179,7 +179,7 @@ extern "C" int sampo_batch_create(const sampo_batch_config* cfg, sampo_batch** o
     uint64_t keep = ~0ull;  // freed pools stay reserved for the next replicates
     cudaMemPoolSetAttribute(b->mempool, cudaMemPoolAttrReleaseThreshold, &keep);
     const size_t n = b->nslots;
-    if ((e = cudaMalloc(&b->sims_dev, n * sizeof(SimDev))) != cudaSuccess ||
+    if ((e = cudaMalloc(&b->sims_dev, n * (sizeof(SimDev) + sizeof(uint4)))) != cudaSuccess ||  // (with read_states' words behind)
         (e = cudaMalloc(&b->reps_dev, n * sizeof(RepParams))) != cudaSuccess ||
         (e = cudaMalloc(&b->bat_dev, sizeof(BatchDev))) != cudaSuccess ||
         (e = cudaMalloc(&b->mc_dev, sizeof(ModelConst))) != cudaSuccess ||
@@ -258,11 +258,12 @@ static void size_grids(sampo_batch* b) {
   drop_day_graphs(b);
 }
 
-// The device state of every slot up to its step constants (one strided copy).
-static int read_headers(sampo_batch* b, std::vector<SimDev>& h) {
-  h.resize(b->nslots);
-  BCK(cudaMemcpy2DAsync(h.data(), sizeof(SimDev), b->sims_dev, sizeof(SimDev), offsetof(SimDev, ctx), b->nslots,
-                        cudaMemcpyDeviceToHost, b->stream), "slot states");
+// {step, active, status bits, pool end} of every slot, once the queued work is done.
+static int read_states(sampo_batch* b, std::vector<uint4>& v) {
+  v.resize(b->nslots);
+  uint4* const out = reinterpret_cast<uint4*>(b->sims_dev + b->nslots);
+  BCK(launch_slot_states(b->sims_dev, b->nslots, out, b->stream), "slot states");
+  BCK(cudaMemcpyAsync(v.data(), out, v.size() * sizeof(uint4), cudaMemcpyDeviceToHost, b->stream), "slot states");
   BCK(cudaStreamSynchronize(b->stream), "slot states");
   return SAMPO_OK;
 }
@@ -270,15 +271,15 @@ static int read_headers(sampo_batch* b, std::vector<SimDev>& h) {
 // The host mirrors of the replicates' steps and activity from the device (a
 // replicate that paused for capacity did not advance).
 static int refresh_mirrors(sampo_batch* b) {
-  std::vector<SimDev> h;
-  const int rc = read_headers(b, h);
+  std::vector<uint4> v;
+  const int rc = read_states(b, v);
   if (rc) return rc;
   for (uint32_t i = 0; i < b->nslots; i++) {
     Replicate& r = b->reps[i];
     if (!r.used || !r.have_pop) continue;
-    r.step = h[i].step;
-    r.active = h[i].active != 0;
-    r.known_end = h[i].pop.r[7].end;
+    r.step = v[i].x;
+    r.active = v[i].y != 0;
+    r.known_end = v[i].w;
   }
   return SAMPO_OK;
 }
@@ -754,16 +755,16 @@ extern "C" int sampo_batch_sync(sampo_batch* b) {
 extern "C" int sampo_batch_states(sampo_batch* b, sampo_slot_state* out, uint32_t nslots) {
   if (!b || !out || nslots > b->nslots) return SAMPO_ERR_ARG;
   cudaSetDevice(b->device);
-  std::vector<SimDev> h;
-  const int rc = read_headers(b, h);
+  std::vector<uint4> v;
+  const int rc = read_states(b, v);
   if (rc) return rc;
   for (uint32_t i = 0; i < nslots; i++) {
     const Replicate& r = b->reps[i];
     sampo_slot_state& o = out[i];
-    o.step = h[i].step;
-    o.active = h[i].active;
-    o.status = h[i].error | h[i].warn;
-    o.end = r.have_pop ? h[i].pop.r[7].end : 0u;
+    o.step = v[i].x;
+    o.active = v[i].y;
+    o.status = v[i].z;
+    o.end = r.have_pop ? v[i].w : 0u;
     o.capacity = r.used ? r.capacity : 0u;
   }
   return SAMPO_OK;
@@ -775,10 +776,9 @@ extern "C" int sampo_batch_grow(sampo_batch* b, uint32_t slot, uint64_t capacity
   if (!r->have_pop) return bfail(b, SAMPO_ERR_STATE, "no population");
   if (capacity > 0xFFFFFF00ull) return bfail(b, SAMPO_ERR_ARG, "capacity above 0xFFFFFF00 slots");
   cudaSetDevice(b->device);
-  std::vector<SimDev> hs;
-  int rc = read_headers(b, hs);  // waits for the queued work
-  if (rc) return rc;
-  SimDev h = hs[slot];
+  SimDev h = initial_sim_state(0, 1.0f);
+  BCK(cudaMemcpyAsync(&h, b->sims_dev + slot, offsetof(SimDev, ctx), cudaMemcpyDeviceToHost, b->stream), "state");
+  BCK(cudaStreamSynchronize(b->stream), "state");  // (waits for the queued work)
   const uint32_t end = h.pop.r[7].end;
   if (capacity < end || capacity < 128) return bfail(b, SAMPO_ERR_ARG, "capacity below the pool's end");
   const RepLayout L(capacity, b->ring), L0(r->capacity, b->ring);

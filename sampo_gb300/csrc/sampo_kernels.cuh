@@ -273,6 +273,8 @@ cudaError_t launch_begin_step(const KParams& p, const CtxInputs& in, uint32_t sl
 // the decisions taken out of the flags (before a pool is read back)
 cudaError_t launch_widen(const KParams& p, cudaStream_t st);
 cudaError_t launch_histogram(const KParams& p, uint32_t* hist_dev, cudaStream_t st);
+// {step, active, status bits, pool end} of each of n states (n >= 1).
+cudaError_t launch_slot_states(const SimDev* sims, uint32_t n, uint4* out, cudaStream_t st);
 cudaError_t launch_eval_math(int fn, const float* x, const float* y, float* out, uint32_t n, cudaStream_t st);
 // Kernel nodes in a captured graph (the launches one replay makes).
 cudaError_t graph_kernel_nodes(cudaGraph_t g, uint32_t* kernels);
