@@ -1382,7 +1382,7 @@ __device__ __noinline__ uint32_t scatter_range(uint32_t lo, uint32_t hi, uint32_
             youngest = min(youngest, days);
             oldest = max(oldest, days);
           }
-          put_if<RG>(live, dst, d, age, delay, cld, (fl & 15u) | (lives ? (due ? DEC_MOVES << 4 : DEC_STAYS << 4) : 0u));
+          put_if<RG>(live, dst, d, age, delay, cld, RG | (fl & 8u) | (lives ? (due ? DEC_MOVES << 4 : DEC_STAYS << 4) : 0u));
         }
         if (crosses.value) {
           ts.cnt -= past;
@@ -1443,7 +1443,7 @@ __device__ __noinline__ uint32_t scatter_range(uint32_t lo, uint32_t hi, uint32_
             inf += a.sporo >= 1.0f ? 1u : 0u;
           }
           if (AHEAD) code1 = decide<RG, WIDE>(w.c1, mc.kill, d, a, da);
-          put(dst.flags + d, (fl & 15u) | (code1 << 4));
+          put(dst.flags + d, RG | (fl & 8u) | (code1 << 4));  // (the range's state: a loaded pool's state bits may differ)
         }
         if (AHEAD) add_tally<RG>(w, ts, bs, n, d, tally_count(code1));
         bs += n;
