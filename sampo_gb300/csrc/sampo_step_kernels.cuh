@@ -1405,7 +1405,7 @@ __device__ __noinline__ uint32_t scatter_range(uint32_t lo, uint32_t hi, uint32_
       if (hatched) da.dmin = da.dmax = 1u;
     } else {
       da.devoob = seen ? w.c1.devOOB : 0u;
-      if (oldest) {
+      if (youngest != 0xffffffffu) {  // (a loaded larva may be in its day 0)
         da.dmin = min(youngest, 99u);
         da.dmax = min(oldest, 99u);
       }

@@ -1,6 +1,6 @@
 """Pools that come from outside hold what no step leaves behind: state bytes
-that do not match the ranges. Every route of a step gives the same records
-for them, the oracle's."""
+that do not match the ranges, larvae in their first day. Every route of a
+step gives the same records for them, the oracle's."""
 import ctypes as C
 
 import numpy as np
@@ -76,3 +76,16 @@ def test_state_bytes_of_caller_owned_pools(gpu_ready, eggs):
     got = _download(tout, int(out.r[7].end))
     for k in range(8):
         assert np.all(got["state"][out.r[k].start:out.r[k].end] == k), k
+
+
+@pytest.mark.parametrize("tiles", [0, None])
+@pytest.mark.parametrize("ages", [(0,), (0, 700), (21,), (5, 30)])
+def test_larvae_younger_than_a_day(gpu_ready, oracle_mod, tiles, ages):
+    """A larva hatches at 24 hours, but a pool may bring younger ones: with
+    hoursInState = age - 24 their records follow from their state, and their
+    day, the 0th, has its mortality like the others."""
+    ranges, arrays, T, env, seeds = _workload((700, 2100, 300, 700), 30, 30000.0, seed=6)
+    s, e = int(ranges[1][0]), int(ranges[1][1])
+    arrays["ageInHours"][s:e] = np.resize(np.array(ages, np.float32), e - s)
+    arrays["hoursInState"][s:e] = arrays["ageInHours"][s:e] - np.float32(24.0)
+    _run_and_compare(ranges, arrays, T, env, seeds, 30000.0, (26, 4), tiles)
