@@ -809,7 +809,10 @@ extern "C" int sampo_batch_grow(sampo_batch* b, uint32_t slot, uint64_t capacity
   // the rings of inputs, seeds and rows (same ring length, same layout)
   BCK(cudaMemcpyAsync((void*)rp.T, old.T, L.T + L.env + L.seeds + L.wt + L.rows, cudaMemcpyDeviceToDevice, b->stream),
       "grow rings");
+  // fresh span arrays: none of their counts is to be cleared (the old ones'
+  // numbers may not even fit a smaller allocation)
   BCK(cudaMemsetAsync(rp.supers, 0, span_array_bytes((uint32_t)capacity), b->stream), "span arrays");
+  h.rot = h.dirty[0] = h.dirty[1] = h.dirty[2] = h.spans_done = 0;
   h.capacity = (uint32_t)capacity;
   h.cur = 0;
   h.error &= ~SAMPO_DEV_ERR_CAPACITY;

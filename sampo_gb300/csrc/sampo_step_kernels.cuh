@@ -610,7 +610,7 @@ __device__ __forceinline__ void load_warp_rep(const RepParams& rp, uint32_t min_
         w.spans1 = rp.spans + (size_t)(rot == 2u ? 0u : rot + 1u) * rp.spanStride;
         const uint32_t old = rot == 0u ? 2u : rot - 1u, units = w.nspans + units_of(w.newEggs, w.span);
         w.spans2 = rp.spans + (size_t)old * rp.spanStride;
-        w.clear = w.ahead ? sim->dirty[old] : 0u;
+        w.clear = w.ahead ? min(sim->dirty[old], rp.spanStride) : 0u;  // (no store leaves the set)
         w.clearPer = units ? (w.clear + units - 1u) / units : 0u;
       }
     }

@@ -1,0 +1,61 @@
+/*
+ * host_batch_check.cu - the host side of the batches (sampo_batch.cu) on
+ * fake_cuda.h: what a call leaves in a slot's device state.
+ */
+#include "fake_cuda.h"
+#include "../sampo_gb300/csrc/sampo_batch.cu"
+
+// A batch of one slot with a population, its ring filled with inputs.
+static sampo_batch* one_slot(uint64_t capacity, uint32_t* slot) {
+  sampo_batch* b = nullptr;
+  sampo_batch_config bc = {2, 16, 0};
+  CHECK(sampo_batch_create(&bc, &b) == SAMPO_OK);
+  sampo_replicate_config rc = {capacity, 1000.0f, 0xffffffffu};
+  CHECK(sampo_batch_add(b, &rc, slot) == SAMPO_OK);
+  float T[16];
+  sampo_environment env[16];
+  memset(env, 0, sizeof(env));
+  for (int i = 0; i < 16; i++) {
+    T[i] = 20.0f + (float)i;
+    env[i].carryingCapacity = 1000.0f;
+  }
+  CHECK(sampo_batch_set_inputs(b, *slot, 0, T, env, 16) == SAMPO_OK);
+  sampo_seeds seeds[4];
+  memset(seeds, 0, sizeof(seeds));
+  CHECK(sampo_batch_init_population(b, *slot, 100, seeds, -1, 0) == SAMPO_OK);
+  return b;
+}
+
+// The update/scatter pass that decides ahead clears dirty[rot - 1] words of
+// the span counts before the decided ones and adds to those after them, which
+// must be zero: whatever a slot brings into a (smaller) allocation, the counts
+// it says are to be cleared lie inside the new arrays and the new arrays are
+// all zero.
+static void grown_slots_have_clean_span_counts() {
+  for (uint32_t rot = 0; rot < 3; rot++) {
+    uint32_t slot = 0;
+    sampo_batch* b = one_slot(1u << 20, &slot);
+    SimDev* sim = b->sims_dev + slot;
+    sim->rot = rot;
+    for (uint32_t k = 0; k < 3; k++) sim->dirty[k] = max_spans(1u << 20) - k;
+    sim->spans_done = 3;
+    CHECK(sampo_batch_grow(b, slot, 1024) == SAMPO_OK);
+    const RepParams& rp = b->reps_dev[slot];
+    CHECK(rp.spanStride == max_spans(1024));
+    CHECK(sim->rot < 3);
+    for (uint32_t k = 0; k < 3; k++) CHECK(sim->dirty[k] == 0);
+    CHECK(sim->spans_done == 0);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(rp.supers);
+    bool zero = true;
+    for (size_t i = 0; i < span_array_bytes(1024) / 4; i++) zero &= w[i] == 0;
+    CHECK(zero);
+    for (int i = 0; i < 16; i++) CHECK(rp.T[i] == 20.0f + (float)i);
+    CHECK(sampo_batch_destroy(b) == SAMPO_OK);
+  }
+}
+
+int main() {
+  grown_slots_have_clean_span_counts();
+  printf(g_checks_failed ? "%d checks failed\n" : "ok\n", g_checks_failed);
+  return g_checks_failed ? 1 : 0;
+}
