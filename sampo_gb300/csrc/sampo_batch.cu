@@ -502,6 +502,11 @@ extern "C" int sampo_batch_checkpoint_load(sampo_batch* b, uint32_t slot, const 
     fclose(f);
     return bfail(b, SAMPO_ERR_IO, std::string("inconsistent checkpoint (") + why + "): " + path);
   }
+  // a stream past the coming step leaves that step's seeds in the file and no more
+  if ((hd.flags & CK_SEED_STREAM) && hd.rnd.next != hd.step && !((hd.flags & CK_COMING_SEEDS) && hd.rnd.next == hd.step + 1u)) {
+    fclose(f);
+    return bfail(b, SAMPO_ERR_IO, std::string("inconsistent checkpoint (seeds of its coming steps are missing): ") + path);
+  }
   cudaSetDevice(b->device);
   BCK(cudaStreamSynchronize(b->stream), "checkpoint");
   const std::string rerr = ck_read_pool(f, hd, r->rp.pool[0]);

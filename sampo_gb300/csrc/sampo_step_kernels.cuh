@@ -164,6 +164,19 @@ __device__ void draw_step_seeds(const RepParams& rp, uint32_t step) {
   if (lane == 0u) s.next = step + 1u;
 }
 
+// Puts back the last step's draws (the step's ring slot keeps them, and the
+// next time they come out the same): the words from 15 on are the draws, draw
+// k less the word three before it is r[k] again.
+__device__ void undraw_step_seeds(const RepParams& rp, uint32_t step) {
+  DevSeedStream& s = rp.sim->rnd;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t x = lane < 31u ? s.st.r[lane] : 0u;
+  const uint32_t draw = __shfl_sync(0xffffffffu, x, (lane + 15u) & 31u), before = __shfl_sync(0xffffffffu, x, (lane + 12u) & 31u);
+  const uint32_t kept = __shfl_sync(0xffffffffu, x, (lane + 16u) & 31u);  // lanes 16 on: word lane - 16
+  if (lane < 31u) s.st.r[lane] = lane < 16u ? draw - before : kept;
+  if (lane == 0u) s.next = step;
+}
+
 template <class T>
 __device__ void load_model_const(const T* g, T& s) {
   const float* src = reinterpret_cast<const float*>(g);
@@ -963,8 +976,8 @@ __device__ __forceinline__ void pause_rep(SimDev* sim) {
 // that does not stop there, the one after, whose pool's size and L1de the
 // decisions already give.
 // When the decided step's layout does not fit the replicate's capacity, the
-// replicate pauses: it becomes inactive at that step with its pool, constants
-// and larval table as they are, and only the step's counters are cleared, so
+// replicate pauses: it becomes inactive at that step with its pool, constants,
+// larval table and seed stream as they are, and only the step's counters are cleared, so
 // that the step runs again, with the same result, once its pool has been
 // moved into a larger one (sampo_batch_grow).
 __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
@@ -981,9 +994,12 @@ __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
   const bool ahead = decided && (mode_bits & PUB_AHEAD) && sd + 1u < stop;
   const bool prepare = !decided || ahead;      // constants and table of step x
   const uint32_t x = decided ? sd + 1u : sd;
+  bool drew = false;  // (warp 0)
   if (tid < 32 && prepare) {
-    // a device seed stream draws a step's seeds once, before thread 0 reads them
-    if (sim->rnd.next == x && x < stop) draw_step_seeds(rp, x);
+    // a device seed stream draws a step's seeds once, before thread 0 reads
+    // them; a replicate that turns out to pause gives them back
+    drew = sim->rnd.next == x && x < stop;
+    if (drew) draw_step_seeds(rp, x);
     __syncwarp();
   }
   if (mode == PUB_REFRESH) {
@@ -1060,9 +1076,8 @@ __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
   }
   __syncthreads();
   if (s_pause) {
-    if (tid == 0) {
-      pause_rep(sim);
-    }
+    if (tid < 32 && drew) undraw_step_seeds(rp, x);
+    if (tid == 0) pause_rep(sim);
     return;
   }
   if (after && decided) {  // the counts of step sd, made while step s was applied
@@ -1126,6 +1141,7 @@ __device__ void publish_rep(const KParams& p, uint32_t r, int mode_bits) {
     // (a replicate that pauses keeps the table of its step: x is the step after)
     for (uint32_t d = tid - 32; d < 100; d += blockDim.x - 32) sim->larvaKill[x & 1u][d] = larva_kill_entry(d, dmin, dmax, l1, cc);
   }
+  if (tid < 32 && drew && __shfl_sync(0xffffffffu, pause, 0)) undraw_step_seeds(rp, x);
 }
 
 // The start of one hour called on its own: its inputs, which come with the
