@@ -71,6 +71,7 @@ struct sampo_sim {
   uint32_t* end_pinned = nullptr;      // behind it: pool ends after a day, copied back one day behind the queue
   SimDev* status = nullptr;            // page-locked: the state's head (kStatusBytes), as check_device last read it
   cudaEvent_t ev_day[2] = {nullptr, nullptr};
+  bool rows_undefined = false;         // a one-launch step gave up since the rows were last cleared
   int last_day_kind = 0;               // DG_* of the last day launched
   uint64_t days_small = 0, days_three = 0;
   bool timing = false;
@@ -324,6 +325,21 @@ extern "C" int sampo_set_seeds(sampo_sim* s, uint32_t first, const sampo_seeds* 
   return SAMPO_OK;
 }
 
+// Notes the error bits of a one-launch step that gave up waiting: what it
+// leaves in its rows and counters is not defined.
+static void note_error(sampo_sim* s, uint32_t error) {
+  if (error & (SAMPO_DEV_ERR_BARRIER | SAMPO_DEV_ERR_TMA)) s->rows_undefined = true;
+}
+// Before a one-launch step: its rows are as the last one left them, or zero
+// when that one gave up.
+static int ready_small_step(sampo_sim* s) {
+  if (!s->rows_undefined) return SAMPO_OK;
+  CK(cudaMemsetAsync(s->small_mem, 0, small_row_words(units_of((uint32_t)s->capacity, 256)) * 4, s->stream), "row reset");
+  CK(cudaMemsetAsync(&s->bat_dev->bar, 0, 2 * sizeof(uint32_t), s->stream), "barrier reset");
+  s->rows_undefined = false;
+  return SAMPO_OK;
+}
+
 static int reset_state(sampo_sim* s, const sampo_population& pop) {
   SimDev h = s->host_state;
   h.pop = pop;
@@ -331,11 +347,6 @@ static int reset_state(sampo_sim* s, const sampo_population& pop) {
   h.step = 0;
   h.cur = 0;
   CK(cudaMemsetAsync(s->span_mem, 0, span_array_bytes((uint32_t)s->capacity), s->stream), "span reset");
-  // the one-launch step's grid barrier and exit counters start from zero, and
-  // its rows, unless a launch gave up at a barrier, are as it left them
-  if (s->status->error & (SAMPO_DEV_ERR_BARRIER | SAMPO_DEV_ERR_TMA))
-    CK(cudaMemsetAsync(s->small_mem, 0, small_row_words(units_of((uint32_t)s->capacity, 256)) * 4, s->stream), "row reset");
-  CK(cudaMemsetAsync(&s->bat_dev->bar, 0, 2 * sizeof(uint32_t), s->stream), "barrier reset");
   CK(cudaMemcpyAsync(s->sim_dev, &h, sizeof(SimDev), cudaMemcpyHostToDevice, s->stream), "state reset");
   s->step = 0;
   return SAMPO_OK;
@@ -431,6 +442,7 @@ static int check_device(sampo_sim* s) {
   CK(cudaStreamSynchronize(s->stream), "status");
   s->known_end = s->status->pop.r[GRAVID].end;  // the pool end the coming day's graph is picked by
   const uint32_t error = s->status->error;
+  note_error(s, error);
   if (error & SAMPO_DEV_ERR_CAPACITY) return fail(s, SAMPO_ERR_CAPACITY, "not enough capacity for the next layout");
   if (error & SAMPO_DEV_ERR_DEVRATES) return fail(s, SAMPO_ERR_TEMPERATURE, "temperature >= 44 C: the reference reads past devRates");
   if (error) return fail(s, SAMPO_ERR_INTERNAL, "device consistency check failed (bits " + std::to_string(error) + ")");
@@ -466,6 +478,8 @@ extern "C" int sampo_step(sampo_sim* s, const sampo_environment* env, float temp
   KParams p = make_params(s);
   uint32_t n = 1;
   if (!s->timing && takes_small_step(s)) {
+    const int rc = ready_small_step(s);
+    if (rc) return rc;
     // (the pool's end is exact here: the tiles need no room to grow)
     CK(launch_begin_step(p, in, slot, s->stream), "step inputs");
     const int items = s->small_items ? s->small_items : small_items_for(s->known_end, 1, s->small_grid);
@@ -554,6 +568,8 @@ static cudaError_t build_small_graph(sampo_sim* s, int items, int b) {
 static int day_graph_for(sampo_sim* s, cudaGraphExec_t* gx, uint32_t* kernels, int* kind) {
   const uint32_t end = s->known_end;
   if (takes_small_step(s)) {
+    const int rc = ready_small_step(s);
+    if (rc) return rc;
     const int items = s->small_items ? s->small_items : small_items_for(end, kSmallGrowth, 2 * s->small_grid);
     const uint64_t want = ((uint64_t)std::max(units_of(end, (uint32_t)(kBlock * items)), 1u) * kSmallGrowth + 1u) / 2u;
     const int ti = items == 1 ? 0 : items == 2 ? 1 : 2;
@@ -1019,6 +1035,7 @@ extern "C" int sampo_device_status(sampo_sim* s, uint32_t* bits, int clear) {
   uint32_t st[2];
   CK(cudaMemcpyAsync(st, &s->sim_dev->error, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream), "status");
   CK(cudaStreamSynchronize(s->stream), "status");
+  note_error(s, st[0]);
   *bits = st[0] | st[1];
   if (clear) {
     uint32_t z[2] = {0, 0};

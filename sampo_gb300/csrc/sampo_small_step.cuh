@@ -298,7 +298,8 @@ struct SmallRows {
   uint4* tiles;
   uint32_t* groups;    // [3][stride][16]
   uint32_t* state;     // the set the next launch starts with (all zero); records of the next one and of the one after that
-                       // that may not be
+                       // that may not be; whether a launch gave up waiting. Its records are not defined then, and the launches
+                       // queued behind it do nothing, until the host has cleared them
   uint32_t stride;     // records of a set
 };
 constexpr uint32_t kGroupTiles = kSmallGroupTiles, kGroupWords = kSmallGroupWords, SA_YOUNG = 128;
@@ -506,8 +507,9 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
   if (tid == 0) {
     mbar_init(&s_mbar);
     fence_mbar_init();
-    const uint32_t active = sim->active;
     rows = small_rows(rp);
+    const uint32_t gave_up = __ldcg(rows.state + 3), active = gave_up ? 0u : sim->active;
+    if (gave_up && b == 0) atomicOr(&sim->error, SAMPO_DEV_ERR_BARRIER);
     s_set = __ldcg(rows.state);
     s_dirty[1] = __ldcg(rows.state + 1);
     s_dirty[2] = __ldcg(rows.state + 2);
@@ -792,6 +794,7 @@ __global__ void __launch_bounds__(kSmallThreads, kSmallMinBlocks) k_step_small(K
     }
   }
   if (!met && tid == 0) atomicOr(&sim->error, SAMPO_DEV_ERR_BARRIER);
+  if ((!met || !ok) && tid == 0) __stcg(rows.state + 3, 1u);
   // a copy that did not land in time may still be in flight: let it land
   // (bounded) before the CTA can exit
   if (tid == 0 && !ok) (void)mbar_wait(&s_mbar, phase ^ 1u);  // the phase whose wait ran out

@@ -137,8 +137,16 @@ cudaError_t launch_slot_states(const SimDev* sims, uint32_t n, uint4* out, cudaS
 }
 cudaError_t launch_eval_math(int, const float*, const float*, float*, uint32_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t graph_kernel_nodes(cudaGraph_t, uint32_t* k) { *k = 1; return cudaSuccess; }
-cudaError_t launch_small_hour(const KParams&, uint32_t, int, int, cudaStream_t) { note("small"); return g_small_answer; }
-cudaError_t launch_small(const KParams&, int, bool, uint32_t, cudaStream_t, int) { note("small day"); return g_small_answer; }
+static cudaError_t note_small(const KParams& p, const char* what) {
+  const RepParams& rp = p.reps[0];
+  bool clean = p.bat->bar == 0 && p.bat->done == 0;
+  for (size_t i = 0; i < small_row_words(rp.smallTiles); i++) clean &= rp.smallRows[i] == 0;
+  note(what);
+  if (clean) note("small on clean rows");
+  return g_small_answer;
+}
+cudaError_t launch_small_hour(const KParams& p, uint32_t, int, int, cudaStream_t) { return note_small(p, "small"); }
+cudaError_t launch_small(const KParams& p, int, bool, uint32_t, cudaStream_t, int) { return note_small(p, "small day"); }
 cudaError_t tune_grids(const KParams&, cudaStream_t, int* c, int* s, int* items, double*) {
   *c = 2 * kFakeSms;
   *s = kFakeSms;

@@ -1,0 +1,80 @@
+/*
+ * host_api_check.cu - the host side of a single simulation (sampo_api.cu) on
+ * fake_cuda.h.
+ */
+#include "fake_cuda.h"
+#include "../sampo_gb300/csrc/sampo_api.cu"
+
+// A simulation with inputs and a population of 100 eggs.
+static sampo_sim* with_pool() {
+  sampo_sim* s = nullptr;
+  const sampo_config cfg = {4096, 1000.0f, 0, 16};
+  CHECK(sampo_create(&cfg, &s) == SAMPO_OK);
+  float T[16];
+  sampo_environment env[16];
+  sampo_seeds seeds[64];
+  memset(env, 0, sizeof(env));
+  memset(seeds, 0, sizeof(seeds));
+  for (int i = 0; i < 16; i++) {
+    T[i] = 25.0f;
+    env[i].carryingCapacity = 1000.0f;
+  }
+  CHECK(sampo_set_inputs(s, 0, T, env, 16) == SAMPO_OK);
+  CHECK(sampo_set_seeds(s, 0, seeds, 16) == SAMPO_OK);
+  CHECK(sampo_init_population(s, 100, seeds, 0, 0) == SAMPO_OK);
+  return s;
+}
+static int one_step(sampo_sim* s) {
+  sampo_environment env;
+  memset(&env, 0, sizeof(env));
+  env.carryingCapacity = 1000.0f;
+  sampo_seeds seeds[4];
+  memset(seeds, 0, sizeof(seeds));
+  sampo_stats_row row;
+  return sampo_step(s, &env, 25.0f, 0, seeds, &row);
+}
+
+// A one-launch hour that gave up (here: the bits such a launch sets, and
+// counts left in its records) leaves records that the next one adds to: they
+// are zero again before the next one-launch hour, whichever call comes first
+// and whether the bits have been read and cleared since.
+static void records_are_zero_after_a_launch_that_gave_up() {
+  for (uint32_t bit : {(uint32_t)SAMPO_DEV_ERR_BARRIER, (uint32_t)SAMPO_DEV_ERR_TMA})
+    for (int clear_by : {0, 1, 2})
+      for (int go_on : {0, 1, 2}) {
+        sampo_sim* s = with_pool();
+        const char* path = "sampo_fake.ck";
+        CHECK(sampo_checkpoint_save(s, path) == SAMPO_OK);
+        CHECK(one_step(s) == SAMPO_OK);
+        const size_t words = small_row_words(units_of(4096, 256));
+        memset(s->small_mem, 0x11, words * 4);
+        s->bat_dev->bar = s->bat_dev->done = 7;
+        s->sim_dev->error = bit;
+        if (clear_by != 2) CHECK(one_step(s) == SAMPO_ERR_INTERNAL);
+        uint32_t bits = 0;
+        if (clear_by) {
+          CHECK(sampo_device_status(s, &bits, 1) == SAMPO_OK && bits == bit);
+          // hours of the three kernels meanwhile: the status words read last are clean
+          CHECK(sampo_set_small_step(s, 0) == SAMPO_OK);
+          CHECK(one_step(s) == SAMPO_OK);
+          CHECK(sampo_set_small_step(s, SAMPO_SMALL_STEP_DEFAULT) == SAMPO_OK);
+        }
+        if (go_on == 1) CHECK(sampo_checkpoint_load(s, path) == SAMPO_OK);
+        if (go_on == 2) {
+          sampo_seeds seeds[4];
+          memset(seeds, 0, sizeof(seeds));
+          CHECK(sampo_init_population(s, 100, seeds, 0, 0) == SAMPO_OK);
+        }
+        g_launches.clear();
+        (void)one_step(s);
+        CHECK(g_launches["small"] == 1 && g_launches["small on clean rows"] == 1);
+        CHECK(sampo_destroy(s) == SAMPO_OK);
+        remove(path);
+      }
+}
+
+int main() {
+  records_are_zero_after_a_launch_that_gave_up();
+  printf(g_checks_failed ? "%d checks failed\n" : "ok\n", g_checks_failed);
+  return g_checks_failed ? 1 : 0;
+}

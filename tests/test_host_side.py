@@ -11,7 +11,7 @@ from sampo_gb300 import build
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
-@pytest.mark.parametrize("name", ["batch"])
+@pytest.mark.parametrize("name", ["api", "batch"])
 def test_host_side(tmp_path, name):
     try:
         nvcc = build.nvcc()
@@ -20,5 +20,16 @@ def test_host_side(tmp_path, name):
     exe = str(tmp_path / "check")
     subprocess.run([nvcc, *build.ARCH, "-O1", "-std=c++17", "--fmad=false", "-Xcompiler", "-ffp-contract=off",
                     os.path.join(HERE, f"host_{name}_check.cu"), "-o", exe], check=True, capture_output=True, text=True)
-    out = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    out = subprocess.run([exe], cwd=tmp_path, capture_output=True, text=True, timeout=120)
+    assert out.returncode == 0, out.stdout + out.stderr
+
+
+@pytest.mark.gpu
+def test_days_behind_a_launch_that_gave_up(gpu_ready, tmp_path):
+    exe = str(tmp_path / "check")
+    objs = [os.path.join(build.OUT, o + ".o") for o in
+            ("sampo_kernels.cu", "sampo_host.cpp", "sampo_species.cu", "sampo_jit_sources.cpp")]
+    subprocess.run([build.nvcc(), *build.NVFLAGS, os.path.join(HERE, "device_rows_check.cu"), *objs, "-o", exe, "-ldl", "-lpthread"],
+                   check=True, capture_output=True, text=True)
+    out = subprocess.run([exe, str(tmp_path / "a.ck")], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
