@@ -477,18 +477,20 @@ extern "C" int sampo_step(sampo_sim* s, const sampo_environment* env, float temp
   s->seed_step[slot] = s->step;
   KParams p = make_params(s);
   uint32_t n = 1;
-  if (!s->timing && takes_small_step(s)) {
+  bool small = !s->timing && takes_small_step(s);
+  if (small) {
     const int rc = ready_small_step(s);
     if (rc) return rc;
-    // (the pool's end is exact here: the tiles need no room to grow)
-    CK(launch_begin_step(p, in, slot, s->stream), "step inputs");
-    const int items = s->small_items ? s->small_items : small_items_for(s->known_end, 1, s->small_grid);
-    CK(launch_small_hour(p, s->known_end, items, s->small_grid, s->stream), "one-launch step");
-    n++;
-  } else {
-    CK(launch_begin_step(p, in, slot, s->stream), "step inputs");
-    CK(launch_hours(s, p, 1, &n), "step kernels");
   }
+  CK(launch_begin_step(p, in, slot, s->stream), "step inputs");
+  if (small) {
+    // (the pool's end is exact here: the tiles need no room to grow)
+    const int items = s->small_items ? s->small_items : small_items_for(s->known_end, 1, s->small_grid);
+    small = launch_small_hour(p, s->known_end, items, s->small_grid, s->stream) == cudaSuccess;
+    if (small) n++;
+    else (void)cudaGetLastError();  // a cooperative launch may be refused (part of the SMs only): three kernels then
+  }
+  if (!small) CK(launch_hours(s, p, 1, &n), "step kernels");
   s->launches += n;
   s->step++;
   const int rc = check_device(s);

@@ -179,11 +179,14 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
   // previous call's contents: the supers the passes add to are cleared.
   const uint32_t end = pop_in->r[7].end;
   const int grid = small_grid(device);
-  const bool small = units_of(end, (uint32_t)kTile) <= std::min((uint32_t)grid, kSmallTiles);
+  bool small = units_of(end, (uint32_t)kTile) <= std::min((uint32_t)grid, kSmallTiles);
   if (launch_publish_start(p, small ? 0u : (uint32_t)PS_CLEAR, end, st) != cudaSuccess) return SAMPO_ERR_CUDA;
-  if (small) {
-    if (launch_small_hour(p, end, small_items_for(end, 1, grid), grid, st) != cudaSuccess) return SAMPO_ERR_CUDA;
-  } else {
+  if (small && launch_small_hour(p, end, small_items_for(end, 1, grid), grid, st) != cudaSuccess) {
+    (void)cudaGetLastError();  // a cooperative launch may be refused (a stream with part of the SMs): the passes then
+    small = false;
+    if (cudaMemsetAsync(rp.supers, 0, max_supers(SAMPO_NOALLOC_MAX_SLOTS) * sizeof(uint4), st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  }
+  if (!small) {
     if (launch_count(p, grid_blocks_count(1, nullptr, kItems, true), st) != cudaSuccess) return SAMPO_ERR_CUDA;
     if (launch_scatter(p, grid_blocks_scatter(1, nullptr, kItems, true), st) != cudaSuccess) return SAMPO_ERR_CUDA;
     if (launch_publish(p, PUB_AFTER_STEP, st) != cudaSuccess) return SAMPO_ERR_CUDA;

@@ -71,6 +71,12 @@ static inline cudaError_t fake_cudaEventDestroy(cudaEvent_t) { return cudaSucces
 static inline cudaError_t fake_cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 static inline cudaError_t fake_cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 static inline cudaError_t fake_cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0; return cudaSuccess; }
+alignas(256) static unsigned char g_fake_symbol[32u << 20];  // the one __device__ array of the library
+template <class T>
+static inline cudaError_t fake_cudaGetSymbolAddress(void** p, const T& t) {
+  *p = g_fake_symbol;
+  return sizeof(t) <= sizeof(g_fake_symbol) ? cudaSuccess : cudaErrorInvalidSymbol;
+}
 static inline cudaError_t fake_cudaGetLastError(void) { return cudaSuccess; }
 static inline const char* fake_cudaGetErrorString(cudaError_t) { return "fake"; }
 #define cudaSetDevice fake_cudaSetDevice
@@ -105,6 +111,7 @@ static inline const char* fake_cudaGetErrorString(cudaError_t) { return "fake"; 
 #define cudaEventRecord fake_cudaEventRecord
 #define cudaEventSynchronize fake_cudaEventSynchronize
 #define cudaEventElapsedTime fake_cudaEventElapsedTime
+#define cudaGetSymbolAddress fake_cudaGetSymbolAddress
 #define cudaGetLastError fake_cudaGetLastError
 #define cudaGetErrorString fake_cudaGetErrorString
 
@@ -115,7 +122,13 @@ static cudaError_t note(const char* what) { g_launches[what]++; return cudaSucce
 int grid_blocks_count(uint32_t, const void*, int, bool wide) { return kFakeSms * (wide ? g_resident_wide : g_resident); }
 int grid_blocks_scatter(uint32_t, const void*, int, bool wide) { return kFakeSms * (wide ? g_resident_wide : g_resident); }
 int grid_blocks_small_all(const void*) { return kFakeSms * 3; }
-cudaError_t launch_count(const KParams&, int, cudaStream_t, int) { return note("count"); }
+cudaError_t launch_count(const KParams& p, int, cudaStream_t, int) {
+  const uint32_t n = units_of(span_count(p.reps[0].sim->pop.r[7].end, 0), 32) * 4, *w = reinterpret_cast<const uint32_t*>(p.reps[0].supers);
+  bool clean = true;
+  for (uint32_t i = 0; i < n; i++) clean &= w[i] == 0;
+  if (clean) note("count on clean supers");
+  return note("count");
+}
 cudaError_t launch_scatter(const KParams&, int, cudaStream_t, int, bool) { return note("scatter"); }
 cudaError_t launch_steps(const KParams& p, uint32_t n, bool, int, int, int, cudaStream_t, uint32_t* launches) {
   if (launches) *launches += 3 * n;
@@ -126,6 +139,7 @@ cudaError_t launch_publish(const KParams&, int, cudaStream_t) { return note("pub
 cudaError_t launch_init_eggs(const KParams&, uint32_t, float, const sampo_seeds*, int, uint64_t, bool, cudaStream_t) { return note("init"); }
 cudaError_t launch_publish_start(const KParams& p, uint32_t flags, uint32_t, cudaStream_t) {
   if (flags & PS_CHECK) p.reps[0].sim->wide = g_wide_found;
+  if (flags & PS_CLEAR) memset(p.reps[0].supers, 0, units_of(span_count(p.reps[0].sim->pop.r[7].end, 0), 32) * sizeof(uint4));
   return note(flags & PS_CLEAR ? "start, clearing" : "start");
 }
 cudaError_t launch_begin_step(const KParams&, const CtxInputs&, uint32_t, cudaStream_t) { return note("begin"); }

@@ -73,7 +73,25 @@ static void records_are_zero_after_a_launch_that_gave_up() {
       }
 }
 
+// Where the device refuses the cooperative launch (a stream that owns part of
+// the SMs, say), the hour is stepped by the three kernels.
+static void refused_launches_take_the_three_kernels() {
+  sampo_sim* s = with_pool();
+  g_small_answer = cudaErrorCooperativeLaunchTooLarge;
+  g_launches.clear();
+  const uint64_t before = s->launches;
+  CHECK(one_step(s) == SAMPO_OK);
+  CHECK(g_launches["begin"] == 1 && g_launches["small"] == 1 && g_launches["steps"] == 1);
+  CHECK(s->launches - before == 4);  // (the refused one did not run)
+  g_small_answer = cudaSuccess;
+  g_launches.clear();
+  CHECK(one_step(s) == SAMPO_OK);
+  CHECK(g_launches["small"] == 1 && g_launches["steps"] == 0);
+  CHECK(sampo_destroy(s) == SAMPO_OK);
+}
+
 int main() {
+  refused_launches_take_the_three_kernels();
   records_are_zero_after_a_launch_that_gave_up();
   printf(g_checks_failed ? "%d checks failed\n" : "ok\n", g_checks_failed);
   return g_checks_failed ? 1 : 0;

@@ -11,7 +11,7 @@ from sampo_gb300 import build
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
-@pytest.mark.parametrize("name", ["api", "batch"])
+@pytest.mark.parametrize("name", ["api", "batch", "noalloc"])
 def test_host_side(tmp_path, name):
     try:
         nvcc = build.nvcc()
