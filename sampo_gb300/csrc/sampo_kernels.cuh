@@ -96,9 +96,10 @@ struct CtxInputs {
 // (sampo_small_step.cuh): three sets of group records, a 16-byte word per
 // tile, four words of state. The records and the state start from zero.
 constexpr uint32_t kSmallGroupTiles = 16, kSmallGroupWords = 16;
-__host__ __device__ constexpr size_t small_row_words(uint32_t tiles) {
-  return 3 * (size_t)units_of(tiles, kSmallGroupTiles) * kSmallGroupWords + 4 * (size_t)tiles + 4;
+__host__ __device__ constexpr size_t small_group_words(uint32_t tiles) {
+  return 3 * (size_t)units_of(tiles, kSmallGroupTiles) * kSmallGroupWords;
 }
+__host__ __device__ constexpr size_t small_row_words(uint32_t tiles) { return small_group_words(tiles) + 4 * (size_t)tiles + 4; }
 
 // Spans: the slots a warp of the two passes takes at once, a multiple of 32.
 // A span costs a warp about a thousand instructions besides its rows (its
@@ -167,7 +168,7 @@ struct KParams {
 // update/scatter pass decides ahead. PUB_DECIDED and PUB_AFTER_STEP take
 // PUB_AHEAD when the update/scatter pass that comes next decides ahead.
 // Flags of k_pool_stats.
-enum : uint32_t { PS_CHECK = 1, PS_CLEAR = 2 };
+enum : uint32_t { PS_CHECK = 1, PS_CLEAR = 2, PS_ROWS = 4 };
 enum : int { PUB_INITIAL = 0, PUB_AFTER_STEP = 1, PUB_REFRESH = 2, PUB_DECIDED = 3, PUB_MODE = 3, PUB_AHEAD = 4 };
 
 #ifndef __CUDACC_RTC__  // host side (the run-time compiler sees the device part only)
@@ -265,7 +266,7 @@ cudaError_t launch_init_eggs(const KParams& p, uint32_t n, float T0, const sampo
                              int age_days_max, uint64_t age_seed, bool full, cudaStream_t st);
 // statistics of p.reps[0]'s current pool, then its publish (PUB_INITIAL);
 // `check` also finds out whether the pool is a wide one (SimDev::wide)
-// (flags: PS_CHECK | PS_CLEAR; end: the pool's end, which sizes the grid)
+// (flags: PS_*; end: the pool's end, which sizes the grid)
 cudaError_t launch_publish_start(const KParams& p, uint32_t flags, uint32_t end, cudaStream_t st);
 // The coming step's inputs into ring slot `slot`, and its constants.
 cudaError_t launch_begin_step(const KParams& p, const CtxInputs& in, uint32_t slot, cudaStream_t st);

@@ -52,7 +52,7 @@ constexpr uint32_t kSmallTiles = 512;
 struct Scratch {
   __align__(16) uint4 spans[span_array_words(SAMPO_NOALLOC_MAX_SLOTS)];
   uint8_t dec[SAMPO_NOALLOC_MAX_SLOTS];  // the count pass's decisions (the caller's pool is only read)
-  __align__(16) uint32_t small[small_row_words(kSmallTiles * 4)];  // (256-slot tiles; zero when the library is loaded)
+  __align__(16) uint32_t small[small_row_words(kSmallTiles * 4)];  // (256-slot tiles)
   sampo_stats_row rows[2];
   alignas(16) CallState call;
 };
@@ -176,11 +176,12 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
   // The one-launch step for a pool of at most one 1024-slot tile per CTA (as
   // in sampo_step), else the passes. (5,000 agents: 104 us with the passes and
   // ten copies, 57 with one launch and two copies.) The array keeps the
-  // previous call's contents: the supers the passes add to are cleared.
+  // previous call's contents: what the kernels add to is cleared (the supers,
+  // or the rows: a call that went wrong, or two at once, leave nothing to the next).
   const uint32_t end = pop_in->r[7].end;
   const int grid = small_grid(device);
   bool small = units_of(end, (uint32_t)kTile) <= std::min((uint32_t)grid, kSmallTiles);
-  if (launch_publish_start(p, small ? 0u : (uint32_t)PS_CLEAR, end, st) != cudaSuccess) return SAMPO_ERR_CUDA;
+  if (launch_publish_start(p, small ? PS_ROWS : PS_CLEAR, end, st) != cudaSuccess) return SAMPO_ERR_CUDA;
   if (small && launch_small_hour(p, end, small_items_for(end, 1, grid), grid, st) != cudaSuccess) {
     (void)cudaGetLastError();  // a cooperative launch may be refused (a stream with part of the SMs): the passes then
     small = false;
@@ -200,9 +201,6 @@ static int run_step(const sampo_device_pool* in, uint32_t in_capacity, const sam
   *row = down.rows[0];
   memcpy(pop_out, down.sim + offsetof(SimDev, pop), sizeof(*pop_out));
   memcpy(bnc_out, down.sim + offsetof(SimDev, bnc), sizeof(*bnc_out));
-  // a launch that gave up at a barrier leaves its rows in no defined state
-  if ((err & (SAMPO_DEV_ERR_BARRIER | SAMPO_DEV_ERR_TMA)) && cudaMemsetAsync(sc->small, 0, sizeof(sc->small), st) != cudaSuccess)
-    return SAMPO_ERR_CUDA;
   if (err & SAMPO_DEV_ERR_CAPACITY) return SAMPO_ERR_CAPACITY;
   if (err & SAMPO_DEV_ERR_DEVRATES) return SAMPO_ERR_TEMPERATURE;
   if (err) return SAMPO_ERR_INTERNAL;

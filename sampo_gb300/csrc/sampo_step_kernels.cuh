@@ -1700,7 +1700,8 @@ __device__ __forceinline__ bool wide_record(const DevPool& s, uint32_t g, int rg
 }
 
 // Statistics of p.reps[0]'s current pool, accumulated into acc_*; PS_CHECK:
-// also whether its records are wide, PS_CLEAR: also clears the supers. Only
+// also whether its records are wide, PS_CLEAR: also clears the supers,
+// PS_ROWS: the records and state of the one-launch step's rows. Only
 // the ranges that the statistics come from are read (larvae and adults; with
 // PS_CHECK all), as one sequence of four-slot groups (16-byte loads), so that
 // a thread has few turns of a load latency each; a loop over all slots that
@@ -1719,6 +1720,11 @@ __global__ void __launch_bounds__(256) k_pool_stats(KParams p, uint32_t flags) {
   if (flags & PS_CLEAR) {
     const uint32_t n = units_of(span_count(pop.r[GRAVID].end, 0), 32);
     for (uint32_t i = tid; i < n; i += threads) rp.supers[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  if (flags & PS_ROWS) {
+    const uint32_t n = (uint32_t)small_group_words(rp.smallTiles) / 4u;
+    uint4* const groups = reinterpret_cast<uint4*>(rp.smallRows);
+    for (uint32_t i = tid; i <= n; i += threads) groups[i < n ? i : n + rp.smallTiles] = make_uint4(0u, 0u, 0u, 0u);  // (the state lies behind the tiles)
   }
   uint32_t upto[8], groups = 0;  // groups of the ranges up to each
 #pragma unroll

@@ -49,7 +49,7 @@ int main(int argc, char** argv) {
   SimDev before, after;
   CHECK(cudaMemcpy(&before, s->sim_dev, sizeof(before), cudaMemcpyDeviceToHost) == cudaSuccess);
   const uint32_t tiles = units_of(1 << 16, 256);
-  const size_t groups = 3 * (size_t)units_of(tiles, kSmallGroupTiles) * kSmallGroupWords, words = small_row_words(tiles);
+  const size_t groups = small_group_words(tiles), words = small_row_words(tiles);
   std::vector<uint32_t> left(words, 0u);
   for (size_t i = 0; i < groups; i++) left[i] = 0x00010001u;
   left[words - 1] = 1u;

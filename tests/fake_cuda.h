@@ -140,7 +140,8 @@ cudaError_t launch_init_eggs(const KParams&, uint32_t, float, const sampo_seeds*
 cudaError_t launch_publish_start(const KParams& p, uint32_t flags, uint32_t, cudaStream_t) {
   if (flags & PS_CHECK) p.reps[0].sim->wide = g_wide_found;
   if (flags & PS_CLEAR) memset(p.reps[0].supers, 0, units_of(span_count(p.reps[0].sim->pop.r[7].end, 0), 32) * sizeof(uint4));
-  return note(flags & PS_CLEAR ? "start, clearing" : "start");
+  if (flags & PS_ROWS) memset(p.reps[0].smallRows, 0, small_row_words(p.reps[0].smallTiles) * 4);
+  return note("start");
 }
 cudaError_t launch_begin_step(const KParams&, const CtxInputs&, uint32_t, cudaStream_t) { return note("begin"); }
 cudaError_t launch_widen(const KParams&, cudaStream_t) { return note("widen"); }
@@ -154,7 +155,8 @@ cudaError_t graph_kernel_nodes(cudaGraph_t, uint32_t* k) { *k = 1; return cudaSu
 static cudaError_t note_small(const KParams& p, const char* what) {
   const RepParams& rp = p.reps[0];
   bool clean = p.bat->bar == 0 && p.bat->done == 0;
-  for (size_t i = 0; i < small_row_words(rp.smallTiles); i++) clean &= rp.smallRows[i] == 0;
+  for (size_t i = 0; i < small_row_words(rp.smallTiles); i++)  // (the tiles' words between are written before they are read)
+    clean &= rp.smallRows[i] == 0 || (i >= small_group_words(rp.smallTiles) && i < small_row_words(rp.smallTiles) - 4);
   note(what);
   if (clean) note("small on clean rows");
   return g_small_answer;
