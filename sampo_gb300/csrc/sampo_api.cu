@@ -54,6 +54,7 @@ struct sampo_sim {
   uint32_t step = 0;                   // host mirror of the device step index
   bool have_pop = false;
   bool pending = false;                // steps queued by sampo_run_async, not yet synced
+  ChosenGrids chosen;
   int grid_count = 0, grid_scatter = 0;
   int items = kItems;                  // slots per thread of the count and update/scatter passes (2 or 4)
   cudaGraphExec_t day_graph = nullptr;  // 24 three-kernel steps
@@ -355,14 +356,20 @@ static int reset_state(sampo_sim* s, const sampo_population& pop) {
 static void drop_day_graph(sampo_sim* s);
 static void drop_small_graphs(sampo_sim* s);
 
-// The passes and grids for narrow or wide pools (state_cols).
+// The grids of the passes the simulation runs; a day graph captured with
+// other kernels or grids goes.
+static void size_grids(sampo_sim* s) {
+  s->grid_count = chosen_grid(s->chosen.count, grid_blocks_count(1, s->species, s->items, s->wide));
+  s->grid_scatter = chosen_grid(s->chosen.scatter, grid_blocks_scatter(1, s->species, s->items, s->wide));
+  drop_day_graph(s);
+}
+
+// The passes for narrow or wide pools (state_cols).
 static void set_wide(sampo_sim* s, bool wide) {
   if (wide == s->wide) return;
   s->wide = wide;
-  s->grid_count = grid_blocks_count(1, s->species, s->items, wide);
-  s->grid_scatter = grid_blocks_scatter(1, s->species, s->items, wide);
-  drop_day_graph(s);  // captured with the other kernels
-  drop_small_graphs(s);
+  size_grids(s);
+  drop_small_graphs(s);  // captured with the other kernels
 }
 
 // Statistics and publish of the pool, of that end, that the caller has just put in buffer 0;
@@ -958,17 +965,14 @@ extern "C" int sampo_autotune(sampo_sim* s, uint32_t* count_ctas_per_sm, uint32_
   CK(launch_publish(p, PUB_REFRESH, s->stream), "step constants");
   int gc = 0, gs = 0, items = kItems;
   CK(tune_grids(p, s->stream, &gc, &gs, &items, nullptr), "autotune");
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-  if (sms <= 0) sms = 1;
+  const int sms = device_sms();
+  s->chosen = {(uint32_t)(gc / sms), (uint32_t)(gs / sms)};
   if (gc != s->grid_count || gs != s->grid_scatter || items != s->items) {
-    s->grid_count = gc;
-    s->grid_scatter = gs;
     s->items = items;
-    drop_day_graph(s);  // captured with the old grids
+    size_grids(s);
   }
-  if (count_ctas_per_sm) *count_ctas_per_sm = (uint32_t)(gc / sms);
-  if (scatter_ctas_per_sm) *scatter_ctas_per_sm = (uint32_t)(gs / sms);
+  if (count_ctas_per_sm) *count_ctas_per_sm = s->chosen.count;
+  if (scatter_ctas_per_sm) *scatter_ctas_per_sm = s->chosen.scatter;
   return check_device(s);
 }
 
@@ -980,9 +984,8 @@ extern "C" int sampo_set_species(sampo_sim* s, const sampo_species* sp) {
   if (s->species == sp) return SAMPO_OK;
   s->species = sp;
   if (sp) s->items = kItems;  // a run-time species is built for 4 slots per thread
-  s->grid_count = grid_blocks_count(1, sp, s->items, s->wide);
-  s->grid_scatter = grid_blocks_scatter(1, sp, s->items, s->wide);
-  drop_day_graph(s);  // captured with the other kernels
+  s->chosen = ChosenGrids();
+  size_grids(s);
   drop_small_graphs(s);
   size_small_step(s);
   return SAMPO_OK;
@@ -992,20 +995,14 @@ extern "C" int sampo_set_grids(sampo_sim* s, uint32_t count_ctas_per_sm, uint32_
   if (!s) return SAMPO_ERR_ARG;
   SETTLE(s);
   cudaSetDevice(s->device);
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-  if (sms <= 0) sms = 1;
+  const int sms = device_sms();
   const uint32_t max_c = (uint32_t)(grid_blocks_count(1, s->species, s->items, s->wide) / sms);
   const uint32_t max_s = (uint32_t)(grid_blocks_scatter(1, s->species, s->items, s->wide) / sms);
   if (count_ctas_per_sm < 1 || count_ctas_per_sm > max_c || scatter_ctas_per_sm < 1 || scatter_ctas_per_sm > max_s)
     return fail(s, SAMPO_ERR_ARG, "CTAs per SM outside 1.." + std::to_string(max_c) + " (count) / 1.." + std::to_string(max_s) +
                                       " (update/scatter)");
-  const int gc = (int)count_ctas_per_sm * sms, gs = (int)scatter_ctas_per_sm * sms;
-  if (gc != s->grid_count || gs != s->grid_scatter) {
-    s->grid_count = gc;
-    s->grid_scatter = gs;
-    drop_day_graph(s);  // captured with the old grids
-  }
+  s->chosen = {count_ctas_per_sm, scatter_ctas_per_sm};
+  if ((int)count_ctas_per_sm * sms != s->grid_count || (int)scatter_ctas_per_sm * sms != s->grid_scatter) size_grids(s);
   return SAMPO_OK;
 }
 
@@ -1017,9 +1014,8 @@ extern "C" int sampo_set_items_per_thread(sampo_sim* s, uint32_t items) {
   cudaSetDevice(s->device);
   if ((int)items != s->items) {
     s->items = (int)items;
-    s->grid_count = grid_blocks_count(1, s->species, s->items, s->wide);
-    s->grid_scatter = grid_blocks_scatter(1, s->species, s->items, s->wide);
-    drop_day_graph(s);
+    s->chosen = ChosenGrids();
+    size_grids(s);
   }
   return SAMPO_OK;
 }

@@ -74,6 +74,7 @@ struct sampo_batch {
   uint32_t* hist_dev = nullptr;
   std::vector<Replicate> reps;
   std::vector<uint32_t> wt_staging;
+  ChosenGrids chosen;
   int grid_count = 0, grid_scatter = 0;
   int items = kItems;                // slots per thread of the count and update/scatter passes (2 or 4)
   uint32_t min_span = 0;             // BatchDev::minSpan as last set
@@ -250,11 +251,11 @@ static RepParams carve(const RepLayout& L, void* mem, SimDev* sim, uint64_t capa
   return rp;
 }
 
-// The largest grids of the passes the batch runs; a day graph captured with
-// other kernels or grids goes.
+// The grids of the passes the batch runs; a day graph captured with other
+// kernels or grids goes.
 static void size_grids(sampo_batch* b) {
-  b->grid_count = grid_blocks_count(b->nslots, b->species, b->items, b->wide);
-  b->grid_scatter = grid_blocks_scatter(b->nslots, b->species, b->items, b->wide);
+  b->grid_count = chosen_grid(b->chosen.count, grid_blocks_count(b->nslots, b->species, b->items, b->wide));
+  b->grid_scatter = chosen_grid(b->chosen.scatter, grid_blocks_scatter(b->nslots, b->species, b->items, b->wide));
   drop_day_graphs(b);
 }
 
@@ -687,17 +688,14 @@ extern "C" int sampo_batch_autotune(sampo_batch* b, uint32_t* count_ctas_per_sm,
   BCK(launch_publish(p, PUB_REFRESH, b->stream), "step constants");
   int gc = 0, gs = 0, items = kItems;
   BCK(tune_grids(p, b->stream, &gc, &gs, &items, nullptr), "autotune");
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-  if (sms <= 0) sms = 1;
+  const int sms = device_sms();
+  b->chosen = {(uint32_t)(gc / sms), (uint32_t)(gs / sms)};
   if (gc != b->grid_count || gs != b->grid_scatter || items != b->items) {
-    b->grid_count = gc;
-    b->grid_scatter = gs;
     b->items = items;
-    drop_day_graphs(b);
+    size_grids(b);
   }
-  if (count_ctas_per_sm) *count_ctas_per_sm = (uint32_t)(gc / sms);
-  if (scatter_ctas_per_sm) *scatter_ctas_per_sm = (uint32_t)(gs / sms);
+  if (count_ctas_per_sm) *count_ctas_per_sm = b->chosen.count;
+  if (scatter_ctas_per_sm) *scatter_ctas_per_sm = b->chosen.scatter;
   return SAMPO_OK;
 }
 
@@ -708,6 +706,7 @@ extern "C" int sampo_batch_set_species(sampo_batch* b, const sampo_species* sp) 
   if (b->species == sp) return SAMPO_OK;
   b->species = sp;
   if (sp) b->items = kItems;  // a run-time species is built for 4 slots per thread
+  b->chosen = ChosenGrids();
   size_grids(b);
   return SAMPO_OK;
 }
@@ -715,20 +714,14 @@ extern "C" int sampo_batch_set_species(sampo_batch* b, const sampo_species* sp) 
 extern "C" int sampo_batch_set_grids(sampo_batch* b, uint32_t count_ctas_per_sm, uint32_t scatter_ctas_per_sm) {
   if (!b) return SAMPO_ERR_ARG;
   cudaSetDevice(b->device);
-  int sms = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-  if (sms <= 0) sms = 1;
+  const int sms = device_sms();
   const uint32_t max_c = (uint32_t)(grid_blocks_count(b->nslots, b->species, b->items, b->wide) / sms);
   const uint32_t max_s = (uint32_t)(grid_blocks_scatter(b->nslots, b->species, b->items, b->wide) / sms);
   if (count_ctas_per_sm < 1 || count_ctas_per_sm > max_c || scatter_ctas_per_sm < 1 || scatter_ctas_per_sm > max_s)
     return bfail(b, SAMPO_ERR_ARG, "CTAs per SM outside 1.." + std::to_string(max_c) + " (count) / 1.." +
                                        std::to_string(max_s) + " (update/scatter)");
-  const int gc = (int)count_ctas_per_sm * sms, gs = (int)scatter_ctas_per_sm * sms;
-  if (gc != b->grid_count || gs != b->grid_scatter) {
-    b->grid_count = gc;
-    b->grid_scatter = gs;
-    drop_day_graphs(b);
-  }
+  b->chosen = {count_ctas_per_sm, scatter_ctas_per_sm};
+  if ((int)count_ctas_per_sm * sms != b->grid_count || (int)scatter_ctas_per_sm * sms != b->grid_scatter) size_grids(b);
   return SAMPO_OK;
 }
 
@@ -739,6 +732,7 @@ extern "C" int sampo_batch_set_items_per_thread(sampo_batch* b, uint32_t items) 
   cudaSetDevice(b->device);
   if ((int)items != b->items) {
     b->items = (int)items;
+    b->chosen = ChosenGrids();
     size_grids(b);
   }
   return SAMPO_OK;

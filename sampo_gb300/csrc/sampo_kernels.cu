@@ -46,6 +46,7 @@ static int sm_count() {
   std::call_once(once[dev], [&] { sms[dev] = setup_device(dev); });
   return sms[dev];
 }
+int device_sms() { return sm_count(); }
 size_t pass_smem_max() { return pass_smem(kMaxRep); }
 
 // Resident CTAs per SM of a pass, built in or of ks (4 rows at once).

@@ -236,6 +236,15 @@ inline SimDev initial_sim_state(uint32_t capacity, float cc) {
 // persistent grid sizes (CTAs resident on all SMs) for batches of nrep replicates
 int grid_blocks_count(uint32_t nrep, const void* ks = nullptr, int items = kItems, bool wide = false);
 int grid_blocks_scatter(uint32_t nrep, const void* ks = nullptr, int items = kItems, bool wide = false);
+// The current device's SMs.
+int device_sms();
+// The grids that sampo_set_grids or the tuner chose, in CTAs per SM of the
+// count and update/scatter passes; 0: the largest. They hold for every pool
+// the passes run on, as far as the grid of its kernels reaches.
+struct ChosenGrids {
+  uint32_t count = 0, scatter = 0;
+};
+inline int chosen_grid(uint32_t chosen, int largest) { return chosen ? std::min((int)chosen * device_sms(), largest) : largest; }
 // The kernels of a run-time species (sampo_species.cu): launch one, and its
 // resident CTAs per SM.
 enum : int {

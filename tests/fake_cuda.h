@@ -121,6 +121,7 @@ namespace sampo {
 static cudaError_t note(const char* what) { g_launches[what]++; return cudaSuccess; }
 int grid_blocks_count(uint32_t, const void*, int, bool wide) { return kFakeSms * (wide ? g_resident_wide : g_resident); }
 int grid_blocks_scatter(uint32_t, const void*, int, bool wide) { return kFakeSms * (wide ? g_resident_wide : g_resident); }
+int device_sms() { return kFakeSms; }
 int grid_blocks_small_all(const void*) { return kFakeSms * 3; }
 cudaError_t launch_count(const KParams& p, int, cudaStream_t, int) {
   const uint32_t n = units_of(span_count(p.reps[0].sim->pop.r[7].end, 0), 32) * 4, *w = reinterpret_cast<const uint32_t*>(p.reps[0].supers);

@@ -90,7 +90,64 @@ static void refused_launches_take_the_three_kernels() {
   CHECK(sampo_destroy(s) == SAMPO_OK);
 }
 
+// Puts a pool in place whose records are, or are not, implied by their states.
+static void load_pool(sampo_sim* s, bool wide) {
+  uint32_t words[128];
+  uint8_t bytes[128];
+  memset(words, 0, sizeof(words));
+  memset(bytes, 0, sizeof(bytes));
+  sampo_population pop;
+  memset(&pop, 0, sizeof(pop));
+  pop.r[0].end = 16;
+  for (uint32_t k = 1; k < 8; k++) pop.r[k].start = pop.r[k].end = 16 + k;
+  sampo_pool_view v = {(float*)words, (float*)words, (float*)words, (float*)words, words, words, words, words, words, bytes, bytes};
+  g_wide_found = wide;
+  CHECK(sampo_load_pool(s, &pop, &v) == SAMPO_OK);
+  CHECK(s->wide == wide);
+}
+static bool grids_are(const sampo_sim* s, int count, int scatter) {
+  return s->grid_count == count * kFakeSms && s->grid_scatter == scatter * kFakeSms;
+}
+
+// Grids that the caller or the tuner chose stay chosen when a pool of the
+// other kind of records is loaded, as far as its passes reach; the calls that
+// reset them to the largest (the number of rows at once, the species) do.
+static void chosen_grids_outlive_the_pool() {
+  for (bool tuned : {false, true}) {
+    sampo_sim* s = with_pool();
+    g_resident = 3;
+    g_resident_wide = 3;
+    CHECK(grids_are(s, 3, 3));
+    load_pool(s, true);
+    CHECK(grids_are(s, 3, 3));
+    g_resident_wide = 2;  // (as the largest grids of the passes differ)
+    load_pool(s, false);
+    load_pool(s, true);
+    CHECK(grids_are(s, 2, 2));
+    load_pool(s, false);
+    if (tuned) {  // picks (2, 1)
+      CHECK(sampo_autotune(s, nullptr, nullptr) == SAMPO_OK);
+    } else {
+      CHECK(sampo_set_grids(s, 2, 1) == SAMPO_OK);
+    }
+    CHECK(grids_are(s, 2, 1));
+    load_pool(s, true);
+    CHECK(grids_are(s, 2, 1));
+    load_pool(s, false);
+    CHECK(grids_are(s, 2, 1));
+    g_resident_wide = 1;
+    load_pool(s, true);
+    CHECK(grids_are(s, 1, 1));
+    load_pool(s, false);
+    CHECK(grids_are(s, 2, 1));
+    CHECK(sampo_set_items_per_thread(s, 2) == SAMPO_OK);
+    CHECK(grids_are(s, 3, 3));
+    CHECK(sampo_destroy(s) == SAMPO_OK);
+  }
+}
+
 int main() {
+  chosen_grids_outlive_the_pool();
   refused_launches_take_the_three_kernels();
   records_are_zero_after_a_launch_that_gave_up();
   printf(g_checks_failed ? "%d checks failed\n" : "ok\n", g_checks_failed);

@@ -22,7 +22,7 @@ static sampo_batch* one_slot(uint64_t capacity, uint32_t* slot) {
   CHECK(sampo_batch_set_inputs(b, *slot, 0, T, env, 16) == SAMPO_OK);
   sampo_seeds seeds[4];
   memset(seeds, 0, sizeof(seeds));
-  CHECK(sampo_batch_init_population(b, *slot, 100, seeds, -1, 0) == SAMPO_OK);
+  CHECK(sampo_batch_init_population(b, *slot, 100, seeds, 0, 0) == SAMPO_OK);
   return b;
 }
 
@@ -54,7 +54,42 @@ static void grown_slots_have_clean_span_counts() {
   }
 }
 
+// Resumes a slot from a checkpoint whose records are, or are not, implied by
+// their states.
+static void resume(sampo_batch* b, uint32_t slot, const char* path, bool wide) {
+  g_wide_found = wide;
+  CHECK(sampo_batch_checkpoint_load(b, slot, path) == SAMPO_OK);
+}
+static bool grids_are(const sampo_batch* b, int count, int scatter) {
+  return b->grid_count == count * kFakeSms && b->grid_scatter == scatter * kFakeSms;
+}
+
+// Chosen grids stay chosen when a slot's pool makes the batch move whole records.
+static void chosen_grids_outlive_a_wide_pool() {
+  const char* path = "sampo_fake_batch.ck";
+  for (bool tuned : {false, true}) {
+    uint32_t slot = 0;
+    sampo_batch* b = one_slot(4096, &slot);
+    CHECK(sampo_batch_checkpoint_save(b, slot, path) == SAMPO_OK);
+    CHECK(grids_are(b, 3, 3));
+    if (tuned) {
+      b->reps[slot].seed_step[0] = 0;
+      CHECK(sampo_batch_autotune(b, nullptr, nullptr) == SAMPO_OK);
+    } else {
+      CHECK(sampo_batch_set_grids(b, 2, 1) == SAMPO_OK);
+    }
+    resume(b, slot, path, true);
+    CHECK(b->wide);
+    CHECK(grids_are(b, 2, 1));
+    CHECK(sampo_batch_set_items_per_thread(b, 2) == SAMPO_OK);
+    CHECK(grids_are(b, 3, 3));
+    CHECK(sampo_batch_destroy(b) == SAMPO_OK);
+  }
+  remove(path);
+}
+
 int main() {
+  chosen_grids_outlive_a_wide_pool();
   grown_slots_have_clean_span_counts();
   printf(g_checks_failed ? "%d checks failed\n" : "ok\n", g_checks_failed);
   return g_checks_failed ? 1 : 0;
