@@ -182,7 +182,10 @@ int sampo_checkpoint_save(sampo_sim* s, const char* path);
  * unchanged. Needs the coming step's inputs. */
 int sampo_autotune(sampo_sim* s, uint32_t* count_ctas_per_sm, uint32_t* scatter_ctas_per_sm);
 /* Sets the grid sizes sampo_autotune would pick, e.g. a choice tuned earlier
- * on the same workload: 1 .. the occupancy limit of each pass. */
+ * on the same workload: 1 .. the occupancy limit of each pass. (Up to 5 CTAs
+ * per SM of the count pass are taken, for choices tuned with kernels of which
+ * more were resident, and run as the largest grid.) The choice holds for
+ * every pool until it is tuned or set again, or a call below resets it. */
 int sampo_set_grids(sampo_sim* s, uint32_t count_ctas_per_sm, uint32_t scatter_ctas_per_sm);
 /* Slots per thread of the count and update/scatter passes: 4 (1024-slot
  * tiles, the default) or 2 (512-slot tiles); results do not depend on it. A

@@ -356,12 +356,13 @@ static int reset_state(sampo_sim* s, const sampo_population& pop) {
 static void drop_day_graph(sampo_sim* s);
 static void drop_small_graphs(sampo_sim* s);
 
-// The grids of the passes the simulation runs; a day graph captured with
-// other kernels or grids goes.
-static void size_grids(sampo_sim* s) {
+// The grids of the passes the simulation runs; a day graph captured with other
+// grids goes, and with `other` kernels.
+static void size_grids(sampo_sim* s, bool other = true) {
+  const int gc = s->grid_count, gs = s->grid_scatter;
   s->grid_count = chosen_grid(s->chosen.count, grid_blocks_count(1, s->species, s->items, s->wide));
   s->grid_scatter = chosen_grid(s->chosen.scatter, grid_blocks_scatter(1, s->species, s->items, s->wide));
-  drop_day_graph(s);
+  if (other || gc != s->grid_count || gs != s->grid_scatter) drop_day_graph(s);
 }
 
 // The passes for narrow or wide pools (state_cols).
@@ -996,13 +997,13 @@ extern "C" int sampo_set_grids(sampo_sim* s, uint32_t count_ctas_per_sm, uint32_
   SETTLE(s);
   cudaSetDevice(s->device);
   const int sms = device_sms();
-  const uint32_t max_c = (uint32_t)(grid_blocks_count(1, s->species, s->items, s->wide) / sms);
+  const uint32_t max_c = (uint32_t)std::max(grid_blocks_count(1, s->species, s->items, s->wide) / sms, kCountGrids);
   const uint32_t max_s = (uint32_t)(grid_blocks_scatter(1, s->species, s->items, s->wide) / sms);
   if (count_ctas_per_sm < 1 || count_ctas_per_sm > max_c || scatter_ctas_per_sm < 1 || scatter_ctas_per_sm > max_s)
     return fail(s, SAMPO_ERR_ARG, "CTAs per SM outside 1.." + std::to_string(max_c) + " (count) / 1.." + std::to_string(max_s) +
                                       " (update/scatter)");
   s->chosen = {count_ctas_per_sm, scatter_ctas_per_sm};
-  if ((int)count_ctas_per_sm * sms != s->grid_count || (int)scatter_ctas_per_sm * sms != s->grid_scatter) size_grids(s);
+  size_grids(s, false);
   return SAMPO_OK;
 }
 

@@ -252,11 +252,12 @@ static RepParams carve(const RepLayout& L, void* mem, SimDev* sim, uint64_t capa
 }
 
 // The grids of the passes the batch runs; a day graph captured with other
-// kernels or grids goes.
-static void size_grids(sampo_batch* b) {
+// grids goes, and with `other` kernels.
+static void size_grids(sampo_batch* b, bool other = true) {
+  const int gc = b->grid_count, gs = b->grid_scatter;
   b->grid_count = chosen_grid(b->chosen.count, grid_blocks_count(b->nslots, b->species, b->items, b->wide));
   b->grid_scatter = chosen_grid(b->chosen.scatter, grid_blocks_scatter(b->nslots, b->species, b->items, b->wide));
-  drop_day_graphs(b);
+  if (other || gc != b->grid_count || gs != b->grid_scatter) drop_day_graphs(b);
 }
 
 // {step, active, status bits, pool end} of every slot, once the queued work is done.
@@ -715,13 +716,13 @@ extern "C" int sampo_batch_set_grids(sampo_batch* b, uint32_t count_ctas_per_sm,
   if (!b) return SAMPO_ERR_ARG;
   cudaSetDevice(b->device);
   const int sms = device_sms();
-  const uint32_t max_c = (uint32_t)(grid_blocks_count(b->nslots, b->species, b->items, b->wide) / sms);
+  const uint32_t max_c = (uint32_t)std::max(grid_blocks_count(b->nslots, b->species, b->items, b->wide) / sms, kCountGrids);
   const uint32_t max_s = (uint32_t)(grid_blocks_scatter(b->nslots, b->species, b->items, b->wide) / sms);
   if (count_ctas_per_sm < 1 || count_ctas_per_sm > max_c || scatter_ctas_per_sm < 1 || scatter_ctas_per_sm > max_s)
     return bfail(b, SAMPO_ERR_ARG, "CTAs per SM outside 1.." + std::to_string(max_c) + " (count) / 1.." +
                                        std::to_string(max_s) + " (update/scatter)");
   b->chosen = {count_ctas_per_sm, scatter_ctas_per_sm};
-  if ((int)count_ctas_per_sm * sms != b->grid_count || (int)scatter_ctas_per_sm * sms != b->grid_scatter) size_grids(b);
+  size_grids(b, false);
   return SAMPO_OK;
 }
 

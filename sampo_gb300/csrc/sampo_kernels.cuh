@@ -241,6 +241,9 @@ int device_sms();
 // The grids that sampo_set_grids or the tuner chose, in CTAs per SM of the
 // count and update/scatter passes; 0: the largest. They hold for every pool
 // the passes run on, as far as the grid of its kernels reaches.
+// (Choices of up to kCountGrids CTAs of the count pass are taken: five were
+// resident before it kept a ring of chunks per warp, three are now.)
+constexpr int kCountGrids = 5;
 struct ChosenGrids {
   uint32_t count = 0, scatter = 0;
 };

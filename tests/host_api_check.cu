@@ -146,7 +146,24 @@ static void chosen_grids_outlive_the_pool() {
   }
 }
 
+// What an earlier build's tuner chose, with up to 5 CTAs of the count pass on
+// an SM, is still taken, and runs as the largest grid.
+static void choices_of_smaller_kernels_are_taken() {
+  sampo_sim* s = with_pool();
+  g_resident = 3;
+  for (uint32_t c = 1; c <= 5; c++) {
+    CHECK(sampo_set_grids(s, c, 2) == SAMPO_OK);
+    CHECK(grids_are(s, (int)std::min(c, 3u), 2));
+  }
+  CHECK(sampo_set_grids(s, 6, 2) == SAMPO_ERR_ARG);
+  CHECK(sampo_set_grids(s, 1, 4) == SAMPO_ERR_ARG);
+  CHECK(sampo_set_grids(s, 0, 1) == SAMPO_ERR_ARG);
+  CHECK(grids_are(s, 3, 2));
+  CHECK(sampo_destroy(s) == SAMPO_OK);
+}
+
 int main() {
+  choices_of_smaller_kernels_are_taken();
   chosen_grids_outlive_the_pool();
   refused_launches_take_the_three_kernels();
   records_are_zero_after_a_launch_that_gave_up();

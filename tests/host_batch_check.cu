@@ -88,7 +88,16 @@ static void chosen_grids_outlive_a_wide_pool() {
   remove(path);
 }
 
+static void choices_of_smaller_kernels_are_taken() {
+  uint32_t slot = 0;
+  sampo_batch* b = one_slot(4096, &slot);
+  CHECK(sampo_batch_set_grids(b, 5, 2) == SAMPO_OK && grids_are(b, 3, 2));
+  CHECK(sampo_batch_set_grids(b, 6, 2) == SAMPO_ERR_ARG);
+  CHECK(sampo_batch_destroy(b) == SAMPO_OK);
+}
+
 int main() {
+  choices_of_smaller_kernels_are_taken();
   chosen_grids_outlive_a_wide_pool();
   grown_slots_have_clean_span_counts();
   printf(g_checks_failed ? "%d checks failed\n" : "ok\n", g_checks_failed);
