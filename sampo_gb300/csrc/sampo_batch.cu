@@ -50,6 +50,7 @@ struct Replicate {
   uint32_t stop_step = 0xffffffffu;
   uint64_t capacity = 0;
   uint32_t known_end = 0;      // its pool's end as the host last saw it
+  bool wide = false;           // its pool came with whole records (state_cols)
   float cc = 0.0f;
   void* mem = nullptr;
   RepParams rp;                // host copy of the kernels' view
@@ -78,7 +79,7 @@ struct sampo_batch {
   int grid_count = 0, grid_scatter = 0;
   int items = kItems;                // slots per thread of the count and update/scatter passes (2 or 4)
   uint32_t min_span = 0;             // BatchDev::minSpan as last set
-  bool wide = false;                 // every slot's pool holds whole records (state_cols): set by the first loaded one that has to
+  bool wide = false;                 // the passes move whole records (state_cols): while a slot's pool has to be moved so
   cudaGraphExec_t day_graph[2] = {nullptr, nullptr};  // three kernels every hour, and deciding ahead
   uint32_t day_graph_kernels[2] = {0, 0};             // kernel nodes of each
   uint64_t launches = 0;             // kernels sampo_batch_run launched
@@ -260,6 +261,23 @@ static void size_grids(sampo_batch* b, bool other = true) {
   if (other || gc != b->grid_count || gs != b->grid_scatter) drop_day_graphs(b);
 }
 
+// The passes for whole records take over when a slot's pool needs them (its
+// own columns are complete; the other slots' pools get theirs), and leave
+// again with the last such pool: whole records of the others obey their
+// states' implications all along, so nothing is to be converted back.
+static int update_wide(sampo_batch* b) {
+  bool wide = false;
+  for (const Replicate& r : b->reps) wide |= r.used && r.wide;
+  if (wide == b->wide) return SAMPO_OK;
+  for (uint32_t i = 0; wide && i < b->nslots; i++) {
+    const Replicate& r = b->reps[i];
+    if (r.used && r.have_pop && !r.wide) BCK(launch_widen(slot_params(b, i), b->stream), "whole records");
+  }
+  b->wide = wide;
+  size_grids(b);
+  return SAMPO_OK;
+}
+
 // {step, active, status bits, pool end} of every slot, once the queued work is done.
 static int read_states(sampo_batch* b, std::vector<uint4>& v) {
   v.resize(b->nslots);
@@ -342,7 +360,7 @@ extern "C" int sampo_batch_remove(sampo_batch* b, uint32_t slot) {
   const int st = upload_slot(b, slot, h);
   if (st) return st;
   BCK(cudaFreeAsync(mem, b->stream), "free replicate");
-  return SAMPO_OK;
+  return update_wide(b);
 }
 
 extern "C" int sampo_batch_set_inputs(sampo_batch* b, uint32_t slot, uint32_t first, const float* temperature,
@@ -422,6 +440,9 @@ extern "C" int sampo_batch_init_population(sampo_batch* b, uint32_t slot, uint32
   BCK(cudaMemsetAsync(r->rp.supers, 0, span_array_bytes((uint32_t)r->capacity), b->stream), "span arrays");
   BCK(cudaMemcpyAsync(b->init_seeds_dev + (size_t)slot * 4, init_seeds, 4 * sizeof(sampo_seeds), cudaMemcpyHostToDevice, b->stream),
       "seeds");
+  r->wide = false;
+  const int wrc = update_wide(b);
+  if (wrc) return wrc;
   const KParams p = slot_params(b, slot);
   BCK(launch_init_eggs(p, n, r->T_host[0], b->init_seeds_dev + (size_t)slot * 4, age_days_max, age_seed, b->wide, b->stream), "initAgents");
   BCK(launch_publish_start(p, 0, pop.r[7].end, b->stream), "initial statistics");
@@ -534,16 +555,12 @@ extern "C" int sampo_batch_checkpoint_load(sampo_batch* b, uint32_t slot, const 
   SimDev back;
   BCK(cudaMemcpyAsync(&back, b->sims_dev + slot, sizeof(SimDev), cudaMemcpyDeviceToHost, b->stream), "state");
   BCK(cudaStreamSynchronize(b->stream), "state");
+  r->wide = back.wide != 0;
+  const int wrc = update_wide(b);
+  if (wrc) return wrc;
   if (back.pop.numLarvae1DayEquiv != hd.pop.numLarvae1DayEquiv || back.pop.numFemale != hd.pop.numFemale ||
       back.pop.numPotentiallyInfective != hd.pop.numPotentiallyInfective)
     return bfail(b, SAMPO_ERR_INTERNAL, "checkpoint statistics do not match its pool");
-  if (back.wide && !b->wide) {
-    // the passes for whole records take over: the other slots' pools get theirs
-    for (uint32_t i = 0; i < b->nslots; i++)
-      if (i != slot && b->reps[i].used && b->reps[i].have_pop) BCK(launch_widen(slot_params(b, i), b->stream), "whole records");
-    b->wide = true;
-    size_grids(b);
-  }
   r->have_pop = true;
   r->known_end = hd.pop.r[7].end;
   r->step = hd.step;

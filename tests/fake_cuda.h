@@ -137,7 +137,9 @@ cudaError_t launch_steps(const KParams& p, uint32_t n, bool, int, int, int, cuda
   return note("steps");
 }
 cudaError_t launch_publish(const KParams&, int, cudaStream_t) { return note("publish"); }
-cudaError_t launch_init_eggs(const KParams&, uint32_t, float, const sampo_seeds*, int, uint64_t, bool, cudaStream_t) { return note("init"); }
+cudaError_t launch_init_eggs(const KParams&, uint32_t, float, const sampo_seeds*, int, uint64_t, bool full, cudaStream_t) {
+  return note(full ? "init, whole" : "init");
+}
 cudaError_t launch_publish_start(const KParams& p, uint32_t flags, uint32_t, cudaStream_t) {
   if (flags & PS_CHECK) p.reps[0].sim->wide = g_wide_found;
   if (flags & PS_CLEAR) memset(p.reps[0].supers, 0, units_of(span_count(p.reps[0].sim->pop.r[7].end, 0), 32) * sizeof(uint4));

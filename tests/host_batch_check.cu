@@ -96,7 +96,43 @@ static void choices_of_smaller_kernels_are_taken() {
   CHECK(sampo_batch_destroy(b) == SAMPO_OK);
 }
 
+// A batch moves whole records while a slot of it holds a pool that needs
+// them, and no longer: removing the slot, or putting another population into
+// it, ends it; the other slots' pools get their implied columns at its start.
+static void whole_records_only_while_a_slot_needs_them() {
+  const char* path = "sampo_fake_batch.ck";
+  for (int end : {0, 1, 2}) {
+    uint32_t slot = 0, other = 0;
+    sampo_batch* b = one_slot(4096, &slot);
+    CHECK(sampo_batch_checkpoint_save(b, slot, path) == SAMPO_OK);
+    const sampo_replicate_config rc = {4096, 1000.0f, 0xffffffffu};
+    CHECK(sampo_batch_add(b, &rc, &other) == SAMPO_OK && other != slot);
+    g_launches.clear();
+    resume(b, other, path, true);
+    CHECK(b->wide && g_launches["widen"] == 1);
+    if (end == 0) {
+      CHECK(sampo_batch_remove(b, other) == SAMPO_OK);
+    } else if (end == 1) {
+      resume(b, other, path, false);
+    } else {
+      sampo_seeds seeds[4];
+      memset(seeds, 0, sizeof(seeds));
+      b->reps[other].input_step[0] = 0;
+      CHECK(sampo_batch_init_population(b, other, 100, seeds, 0, 0) == SAMPO_OK);
+      CHECK(g_launches["init, whole"] == 0);
+    }
+    CHECK(!b->wide);
+    resume(b, slot, path, true);
+    CHECK(b->wide);
+    resume(b, slot, path, true);
+    CHECK(b->wide);
+    CHECK(sampo_batch_destroy(b) == SAMPO_OK);
+  }
+  remove(path);
+}
+
 int main() {
+  whole_records_only_while_a_slot_needs_them();
   choices_of_smaller_kernels_are_taken();
   chosen_grids_outlive_a_wide_pool();
   grown_slots_have_clean_span_counts();

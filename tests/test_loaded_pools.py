@@ -89,3 +89,53 @@ def test_larvae_younger_than_a_day(gpu_ready, oracle_mod, tiles, ages):
     arrays["ageInHours"][s:e] = np.resize(np.array(ages, np.float32), e - s)
     arrays["hoursInState"][s:e] = arrays["ageInHours"][s:e] - np.float32(24.0)
     _run_and_compare(ranges, arrays, T, env, seeds, 30000.0, (26, 4), tiles)
+
+
+def test_batch_with_a_pool_of_whole_records(gpu_ready, tmp_path):
+    """A slot resumed from a pool with free records makes its batch move whole
+    records (three kernels an hour) until it is removed; the replicates beside
+    it, which decide ahead before and after (one count pass a day), and the
+    slot itself equal their plain runs."""
+    import dataclasses
+    from sampo_gb300.batch import Batch, admit
+    from sampo_gb300.sim import Simulation
+    from tests.test_batch import SPECS, compare
+    n, cc, cap = 30, 30000.0, 1 << 18
+    ranges, arrays, T, env, seeds = _workload((9000, 7000, 2000, 5000), n, cc, seed=8)
+    s, e = int(ranges[1][0]), int(ranges[1][1])
+    arrays["hoursInState"][s:e:2] += np.float32(0.25)
+    ck = str(tmp_path / "whole.ck")
+    with Simulation(capacity=cap, carrying_capacity=cc, max_steps=n + 1) as sim:
+        sim.set_inputs(T, env)
+        sim.set_seeds(0, seeds)
+        sim.load_pool(ranges, arrays)
+        sim.checkpoint(ck)
+        sim.run(n)
+        want, (pop, pool) = sim.current_row(), sim.read_pool()
+    big = dataclasses.replace(SPECS[4], initial=90000, days=6, capacity=1800000)
+    small = dataclasses.replace(SPECS[1], days=6)
+    with Batch(max_replicates=4, ring_steps=150) as b:
+        slots = [admit(b, x, 144) for x in (big, small)]
+
+        def kernels(hours):
+            before = b.launches()
+            b.run(hours)
+            return b.launches() - before
+
+        assert kernels(24) == 1 + 50          # count, publish, 24 x (scatter, publish)
+        w = b.add(cap, cc, stop_step=n)
+        b.set_inputs(w, T, env)
+        b.set_seeds(w, 0, seeds)
+        b.resume(w, ck)
+        assert kernels(24) == 1 + 72
+        late = admit(b, small, 72)            # admitted into whole records
+        assert kernels(24) == 1 + 72
+        assert b.rows(w, n, 1)[0].tobytes() == want.tobytes()
+        bpop, bpool = b.read_pool(w)
+        assert np.array_equal(bpop["ranges"], pop["ranges"])
+        _same_pools(pop["ranges"], bpool, pool)
+        b.remove(w)
+        assert kernels(72) == 1 + 150
+        compare(b, slots[0], big, 144, "large replicate")
+        compare(b, slots[1], small, 144, "small replicate")
+        compare(b, late, small, 72, "late replicate")
