@@ -190,9 +190,11 @@ namespace sampo {
 // narrow pools, see state_cols): half an hour past it the quotient is at
 // least 1/48 away from every whole number, far more than the two roundings,
 // so truncating it gives the same days as the exact division.
-__device__ __forceinline__ uint32_t whole_age_days(float age) {
-  return __float_as_uint(__fadd_rz(__fmul_rn(__fadd_rn(age, 0.5f), 1.0f / 24.0f), 8388608.0f)) - 0x4B000000u;
-}
+__device__ __forceinline__ float whole_age_quotient(float age) { return __fmul_rn(__fadd_rn(age, 0.5f), 1.0f / 24.0f); }
+__device__ __forceinline__ uint32_t whole_days(float quotient) { return __float_as_uint(__fadd_rz(quotient, 8388608.0f)) - 0x4B000000u; }
+__device__ __forceinline__ uint32_t whole_age_days(float age) { return whole_days(whole_age_quotient(age)); }
+// The days an hour on (the same margin covers this sum too).
+__device__ __forceinline__ uint32_t whole_days_next(float quotient) { return whole_days(__fadd_rn(quotient, 1.0f / 24.0f)); }
 template <bool WHOLE = false>
 __device__ __forceinline__ uint32_t age_days(float age) {
   if (WHOLE) {

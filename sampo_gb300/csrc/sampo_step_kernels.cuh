@@ -1379,10 +1379,10 @@ __device__ __noinline__ uint32_t scatter_range(uint32_t lo, uint32_t hi, uint32_
           bs += __popc(ms[k]);
           // the step after: mortality, then the transition (update_agent<false>)
           uint32_t kill = hkill;
-          float q = 0.0f;  // (age + 1/2) / 24: whole_age_days before truncation
+          float q = 0.0f;
           if (RG == LARVA) {
-            q = __fmul_rn(__fadd_rn(live ? age : 24.0f, 0.5f), 1.0f / 24.0f);
-            const uint32_t days = __float_as_uint(__fadd_rz(q, 8388608.0f)) - 0x4B000000u;
+            q = whole_age_quotient(live ? age : 24.0f);
+            const uint32_t days = whole_days(q);
             kill = w.larvaKill1[days < 99u ? days : 99u];
             if (live && kill == 0u) da.acc.bad = 1u;
           }
@@ -1392,8 +1392,8 @@ __device__ __noinline__ uint32_t scatter_range(uint32_t lo, uint32_t hi, uint32_
           const uint32_t c = lives ? (due ? 1u << 16 : 1u) : 0u;
           ts.cnt += c;
           if (crosses.value && d >= ts.end) past += c;
-          if (RG == LARVA && lives && !due) {  // its whole days an hour on (the margin of whole_age_days covers this sum too)
-            const uint32_t days = __float_as_uint(__fadd_rz(__fadd_rn(q, 1.0f / 24.0f), 8388608.0f)) - 0x4B000000u;
+          if (RG == LARVA && lives && !due) {  // its whole days an hour on
+            const uint32_t days = whole_days_next(q);
             da.l1 += days;
             youngest = min(youngest, days);
             oldest = max(oldest, days);
