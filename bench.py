@@ -137,8 +137,8 @@ class ClockSampler:
 
 
 def traffic_from_profile():
-    """dram bytes per live agent of the update/scatter kernel from the
-    committed ncu summary (profiles/k_scatter_dram.json), or None."""
+    """The committed ncu summary of the deciding update/scatter pass's DRAM
+    bytes (profiles/k_scatter_dram.json), or None."""
     p = os.path.join(REPO, "profiles", "k_scatter_dram.json")
     if not os.path.exists(p):
         return None
@@ -199,7 +199,9 @@ def gpu_arm(args, wl, rank, world, device):
     gpu_launches = sim.kernel_times()[1] - launches0
     small = sim.small_step_info()
 
-    # ---- roofline: the same days again, each kernel between CUDA events ----
+    # ---- passes: the same days again, each kernel between CUDA events (these
+    # hours take the count pass and the update/scatter pass that does not
+    # decide; the day graphs run that one an hour in 24) ----
     fresh()
     sim.set_timing(True)
     rows2 = sim.run(24 * args.steps)
@@ -217,11 +219,17 @@ def gpu_arm(args, wl, rank, world, device):
     # the step in timing mode minus the two passes: k_publish and the gaps between the launches
     publish_ms = (times[2] - times[0] - times[1]) / n_launch
     peak, peak_kind = peaks()
-    achieved = scatter_bytes.mean() / (scatter_ms * 1e-3) / 1e9
+    # the roofline's line is the hour of the timed days, its time and its bytes:
+    # by far most of it the update/scatter pass that decides the next hour
+    # (k_count's bytes once a day)
+    step_ms_graph = ms / (24 * args.steps)
+    step_bytes = float(count_bytes.mean() / 24 + scatter_bytes.mean())
+    achieved = step_bytes / (step_ms_graph * 1e-3) / 1e9
     prof = traffic_from_profile()
     traffic = None
-    if prof:
-        traffic = float(prof["dram_bytes_per_live_agent"] * tot.mean())
+    days_three = small["days_three_kernel"] - small0["days_three_kernel"]
+    if prof and days_three == args.steps:
+        traffic = float(prof["dram_over_algorithmic"] * scatter_bytes.mean())
 
     # ---- e2e: through the C ABI with page-locked host buffers, per day ----
     from sampo_gb300._lib import ENV_DTYPE, ROW_DTYPE
@@ -250,21 +258,20 @@ def gpu_arm(args, wl, rank, world, device):
     for h in (hT, hE, hS, hR):
         h.free()
     sim.close()
-    # each pass against the peak, and the whole step as the day graphs run it
-    step_ms_graph = ms / (24 * args.steps)
-    step_bytes = float(count_bytes.mean() / 24 + scatter_bytes.mean())
 
+    # each pass against the peak, and the whole step as the day graphs run it
     def pass_line(nbytes, t_ms):
         gbs = nbytes / (t_ms * 1e-3) / 1e9
         return {"bytes_per_launch": nbytes, "ms_per_launch": t_ms, "gbs": gbs, "frac": gbs / peak}
     passes = {
         "k_count: decisions (10-14 B per live agent; once a day in the day graphs)": pass_line(float(count_bytes.mean()), count_ms),
-        "k_scatter: update + compaction (9-37 B read and written per agent, by its state)": pass_line(float(scatter_bytes.mean()), scatter_ms),
-        "hourly step in the day graphs (the update/scatter pass, which decides the next hour too, and k_publish)": pass_line(step_bytes, step_ms_graph),
+        "k_scatter, not deciding (timing mode, single hours, a day's last hour): 9-37 B read and written per agent, by its state": pass_line(float(scatter_bytes.mean()), scatter_ms),
+        "hourly step in the timed days (of large pools: the update/scatter pass, which decides the next hour too, and k_publish)": pass_line(step_bytes, step_ms_graph),
     }
     return dict(agent_days=agent_days, ms=ms, wall=wall, live=live, rows=rows, clocks=clk.summary(), passes=passes,
                 gpu_launches=gpu_launches, scatter_ms=scatter_ms, count_ms=count_ms, publish_ms=publish_ms, achieved=achieved, peak=peak,
-                peak_kind=peak_kind, traffic=traffic, e2e_agent_days=e2e_live / 24.0, e2e_wall=e2e_wall,
+                peak_kind=peak_kind, traffic=traffic, step_ms_graph=step_ms_graph,
+                days_small=small["days_one_launch"] - small0["days_one_launch"], e2e_agent_days=e2e_live / 24.0, e2e_wall=e2e_wall,
                 count_gbs=count_bytes.mean() / (count_ms * 1e-3) / 1e9, days=days, tuned=tuned, items=items, small=small, small0=small0)
 
 
@@ -668,13 +675,16 @@ def main():
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32+u32 (f64 where the reference promotes)",
         "data": "synthetic", "config": cfg, "details": details,
         "roofline": {"bound": "hbm", "achieved": r["achieved"], "peak": r["peak"], "unit": "GB/s",
-                     "frac": r["achieved"] / r["peak"], "traffic": r["traffic"], "kernel": "k_scatter (update + stable scatter)",
-                     "traffic_from": "scaled: DRAM bytes per live agent of a single-pass ncu capture of k_scatter on the "
-                                     "roofline workload at 5.7e7 live agents (profiles/k_scatter_dram.json: 1.10 of the "
-                                     "algorithmic bytes) x this run's mean live pool",
-                     "peak_kind": r["peak_kind"], "scatter_ms_per_launch": r["scatter_ms"], "count_ms_per_launch": r["count_ms"],
-                     "publish_and_gaps_ms_per_step": r["publish_ms"],
-                     "count_pass_gbs": r["count_gbs"],
+                     "frac": r["achieved"] / r["peak"], "traffic": r["traffic"], "ms_per_launch": r["step_ms_graph"],
+                     "kernel": ("an hour of the one-launch days (k_step_small)" if r["days_small"] == args.steps else
+                                "an hour of the timed days: k_scatter deciding ahead (update + stable scatter + the next hour's "
+                                "decisions), k_publish, and a 24th of k_count"),
+                     "traffic_from": "scaled: DRAM bytes over algorithmic bytes (1.05) of a single-pass ncu capture of the deciding "
+                                     "k_scatter on the roofline workload at 5.7e7 live agents (profiles/k_scatter_dram.json) x "
+                                     "this run's mean algorithmic bytes of the pass",
+                     "peak_kind": r["peak_kind"], "timing_mode": {"scatter_ms_per_launch": r["scatter_ms"], "count_ms_per_launch": r["count_ms"],
+                                                                  "publish_and_gaps_ms_per_step": r["publish_ms"],
+                                                                  "count_pass_gbs": r["count_gbs"]},
                      "algorithmic_bytes": "k_scatter: the fields that an agent's state does not imply and its flags (9-37 B), read per live "
                                           "agent and written per agent of the next pool",
                      "passes": r["passes"]},
