@@ -173,12 +173,14 @@ int sampo_read_pool(sampo_sim* s, sampo_population* pop, sampo_pool_view* pool);
  * after 16 x (step + 1) draws). Loading needs a handle with the file's
  * carrying capacity and room for its pool. */
 int sampo_checkpoint_save(sampo_sim* s, const char* path);
-/* Autotuner (no counterpart in the reference): times the step kernels on the
- * coming step of this simulation for each tile size (1024- and 512-slot
- * tiles: 4 or 2 slots per thread) at every persistent grid size the
- * occupancy allows (CTAs per SM of the count and update/scatter passes),
- * keeps the fastest for the following steps and returns the grids (the tile
- * size: sampo_items_per_thread). The trials leave the simulation's course
+/* Autotuner (no counterpart in the reference): times the kernels of one hour
+ * taken by itself (the count pass and the update/scatter pass that does not
+ * decide ahead) on the coming step of this simulation, for 4 and 2 rows of 32
+ * agents at once and at every persistent grid size the occupancy allows (CTAs
+ * per SM of the two passes), keeps the fastest for the following steps and
+ * returns the grids (the rows: sampo_items_per_thread). The days of large
+ * pools, whose update/scatter pass decides the next hour too, run with what is
+ * fastest for the single hour. The trials leave the simulation's course
  * unchanged. Needs the coming step's inputs. */
 int sampo_autotune(sampo_sim* s, uint32_t* count_ctas_per_sm, uint32_t* scatter_ctas_per_sm);
 /* Sets the grid sizes sampo_autotune would pick, e.g. a choice tuned earlier
@@ -187,9 +189,9 @@ int sampo_autotune(sampo_sim* s, uint32_t* count_ctas_per_sm, uint32_t* scatter_
  * more were resident, and run as the largest grid.) The choice holds for
  * every pool until it is tuned or set again, or a call below resets it. */
 int sampo_set_grids(sampo_sim* s, uint32_t count_ctas_per_sm, uint32_t scatter_ctas_per_sm);
-/* Slots per thread of the count and update/scatter passes: 4 (1024-slot
- * tiles, the default) or 2 (512-slot tiles); results do not depend on it. A
- * run-time species runs 4. Setting it resets the grids to the largest the
+/* Rows of 32 agents that a warp of the count and update/scatter passes takes
+ * at once: 4 (the default) or 2; results do not depend on it. A run-time
+ * species and whole records run 4. Setting it resets the grids to the largest the
  * occupancy allows. */
 int sampo_set_items_per_thread(sampo_sim* s, uint32_t items);
 int sampo_items_per_thread(sampo_sim* s, uint32_t* items);
@@ -200,8 +202,9 @@ int sampo_items_per_thread(sampo_sim* s, uint32_t* items);
  * a pool of at most max_tiles 1024-slot tiles takes one launch of a
  * cooperative kernel that runs the day's 24 hourly steps (update, scan and
  * compaction with two bounded grid barriers per hour) on a grid sized to the
- * pool, a larger one the count, update/scatter and publish kernels every
- * hour. Both give the same results at any size. SAMPO_SMALL_STEP_DEFAULT:
+ * pool, a larger one a count kernel and then update/scatter and publish
+ * kernels every hour (with whole records or a run-time species all three every
+ * hour: "three-kernel" below is either). Both give the same results at any size. SAMPO_SMALL_STEP_DEFAULT:
  * the largest co-resident grid of the one-launch kernel, one tile per CTA
  * (the default); 0: never. sampo_run_async picks by the size seen at its
  * call, sampo_step by the size at its hour (one launch of one hourly step);
@@ -337,8 +340,9 @@ int sampo_eval_math(int fn, const float* x, const float* y, float* out, uint32_t
  * A batch owns up to max_replicates slots on one GPU; every slot holds one
  * simulation (a "replicate": its own pool, carrying capacity, seeds, inputs
  * and step counter). sampo_batch_run advances every active replicate by the
- * same number of steps in one pass of the step kernels per hour (tiles of all
- * replicates share the persistent CTAs), replayed as a CUDA graph per day.
+ * same number of steps in one pass of the step kernels per hour (the resident
+ * warps take spans of all replicates' slots in turn), replayed as a CUDA graph
+ * per day.
  * Each replicate's results are bit-identical to the same simulation run
  * alone through sampo_step / sampo_run. Slots can be filled and emptied
  * between runs (continuous batching); pools are allocated stream-ordered

@@ -586,8 +586,12 @@ static cudaError_t launch_hours(sampo_batch* b, const KParams& p, uint32_t nstep
 }
 
 // Whether a run's days decide ahead: the pools the host has last seen come to
-// more than kAheadSlots slots. Below that a step is three launches' latency
-// either way.
+// more than kAheadSlots slots. Measured both ways (us an hour, three kernels
+// against deciding ahead): one replicate of 8,192 slots 21.8 / 18.8, of
+// 262,144 24.3 / 21.1; 8 of 1,024 23.4 / 19.5, of 32,768 25.0 / 21.5; 64 of 128
+// 25.5 / 21.5, of 4,096 26.3 / 23.3. Deciding ahead is ahead on both sides of
+// the line by the count pass's launch, so the line could lie lower; below it a
+// batch keeps three launches an hour, whatever the length of its runs.
 constexpr uint64_t kAheadSlots = 65536;
 static uint64_t known_slots(const sampo_batch* b) {
   uint64_t slots = 0;

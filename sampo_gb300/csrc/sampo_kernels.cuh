@@ -105,11 +105,15 @@ __host__ __device__ constexpr size_t small_row_words(uint32_t tiles) { return sm
 // A span costs a warp about a thousand instructions besides its rows (its
 // prefix, the start and end of its range, the agents that move on in a
 // partly filled warp), a row of 32 agents 60 to 150, so a pool is cut into as
-// few spans as keep every warp of the resident grid (kSpanWarps on 152 SMs)
-// equally busy: the smallest multiple of kSpanWarps that keeps them at
-// kSpanMax slots. A batch sets a larger smallest span (BatchDev::minSpan),
-// since its replicates share the warps.
-constexpr uint32_t kSpanMin = 128, kSpanMax = 1024, kSpanWarps = 3648;
+// few spans as keep every warp of the resident grid equally busy: the smallest
+// multiple of kSpanWarps that keeps them at kSpanMax slots. kSpanWarps is the
+// resident grid of a GB300, 152 SMs x 3 CTAs (what the passes' 80 registers
+// and 59 KB of shared memory allow) x 8 warps; a constant, because the spans
+// are sized where no host call can ask (the kernels and the sizes of the span
+// arrays). A grid of fewer warps takes the spans in more turns, to the same
+// results. A batch sets a larger smallest span (BatchDev::minSpan), since its
+// replicates share the warps.
+constexpr uint32_t kSpanMin = 128, kSpanMax = 1024, kSpanWarps = 152 * 3 * 8;
 __host__ __device__ constexpr uint32_t span_size(uint32_t end, uint32_t min_span) {
   const uint32_t warps = kSpanWarps * (end / (kSpanWarps * kSpanMax) + 1u);
   uint32_t s = units_of(end, warps);
@@ -312,8 +316,12 @@ cudaError_t launch_small(const KParams& p, int grid, bool cooperative, uint32_t 
                          int items = kItems);
 // Times count + scatter of the coming step for each number of rows at once
 // (4 and, for the built-in species, 2) at every (count, scatter) number of
-// CTAs per SM the occupancy allows, and returns the fastest. The trials leave the simulations' course unchanged (k_trial_reset);
-// the coming step's constants must be current (PUB_REFRESH) before the call.
+// CTAs per SM the occupancy allows, and returns the fastest. The scatter pass
+// timed is the one that does not decide ahead (single hours, whole records,
+// run-time species, small batches); days that decide ahead run it one hour in
+// 24 and k_count once, and take its picks over. The trials leave the
+// simulations' course unchanged (k_trial_reset); the coming step's constants
+// must be current (PUB_REFRESH) before the call.
 cudaError_t tune_grids(const KParams& p, cudaStream_t st, int* grid_count, int* grid_scatter, int* items, double* best_ms);
 
 #endif  // __CUDACC_RTC__

@@ -10,13 +10,14 @@
 // promotes to double (include/properties.h:134, kernel/updateAgents.cl:69-70)
 // stay double.
 //
-// update_agent<FULL> is used twice per step: FULL=false by the counting pass
-// (only the fields that decide survival, the next state and the number of
-// eggs laid) and FULL=true by the scatter pass (the complete record), which
-// takes the counting pass's decision (DECIDED: `code`, DEC_STAYS or
-// DEC_MOVES) instead of drawing it again. EGGS adds the eggs laid to
-// Acc::newEggs (the counting pass, and the one-launch step, whose single
-// update decides and writes).
+// update_agent<FULL=false> decides (only the fields that decide survival, the
+// next state and the number of eggs laid): in the count pass, and for the hour
+// after in an update/scatter pass that decides ahead. FULL=true updates the
+// record: in the update/scatter pass, with the decision taken before (DECIDED:
+// `code`, DEC_STAYS or DEC_MOVES) instead of drawing it again, and in the
+// one-launch step, whose single update decides and writes. EGGS adds the eggs
+// laid to Acc::newEggs (wherever an agent is decided). That path has eggs and
+// larvae that stay in a form of its own (scatter_range).
 // WHOLE: the ages are whole hours (a narrow pool).
 // LDG reads the larval mortality table through the read-only cache; the
 // one-launch step, which rewrites the table between the hours of one launch,

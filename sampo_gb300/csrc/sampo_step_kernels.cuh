@@ -3,15 +3,20 @@
 // the library by nvcc (sampo_kernels.cu) and, for a user species header, at
 // run time by NVRTC (sampo_species.cu).
 //
-// A step of a batch of simulations is two kernels over every active
-// replicate's current pool buffer and a small one with a CTA per replicate:
+// A day of a batch of simulations is one k_count, then 24 k_scatter, each of
+// which decides the hour after its own as it writes, and after each of these
+// kernels a k_publish (launch_steps); a single hour, a run-time species, whole
+// records and small batches take all three kernels every hour. k_count and
+// k_scatter go over every active replicate's current pool buffer, k_publish
+// has a CTA per replicate:
 //
-//  k_count   reads the ~8-12 bytes per agent that decide survival, the next
-//            state and the eggs laid (killAgents + the decision part of
-//            updateAgents), notes each decision in two bits of the agent's
-//            flags, and counts the survivors by next state per span of slots
-//            and the replicate's new eggs.
-//  k_scatter applies the decisions to the complete records, obtains each
+//  k_count   reads the columns that decide survival, the next state and the
+//            eggs laid (killAgents + the decision part of updateAgents; 9 to
+//            13 bytes of an agent with its flags, decide_cols), notes each
+//            decision in two bits of the agent's flags, and counts the
+//            survivors by next state per span of slots and the replicate's
+//            new eggs.
+//  k_scatter applies the decisions to the records (state_cols), obtains each
 //            survivor's stable rank within its next state (the span counts
 //            of k_count, then ballots), writes the updated record to its
 //            slot in the other buffer (the reference's oldToNewAgents
@@ -1398,7 +1403,7 @@ __device__ __noinline__ uint32_t scatter_range(uint32_t lo, uint32_t hi, uint32_
             youngest = min(youngest, days);
             oldest = max(oldest, days);
           }
-          put_if<RG>(live, dst, d, age, delay, cld, RG | (fl & 8u) | (lives ? (due ? DEC_MOVES << 4 : DEC_STAYS << 4) : 0u));
+          put_if<RG>(live, dst, d, age, delay, cld, (fl & 8u) | (lives ? (due ? RG | DEC_MOVES << 4 : RG | DEC_STAYS << 4) : (uint32_t)RG));
         }
         if (crosses.value) {
           ts.cnt -= past;
